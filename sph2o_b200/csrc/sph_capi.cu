@@ -108,6 +108,7 @@ struct sph_ctx {
     int solver_occ = 8;
     bool staged_lists = false; /* SPH_OPT_LIST_STAGED */
     int solver_tpp = 2;  /* measured best on B200 for the 1M-particle scene (1, 2, 4: 1.03, 0.84, 0.92 ms) */
+    float* stage = nullptr;      /* 3 max(nf, nb) floats: device side of every host transfer (see sph_get_state) */
     float4* braw = nullptr;      /* boundary in caller order (re-sorted when the cell order changes) */
     unsigned* bid = nullptr;
     /* PCISPH boundary method: boundary normals (caller order on the host,
@@ -1103,10 +1104,8 @@ int sph_init(sph_ctx* c)
             }
 
     /* upload: fluid in caller order becomes the first "unsorted" state */
-    float* stage = nullptr;
-    const size_t stage_n = 3 * std::max<size_t>(nmax, 1);
-    CUDA_TRY(c, cudaMalloc(&stage, stage_n * sizeof(float)));
-    c->allocations.push_back(stage);
+    if ((rc = dalloc(c, &c->stage, 3 * nmax)) != SPH_OK) return rc;
+    float* stage = c->stage;
     CUDA_TRY(c, cudaMemcpyAsync(stage, c->h_fluid.data(), 3 * nf * sizeof(float), cudaMemcpyHostToDevice, c->stream));
     launch_pack_v3((int)nf, stage, c->pos, 0.0f, c->stream);
     CUDA_TRY(c, cudaMemcpyAsync(stage, c->h_vel.data(), 3 * nf * sizeof(float), cudaMemcpyHostToDevice, c->stream));
@@ -1279,8 +1278,11 @@ int sph_get_state(sph_ctx* c, float* xyz, float* v, float* rho)
     unsigned na = 0;
     int rc = active_count(c, &na);
     if (rc != SPH_OK) return rc;
-    float* tmp = nullptr;
-    CUDA_TRY(c, cudaMallocAsync((void**)&tmp, 3 * nf * sizeof(float), c->stream));
+    /* The context's own staging buffer: a buffer allocated and freed per call
+       (cudaMallocAsync, cudaFreeAsync and the synchronisation, after which the
+       pool gives its memory back) took ~0.5 ms of host time per call on a
+       1,000-particle scene whose copies and kernels take ~20 us. */
+    float* tmp = c->stage;
     if (na < nf) CUDA_TRY(c, cudaMemsetAsync(tmp, 0, 3 * nf * sizeof(float), c->stream)); /* inactive: 0 */
     auto copy_out = [&](float* dst, size_t count) -> int {
         CUDA_TRY(c, cudaMemcpyAsync(dst, tmp, count * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
@@ -1293,7 +1295,6 @@ int sph_get_state(sph_ctx* c, float* xyz, float* v, float* rho)
         launch_unsort_f((int)na, c->orig, c->rho, tmp, c->stream);
         rc = copy_out(rho, nf);
     }
-    cudaFreeAsync(tmp, c->stream);
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     if (rc != SPH_OK) return rc;
     return check_launch(c, "get_state");
@@ -1307,8 +1308,7 @@ int sph_set_state(sph_ctx* c, const float* xyz, const float* v)
     unsigned na = 0;
     int rc0 = active_count(c, &na);
     if (rc0 != SPH_OK) return rc0;
-    float* tmp = nullptr;
-    CUDA_TRY(c, cudaMallocAsync((void**)&tmp, 3 * nf * sizeof(float), c->stream));
+    float* tmp = c->stage;
     if (xyz) {
         CUDA_TRY(c, cudaMemcpyAsync(tmp, xyz, 3 * nf * sizeof(float), cudaMemcpyHostToDevice, c->stream));
         launch_sort_v3((int)na, c->orig, tmp, c->pos, c->stream);
@@ -1319,17 +1319,16 @@ int sph_set_state(sph_ctx* c, const float* xyz, const float* v)
         CUDA_TRY(c, cudaMemcpyAsync(tmp, v, 3 * nf * sizeof(float), cudaMemcpyHostToDevice, c->stream));
         launch_sort_v3((int)na, c->orig, tmp, c->vel, c->stream);
     }
-    cudaFreeAsync(tmp, c->stream);
-    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     c->lists_valid = false;
+    int rc = SPH_OK;
     if (xyz && c->desc.simulation_method == SPH_DFSPH) {
         /* DFSPH keeps densities/alpha of the current positions between steps */
-        int rc = neighbor_search(c);
-        if (rc != SPH_OK) return rc;
-        launch_density(c->P, arrays(c), true, false, c->pass_block, c->stream);
-        CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+        rc = neighbor_search(c);
+        if (rc == SPH_OK) launch_density(c->P, arrays(c), true, false, c->pass_block, c->stream);
     }
-    return check_launch(c, "set_state");
+    /* one wait: the caller's arrays have been read and the search has run */
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    return rc != SPH_OK ? rc : check_launch(c, "set_state");
 }
 
 int sph_get_boundary_state(sph_ctx* c, float* density, float* pressure)
@@ -1338,8 +1337,7 @@ int sph_get_boundary_state(sph_ctx* c, float* density, float* pressure)
     if (!c->initialized) return fail(c, SPH_ERR_STATE, "sph_get_boundary_state before sph_init");
     if (!c->P.pcib) return fail(c, SPH_ERR_ARG, "boundary densities exist for the PCISPH boundary method only");
     if (c->nb == 0) return SPH_OK;
-    float* tmp = nullptr;
-    CUDA_TRY(c, cudaMallocAsync((void**)&tmp, c->nb * sizeof(float), c->stream));
+    float* tmp = c->stage;
     for (int k = 0; k < 2; ++k) {
         float* out = k == 0 ? density : pressure;
         if (!out) continue;
@@ -1347,8 +1345,6 @@ int sph_get_boundary_state(sph_ctx* c, float* density, float* pressure)
         CUDA_TRY(c, cudaMemcpyAsync(out, tmp, c->nb * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     }
-    cudaFreeAsync(tmp, c->stream);
-    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     return check_launch(c, "get_boundary_state");
 }
 
@@ -1358,11 +1354,9 @@ int sph_get_boundary_volume(sph_ctx* c, float* vol)
     if (!c->initialized) return fail(c, SPH_ERR_STATE, "sph_get_boundary_volume before sph_init");
     if (c->P.pcib) return fail(c, SPH_ERR_ARG, "boundary volumes exist for the Akinci boundary method only");
     if (c->nb == 0) return SPH_OK;
-    float* tmp = nullptr;
-    CUDA_TRY(c, cudaMallocAsync((void**)&tmp, c->nb * sizeof(float), c->stream));
+    float* tmp = c->stage;
     launch_unsort_f((int)c->nb, c->borig, c->bvol, tmp, c->stream);
     CUDA_TRY(c, cudaMemcpyAsync(vol, tmp, c->nb * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
-    cudaFreeAsync(tmp, c->stream);
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     return check_launch(c, "get_boundary_volume");
 }
@@ -1406,12 +1400,8 @@ int sph_set_time(sph_ctx* c, double time, float dt)
     if (!c) return SPH_ERR_ARG;
     if (!c->initialized) return fail(c, SPH_ERR_STATE, "sph_set_time before sph_init");
     if (!(dt > 0.0f)) return fail(c, SPH_ERR_ARG, "dt must be positive");
-    DevState s{};
-    int rc = read_state(c, &s);
-    if (rc != SPH_OK) return rc;
-    s.time = time;
-    s.dt = dt;
-    CUDA_TRY(c, cudaMemcpyAsync(c->st, &s, sizeof s, cudaMemcpyHostToDevice, c->stream));
+    CUDA_TRY(c, cudaMemcpyAsync(&c->st->time, &time, sizeof time, cudaMemcpyHostToDevice, c->stream));
+    CUDA_TRY(c, cudaMemcpyAsync(&c->st->dt, &dt, sizeof dt, cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     c->last.time = time;
     c->last.dt = dt;
@@ -1458,8 +1448,7 @@ int sph_compute_phase(sph_ctx* c, int phase, float* out)
        boundary particles too (SPHSolver.cpp:126-137), WCSPH their pressures */
     if (c->P.pcib) launch_boundary_density(c->P, A, c->stream);
     const size_t nf = c->nf;
-    float* tmp = nullptr;
-    CUDA_TRY(c, cudaMallocAsync((void**)&tmp, 3 * nf * sizeof(float), c->stream));
+    float* tmp = c->stage;
     CUDA_TRY(c, cudaMemsetAsync(tmp, 0, 3 * nf * sizeof(float), c->stream)); /* inactive particles read 0 */
     size_t count = nf;
     switch (phase) {
@@ -1481,7 +1470,6 @@ int sph_compute_phase(sph_ctx* c, int phase, float* out)
     CUDA_TRY(c, cudaMemcpyAsync(out, tmp, count * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
     if (phase == SPH_PHASE_NONPRESSURE_ACC || phase == SPH_PHASE_PRESSURE_ACC)
         CUDA_TRY(c, cudaMemsetAsync(c->acc, 0, nf * sizeof(float4), c->stream));
-    cudaFreeAsync(tmp, c->stream);
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     return check_launch(c, "compute_phase");
 }
