@@ -219,10 +219,12 @@ enum sph_option {
     SPH_OPT_CUDA_GRAPHS = 0,      /* 1 (default): steps replay captured CUDA graphs of two steps (one
                                      for an odd remainder), keyed by the buffer assignment */
     SPH_OPT_CELL_ORDER = 1,       /* 0 (default): 4x4x4 cell bricks, Morton inside; 1: linear, x fastest */
-    SPH_OPT_SOLVER_OCCUPANCY = 2, /* DFSPH persistent solver blocks per SM: 8 (default) or 4 */
+    SPH_OPT_SOLVER_OCCUPANCY = 2, /* DFSPH persistent solver blocks per SM: 8 or 4; until set it reads 8 and
+                                     the library chooses */
     SPH_OPT_PASS_BLOCK = 3,       /* threads per block of the particle-pass kernels: 256 (default) or 128 */
     SPH_OPT_SOLVER_LANES = 4,     /* lanes sharing one particle's neighbour list in the persistent DFSPH
-                                     solver: 1, 2 (default) or 4 */
+                                     solver: 1, 2 or 4; 1 and 2 give the same bits; until set it reads 2 and
+                                     the library chooses 1 or 2 by size */
     SPH_OPT_POSITION_RESIDUAL = 5,/* 1: every position keeps the rounding residual of its integration
                                      (float pair, error-free sums), so long runs of small steps keep about
                                      twice float precision; 0 (default): FP32 positions rounded as the

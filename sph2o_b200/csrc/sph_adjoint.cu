@@ -134,7 +134,6 @@ __global__ void __launch_bounds__(256, 4) k_adj_forces(SimParams P, AdjointArray
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = t / TPP;
     const unsigned sub = (unsigned)t % TPP;
-    const size_t nf = (size_t)P.nf;
     double kbar = 0.0, nubar = 0.0;
     float sA = 0.0f, sB = 0.0f, rv = 0.0f, sbv = 0.0f, nup = 0.0f;
     float xrx = 0.0f, xry = 0.0f, xrz = 0.0f, vrx = 0.0f, vry = 0.0f, vrz = 0.0f;
@@ -153,7 +152,7 @@ __global__ void __launch_bounds__(256, 4) k_adj_forces(SimParams P, AdjointArray
         const float inv_rho_i = 1.0f / rho_i;
         const unsigned nF = J.cnt_f[i];
         for (unsigned kk = sub; kk < nF; kk += TPP) {
-            const unsigned j = list_at(J.nbr_f, kk, nf, i);
+            const unsigned j = list_at(J.nbr_f, kk, P.capF, i);
             const float4 xj = J.pos[j];
             float rx, ry, rz, s, rl, inv_rl, f, g;
             pair_of(xi, xj, rx, ry, rz, s, rl, inv_rl);
@@ -196,7 +195,7 @@ __global__ void __launch_bounds__(256, 4) k_adj_forces(SimParams P, AdjointArray
         }
         const unsigned nB = J.cnt_b[i];
         for (unsigned kk = sub; kk < nB; kk += TPP) {
-            const float4 xb = J.bpos[list_at(J.nbr_b, kk, nf, i)];
+            const float4 xb = J.bpos[list_at(J.nbr_b, kk, P.capB, i)];
             float rx, ry, rz, s, rl, inv_rl, f, g;
             pair_of(xi, xb, rx, ry, rz, s, rl, inv_rl);
             cs_grad_fg(rl, inv_rl, P, f, g);
@@ -292,13 +291,12 @@ __global__ void __launch_bounds__(256, 6) k_adj_density(SimParams P, AdjointArra
     const unsigned sub = (unsigned)t % TPP;
     /* a group's lanes share i, so a group leaves together */
     if (i >= P.nf) return;
-    const size_t nf = (size_t)P.nf;
     const float4 xi = J.pos[i];
     const float rbi = J.rhobar[i];
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
     const unsigned nF = J.cnt_f[i];
     for (unsigned kk = sub; kk < nF; kk += TPP) {
-        const unsigned j = list_at(J.nbr_f, kk, nf, i);
+        const unsigned j = list_at(J.nbr_f, kk, P.capF, i);
         float rx, ry, rz, s, rl, inv_rl;
         pair_of(xi, J.pos[j], rx, ry, rz, s, rl, inv_rl);
         const float f = cs_gradf(rl, inv_rl, P);
@@ -308,7 +306,7 @@ __global__ void __launch_bounds__(256, 6) k_adj_density(SimParams P, AdjointArra
     }
     const unsigned nB = J.cnt_b[i];
     for (unsigned kk = sub; kk < nB; kk += TPP) {
-        const float4 xb = J.bpos[list_at(J.nbr_b, kk, nf, i)];
+        const float4 xb = J.bpos[list_at(J.nbr_b, kk, P.capB, i)];
         float rx, ry, rz, s, rl, inv_rl;
         pair_of(xi, xb, rx, ry, rz, s, rl, inv_rl);
         const float c = xb.w * rbi * cs_gradf(rl, inv_rl, P);

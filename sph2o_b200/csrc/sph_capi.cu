@@ -63,13 +63,14 @@ struct sph_ctx {
     unsigned *orig = nullptr, *orig2 = nullptr;
     float *kws = nullptr, *kws2 = nullptr, *kvws = nullptr, *kvws2 = nullptr;
     float4 *acc = nullptr, *normal = nullptr, *predr = nullptr, *pacc = nullptr;
-    float *rho = nullptr, *alpha = nullptr, *k = nullptr, *press = nullptr;
+    float *rho = nullptr, *alpha = nullptr, *press = nullptr;
     unsigned *cell_of = nullptr, *slot = nullptr, *tmp_key = nullptr, *tmp_src = nullptr, *cell_sorted = nullptr;
     unsigned *cell_count = nullptr, *cell_start = nullptr, *bcell_start = nullptr, *block_sums = nullptr;
     float4* bpos = nullptr;
     float* bvol = nullptr;
     unsigned* borig = nullptr;
     unsigned *nbr_f = nullptr, *cnt_f = nullptr, *nbr_b = nullptr, *cnt_b = nullptr;
+    uint2 *pair_f = nullptr, *pair_b = nullptr; /* DFSPH: list entries with their kernel factors */
     DevState* st = nullptr;
     DevState* st_host = nullptr; /* pinned mirror */
     double* accum = nullptr;
@@ -105,9 +106,9 @@ struct sph_ctx {
     bool use_graphs = true;
     /* tunables (sph_set_option / sph_autotune) */
     int pass_block = 256;
-    int solver_occ = 8;
+    int solver_occ = 0;  /* blocks per SM and lanes of the persistent DFSPH solver; 0: not set, by size */
     bool staged_lists = false; /* SPH_OPT_LIST_STAGED */
-    int solver_tpp = 2;  /* measured best on B200 for the 1M-particle scene (1, 2, 4: 1.03, 0.84, 0.92 ms) */
+    int solver_tpp = 0;
     float* stage = nullptr;      /* 3 max(nf, nb) floats: device side of every host transfer (see sph_get_state) */
     float4* braw = nullptr;      /* boundary in caller order (re-sorted when the cell order changes) */
     unsigned* bid = nullptr;
@@ -125,6 +126,7 @@ struct sph_ctx {
     float4 *plo = nullptr, *plo2 = nullptr;
     float4* snap_plo = nullptr;
     float* divres = nullptr;  /* DFSPH: divergence error of the density pass */
+    float4* rec = nullptr;    /* DFSPH: the solvers' working records (DeviceArrays::rec) */
     /* autotune snapshot */
     float4 *snap_pos = nullptr, *snap_vel = nullptr;
     unsigned* snap_orig = nullptr;
@@ -348,16 +350,18 @@ DeviceArrays arrays(sph_ctx* c)
     DeviceArrays A{};
     A.pos = c->pos; A.vel = c->vel; A.pos_alt = c->pos2; A.vel_alt = c->vel2;
     A.acc = c->acc; A.normal = c->normal; A.predr = c->predr; A.pacc = c->pacc;
-    A.rho = c->rho; A.alpha = c->alpha; A.k = c->k; A.kws = c->kws; A.kvws = c->kvws; A.press = c->press;
+    A.rho = c->rho; A.alpha = c->alpha; A.kws = c->kws; A.kvws = c->kvws; A.press = c->press;
     A.orig_w = c->orig;
     A.cell_start = c->cell_start; A.cell_sorted = c->cell_sorted;
     A.bpos = c->bpos; A.bcell_start = c->bcell_start;
     A.nbr_f = c->nbr_f; A.cnt_f = c->cnt_f; A.nbr_b = c->nbr_b; A.cnt_b = c->cnt_b;
+    A.pair_f = c->pair_f; A.pair_b = c->pair_b;
     A.accum = c->accum; A.st = c->st;
     A.bnormal = c->bnormal; A.bdens = c->bdens; A.bpress = c->bpress; A.bdp = c->bdp;
     A.predv = c->predv; A.cell_entry = c->cell_entry;
     A.plo = c->P.pos_lo ? c->plo : nullptr;
     A.divres = c->divres;
+    A.rec = c->rec;
     A.plo_alt = c->P.pos_lo ? c->plo2 : nullptr;
     if (c->nscenes) {
         A.sref.scenes = c->d_scenes;
@@ -428,8 +432,12 @@ void drain_profile(sph_ctx* c)
 int alloc_lists(sph_ctx* c)
 {
     int rc;
-    if ((rc = dalloc(c, &c->nbr_f, (size_t)c->P.capF * c->nf)) != SPH_OK) return rc;
-    if ((rc = dalloc(c, &c->nbr_b, (size_t)c->P.capB * c->nf)) != SPH_OK) return rc;
+    if ((rc = dalloc(c, &c->nbr_f, list_len(c->nf, c->P.capF))) != SPH_OK) return rc;
+    if ((rc = dalloc(c, &c->nbr_b, list_len(c->nf, c->P.capB))) != SPH_OK) return rc;
+    if (c->desc.simulation_method == SPH_DFSPH) {
+        if ((rc = dalloc(c, &c->pair_f, list_len(c->nf, c->P.capF))) != SPH_OK) return rc;
+        if ((rc = dalloc(c, &c->pair_b, list_len(c->nf, c->P.capB))) != SPH_OK) return rc;
+    }
     return SPH_OK;
 }
 
@@ -543,11 +551,23 @@ int step_pcisph(sph_ctx* c)
     return check_launch(c, "pcisph step");
 }
 
+/* Blocks per SM of the persistent DFSPH solver: 4 (64 registers, four gathers
+   in flight) unless set; 8 (32 registers, two) measured slower at every size
+   (26k 153 against 136 us of density solver per step, 125k 223 against 205,
+   1M 1,282 against 1,231). */
+int solver_occ(const sph_ctx* c) { return c->solver_occ ? c->solver_occ : 4; }
+
+/* Lanes per particle of the persistent DFSPH solver unless set: one from 2^16
+   particles on, where they fill the 148 x 4 x 256 resident threads (125k: 205
+   us of density solver per step against 209 with two lanes; 1M: 1,231 against
+   1,361); two below (26k: 136 against 149). Both give the same bits. */
+int solver_lanes(const sph_ctx* c) { return c->solver_tpp ? c->solver_tpp : c->nf >= (1u << 16) ? 1 : 2; }
+
 int tpp_index(int tpp) { return tpp == 4 ? 2 : tpp == 2 ? 1 : 0; }
 
 int solve_grid(const sph_ctx* c, bool divergence)
 {
-    return c->grid_solve[divergence ? 1 : 0][c->solver_occ == 4 ? 1 : 0][tpp_index(c->solver_tpp)];
+    return c->grid_solve[divergence ? 1 : 0][solver_occ(c) == 4 ? 1 : 0][tpp_index(solver_lanes(c))];
 }
 
 int step_dfsph(sph_ctx* c)
@@ -561,7 +581,7 @@ int step_dfsph(sph_ctx* c)
     {
         Phase ph(c, SPH_PROF_DENSITY_SOLVE, 1);
         e = c->nscenes ? launch_dfsph_solve_batch(c->P, A, false, c->grid_batch_density, c->stream)
-                       : launch_dfsph_solve(c->P, A, false, solve_grid(c, false), c->solver_occ, c->solver_tpp, c->stream);
+                       : launch_dfsph_solve(c->P, A, false, solve_grid(c, false), solver_occ(c), solver_lanes(c), c->stream);
     }
     if (e != 0) return fail(c, SPH_ERR_CUDA, std::string("dfsph density solver launch: ") + cudaGetErrorString((cudaError_t)e));
     if (c->P.pcib) { /* DFSPHSolver.cpp:60-70 */
@@ -577,7 +597,7 @@ int step_dfsph(sph_ctx* c)
     {
         Phase ph(c, SPH_PROF_DIVERGENCE_SOLVE, 1);
         e = c->nscenes ? launch_dfsph_solve_batch(c->P, A, true, c->grid_batch_div, c->stream)
-                       : launch_dfsph_solve(c->P, A, true, solve_grid(c, true), c->solver_occ, c->solver_tpp, c->stream);
+                       : launch_dfsph_solve(c->P, A, true, solve_grid(c, true), solver_occ(c), solver_lanes(c), c->stream);
     }
     if (e != 0) return fail(c, SPH_ERR_CUDA, std::string("dfsph divergence solver launch: ") + cudaGetErrorString((cudaError_t)e));
     cube_correct(c); /* DFSPHSolver.cpp:94-103 */
@@ -588,9 +608,10 @@ int step_dfsph(sph_ctx* c)
            particle's current position, with the cell contents of the last
            insertion, and evaluate distances at current positions: rebuild
            the lists from the current positions against the same cell table. */
-        Phase ph(c, SPH_PROF_LISTS, 1);
+        Phase ph(c, SPH_PROF_LISTS, 2);
         launch_build_lists(c->P, SceneRef{c->d_scenes, c->d_scene_of}, c->pos, c->cell_start, c->bpos, c->bcell_start,
                            c->nbr_f, c->cnt_f, c->nbr_b, c->cnt_b, c->st, c->stream);
+        launch_pair_factors(c->P, arrays(c), c->stream);
     }
     return check_launch(c, "dfsph step");
 }
@@ -630,13 +651,15 @@ int recover_overflow(sph_ctx* c)
     CUDA_TRY(c, cudaMemcpyAsync(&c->st->err, &zero, sizeof(int), cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(c, cudaMemcpyAsync(&c->st->overflow, &uzero, sizeof(unsigned), cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-    auto drop = [&](unsigned* p) {
-        auto it = std::find(c->allocations.begin(), c->allocations.end(), (void*)p);
+    auto drop = [&](void* p) {
+        auto it = std::find(c->allocations.begin(), c->allocations.end(), p);
         if (it != c->allocations.end()) { cudaFree(p); c->allocations.erase(it); }
     };
     drop_graphs(c);
     drop(c->nbr_f);
     drop(c->nbr_b);
+    drop(c->pair_f);
+    drop(c->pair_b);
     c->P.capF = c->P.capF + c->P.capF / 2;
     c->P.capB = c->P.capB + c->P.capB / 2;
     c->lists_valid = false;
@@ -1037,7 +1060,7 @@ int sph_init(sph_ctx* c)
     ALLOC(pos, nf); ALLOC(vel, nf); ALLOC(pos2, nf); ALLOC(vel2, nf);
     ALLOC(orig, nf); ALLOC(orig2, nf);
     ALLOC(kws, nf); ALLOC(kws2, nf); ALLOC(kvws, nf); ALLOC(kvws2, nf);
-    ALLOC(acc, nf); ALLOC(rho, nf); ALLOC(alpha, nf); ALLOC(k, nf); ALLOC(press, nf);
+    ALLOC(acc, nf); ALLOC(rho, nf); ALLOC(alpha, nf); ALLOC(press, nf);
     ALLOC(normal, nf); ALLOC(predr, nf); ALLOC(pacc, nf);
     ALLOC(cell_of, nmax); ALLOC(slot, nmax); ALLOC(tmp_key, nmax); ALLOC(tmp_src, nmax); ALLOC(cell_sorted, nmax);
     ALLOC(cell_count, (size_t)P.ncells); ALLOC(cell_start, (size_t)P.ncells + 1);
@@ -1055,7 +1078,10 @@ int sph_init(sph_ctx* c)
     c->orig_base = c->orig;
     c->kws_base = c->kws;
     if ((rc = alloc_lists(c)) != SPH_OK) return rc;
-    if (c->desc.simulation_method == SPH_DFSPH && (rc = dalloc(c, &c->divres, nf)) != SPH_OK) return rc;
+    if (c->desc.simulation_method == SPH_DFSPH) {
+        if ((rc = dalloc(c, &c->divres, nf)) != SPH_OK) return rc;
+        if ((rc = dalloc(c, &c->rec, 2 * nf)) != SPH_OK) return rc;
+    }
     if (c->pos_lo) {
         if (c->nscenes) return fail(c, SPH_ERR_ARG, "position residuals apply to single scenes, not to batches");
         if ((rc = dalloc(c, &c->plo, nf)) != SPH_OK) return rc;
@@ -1686,9 +1712,9 @@ int sph_get_option(const sph_ctx* c, int option, int* value)
     switch (option) {
     case SPH_OPT_CUDA_GRAPHS: *value = c->use_graphs ? 1 : 0; return SPH_OK;
     case SPH_OPT_CELL_ORDER: *value = c->P.cell_order; return SPH_OK;
-    case SPH_OPT_SOLVER_OCCUPANCY: *value = c->solver_occ; return SPH_OK;
+    case SPH_OPT_SOLVER_OCCUPANCY: *value = c->solver_occ ? c->solver_occ : 8; return SPH_OK;
     case SPH_OPT_PASS_BLOCK: *value = c->pass_block; return SPH_OK;
-    case SPH_OPT_SOLVER_LANES: *value = c->solver_tpp; return SPH_OK;
+    case SPH_OPT_SOLVER_LANES: *value = c->solver_tpp ? c->solver_tpp : 2; return SPH_OK;
     case SPH_OPT_POSITION_RESIDUAL: *value = c->pos_lo; return SPH_OK;
     case SPH_OPT_LIST_STAGED: *value = c->staged_lists ? 1 : 0; return SPH_OK;
     default: return SPH_ERR_ARG;
@@ -1704,7 +1730,7 @@ int sph_autotune(sph_ctx* c, int trial_steps, const char* cache_path, int* confi
         /* trial steps would advance the carried normals and the per-cell search record */
         return fail(c, SPH_ERR_ARG, "sph_autotune is not available with the PCISPH boundary method");
     const std::string key = tune_key(c);
-    int best[SPH_TUNE_COUNT] = {c->P.cell_order, c->solver_occ, c->pass_block, c->solver_tpp};
+    int best[SPH_TUNE_COUNT] = {c->P.cell_order, solver_occ(c), c->pass_block, solver_lanes(c)};
     int rc;
     if (tune_lookup(cache_path, key, best)) {
         if ((rc = apply_config(c, best)) != SPH_OK) return rc;
@@ -1879,9 +1905,10 @@ int sph_debug_neighbors(sph_ctx* c, unsigned* f_offsets, unsigned* f_index, size
     if (!c->initialized) return fail(c, SPH_ERR_STATE, "sph_debug_neighbors before sph_init");
     int rc = neighbor_search(c);
     if (rc != SPH_OK) return rc;
+    if (c->pair_f) launch_pair_factors(c->P, arrays(c), c->stream); /* the next DFSPH step reads them */
     const size_t nf = c->nf, nb = c->nb;
     std::vector<unsigned> cntf(nf), cntb(nf), orig(nf), borig(nb);
-    std::vector<unsigned> nbrf((size_t)c->P.capF * nf), nbrb((size_t)c->P.capB * nf);
+    std::vector<unsigned> nbrf(list_len(nf, c->P.capF)), nbrb(list_len(nf, c->P.capB));
     CUDA_TRY(c, cudaMemcpyAsync(cntf.data(), c->cnt_f, nf * 4, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaMemcpyAsync(cntb.data(), c->cnt_b, nf * 4, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaMemcpyAsync(orig.data(), c->orig, nf * 4, cudaMemcpyDeviceToHost, c->stream));
@@ -1902,9 +1929,9 @@ int sph_debug_neighbors(sph_ctx* c, unsigned* f_offsets, unsigned* f_index, size
         if (b_offsets) b_offsets[o] = (unsigned)tb;
         if (i == (size_t)-1) continue; /* inactive (emitter) particle: no neighbours */
         for (unsigned k = 0; k < cntf[i]; ++k, ++tf)
-            if (f_index && tf < f_cap) f_index[tf] = orig[nbrf[(size_t)k * nf + i]];
+            if (f_index && tf < f_cap) f_index[tf] = orig[nbrf[list_index(k, c->P.capF, (unsigned)i)]];
         for (unsigned k = 0; k < cntb[i]; ++k, ++tb)
-            if (b_index && tb < b_cap) b_index[tb] = borig[nbrb[(size_t)k * nf + i]];
+            if (b_index && tb < b_cap) b_index[tb] = borig[nbrb[list_index(k, c->P.capB, (unsigned)i)]];
     }
     if (f_offsets) f_offsets[nf] = (unsigned)tf;
     if (b_offsets) b_offsets[nf] = (unsigned)tb;
@@ -1979,7 +2006,7 @@ int adj_reserve(sph_ctx* c, int nseg, int every)
         AALLOC(ck_pos, (size_t)nseg * nf); AALLOC(ck_vel, (size_t)nseg * nf); AALLOC(ck_orig, (size_t)nseg * nf);
         a.cap_seg = nseg;
     }
-    const size_t list_bytes = (size_t)every * nf * ((size_t)(c->P.capF + c->P.capB) * 4 + 16);
+    const size_t list_bytes = (size_t)every * (list_len(nf, c->P.capF + c->P.capB) * 4 + nf * 16);
     const bool keep = list_bytes <= kAdjointListBudget;
     if (every > a.cap_every || keep != a.keep_lists ||
         (keep && (a.sl_capF != c->P.capF || a.sl_capB != c->P.capB))) {
@@ -1993,7 +2020,7 @@ int adj_reserve(sph_ctx* c, int nseg, int every)
         a.cap_every = 0;
         AALLOC(sl_pos, (size_t)cap * nf); AALLOC(sl_vel, (size_t)cap * nf); AALLOC(sl_orig, (size_t)cap * nf);
         if (keep) {
-            AALLOC(sl_nbr_f, (size_t)cap * c->P.capF * nf); AALLOC(sl_nbr_b, (size_t)cap * c->P.capB * nf);
+            AALLOC(sl_nbr_f, cap * list_len(nf, c->P.capF)); AALLOC(sl_nbr_b, cap * list_len(nf, c->P.capB));
             AALLOC(sl_cnt_f, (size_t)cap * nf); AALLOC(sl_cnt_b, (size_t)cap * nf);
             AALLOC(sl_rho, (size_t)cap * nf); AALLOC(sl_press, (size_t)cap * nf);
             a.sl_capF = c->P.capF;
@@ -2045,7 +2072,7 @@ AdjointArrays adj_arrays_kept(sph_ctx* c, int n)
     AdjointArrays J = adj_arrays(c);
     J.pos = a.sl_pos + n * nf; J.vel = a.sl_vel + n * nf; J.orig = a.sl_orig + n * nf;
     J.rho = a.sl_rho + n * nf; J.press = a.sl_press + n * nf;
-    J.nbr_f = a.sl_nbr_f + (size_t)n * a.sl_capF * nf; J.nbr_b = a.sl_nbr_b + (size_t)n * a.sl_capB * nf;
+    J.nbr_f = a.sl_nbr_f + n * list_len(nf, a.sl_capF); J.nbr_b = a.sl_nbr_b + n * list_len(nf, a.sl_capB);
     J.cnt_f = a.sl_cnt_f + n * nf; J.cnt_b = a.sl_cnt_b + n * nf;
     return J;
 }
@@ -2063,7 +2090,7 @@ int adj_segment_body(sph_ctx* c, int len)
             /* the step builds its lists and densities straight into slot n */
             unsigned *lf = c->nbr_f, *cf = c->cnt_f, *lb = c->nbr_b, *cb = c->cnt_b;
             float *rho = c->rho, *press = c->press;
-            c->nbr_f = a.sl_nbr_f + (size_t)n * a.sl_capF * nf; c->nbr_b = a.sl_nbr_b + (size_t)n * a.sl_capB * nf;
+            c->nbr_f = a.sl_nbr_f + n * list_len(nf, a.sl_capF); c->nbr_b = a.sl_nbr_b + n * list_len(nf, a.sl_capB);
             c->cnt_f = a.sl_cnt_f + n * nf; c->cnt_b = a.sl_cnt_b + n * nf;
             c->rho = a.sl_rho + n * nf; c->press = a.sl_press + n * nf;
             rc = step_wcsph(c);

@@ -8,9 +8,10 @@
  *   rho, alpha, k, kws, kvws, press    float scalars (SoA)
  *   orig uint32 caller-order id of each sorted slot
  *   bpos float4 (x, y, z, psi = rho0 * V_b) for the static boundary
- *   neighbour lists: column-major uint32 nbrF[k * nf + i] / nbrB[k * nf + i]
- *   with counts cntF[i] / cntB[i], so a warp of consecutive particles reads
- *   its k-th neighbours as one coalesced 128-byte line.
+ *   neighbour lists: uint32 entries in tiles of 32 particles, entry k of
+ *   particle i at list_index(k, capacity, i), counts cntF[i] / cntB[i]: a warp
+ *   of 32 consecutive particles reads its k-th neighbours as one coalesced
+ *   128-byte line and its whole lists from one contiguous stretch.
  */
 #ifndef SPH2O_DEVICE_CUH
 #define SPH2O_DEVICE_CUH
@@ -396,13 +397,24 @@ static inline float sqrt_le_bound(float h)
     return s;
 }
 
-/* Entry kk of sorted particle i's neighbour list (column-major). The lists
+/* Place of entry kk of sorted particle i in a neighbour-list array of `cap`
+   entries per particle: tiles of 32 particles, 32 consecutive entries per
+   row, the rows of a tile one after the other. */
+__host__ __device__ __forceinline__ size_t list_index(unsigned kk, unsigned cap, unsigned i)
+{
+    return ((size_t)(i >> 5) * cap + kk) * 32 + (i & 31u);
+}
+
+/* Entries of a list array of n particles. */
+static inline size_t list_len(size_t n, unsigned cap) { return (n + 31) / 32 * 32 * cap; }
+
+/* Entry kk of sorted particle i's neighbour list. The lists
    are streamed once per pass and at 1M particles are larger than the L2, so
    they are loaded with the evict-first hint (ld.global.cs): they must not
    push out of L2 the particle state that the neighbour gathers read. */
-__device__ __forceinline__ unsigned list_at(const unsigned* list, unsigned kk, size_t nf, int i)
+__device__ __forceinline__ unsigned list_at(const unsigned* list, unsigned kk, unsigned cap, int i)
 {
-    return __ldcs(list + kk * nf + i);
+    return __ldcs(list + list_index(kk, cap, (unsigned)i));
 }
 
 /* ---------------------------------------------------------------------- */

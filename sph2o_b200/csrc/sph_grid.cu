@@ -145,7 +145,6 @@ __device__ __forceinline__ void build_lists_at(const SimParams& P, const SceneRe
                                                DevState* st)
 {
     const float4 xi = pos[i];
-    const size_t nf = (size_t)P.nf;
     /* |r| <= h as the reference rounds it, without the square root */
     const float s2max = P.h2_exact;
     unsigned nF = 0, nB = 0;
@@ -153,7 +152,7 @@ __device__ __forceinline__ void build_lists_at(const SimParams& P, const SceneRe
         const unsigned s = cell_start[c], e = cell_start[c + 1];
         for (unsigned q = s; q < e; ++q) {
             if (dist2_exact(xi, pos[q]) <= s2max) {
-                if (nF < P.capF) __stcs(nbr_f + (size_t)nF * nf + i, q);
+                if (nF < P.capF) __stcs(nbr_f + list_index(nF, P.capF, i), q);
                 ++nF;
             }
         }
@@ -161,7 +160,7 @@ __device__ __forceinline__ void build_lists_at(const SimParams& P, const SceneRe
             const unsigned bs = bcell_start[c], be = bcell_start[c + 1];
             for (unsigned q = bs; q < be; ++q) {
                 if (dist2_exact(xi, bpos[q]) <= s2max) {
-                    if (nB < P.capB) __stcs(nbr_b + (size_t)nB * nf + i, q);
+                    if (nB < P.capB) __stcs(nbr_b + list_index(nB, P.capB, i), q);
                     ++nB;
                 }
             }
@@ -282,7 +281,6 @@ __global__ void __launch_bounds__(kStagedBlock) k_ns_build_lists_staged(
             for (unsigned k = (unsigned)lane; k < n; k += 32u) s_pos[o + k] = pos[s + k];
         }
     __syncthreads();
-    const size_t nf = (size_t)P.nf;
     const float s2max = P.h2_exact;
     for (unsigned i = ps + threadIdx.x; i < pe; i += kStagedBlock) {
         const float4 xi = pos[i];
@@ -307,13 +305,13 @@ __global__ void __launch_bounds__(kStagedBlock) k_ns_build_lists_staged(
                     for (unsigned k = 0; k < n; ++k) {
                         const float4 xq = staged ? s_pos[o + k] : pos[s + k];
                         if (dist2_exact(xi, xq) <= s2max) {
-                            if (nF < P.capF) __stcs(nbr_f + (size_t)nF * nf + i, s + k);
+                            if (nF < P.capF) __stcs(nbr_f + list_index(nF, P.capF, i), s + k);
                             ++nF;
                         }
                     }
                     for (unsigned q = s_bs[h]; q < s_be[h]; ++q) {
                         if (dist2_exact(xi, bpos[q]) <= s2max) {
-                            if (nB < P.capB) __stcs(nbr_b + (size_t)nB * nf + i, q);
+                            if (nB < P.capB) __stcs(nbr_b + list_index(nB, P.capB, i), q);
                             ++nB;
                         }
                     }

@@ -82,7 +82,7 @@ __device__ __forceinline__ void ns_rank_gather_at(int p, const unsigned* __restr
    particle shrinks from ~216 candidates (or 27 cells) to ~7 rounds. */
 __device__ __forceinline__ void warp_candidates(const float4* __restrict__ xs, unsigned s, unsigned e, float4 xi,
                                                 float s2max, unsigned lane, unsigned cap, unsigned* __restrict__ list,
-                                                size_t nf, int i, unsigned& n)
+                                                int i, unsigned& n)
 {
     const unsigned cnt = e - s;
     unsigned incl = cnt;
@@ -105,7 +105,7 @@ __device__ __forceinline__ void warp_candidates(const float4* __restrict__ xs, u
         const unsigned bits = __ballot_sync(0xffffffffu, in);
         if (in) {
             const unsigned r = n + __popc(bits & ((1u << lane) - 1u));
-            if (r < cap) __stcs(list + (size_t)r * nf + i, q);
+            if (r < cap) __stcs(list + list_index(r, cap, i), q);
         }
         n += __popc(bits);
     }
@@ -140,10 +140,9 @@ __device__ __forceinline__ void build_lists_warp_at(const SimParams& P, const Sc
             }
         }
     }
-    const size_t nf = (size_t)P.nf;
     unsigned nF = 0, nB = 0;
-    warp_candidates(pos, s, e, xi, P.h2_exact, lane, P.capF, nbr_f, nf, i, nF);
-    if (P.nb > 0) warp_candidates(bpos, bs, be, xi, P.h2_exact, lane, P.capB, nbr_b, nf, i, nB);
+    warp_candidates(pos, s, e, xi, P.h2_exact, lane, P.capF, nbr_f, i, nF);
+    if (P.nb > 0) warp_candidates(bpos, bs, be, xi, P.h2_exact, lane, P.capB, nbr_b, i, nB);
     if (lane != 0) return;
     cnt_f[i] = min(nF, P.capF);
     cnt_b[i] = min(nB, P.capB);

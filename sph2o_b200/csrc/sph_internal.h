@@ -28,7 +28,6 @@ struct DeviceArrays {
     float4* pacc;         /* PCISPH pressure acceleration */
     float* rho;
     float* alpha;
-    float* k;
     float* kws;
     float* kvws;
     float* press;
@@ -40,6 +39,13 @@ struct DeviceArrays {
     const unsigned* cnt_f;
     const unsigned* nbr_b;
     const unsigned* cnt_b;
+    /* DFSPH: the lists with each entry's kernel factor, (slot, bits of f with
+       gradW = f r), in the layout of nbr_f / nbr_b (see k_density) */
+    uint2* pair_f;
+    uint2* pair_b;
+    /* DFSPH solvers' working state, two float4 per particle: (x, y, z, k) and
+       (vx, vy, vz, 0), so a neighbour's half or whole record is one load */
+    float4* rec;
     unsigned* orig_w;     /* caller-order ids of the sorted slots (emitters write new ones) */
     double* accum;        /* per-iteration residual accumulators, zeroed per solve */
     DevState* st;
@@ -61,9 +67,7 @@ struct DeviceArrays {
        integration target */
     float4* plo;
     float4* plo_alt;
-    /* DFSPH: divergence error of the density pass (NULL: the divergence
-       solver computes its warm-start residual itself) */
-    float* divres;
+    float* divres;        /* DFSPH: divergence error of the density pass */
 };
 
 /* sph_grid.cu */
@@ -93,6 +97,9 @@ enum ForceMode : int {
 
 /* block: threads per block of the pass kernels (128 or 256, autotuned) */
 void launch_density(const SimParams& P, const DeviceArrays& A, bool alpha, bool eos, int block, cudaStream_t s);
+/* pair_f / pair_b from the current lists and positions, where a list build is
+   not followed by the density pass that writes them */
+void launch_pair_factors(const SimParams& P, const DeviceArrays& A, cudaStream_t s);
 void launch_normals(const SimParams& P, const DeviceArrays& A, int block, cudaStream_t s);
 void launch_forces(const SimParams& P, const DeviceArrays& A, int mode, int block, cudaStream_t s);
 /* occ: blocks per SM of the persistent DFSPH solver variant (4 or 8);

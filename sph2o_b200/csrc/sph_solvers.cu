@@ -35,6 +35,7 @@
 #include "sph_device.cuh"
 #include "sph_internal.h"
 
+#include <type_traits>
 
 
 namespace sph {
@@ -54,13 +55,13 @@ __device__ __forceinline__ Pair make_pair(float4 a, float4 b)
     return p;
 }
 
-/* Calls f(j, x_j) for the fluid neighbours of sorted particle i in list
+/* Calls f(kk, j, x_j) for the fluid neighbours (list entry kk) of sorted particle i in list
    order, issuing the list loads and position gathers of U entries before the
    first of them is used (more loads in flight per thread; same order, so the
    sums it feeds are unchanged). With TPP lanes per particle, lane sub visits
    the entries sub, sub + TPP, ... */
 template <int U, int TPP = 1, typename F>
-__device__ __forceinline__ void for_fluid_neighbors(const DeviceArrays& A, int i, size_t nf, unsigned n, F&& f,
+__device__ __forceinline__ void for_fluid_neighbors(const SimParams& P, const DeviceArrays& A, int i, unsigned n, F&& f,
                                                     unsigned sub = 0)
 {
     unsigned kk = sub;
@@ -68,15 +69,15 @@ __device__ __forceinline__ void for_fluid_neighbors(const DeviceArrays& A, int i
         unsigned jj[U];
         float4 xj[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) jj[u] = list_at(A.nbr_f, kk + u * TPP, nf, i);
+        for (int u = 0; u < U; ++u) jj[u] = list_at(A.nbr_f, kk + u * TPP, P.capF, i);
 #pragma unroll
         for (int u = 0; u < U; ++u) xj[u] = A.pos[jj[u]];
 #pragma unroll
-        for (int u = 0; u < U; ++u) f(jj[u], xj[u]);
+        for (int u = 0; u < U; ++u) f(kk + u * TPP, jj[u], xj[u]);
     }
     for (; kk < n; kk += TPP) {
-        const unsigned j = list_at(A.nbr_f, kk, nf, i);
-        f(j, A.pos[j]);
+        const unsigned j = list_at(A.nbr_f, kk, P.capF, i);
+        f(kk, j, A.pos[j]);
     }
 }
 
@@ -197,16 +198,16 @@ __global__ void __launch_bounds__(256, 8) k_density(SimParams P, DeviceArrays A)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= active_n(P, A.st)) return;
-    const size_t nf = (size_t)P.nf;
     const float4 xi = A.pos[i];
     const float4 vi = DIVRES ? A.vel[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float rho = 0.0f, sgx = 0.0f, sgy = 0.0f, sgz = 0.0f, ssq = 0.0f, div = 0.0f;
     const unsigned nF = A.cnt_f[i];
-    for_fluid_neighbors<2>(A, i, nf, nF, [&](unsigned j, const float4& xj) {
+    for_fluid_neighbors<2>(P, A, i, nF, [&](unsigned kk, unsigned j, const float4& xj) {
         rho = __fadd_rn(rho, __fmul_rn(P.mass, cs_W_exact(dist2_exact(xi, xj), P)));
         if (ALPHA) {
             const Pair p = make_pair(xi, xj);
             const float fg = cs_gradf(p.rl, p.inv_rl, P);
+            if (DIVRES) __stcs(A.pair_f + list_index(kk, P.capF, i), make_uint2(j, __float_as_uint(fg)));
             const float f = P.mass * fg;
             const float gx = f * p.rx, gy = f * p.ry, gz = f * p.rz;
             sgx += gx; sgy += gy; sgz += gz;
@@ -219,11 +220,13 @@ __global__ void __launch_bounds__(256, 8) k_density(SimParams P, DeviceArrays A)
     });
     const unsigned nB = A.cnt_b[i];
     for (unsigned kk = 0; kk < nB; ++kk) {
-        const float4 xb = A.bpos[list_at(A.nbr_b, kk, nf, i)];
+        const unsigned bq = list_at(A.nbr_b, kk, P.capB, i);
+        const float4 xb = A.bpos[bq];
         rho = __fadd_rn(rho, __fmul_rn(xb.w, cs_W_exact(dist2_exact(xi, xb), P)));
         if (ALPHA) {
             const Pair p = make_pair(xi, xb);
             const float fg = cs_gradf(p.rl, p.inv_rl, P);
+            if (DIVRES) __stcs(A.pair_b + list_index(kk, P.capB, i), make_uint2(bq, __float_as_uint(fg)));
             const float f = xb.w * fg;
             sgx += f * p.rx; sgy += f * p.ry; sgz += f * p.rz;
             if (DIVRES) div += xb.w * (fg * ((vi.x * p.rx + vi.y * p.ry) + vi.z * p.rz));
@@ -236,7 +239,31 @@ __global__ void __launch_bounds__(256, 8) k_density(SimParams P, DeviceArrays A)
     }
     if (EOS) A.press[i] = tait_pressure(rho, P, P.kr_g);
     /* fewer than 20 neighbours within h: no correction (DFSPHSolver.cpp:608-611) */
-    if (DIVRES) A.divres[i] = (nF + nB < 20u) ? 0.0f : fmaxf(div, 0.0f);
+    if (DIVRES) {
+        A.divres[i] = (nF + nB < 20u) ? 0.0f : fmaxf(div, 0.0f);
+        /* the divergence solver's record */
+        A.rec[2 * (size_t)i] = make_float4(xi.x, xi.y, xi.z, 0.0f);
+        A.rec[2 * (size_t)i + 1] = vi;
+    }
+}
+
+/* What the density pass writes into pair_f / pair_b, alone: after a list
+   build that no density pass follows. */
+__global__ void __launch_bounds__(256) k_pair_factors(SimParams P, DeviceArrays A)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= active_n(P, A.st)) return;
+    const float4 xi = A.pos[i];
+    const unsigned nF = A.cnt_f[i], nB = A.cnt_b[i];
+    for_fluid_neighbors<2>(P, A, i, nF, [&](unsigned kk, unsigned j, const float4& xj) {
+        const Pair p = make_pair(xi, xj);
+        __stcs(A.pair_f + list_index(kk, P.capF, i), make_uint2(j, __float_as_uint(cs_gradf(p.rl, p.inv_rl, P))));
+    });
+    for (unsigned kk = 0; kk < nB; ++kk) {
+        const unsigned bq = list_at(A.nbr_b, kk, P.capB, i);
+        const Pair p = make_pair(xi, A.bpos[bq]);
+        __stcs(A.pair_b + list_index(kk, P.capB, i), make_uint2(bq, __float_as_uint(cs_gradf(p.rl, p.inv_rl, P))));
+    }
 }
 
 /* Density (and the Tait pressure when EOS) of small scenes with TPP lanes per
@@ -252,14 +279,13 @@ __device__ __forceinline__ void density_lanes_at(const SimParams& P, const Devic
     if (i >= active_n(P, A.st)) return;
     const unsigned lane = threadIdx.x & 31u, sub = lane % TPP, first = lane - sub;
     const unsigned gmask = ((1u << TPP) - 1u) << first;
-    const size_t nf = (size_t)P.nf;
     const float4 xi = A.pos[i];
     float rho = 0.0f;
     const unsigned nF = A.cnt_f[i];
     for (unsigned k0 = 0; k0 < nF; k0 += TPP) {
         const unsigned kk = k0 + sub;
         float w = 0.0f;
-        if (kk < nF) w = __fmul_rn(P.mass, cs_W_exact(dist2_exact(xi, A.pos[list_at(A.nbr_f, kk, nf, i)]), P));
+        if (kk < nF) w = __fmul_rn(P.mass, cs_W_exact(dist2_exact(xi, A.pos[list_at(A.nbr_f, kk, P.capF, i)]), P));
 #pragma unroll
         for (int l = 0; l < TPP; ++l) rho = __fadd_rn(rho, __shfl_sync(gmask, w, first + l));
     }
@@ -268,7 +294,7 @@ __device__ __forceinline__ void density_lanes_at(const SimParams& P, const Devic
         const unsigned kk = k0 + sub;
         float w = 0.0f;
         if (kk < nB) {
-            const float4 xb = A.bpos[list_at(A.nbr_b, kk, nf, i)];
+            const float4 xb = A.bpos[list_at(A.nbr_b, kk, P.capB, i)];
             w = __fmul_rn(xb.w, cs_W_exact(dist2_exact(xi, xb), P));
         }
 #pragma unroll
@@ -289,12 +315,11 @@ __global__ void __launch_bounds__(256, 8) k_normals(SimParams P, DeviceArrays A)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= active_n(P, A.st)) return;
-    const size_t nf = (size_t)P.nf;
     const float4 xi = A.pos[i];
     float nx = 0.0f, ny = 0.0f, nz = 0.0f;
     const unsigned nF = A.cnt_f[i];
     for (unsigned kk = 0; kk < nF; ++kk) {
-        const unsigned j = list_at(A.nbr_f, kk, nf, i);
+        const unsigned j = list_at(A.nbr_f, kk, P.capF, i);
         const Pair p = make_pair(xi, A.pos[j]);
         const float f = (P.mass / A.rho[j]) * cs_gradf(p.rl, p.inv_rl, P);
         nx += f * p.rx; ny += f * p.ry; nz += f * p.rz;
@@ -313,7 +338,6 @@ __device__ __forceinline__ void forces_at(const SimParams& P, const DeviceArrays
     const int i = t / TPP;
     const unsigned sub = (unsigned)t % TPP;
     const bool active = i < active_n(P, A.st);
-    const size_t nf = (size_t)P.nf;
     /* per-scene coefficients and time step of a batch */
     const unsigned scene = (A.sst && active) ? A.sref.scene_of[i] : 0u;
     const float dt = A.sst ? (active ? A.sst[scene].dt : 0.0f) : A.st->dt;
@@ -335,7 +359,7 @@ __device__ __forceinline__ void forces_at(const SimParams& P, const DeviceArrays
         const float4 ni = st_on ? A.normal[i] : make_float4(0, 0, 0, 0);
         const float eps_h2 = 0.01f * P.h2;
         float svx = 0.0f, svy = 0.0f, svz = 0.0f; /* standard viscosity sum */
-        for_fluid_neighbors<2, TPP>(A, i, nf, nF, [&](unsigned j, const float4& xj) {
+        for_fluid_neighbors<2, TPP>(P, A, i, nF, [&](unsigned, unsigned j, const float4& xj) {
             const Pair p = make_pair(xi, xj);
             const float rho_j = A.rho[j];
             const float f = cs_gradf(p.rl, p.inv_rl, P);
@@ -386,7 +410,7 @@ __device__ __forceinline__ void forces_at(const SimParams& P, const DeviceArrays
         if (pressure || bvisc || (np && P.adh_on)) {
             float bvx = 0.0f, bvy = 0.0f, bvz = 0.0f;
             for (unsigned kk = sub; kk < nB; kk += TPP) {
-                const unsigned bq = list_at(A.nbr_b, kk, nf, i);
+                const unsigned bq = list_at(A.nbr_b, kk, P.capB, i);
                 const float4 xb = A.bpos[bq];
                 const Pair p = make_pair(xi, xb);
                 const float psi = xb.w;
@@ -490,50 +514,71 @@ __global__ void __launch_bounds__(256, 6) k_forces(SimParams P, DeviceArrays A)
 /* ---------------------------------------------------------------------- */
 /* DFSPH pieces                                                             */
 
-/* Sum of the residual terms of particle i over the neighbour-list entries
-   sub, sub + TPP, ... (fluid, then boundary). The fluid loop issues the
-   gathers of U entries before using any of them (more loads in flight per
-   lane) and adds the terms in list order, so U changes no bit. */
-template <bool DIV, int TPP, int U = 1>
-__device__ __forceinline__ float dfsph_residual_part(const SimParams& P, const DeviceArrays& A, int i, int sub,
-                                                     size_t nf)
+/* Entry kk of particle i in a pair array (evict-first, as list_at). */
+__device__ __forceinline__ uint2 pair_at(const uint2* pairs, unsigned kk, unsigned cap, int i)
 {
-    const float4 xi = A.pos[i];
-    const float4 vi = A.vel[i];
-    float sum = 0.0f;
+    return __ldcs(pairs + list_index(kk, cap, (unsigned)i));
+}
+
+/* Record j of DeviceArrays::rec, both halves with one 256-bit load. */
+__device__ __forceinline__ void load_rec(const float4* rec, unsigned j, float4& a, float4& b)
+{
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(rec + 2 * (size_t)j)
+                 : "memory");
+}
+
+/* One fluid term of the residual: m f (v_i - v_j) . r_ij */
+__device__ __forceinline__ float dfsph_residual_term(const SimParams& P, float4 xi, float4 vi, float4 xj, float4 vj,
+                                                     float f)
+{
+    const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
+    return P.mass * (f * (((vi.x - vj.x) * rx + (vi.y - vj.y) * ry) + (vi.z - vj.z) * rz));
+}
+
+/* Sum of the residual terms of particle i over the neighbour-list entries
+   sub, sub + TPP, ... (fluid, then boundary), as ACC interleaved partial sums
+   added at the end. The fluid loop issues the gathers of U entries before
+   using any of them (more loads in flight per lane) and adds the terms in
+   list order, so U changes no bit; TPP * ACC = 2 is one order of additions
+   whichever way it is split. */
+template <int TPP, int ACC, int U>
+__device__ __forceinline__ float dfsph_residual_part(const SimParams& P, const DeviceArrays& A, int i, int sub)
+{
+    static_assert(U % ACC == 0, "an unrolled round holds whole rounds of partial sums");
+    float4 xi, vi;
+    load_rec(A.rec, (unsigned)i, xi, vi);
+    float s[ACC];
+#pragma unroll
+    for (int c = 0; c < ACC; ++c) s[c] = 0.0f;
     const unsigned nF = A.cnt_f[i], nB = A.cnt_b[i];
+    const auto round = [&](unsigned kk, auto count) {
+        constexpr int N = decltype(count)::value;
+        uint2 e[N];
+        float4 xj[N], vj[N];
+#pragma unroll
+        for (int u = 0; u < N; ++u) e[u] = pair_at(A.pair_f, kk + u * TPP, P.capF, i);
+#pragma unroll
+        for (int u = 0; u < N; ++u) load_rec(A.rec, e[u].x, xj[u], vj[u]);
+#pragma unroll
+        for (int u = 0; u < N; ++u) s[u % ACC] += dfsph_residual_term(P, xi, vi, xj[u], vj[u], __uint_as_float(e[u].y));
+    };
     unsigned kk = sub;
-    for (; kk + (U - 1) * TPP < nF; kk += U * TPP) {
-        unsigned jj[U];
-        float4 xj[U], vj[U];
+    for (; kk + (U - 1) * TPP < nF; kk += U * TPP) round(kk, std::integral_constant<int, U>());
+    for (; U > ACC && kk + (ACC - 1) * TPP < nF; kk += ACC * TPP) round(kk, std::integral_constant<int, ACC>());
+    if (ACC > 1 && kk < nF) round(kk, std::integral_constant<int, 1>());
+    for (unsigned kk = sub; kk < nB; kk += TPP * ACC) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) jj[u] = list_at(A.nbr_f, kk + u * TPP, nf, i);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            xj[u] = A.pos[jj[u]];
-            vj[u] = A.vel[jj[u]];
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const Pair p = make_pair(xi, xj[u]);
-            const float f = cs_gradf(p.rl, p.inv_rl, P);
-            sum += P.mass * (f * (((vi.x - vj[u].x) * p.rx + (vi.y - vj[u].y) * p.ry) + (vi.z - vj[u].z) * p.rz));
+        for (int c = 0; c < ACC; ++c) {
+            if (c > 0 && kk + c * TPP >= nB) break;
+            const uint2 e = pair_at(A.pair_b, kk + c * TPP, P.capB, i);
+            const float4 xb = A.bpos[e.x];
+            const float rx = xi.x - xb.x, ry = xi.y - xb.y, rz = xi.z - xb.z;
+            s[c] += xb.w * (__uint_as_float(e.y) * ((vi.x * rx + vi.y * ry) + vi.z * rz));
         }
     }
-    for (; kk < nF; kk += TPP) {
-        const unsigned j = list_at(A.nbr_f, kk, nf, i);
-        const Pair p = make_pair(xi, A.pos[j]);
-        const float4 vj = A.vel[j];
-        const float f = cs_gradf(p.rl, p.inv_rl, P);
-        sum += P.mass * (f * (((vi.x - vj.x) * p.rx + (vi.y - vj.y) * p.ry) + (vi.z - vj.z) * p.rz));
-    }
-    for (unsigned kk = sub; kk < nB; kk += TPP) {
-        const float4 xb = A.bpos[list_at(A.nbr_b, kk, nf, i)];
-        const Pair p = make_pair(xi, xb);
-        const float f = cs_gradf(p.rl, p.inv_rl, P);
-        sum += xb.w * (f * ((vi.x * p.rx + vi.y * p.ry) + vi.z * p.rz));
-    }
-    return sum;
+    return ACC == 2 ? s[0] + s[ACC - 1] : s[0];
 }
 
 /* The residual from the summed terms: predicted density (DIV=false) or
@@ -555,82 +600,89 @@ __device__ __forceinline__ float dfsph_residual_finish(const SimParams& P, const
 
 /* predicted density (DIV=false) or divergence error (DIV=true) of particle i */
 template <bool DIV>
-__device__ __forceinline__ float dfsph_residual(const SimParams& P, const DeviceArrays& A, int i, size_t nf,
-                                                float dt)
+__device__ __forceinline__ float dfsph_residual(const SimParams& P, const DeviceArrays& A, int i, float dt)
 {
-    return dfsph_residual_finish<DIV>(P, A, i, dfsph_residual_part<DIV, 1>(P, A, i, 0, nf), dt);
+    return dfsph_residual_finish<DIV>(P, A, i, dfsph_residual_part<1, 1, 4>(P, A, i, 0), dt);
 }
 
 /* Partial sums over list entries sub, sub + TPP, ... of
    sum_j m (k_i + k_j) gradW  (+ boundary with k_i), the fluid gathers issued
-   U at a time as in dfsph_residual_part. K is written inside the same
-   persistent kernel (before a grid barrier), so it is a plain pointer: a
-   read-only (non-coherent) load path would be wrong for it. */
-template <int TPP, int U = 1>
-__device__ __forceinline__ void dfsph_correct_part(const SimParams& P, const DeviceArrays& A, const float* K, int i,
-                                                   int sub, size_t nf, float& sx, float& sy, float& sz)
+   U at a time and ACC interleaved sums, as in dfsph_residual_part. k is in
+   the records' w, written inside the same persistent kernel (before a grid
+   barrier): a read-only (non-coherent) load path would be wrong for it. */
+template <int TPP, int ACC, int U>
+__device__ __forceinline__ void dfsph_correct_part(const SimParams& P, const DeviceArrays& A, int i, int sub,
+                                                   float& sx, float& sy, float& sz)
 {
-    const float4 xi = A.pos[i];
-    const float ki = K[i];
-    sx = sy = sz = 0.0f;
+    static_assert(U % ACC == 0, "an unrolled round holds whole rounds of partial sums");
+    const float4* rec = A.rec;
+    const float4 xi = rec[2 * (size_t)i];
+    const float ki = xi.w;
+    float tx[ACC], ty[ACC], tz[ACC];
+#pragma unroll
+    for (int c = 0; c < ACC; ++c) tx[c] = ty[c] = tz[c] = 0.0f;
     const unsigned nF = A.cnt_f[i];
-    unsigned kk = sub;
-    for (; kk + (U - 1) * TPP < nF; kk += U * TPP) {
-        unsigned jj[U];
-        float kj[U];
-        float4 xj[U];
+    const auto round = [&](unsigned kk, auto count) {
+        constexpr int N = decltype(count)::value;
+        uint2 e[N];
+        float4 xj[N];
 #pragma unroll
-        for (int u = 0; u < U; ++u) jj[u] = list_at(A.nbr_f, kk + u * TPP, nf, i);
+        for (int u = 0; u < N; ++u) e[u] = pair_at(A.pair_f, kk + u * TPP, P.capF, i);
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            kj[u] = K[jj[u]];
-            xj[u] = A.pos[jj[u]];
-        }
+        for (int u = 0; u < N; ++u) xj[u] = rec[2 * (size_t)e[u].x];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const float ks = ki + kj[u];
+        for (int u = 0; u < N; ++u) {
+            const float ks = ki + xj[u].w;
             if (fabsf(ks) > P.eps) {
-                const Pair p = make_pair(xi, xj[u]);
-                const float c = P.mass * ks * cs_gradf(p.rl, p.inv_rl, P);
-                sx += c * p.rx; sy += c * p.ry; sz += c * p.rz;
+                const float c = P.mass * ks * __uint_as_float(e[u].y);
+                tx[u % ACC] += c * (xi.x - xj[u].x);
+                ty[u % ACC] += c * (xi.y - xj[u].y);
+                tz[u % ACC] += c * (xi.z - xj[u].z);
+            }
+        }
+    };
+    unsigned kk = sub;
+    for (; kk + (U - 1) * TPP < nF; kk += U * TPP) round(kk, std::integral_constant<int, U>());
+    for (; U > ACC && kk + (ACC - 1) * TPP < nF; kk += ACC * TPP) round(kk, std::integral_constant<int, ACC>());
+    if (ACC > 1 && kk < nF) round(kk, std::integral_constant<int, 1>());
+    if (fabsf(ki) > P.eps) {
+        const unsigned nB = A.cnt_b[i];
+        for (unsigned kk = sub; kk < nB; kk += TPP * ACC) {
+#pragma unroll
+            for (int c = 0; c < ACC; ++c) {
+                if (c > 0 && kk + c * TPP >= nB) break;
+                const uint2 e = pair_at(A.pair_b, kk + c * TPP, P.capB, i);
+                const float4 xb = A.bpos[e.x];
+                const float w = xb.w * ki * __uint_as_float(e.y);
+                tx[c] += w * (xi.x - xb.x); ty[c] += w * (xi.y - xb.y); tz[c] += w * (xi.z - xb.z);
             }
         }
     }
-    for (; kk < nF; kk += TPP) {
-        const unsigned j = list_at(A.nbr_f, kk, nf, i);
-        const float ks = ki + K[j];
-        if (fabsf(ks) > P.eps) {
-            const Pair p = make_pair(xi, A.pos[j]);
-            const float c = P.mass * ks * cs_gradf(p.rl, p.inv_rl, P);
-            sx += c * p.rx; sy += c * p.ry; sz += c * p.rz;
-        }
-    }
-    if (fabsf(ki) > P.eps) {
-        const unsigned nB = A.cnt_b[i];
-        for (unsigned kk = sub; kk < nB; kk += TPP) {
-            const float4 xb = A.bpos[list_at(A.nbr_b, kk, nf, i)];
-            const Pair p = make_pair(xi, xb);
-            const float c = xb.w * ki * cs_gradf(p.rl, p.inv_rl, P);
-            sx += c * p.rx; sy += c * p.ry; sz += c * p.rz;
-        }
-    }
+    sx = ACC == 2 ? tx[0] + tx[ACC - 1] : tx[0];
+    sy = ACC == 2 ? ty[0] + ty[ACC - 1] : ty[0];
+    sz = ACC == 2 ? tz[0] + tz[ACC - 1] : tz[0];
 }
 
 __device__ __forceinline__ void dfsph_apply(const DeviceArrays& A, int i, float dt, float sx, float sy, float sz)
 {
-    float4 v = A.vel[i];
+    float4 v = A.rec[2 * (size_t)i + 1];
     v.x = __fsub_rn(v.x, __fmul_rn(dt, sx));
     v.y = __fsub_rn(v.y, __fmul_rn(dt, sy));
     v.z = __fsub_rn(v.z, __fmul_rn(dt, sz));
-    A.vel[i] = v;
+    A.rec[2 * (size_t)i + 1] = v;
+}
+
+/* k of particle i, where its neighbours' correction reads it */
+__device__ __forceinline__ void dfsph_set_k(const DeviceArrays& A, int i, float k)
+{
+    reinterpret_cast<float*>(A.rec)[8 * (size_t)i + 3] = k;
 }
 
 /* v_i -= dt * sum_j m (k_i + k_j) gradW  (+ boundary with k_i) */
-__device__ __forceinline__ void dfsph_correct(const SimParams& P, const DeviceArrays& A, const float* K, int i,
-                                              size_t nf, float dt)
+__device__ __forceinline__ void dfsph_correct(const SimParams& P, const DeviceArrays& A, int i, float dt)
 {
     float sx, sy, sz;
-    dfsph_correct_part<1>(P, A, K, i, 0, nf, sx, sy, sz);
+    dfsph_correct_part<1, 1, 4>(P, A, i, 0, sx, sy, sz);
     dfsph_apply(A, i, dt, sx, sy, sz);
 }
 
@@ -671,22 +723,22 @@ __device__ __forceinline__ void for_particles(int n, F&& f)
 }
 
 /* residual of particle i with its list split over TPP lanes (all lanes call) */
-template <bool DIV, int TPP, int U>
+template <bool DIV, int TPP, int ACC, int U>
 __device__ __forceinline__ float dfsph_residual_lanes(const SimParams& P, const DeviceArrays& A, int i, int sub,
-                                                      bool valid, size_t nf, float dt)
+                                                      bool valid, float dt)
 {
-    float part = valid ? dfsph_residual_part<DIV, TPP, U>(P, A, i, sub, nf) : 0.0f;
+    float part = valid ? dfsph_residual_part<TPP, ACC, U>(P, A, i, sub) : 0.0f;
     if (TPP > 1) part = lane_group_sum<TPP>(part);
     return valid ? dfsph_residual_finish<DIV>(P, A, i, part, dt) : 0.0f;
 }
 
 /* velocity correction of particle i with its list split over TPP lanes */
-template <int TPP, int U>
-__device__ __forceinline__ void dfsph_correct_lanes(const SimParams& P, const DeviceArrays& A, const float* K, int i,
-                                                    int sub, bool valid, size_t nf, float dt)
+template <int TPP, int ACC, int U>
+__device__ __forceinline__ void dfsph_correct_lanes(const SimParams& P, const DeviceArrays& A, int i, int sub,
+                                                    bool valid, float dt)
 {
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-    if (valid) dfsph_correct_part<TPP, U>(P, A, K, i, sub, nf, sx, sy, sz);
+    if (valid) dfsph_correct_part<TPP, ACC, U>(P, A, i, sub, sx, sy, sz);
     if (TPP > 1) {
         sx = lane_group_sum<TPP>(sx);
         sy = lane_group_sum<TPP>(sy);
@@ -695,22 +747,27 @@ __device__ __forceinline__ void dfsph_correct_lanes(const SimParams& P, const De
     if (valid && sub == 0) dfsph_apply(A, i, dt, sx, sy, sz);
 }
 
-/* OCC blocks of 256 per SM: 8 (32 registers) by default -- the passes are
-   bound by the latency of dependent neighbour gathers and full occupancy
-   hides most of it; 4 (64 registers, no spills) is the autotuner's other
-   candidate. TPP lanes share a particle in the neighbour passes (1, 2 or 4):
-   more gathers in flight per particle, fewer particles per warp. Each lane
-   issues U gathers before using them: 2 within the 32 registers of the
-   8-block variant, 4 in the 64-register variant (measured best for each on
-   the 1M-particle scene). */
+/* What bounds the passes: the L1's rate for scattered gathers. A warp-visit
+   (32 lanes, one list entry each) takes ~28 SM cycles whatever the occupancy
+   (8, 6, 5, 4 blocks per SM), and halving its instructions by reading the
+   kernel factor f from pair_f instead of recomputing it (rsqrt, spline) alone
+   left the 1M pass at 107 us. What helped, per pass on the 1M double dam break
+   in motion (5.5 + 1.25 iterations per step), density solver 1,424 -> 1,231 us
+   per step: a neighbour's position, velocity and k in one record, fetched with
+   one 256-bit load (residual) or one 128-bit load (correction) instead of two
+   (109 -> 104 us); lists in contiguous tiles of 32 particles (104 -> 98); one
+   lane per particle with 64 registers and four gathers in flight (98 -> 95).
+   OCC blocks of 256 per SM: 4 (64 registers) by default, 8 (32 registers, two
+   gathers) is the autotuner's other candidate. TPP lanes share a particle;
+   1 and 2 lanes add the same two interleaved sums, so they agree bit for bit. */
 template <bool DIV, int OCC, int TPP>
 __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, DeviceArrays A)
 {
     constexpr int U = OCC == 4 ? 4 : 2;
+    constexpr int ACC = TPP == 1 ? 2 : 1;
     __shared__ double s_red[32];
     DevState* st = A.st;
     const int nfi = active_n(P, st);
-    const size_t nf = (size_t)P.nf;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int nthr = gridDim.x * blockDim.x;
 
@@ -730,9 +787,10 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
         hs = fmaxf(hs, P.min_ts);
         hs = fminf(hs, P.max_ts);
         dt = hs;
-        /* DFSPHSolver::predictVelocities */
+        /* DFSPHSolver::predictVelocities, into the records */
         for (int i = tid; i < nfi; i += nthr) {
             const float4 a = A.acc[i];
+            const float4 x = A.pos[i];
             float4 v = A.vel[i];
             v.x = __fadd_rn(v.x, __fmul_rn(__fadd_rn(a.x, P.gx), dt));
             v.y = __fadd_rn(v.y, __fmul_rn(__fadd_rn(a.y, P.gy), dt));
@@ -741,8 +799,8 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
                with the normals left by the last collision pass (or by the
                surface-tension pass of this step, which shares the array) */
             if (P.pcib) pcib_velocity(P, A.normal[i], v, v);
-            A.vel[i] = v;
-            A.acc[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            A.rec[2 * (size_t)i] = make_float4(x.x, x.y, x.z, 0.0f);
+            A.rec[2 * (size_t)i + 1] = v;
         }
         if (!grid_barrier(st)) return;
     } else {
@@ -751,24 +809,20 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
     const float ts2 = dt * dt;
     float* kws = DIV ? A.kvws : A.kws;
 
-    /* warm start: residual at the current velocities, keep the previous
-       step's accumulated k only where the residual is positive */
+    /* warm start: residual at the current velocities (the divergence error
+       comes from the density pass), keep the previous step's accumulated k
+       only where the residual is positive */
     for_particles<TPP>(nfi, [&](int i, int sub, bool valid) {
-        /* the divergence error may come from the density pass (A.divres) */
-        const float r = (DIV && A.divres) ? (valid ? A.divres[i] : 0.0f)
-                                          : dfsph_residual_lanes<DIV, TPP, U>(P, A, i, sub, valid, nf, dt);
+        const float r = DIV ? (valid ? A.divres[i] : 0.0f)
+                            : dfsph_residual_lanes<DIV, TPP, ACC, U>(P, A, i, sub, valid, dt);
         if (valid && sub == 0) {
-            if (DIV) kws[i] = r > 0.0f ? kws[i] / dt : 0.0f;
-            else kws[i] = r > P.rho0 ? kws[i] / ts2 : 0.0f;
+            if (DIV) dfsph_set_k(A, i, r > 0.0f ? kws[i] / dt : 0.0f);
+            else dfsph_set_k(A, i, r > P.rho0 ? kws[i] / ts2 : 0.0f);
         }
     });
     if (!grid_barrier(st)) return;
-    for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, U>(P, A, kws, i, sub, valid, nf, dt); });
+    for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U>(P, A, i, sub, valid, dt); });
     if (!grid_barrier(st)) return;
-    /* same particle-to-lane mapping as the accumulation below (no barrier between) */
-    for_particles<TPP>(nfi, [&](int i, int sub, bool valid) {
-        if (valid && sub == 0) kws[i] = 0.0f;
-    });
 
     const double limit = DIV ? (double)(P.eta_v / dt) : (double)P.eta;
     const unsigned min_it = DIV ? P.min_it_v : P.min_it;
@@ -780,7 +834,7 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
     while ((avg > limit || it < min_it) && it < max_it) {
         double local = 0.0;
         for_particles<TPP>(nfi, [&](int i, int sub, bool valid) {
-            const float r = dfsph_residual_lanes<DIV, TPP, U>(P, A, i, sub, valid, nf, dt);
+            const float r = dfsph_residual_lanes<DIV, TPP, ACC, U>(P, A, i, sub, valid, dt);
             if (!valid || sub != 0) return;
             float k;
             if (DIV) {
@@ -790,29 +844,27 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
                 k = __fdiv_rn(__fmul_rn(__fsub_rn(r, P.rho0), A.alpha[i]), __fmul_rn(ts2, A.rho[i]));
                 local += (double)((r - P.rho0) / P.rho0);
             }
-            A.k[i] = k;
-            kws[i] += k;
+            dfsph_set_k(A, i, k);
+            kws[i] = it == 0 ? k : kws[i] + k;
         });
         const double bs = block_sum(local, s_red);
         if (threadIdx.x == 0) atomicAdd(&A.accum[it], bs);
         if (!grid_barrier(st)) return;
         avg = *(volatile double*)&A.accum[it] / (double)nfi;
-        for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, U>(P, A, A.k, i, sub, valid, nf, dt); });
+        for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U>(P, A, i, sub, valid, dt); });
         if (!grid_barrier(st)) return;
         ++it;
     }
 
+    /* the accumulated k as the next step's warm start (0 when no iteration
+       ran), the velocities, and DFSPHSolver::updatePositions */
     const float scale = DIV ? dt : ts2;
-    /* the particle-to-lane mapping of the zeroing and accumulation passes:
-       with no iteration there is no barrier after the zeroing */
-    for_particles<TPP>(nfi, [&](int i, int sub, bool valid) {
-        if (valid && sub == 0) kws[i] *= scale;
-    });
-    if (!DIV) {
-        /* DFSPHSolver::updatePositions */
-        bool bad = false;
-        for (int i = tid; i < nfi; i += nthr) {
-            const float4 v = A.vel[i];
+    bool bad = false;
+    for (int i = tid; i < nfi; i += nthr) {
+        kws[i] = it == 0 ? 0.0f : kws[i] * scale;
+        const float4 v = A.rec[2 * (size_t)i + 1];
+        A.vel[i] = v;
+        if (!DIV) {
             float4 x = A.pos[i];
             float4 lo = P.pos_lo ? A.plo[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             x.x = pos_add(x.x, lo.x, __fmul_rn(v.x, dt), P.pos_lo);
@@ -822,8 +874,8 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
             if (P.pos_lo) A.plo[i] = lo;
             bad |= !isfinite(x.x) || !isfinite(x.y) || !isfinite(x.z);
         }
-        if (bad) atomicOr(&st->err, ERRBIT_NAN);
     }
+    if (bad) atomicOr(&st->err, ERRBIT_NAN);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         if (!DIV) {
             st->dt = dt;
@@ -862,14 +914,13 @@ __device__ __forceinline__ void scene_accumulate(double* accum, unsigned stride,
 }
 
 template <bool DIV>
-__global__ void __launch_bounds__(kSolverBlock, 8) k_dfsph_solve_batch(SimParams P, DeviceArrays A)
+__global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams P, DeviceArrays A)
 {
     DevState* st = A.st;
     SceneState* sst = A.sst;
     const SceneInfo* sc = A.sref.scenes;
     const unsigned* so = A.sref.scene_of;
     const int nfi = P.nf, ns = A.nscenes;
-    const size_t nf = (size_t)nfi;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int nthr = gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
@@ -907,23 +958,26 @@ __global__ void __launch_bounds__(kSolverBlock, 8) k_dfsph_solve_batch(SimParams
             v.x = __fadd_rn(v.x, __fmul_rn(__fadd_rn(a.x, P.gx), dt));
             v.y = __fadd_rn(v.y, __fmul_rn(__fadd_rn(a.y, P.gy), dt));
             v.z = __fadd_rn(v.z, __fmul_rn(__fadd_rn(a.z, P.gz), dt));
-            A.vel[i] = v;
-            A.acc[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 x = A.pos[i];
+            A.rec[2 * (size_t)i] = make_float4(x.x, x.y, x.z, 0.0f);
+            A.rec[2 * (size_t)i + 1] = v;
         }
         if (!grid_barrier(st)) return;
     }
     float* kws = DIV ? A.kvws : A.kws;
     for (int i = tid; i < nfi; i += nthr) {
         const float dt = sst[so[i]].dt_next;
-        /* the divergence error may come from the density pass (A.divres) */
-        const float r = (DIV && A.divres) ? A.divres[i] : dfsph_residual<DIV>(P, A, i, nf, dt);
-        if (DIV) kws[i] = r > 0.0f ? kws[i] / dt : 0.0f;
-        else kws[i] = r > P.rho0 ? kws[i] / (dt * dt) : 0.0f;
+        /* the divergence error comes from the density pass */
+        const float r = DIV ? A.divres[i] : dfsph_residual<DIV>(P, A, i, dt);
+        if (DIV) dfsph_set_k(A, i, r > 0.0f ? kws[i] / dt : 0.0f);
+        else dfsph_set_k(A, i, r > P.rho0 ? kws[i] / (dt * dt) : 0.0f);
     }
     if (!grid_barrier(st)) return;
-    for (int i = tid; i < nfi; i += nthr) dfsph_correct(P, A, kws, i, nf, sst[so[i]].dt_next);
+    for (int i = tid; i < nfi; i += nthr) {
+        dfsph_correct(P, A, i, sst[so[i]].dt_next);
+        kws[i] = 0.0f;
+    }
     if (!grid_barrier(st)) return;
-    for (int i = tid; i < nfi; i += nthr) kws[i] = 0.0f;
 
     /* activity for iteration it lives in bit (it & 1) of SceneState::active;
        the convergence test of iteration it keeps that bit (the correction
@@ -941,7 +995,7 @@ __global__ void __launch_bounds__(kSolverBlock, 8) k_dfsph_solve_batch(SimParams
             double err = 0.0;
             if (on) {
                 const float dt = sst[s].dt_next;
-                const float r = dfsph_residual<DIV>(P, A, i, nf, dt);
+                const float r = dfsph_residual<DIV>(P, A, i, dt);
                 float k;
                 if (DIV) {
                     k = r * A.alpha[i] / (dt * A.rho[i]);
@@ -950,10 +1004,10 @@ __global__ void __launch_bounds__(kSolverBlock, 8) k_dfsph_solve_batch(SimParams
                     k = __fdiv_rn(__fmul_rn(__fsub_rn(r, P.rho0), A.alpha[i]), __fmul_rn(dt * dt, A.rho[i]));
                     err = (double)((r - P.rho0) / P.rho0);
                 }
-                A.k[i] = k;
+                dfsph_set_k(A, i, k);
                 kws[i] += k;
             } else if (valid_i) {
-                A.k[i] = 0.0f;
+                dfsph_set_k(A, i, 0.0f);
             }
             scene_accumulate(A.accum, stride, it, s, on, err);
         }
@@ -978,22 +1032,20 @@ __global__ void __launch_bounds__(kSolverBlock, 8) k_dfsph_solve_batch(SimParams
         }
         for (int i = tid; i < nfi; i += nthr) {
             const unsigned s = so[i];
-            if (sst[s].active & bit) dfsph_correct(P, A, A.k, i, nf, sst[s].dt_next);
+            if (sst[s].active & bit) dfsph_correct(P, A, i, sst[s].dt_next);
         }
         if (!grid_barrier(st)) return;
         any = *(volatile unsigned*)&A.any_active[it + 1u] != 0u;
         ++it;
     }
 
+    bool bad = false;
     for (int i = tid; i < nfi; i += nthr) {
         const float dt = sst[so[i]].dt_next;
         kws[i] *= DIV ? dt : dt * dt;
-    }
-    if (!DIV) {
-        bool bad = false;
-        for (int i = tid; i < nfi; i += nthr) {
-            const float dt = sst[so[i]].dt_next;
-            const float4 v = A.vel[i];
+        const float4 v = A.rec[2 * (size_t)i + 1];
+        A.vel[i] = v;
+        if (!DIV) {
             float4 x = A.pos[i];
             x.x = __fadd_rn(x.x, __fmul_rn(v.x, dt));
             x.y = __fadd_rn(x.y, __fmul_rn(v.y, dt));
@@ -1001,8 +1053,8 @@ __global__ void __launch_bounds__(kSolverBlock, 8) k_dfsph_solve_batch(SimParams
             A.pos[i] = x;
             bad |= !isfinite(x.x) || !isfinite(x.y) || !isfinite(x.z);
         }
-        if (bad) atomicOr(&st->err, ERRBIT_NAN);
     }
+    if (bad) atomicOr(&st->err, ERRBIT_NAN);
     for (int s = tid; s < ns; s += nthr) {
         if (!DIV) {
             if (min_it == 0u || max_it == 0u) sst[s].its = 0u;
@@ -1027,7 +1079,6 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
     __shared__ double s_red[32];
     DevState* st = A.st;
     const int nfi = active_n(P, st);
-    const size_t nf = (size_t)P.nf;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int nthr = gridDim.x * blockDim.x;
     const float dt = st->dt;
@@ -1121,7 +1172,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
             float ax = 0.0f, ay = 0.0f, az = 0.0f;
             const unsigned nF = A.cnt_f[i], nB = A.cnt_b[i];
             for (unsigned kk = 0; kk < nF; ++kk) {
-                const unsigned j = list_at(A.nbr_f, kk, nf, i);
+                const unsigned j = list_at(A.nbr_f, kk, P.capF, i);
                 const float4 xj = A.pos[j];
                 const float rho_j = A.rho[j];
                 float gx, gy, gz;
@@ -1132,7 +1183,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
                 az = __fsub_rn(az, __fmul_rn(c, gz));
             }
             for (unsigned kk = 0; kk < nB; ++kk) {
-                const unsigned bq = list_at(A.nbr_b, kk, nf, i);
+                const unsigned bq = list_at(A.nbr_b, kk, P.capB, i);
                 const float4 xb = A.bpos[bq];
                 float gx, gy, gz, c;
                 if (P.pcib) {
@@ -1440,6 +1491,11 @@ void launch_density(const SimParams& P, const DeviceArrays& A, bool alpha, bool 
     }
     else if (eos) k_density<false, true><<<g, block, 0, s>>>(P, A);
     else k_density<false, false><<<g, block, 0, s>>>(P, A);
+}
+
+void launch_pair_factors(const SimParams& P, const DeviceArrays& A, cudaStream_t s)
+{
+    if (P.nf > 0) k_pair_factors<<<blocks_for(P.nf, 256), 256, 0, s>>>(P, A);
 }
 
 void launch_normals(const SimParams& P, const DeviceArrays& A, int block, cudaStream_t s)
