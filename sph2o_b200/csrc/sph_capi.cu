@@ -62,7 +62,8 @@ struct sph_ctx {
     float4 *pos = nullptr, *vel = nullptr, *pos2 = nullptr, *vel2 = nullptr;
     unsigned *orig = nullptr, *orig2 = nullptr;
     float *kws = nullptr, *kws2 = nullptr, *kvws = nullptr, *kvws2 = nullptr;
-    float4 *acc = nullptr, *normal = nullptr, *predr = nullptr, *pacc = nullptr;
+    float4 *acc = nullptr, *normal = nullptr, *predr = nullptr, *posd = nullptr;
+    float4* pgrad = nullptr; /* PCISPH: gradients of the list entries (DeviceArrays::pgrad) */
     float *rho = nullptr, *alpha = nullptr, *press = nullptr;
     unsigned *cell_of = nullptr, *slot = nullptr, *tmp_key = nullptr, *tmp_src = nullptr, *cell_sorted = nullptr;
     unsigned *cell_count = nullptr, *cell_start = nullptr, *bcell_start = nullptr, *block_sums = nullptr;
@@ -266,6 +267,8 @@ void derive_params(sph_ctx* c)
     P.kr_g = d.gamma != 0.0f ? d.stiffness * d.density0 / d.gamma : 0.0f;
     P.h2_guard = (float)((double)h * (double)h * (1.0 + 1.0e-5));
     P.h2_exact = sqrt_le_bound(h);
+    P.h_rh = 1.0f / h;
+    P.h_rl = (float)(1.0 / (double)h - (double)P.h_rh);
     P.eta = d.eta;
     P.eta_v = d.eta_v;
     P.cfl = d.cfl_factor;
@@ -349,7 +352,7 @@ DeviceArrays arrays(sph_ctx* c)
 {
     DeviceArrays A{};
     A.pos = c->pos; A.vel = c->vel; A.pos_alt = c->pos2; A.vel_alt = c->vel2;
-    A.acc = c->acc; A.normal = c->normal; A.predr = c->predr; A.pacc = c->pacc;
+    A.acc = c->acc; A.normal = c->normal; A.predr = c->predr; A.posd = c->posd; A.pgrad = c->pgrad;
     A.rho = c->rho; A.alpha = c->alpha; A.kws = c->kws; A.kvws = c->kvws; A.press = c->press;
     A.orig_w = c->orig;
     A.cell_start = c->cell_start; A.cell_sorted = c->cell_sorted;
@@ -438,6 +441,9 @@ int alloc_lists(sph_ctx* c)
         if ((rc = dalloc(c, &c->pair_f, list_len(c->nf, c->P.capF))) != SPH_OK) return rc;
         if ((rc = dalloc(c, &c->pair_b, list_len(c->nf, c->P.capB))) != SPH_OK) return rc;
     }
+    if (c->desc.simulation_method == SPH_PCISPH &&
+        (rc = dalloc(c, &c->pgrad, list_len(c->nf, c->P.capF))) != SPH_OK)
+        return rc;
     return SPH_OK;
 }
 
@@ -660,6 +666,7 @@ int recover_overflow(sph_ctx* c)
     drop(c->nbr_b);
     drop(c->pair_f);
     drop(c->pair_b);
+    drop(c->pgrad);
     c->P.capF = c->P.capF + c->P.capF / 2;
     c->P.capB = c->P.capB + c->P.capB / 2;
     c->lists_valid = false;
@@ -1061,7 +1068,7 @@ int sph_init(sph_ctx* c)
     ALLOC(orig, nf); ALLOC(orig2, nf);
     ALLOC(kws, nf); ALLOC(kws2, nf); ALLOC(kvws, nf); ALLOC(kvws2, nf);
     ALLOC(acc, nf); ALLOC(rho, nf); ALLOC(alpha, nf); ALLOC(press, nf);
-    ALLOC(normal, nf); ALLOC(predr, nf); ALLOC(pacc, nf);
+    ALLOC(normal, nf); ALLOC(predr, nf); ALLOC(posd, nf);
     ALLOC(cell_of, nmax); ALLOC(slot, nmax); ALLOC(tmp_key, nmax); ALLOC(tmp_src, nmax); ALLOC(cell_sorted, nmax);
     ALLOC(cell_count, (size_t)P.ncells); ALLOC(cell_start, (size_t)P.ncells + 1);
     ALLOC(bcell_start, (size_t)P.ncells + 1); ALLOC(block_sums, (size_t)P.ncells / 4096 + 1);
@@ -1128,6 +1135,13 @@ int sph_init(sph_ctx* c)
                 c->grid_solve[dv][o][t] = persistent_grid(false, dv == 1, false, o ? 4 : 8, 1 << t);
                 if (c->grid_solve[dv][o][t] <= 0) return fail(c, SPH_ERR_CUDA, "cannot size the persistent solver grid");
             }
+
+    /* the fast division by h, if it is exact for this h (block_sums is free) */
+    unsigned bad_div = 1;
+    launch_check_div_h(P, c->block_sums, c->stream);
+    CUDA_TRY(c, cudaMemcpyAsync(&bad_div, c->block_sums, sizeof bad_div, cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    P.h_div_exact = bad_div ? 0 : 1;
 
     /* upload: fluid in caller order becomes the first "unsorted" state */
     if ((rc = dalloc(c, &c->stage, 3 * nmax)) != SPH_OK) return rc;

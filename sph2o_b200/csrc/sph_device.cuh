@@ -46,6 +46,8 @@ struct SimParams {
     float kr_g;         /* (stiffness * rho0) / gamma, WCSPHSolver.cpp:93            */
     float h2_guard;     /* h^2 (1 + 1e-5): exact-W candidates above it are 0 anyway  */
     float h2_exact;     /* sqrt_le_bound(h): s <= h2_exact exactly when sqrt_rn(s) <= h */
+    float h_rh, h_rl;   /* 1 / h as an unevaluated sum of two floats (div_h)           */
+    int h_div_exact;    /* 1: div_h was checked to equal the division for this h       */
     float eta, eta_v, cfl, min_ts, max_ts;
     unsigned min_it, max_it, min_it_v, max_it_v;
     float pcisph_delta;
@@ -171,9 +173,21 @@ __device__ __forceinline__ float dist2_exact(float4 a, float4 b)
     return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
 }
 
+/* x / h, correctly rounded, by the two-operation division by a divisor known
+   in advance of Brisebarre, Muller and Raina ("Accelerating Correctly Rounded
+   Floating-Point Division When the Divisor Is Known in Advance", IEEE Trans.
+   Computers 53(8), 2004): x rh + x rl with rh + rl = 1 / h to twice float
+   precision, the second product fused. It is correct for most divisors; for
+   this one k_check_div_h compared it with __fdiv_rn over every mantissa of x
+   (the scale of x does not matter above 2^-90), else the division is used. */
+__device__ __forceinline__ float div_h(float x, const SimParams& P)
+{
+    return P.h_div_exact ? __fmaf_rn(x, P.h_rh, __fmul_rn(x, P.h_rl)) : __fdiv_rn(x, P.h);
+}
+
 __device__ __forceinline__ float cs_W_exact(float s, const SimParams& P)
 {
-    const float q = __fdiv_rn(__fsqrt_rn(s), P.h);
+    const float q = div_h(__fsqrt_rn(s), P);
     if (!(q <= 1.0f)) return 0.0f;
     if (q <= 0.5f) {
         const float q2 = __fmul_rn(q, q);
@@ -194,12 +208,12 @@ __device__ __forceinline__ void cs_gradW_exact(float rx, float ry, float rz, con
 {
     const float s = __fadd_rn(__fadd_rn(__fmul_rn(rx, rx), __fmul_rn(ry, ry)), __fmul_rn(rz, rz));
     const float rl = __fsqrt_rn(s);
-    const float q = __fdiv_rn(rl, P.h);
+    const float q = div_h(rl, P);
     gx = gy = gz = 0.0f;
     if (!((double)rl > 1.0e-9) || !(q <= 1.0f)) return;
-    const float qx = __fdiv_rn(__fdiv_rn(rx, rl), P.h);
-    const float qy = __fdiv_rn(__fdiv_rn(ry, rl), P.h);
-    const float qz = __fdiv_rn(__fdiv_rn(rz, rl), P.h);
+    const float qx = div_h(__fdiv_rn(rx, rl), P);
+    const float qy = div_h(__fdiv_rn(ry, rl), P);
+    const float qz = div_h(__fdiv_rn(rz, rl), P);
     float c;
     if (q <= 0.5f) {
         c = __fmul_rn(__fmul_rn(P.cs_l, q), __fsub_rn(__fmul_rn(3.0f, q), 2.0f));

@@ -456,6 +456,21 @@ void launch_build_lists(const SimParams& P, const SceneRef& S, const float4* pos
                                                                 cnt_f, nbr_b, cnt_b, st);
 }
 
+/* bad |= div_h(x) differs from x / h for a mantissa of x (sign and scale of x
+   do not matter: every operation scales exactly). */
+__global__ void __launch_bounds__(256) k_check_div_h(SimParams P, unsigned* bad)
+{
+    const unsigned m = blockIdx.x * blockDim.x + threadIdx.x;
+    P.h_div_exact = 1;
+    const float x = __uint_as_float(0x3f800000u | m);
+    if (div_h(x, P) != __fdiv_rn(x, P.h)) *bad = 1u;
+}
+
+void launch_check_div_h(const SimParams& P, unsigned* bad, cudaStream_t s)
+{
+    k_check_div_h<<<(1 << 23) / 256, 256, 0, s>>>(P, bad);
+}
+
 void launch_boundary_volume(const SimParams& P, const SceneRef& S, float4* bpos, const unsigned* bcell_start,
                             float* bvol, cudaStream_t s)
 {

@@ -25,7 +25,8 @@ struct DeviceArrays {
     float4* acc;
     float4* normal;
     float4* predr;        /* PCISPH predicted position */
-    float4* pacc;         /* PCISPH pressure acceleration */
+    float4* posd;         /* PCISPH: (x, y, z, p / rho^2 of the iteration) */
+    float4* pgrad;        /* PCISPH: (slot, gradW) of each fluid list entry, in the layout of nbr_f */
     float* rho;
     float* alpha;
     float* kws;
@@ -81,6 +82,8 @@ void launch_build_lists(const SimParams& P, const SceneRef& S, const float4* pos
                         unsigned* cnt_b, DevState* st, cudaStream_t s, bool staged = false);
 void launch_boundary_volume(const SimParams& P, const SceneRef& S, float4* bpos, const unsigned* bcell_start,
                             float* bvol, cudaStream_t s);
+/* *bad (zeroed by the caller) becomes 1 if div_h(x) != x / h for some x */
+void launch_check_div_h(const SimParams& P, unsigned* bad, cudaStream_t s);
 void launch_unsort_v4(int n, const unsigned* orig, const float4* in, float* out3, cudaStream_t s);
 void launch_unsort_f(int n, const unsigned* orig, const float* in, float* out, cudaStream_t s);
 void launch_sort_v3(int n, const unsigned* orig, const float* in3, float4* out, cudaStream_t s);

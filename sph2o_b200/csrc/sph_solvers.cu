@@ -1074,67 +1074,137 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams
 /* ---------------------------------------------------------------------- */
 /* PCISPH                                                                   */
 
+/* predictVelocityAndPosition of particle i for the pressure acceleration pa:
+   acc = (a + pacc) + g; predV = v + acc dt; predR = r + predV dt */
+__device__ __forceinline__ void pcisph_predict(const SimParams& P, const DeviceArrays& A, int i, float dt, float4 pa)
+{
+    const float4 a = A.acc[i], v = A.vel[i], x = A.pos[i];
+    const float vx = __fadd_rn(v.x, __fmul_rn(__fadd_rn(__fadd_rn(a.x, pa.x), P.gx), dt));
+    const float vy = __fadd_rn(v.y, __fmul_rn(__fadd_rn(__fadd_rn(a.y, pa.y), P.gy), dt));
+    const float vz = __fadd_rn(v.z, __fmul_rn(__fadd_rn(__fadd_rn(a.z, pa.z), P.gz), dt));
+    float4 pr = make_float4(__fadd_rn(x.x, __fmul_rn(vx, dt)), __fadd_rn(x.y, __fmul_rn(vy, dt)),
+                            __fadd_rn(x.z, __fmul_rn(vz, dt)), 0.0f);
+    if (P.pcib) {
+        /* PCISPHBoundaryObject::correctPredPositions (:390-438): tested at the
+           current position (whose cell holds lists), weighted at the
+           predicted one, which moves */
+        A.predv[i] = make_float4(vx, vy, vz, 0.0f);
+        float wsum, w2sum;
+        float3 avg;
+        pcib_collide(P, A, x, pr, wsum, w2sum, avg);
+        float4 n;
+        pr = pcib_push(pr, wsum, w2sum, avg, n);
+        A.normal[i] = n;
+    }
+    A.predr[i] = pr;
+}
+
+/* PCISPHSolver::integrate of particle i; true when the new position is not finite */
+__device__ __forceinline__ bool pcisph_integrate(const SimParams& P, const DeviceArrays& A, int i, float dt, float4 pa)
+{
+    const float4 a = A.acc[i];
+    float4 v = A.vel[i], x = A.pos[i];
+    /* a += g + pacc; v += a dt; x += v dt */
+    const float axx = __fadd_rn(a.x, __fadd_rn(P.gx, pa.x));
+    const float ayy = __fadd_rn(a.y, __fadd_rn(P.gy, pa.y));
+    const float azz = __fadd_rn(a.z, __fadd_rn(P.gz, pa.z));
+    v.x = __fadd_rn(v.x, __fmul_rn(axx, dt)); v.y = __fadd_rn(v.y, __fmul_rn(ayy, dt));
+    v.z = __fadd_rn(v.z, __fmul_rn(azz, dt));
+    float4 lo = P.pos_lo ? A.plo[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    x.x = pos_add(x.x, lo.x, __fmul_rn(v.x, dt), P.pos_lo);
+    x.y = pos_add(x.y, lo.y, __fmul_rn(v.y, dt), P.pos_lo);
+    x.z = pos_add(x.z, lo.z, __fmul_rn(v.z, dt), P.pos_lo);
+    if (P.pos_lo) A.plo[i] = lo;
+    if (P.pcib) {
+        /* correctPositions (PCISPH branch, :226-262): candidates of the new
+           cell if the last search listed it, weights at the predicted
+           position; then correctVelocities from the predicted velocity */
+        float wsum = 0.0f, w2sum = 0.0f;
+        float3 avg = make_float3(0.0f, 0.0f, 0.0f);
+        if (cell_listed(A.cell_entry, cell_index(x, P.h, grid_single(P)), A.st->ns_epoch))
+            pcib_collide(P, A, x, A.predr[i], wsum, w2sum, avg);
+        float4 n;
+        x = pcib_push(x, wsum, w2sum, avg, n);
+        A.normal[i] = n;
+        pcib_velocity(P, n, A.predv[i], v);
+    }
+    A.vel[i] = v;
+    A.pos[i] = x;
+    A.acc[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    return !isfinite(x.x) || !isfinite(x.y) || !isfinite(x.z);
+}
+
+/* Accepted candidates that a thread of k_pcisph_solve collects before it
+   evaluates their kernel terms. */
+constexpr int kPcisphBatch = 32;
+
+/* The loop of PCISPHSolver::step. Neighbours read posd (current position and
+   p / rho^2) and predr, never pos, so the pass that ends an iteration also
+   predicts the next one's positions, or integrates when it was the last. */
 __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, DeviceArrays A)
 {
     __shared__ double s_red[32];
+    __shared__ float s_s2[kPcisphBatch][kSolverBlock];
     DevState* st = A.st;
     const int nfi = active_n(P, st);
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int nthr = gridDim.x * blockDim.x;
     const float dt = st->dt;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 
-    /* PCISPHSolver::initPressure (boundary pressures too with PCISPH boundary particles) */
+    /* PCISPHSolver::initPressure (boundary pressures too with PCISPH boundary
+       particles) and the first prediction, without pressure. The first test uses
+       the residual left by the previous step (PCISPHSolver.cpp:374) */
+    unsigned it = 0;
+    double avg = st->pcisph_avg;
+    bool more = (avg > (double)P.eta || it < P.min_it) && it < P.max_it;
+    bool bad = false;
     for (int i = tid; i < nfi; i += nthr) {
         A.press[i] = 0.0f;
-        A.pacc[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (!more) {
+            bad |= pcisph_integrate(P, A, i, dt, zero);
+            continue;
+        }
+        const float4 x = A.pos[i];
+        A.posd[i] = make_float4(x.x, x.y, x.z, 0.0f);
+        pcisph_predict(P, A, i, dt, zero);
     }
     if (P.pcib)
         for (int q = tid; q < P.nb; q += nthr) A.bpress[q] = 0.0f;
-    unsigned it = 0;
-    /* the first test uses the residual left by the previous step (PCISPHSolver.cpp:374) */
-    double avg = st->pcisph_avg;
-    while ((avg > (double)P.eta || it < P.min_it) && it < P.max_it) {
-        /* predictVelocityAndPosition */
-        for (int i = tid; i < nfi; i += nthr) {
-            const float4 a = A.acc[i], pa = A.pacc[i], v = A.vel[i], x = A.pos[i];
-            /* acc = (a + pacc) + g; predV = v + acc dt; predR = r + predV dt */
-            const float vx = __fadd_rn(v.x, __fmul_rn(__fadd_rn(__fadd_rn(a.x, pa.x), P.gx), dt));
-            const float vy = __fadd_rn(v.y, __fmul_rn(__fadd_rn(__fadd_rn(a.y, pa.y), P.gy), dt));
-            const float vz = __fadd_rn(v.z, __fmul_rn(__fadd_rn(__fadd_rn(a.z, pa.z), P.gz), dt));
-            float4 pr = make_float4(__fadd_rn(x.x, __fmul_rn(vx, dt)), __fadd_rn(x.y, __fmul_rn(vy, dt)),
-                                    __fadd_rn(x.z, __fmul_rn(vz, dt)), 0.0f);
-            if (P.pcib) {
-                /* PCISPHBoundaryObject::correctPredPositions (:390-438): tested at the
-                   current position (whose cell holds lists), weighted at the
-                   predicted one, which moves */
-                A.predv[i] = make_float4(vx, vy, vz, 0.0f);
-                float wsum, w2sum;
-                float3 avg;
-                pcib_collide(P, A, x, pr, wsum, w2sum, avg);
-                float4 n;
-                pr = pcib_push(pr, wsum, w2sum, avg, n);
-                A.normal[i] = n;
-            }
-            A.predr[i] = pr;
-        }
-        if (!grid_barrier(st)) return;
+    if (more && !grid_barrier(st)) return;
+    while (more) {
         /* predictFluidDensities over the start-of-step candidates of the 27
            cells around the particle's current cell, then updatePressure */
         double local = 0.0;
         for (int i = tid; i < nfi; i += nthr) {
-            const float4 xi = A.pos[i];
+            const float4 xi = A.posd[i];
             const float4 pi = A.predr[i];
             /* all fluid candidates of the 27 cells first, then all boundary
-               candidates: the reference's summation order (PCISPHSolver.cpp:180-206) */
-            const Grid g = grid_for(P, A.sref, (unsigned)i);
+               candidates: the reference's summation order (PCISPHSolver.cpp:180-206).
+               About one candidate in seven is within h, but nearly always one of
+               some lane of the warp: the accepted ones are collected and their
+               kernel (a square root, FP64 products) evaluated afterwards, all
+               lanes together, in the same order. */
+            const Grid g = grid_single(P);
             float rho = 0.0f;
+            int n = 0;
+            const auto add_fluid = [&]() {
+#pragma unroll 1
+                for (int k = 0; k < n; ++k)
+                    rho = __fadd_rn(rho, __fmul_rn(P.mass, cs_W_exact(s_s2[k][threadIdx.x], P)));
+                n = 0;
+            };
             for_cells27(xi, P.h, g, [&](unsigned c) {
                 const unsigned e = A.cell_start[c + 1];
                 for (unsigned q = A.cell_start[c]; q < e; ++q) {
                     const float s2 = dist2_exact(pi, A.predr[q]);
-                    if (s2 <= P.h2_guard) rho = __fadd_rn(rho, __fmul_rn(P.mass, cs_W_exact(s2, P)));
+                    if (s2 <= P.h2_guard) {
+                        if (n == kPcisphBatch) add_fluid();
+                        s_s2[n++][threadIdx.x] = s2;
+                    }
                 }
             });
+            add_fluid();
             if (P.nb > 0)
                 for_cells27(xi, P.h, g, [&](unsigned c) {
                     const unsigned e = A.bcell_start[c + 1];
@@ -1146,7 +1216,9 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
                 });
             A.rho[i] = rho;
             const float err = fmaxf(0.0f, __fsub_rn(rho, P.rho0));
-            A.press[i] = __fadd_rn(A.press[i], __fmul_rn(P.pcisph_delta, err));
+            const float p = __fadd_rn(A.press[i], __fmul_rn(P.pcisph_delta, err));
+            A.press[i] = p;
+            reinterpret_cast<float*>(A.posd)[4 * (size_t)i + 3] = __fdiv_rn(p, __fmul_rn(rho, rho));
             local += (double)(err / P.rho0);
         }
         if (P.pcib)
@@ -1162,25 +1234,39 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
         if (threadIdx.x == 0) atomicAdd(&A.accum[it], bs);
         if (!grid_barrier(st)) return;
         avg = *(volatile double*)&A.accum[it] / (double)nfi;
+        more = (avg > (double)P.eta || it + 1u < P.min_it) && it + 1u < P.max_it;
         /* computePressureAcc at the current positions, with the reference's
            exact gradient arithmetic: the result feeds the next predicted
-           positions, whose densities enter the ill-conditioned p update */
+           positions, whose densities enter the ill-conditioned p update. The
+           gradients do not change within a step: the first iteration keeps
+           them beside their list entries for the later ones. */
         for (int i = tid; i < nfi; i += nthr) {
-            const float4 xi = A.pos[i];
-            const float rho_i = A.rho[i];
-            const float dpi = __fdiv_rn(A.press[i], __fmul_rn(rho_i, rho_i));
+            const float4 xi = A.posd[i];
+            const float dpi = xi.w;
             float ax = 0.0f, ay = 0.0f, az = 0.0f;
             const unsigned nF = A.cnt_f[i], nB = A.cnt_b[i];
-            for (unsigned kk = 0; kk < nF; ++kk) {
-                const unsigned j = list_at(A.nbr_f, kk, P.capF, i);
-                const float4 xj = A.pos[j];
-                const float rho_j = A.rho[j];
-                float gx, gy, gz;
-                cs_gradW_exact(__fsub_rn(xi.x, xj.x), __fsub_rn(xi.y, xj.y), __fsub_rn(xi.z, xj.z), P, gx, gy, gz);
-                const float c = __fmul_rn(P.mass, __fadd_rn(dpi, __fdiv_rn(A.press[j], __fmul_rn(rho_j, rho_j))));
-                ax = __fsub_rn(ax, __fmul_rn(c, gx));
-                ay = __fsub_rn(ay, __fmul_rn(c, gy));
-                az = __fsub_rn(az, __fmul_rn(c, gz));
+            if (it == 0) {
+                for (unsigned kk = 0; kk < nF; ++kk) {
+                    const unsigned j = list_at(A.nbr_f, kk, P.capF, i);
+                    const float4 xj = A.posd[j];
+                    float gx, gy, gz;
+                    cs_gradW_exact(__fsub_rn(xi.x, xj.x), __fsub_rn(xi.y, xj.y), __fsub_rn(xi.z, xj.z), P, gx, gy, gz);
+                    if (more) __stcs(A.pgrad + list_index(kk, P.capF, i), make_float4(__uint_as_float(j), gx, gy, gz));
+                    const float c = __fmul_rn(P.mass, __fadd_rn(dpi, xj.w));
+                    ax = __fsub_rn(ax, __fmul_rn(c, gx));
+                    ay = __fsub_rn(ay, __fmul_rn(c, gy));
+                    az = __fsub_rn(az, __fmul_rn(c, gz));
+                }
+            } else {
+                const float* dp = reinterpret_cast<const float*>(A.posd) + 3;
+#pragma unroll 4
+                for (unsigned kk = 0; kk < nF; ++kk) {
+                    const float4 g = __ldcs(A.pgrad + list_index(kk, P.capF, i));
+                    const float c = __fmul_rn(P.mass, __fadd_rn(dpi, dp[4 * (size_t)__float_as_uint(g.x)]));
+                    ax = __fsub_rn(ax, __fmul_rn(c, g.y));
+                    ay = __fsub_rn(ay, __fmul_rn(c, g.z));
+                    az = __fsub_rn(az, __fmul_rn(c, g.w));
+                }
             }
             for (unsigned kk = 0; kk < nB; ++kk) {
                 const unsigned bq = list_at(A.nbr_b, kk, P.capB, i);
@@ -1199,44 +1285,12 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
                 ay = __fsub_rn(ay, __fmul_rn(c, gy));
                 az = __fsub_rn(az, __fmul_rn(c, gz));
             }
-            A.pacc[i] = make_float4(ax, ay, az, 0.0f);
+            const float4 pa = make_float4(ax, ay, az, 0.0f);
+            if (more) pcisph_predict(P, A, i, dt, pa);
+            else bad |= pcisph_integrate(P, A, i, dt, pa);
         }
         ++it;
-    }
-    if (!grid_barrier(st)) return;
-    /* PCISPHSolver::integrate */
-    bool bad = false;
-    for (int i = tid; i < nfi; i += nthr) {
-        const float4 a = A.acc[i], pa = A.pacc[i];
-        float4 v = A.vel[i], x = A.pos[i];
-        /* a += g + pacc; v += a dt; x += v dt */
-        const float axx = __fadd_rn(a.x, __fadd_rn(P.gx, pa.x));
-        const float ayy = __fadd_rn(a.y, __fadd_rn(P.gy, pa.y));
-        const float azz = __fadd_rn(a.z, __fadd_rn(P.gz, pa.z));
-        v.x = __fadd_rn(v.x, __fmul_rn(axx, dt)); v.y = __fadd_rn(v.y, __fmul_rn(ayy, dt));
-        v.z = __fadd_rn(v.z, __fmul_rn(azz, dt));
-        float4 lo = P.pos_lo ? A.plo[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        x.x = pos_add(x.x, lo.x, __fmul_rn(v.x, dt), P.pos_lo);
-        x.y = pos_add(x.y, lo.y, __fmul_rn(v.y, dt), P.pos_lo);
-        x.z = pos_add(x.z, lo.z, __fmul_rn(v.z, dt), P.pos_lo);
-        if (P.pos_lo) A.plo[i] = lo;
-        if (P.pcib) {
-            /* correctPositions (PCISPH branch, :226-262): candidates of the new
-               cell if the last search listed it, weights at the predicted
-               position; then correctVelocities from the predicted velocity */
-            float wsum = 0.0f, w2sum = 0.0f;
-            float3 avg = make_float3(0.0f, 0.0f, 0.0f);
-            if (cell_listed(A.cell_entry, cell_index(x, P.h, grid_single(P)), st->ns_epoch))
-                pcib_collide(P, A, x, A.predr[i], wsum, w2sum, avg);
-            float4 n;
-            x = pcib_push(x, wsum, w2sum, avg, n);
-            A.normal[i] = n;
-            pcib_velocity(P, n, A.predv[i], v);
-        }
-        A.vel[i] = v;
-        A.pos[i] = x;
-        A.acc[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        bad |= !isfinite(x.x) || !isfinite(x.y) || !isfinite(x.z);
+        if (more && !grid_barrier(st)) return;
     }
     if (bad) atomicOr(&st->err, ERRBIT_NAN);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
