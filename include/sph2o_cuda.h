@@ -218,7 +218,7 @@ int sph_profile_read(sph_ctx* ctx, double* ms, unsigned long long* launches);
 enum sph_option {
     SPH_OPT_CUDA_GRAPHS = 0,      /* 1 (default): steps replay captured CUDA graphs of two steps (one
                                      for an odd remainder), keyed by the buffer assignment */
-    SPH_OPT_CELL_ORDER = 1,       /* 0 (default): 4x4x4 cell bricks, Morton inside; 1: linear, x fastest */
+    SPH_OPT_CELL_ORDER = 1,       /* 0 (default): 4x4x4 cell bricks, z fastest inside; 1: linear, x fastest */
     SPH_OPT_SOLVER_OCCUPANCY = 2, /* DFSPH persistent solver blocks per SM: 8 or 4; until set it reads 8 and
                                      the library chooses */
     SPH_OPT_PASS_BLOCK = 3,       /* threads per block of the particle-pass kernels: 256 (default) or 128 */

@@ -67,6 +67,7 @@ struct sph_ctx {
     float *rho = nullptr, *alpha = nullptr, *press = nullptr;
     unsigned *cell_of = nullptr, *slot = nullptr, *tmp_key = nullptr, *tmp_src = nullptr, *cell_sorted = nullptr;
     unsigned *cell_count = nullptr, *cell_start = nullptr, *bcell_start = nullptr, *block_sums = nullptr;
+    unsigned char* near = nullptr; /* per cell: boundary particles around it (k_mark_near) */
     float4* bpos = nullptr;
     float* bvol = nullptr;
     unsigned* borig = nullptr;
@@ -253,6 +254,7 @@ void derive_params(sph_ctx* c)
     P.mass = d.density0 * volume;
     const float h3 = h * h * h;
     P.cs_k = 8.0f / (pi * h3);
+    P.cs_k2 = 2.0 * (double)P.cs_k;
     P.cs_l = 48.0f / (pi * h3);
     P.cs_l_h2 = P.cs_l / (h * h);
     P.cs_l_h = P.cs_l / h;
@@ -356,7 +358,7 @@ DeviceArrays arrays(sph_ctx* c)
     A.rho = c->rho; A.alpha = c->alpha; A.kws = c->kws; A.kvws = c->kvws; A.press = c->press;
     A.orig_w = c->orig;
     A.cell_start = c->cell_start; A.cell_sorted = c->cell_sorted;
-    A.bpos = c->bpos; A.bcell_start = c->bcell_start;
+    A.bpos = c->bpos; A.bcell_start = c->bcell_start; A.near = c->near;
     A.nbr_f = c->nbr_f; A.cnt_f = c->cnt_f; A.nbr_b = c->nbr_b; A.cnt_b = c->cnt_b;
     A.pair_f = c->pair_f; A.pair_b = c->pair_b;
     A.accum = c->accum; A.st = c->st;
@@ -480,7 +482,7 @@ int neighbor_search(sph_ctx* c)
     }
     {
         Phase ph(c, SPH_PROF_LISTS, 1);
-        launch_build_lists(c->P, SceneRef{c->d_scenes, c->d_scene_of}, c->pos, c->cell_start, c->bpos, c->bcell_start, c->nbr_f, c->cnt_f, c->nbr_b,
+        launch_build_lists(c->P, SceneRef{c->d_scenes, c->d_scene_of}, c->pos, c->cell_start, c->bpos, c->bcell_start, c->near, c->nbr_f, c->cnt_f, c->nbr_b,
                            c->cnt_b, c->st, c->stream, c->staged_lists);
     }
     if (c->P.pcib) {
@@ -615,7 +617,7 @@ int step_dfsph(sph_ctx* c)
            insertion, and evaluate distances at current positions: rebuild
            the lists from the current positions against the same cell table. */
         Phase ph(c, SPH_PROF_LISTS, 2);
-        launch_build_lists(c->P, SceneRef{c->d_scenes, c->d_scene_of}, c->pos, c->cell_start, c->bpos, c->bcell_start,
+        launch_build_lists(c->P, SceneRef{c->d_scenes, c->d_scene_of}, c->pos, c->cell_start, c->bpos, c->bcell_start, c->near,
                            c->nbr_f, c->cnt_f, c->nbr_b, c->cnt_b, c->st, c->stream);
         launch_pair_factors(c->P, arrays(c), c->stream);
     }
@@ -1072,6 +1074,7 @@ int sph_init(sph_ctx* c)
     ALLOC(cell_of, nmax); ALLOC(slot, nmax); ALLOC(tmp_key, nmax); ALLOC(tmp_src, nmax); ALLOC(cell_sorted, nmax);
     ALLOC(cell_count, (size_t)P.ncells); ALLOC(cell_start, (size_t)P.ncells + 1);
     ALLOC(bcell_start, (size_t)P.ncells + 1); ALLOC(block_sums, (size_t)P.ncells / 4096 + 1);
+    ALLOC(near, (size_t)P.ncells);
     ALLOC(bpos, nb); ALLOC(bvol, nb); ALLOC(borig, nb);
     ALLOC(cnt_f, nf); ALLOC(cnt_b, nf);
     ALLOC(st, 1);
@@ -1182,6 +1185,7 @@ int sph_init(sph_ctx* c)
         launch_sort(P, bref, (int)nb, braw, c->cell_count, c->bcell_start, c->block_sums, c->cell_of, c->slot,
                     c->tmp_key, c->tmp_src, bid, g, c->stream);
         if (!P.pcib) launch_boundary_volume(P, bref, c->bpos, c->bcell_start, c->bvol, c->stream);
+        launch_mark_near(P, bref, c->bpos, c->near, c->stream);
     } else {
         CUDA_TRY(c, cudaMemsetAsync(c->bcell_start, 0, ((size_t)P.ncells + 1) * sizeof(unsigned), c->stream));
     }
@@ -1530,6 +1534,8 @@ int resort_boundary(sph_ctx* c)
     launch_sort(c->P, bref, (int)c->nb, c->braw, c->cell_count, c->bcell_start, c->block_sums, c->cell_of, c->slot,
                 c->tmp_key, c->tmp_src, c->bid, g, c->stream);
     launch_boundary_volume(c->P, bref, c->bpos, c->bcell_start, c->bvol, c->stream);
+    CUDA_TRY(c, cudaMemsetAsync(c->near, 0, c->P.ncells, c->stream));
+    launch_mark_near(c->P, bref, c->bpos, c->near, c->stream);
     return check_launch(c, "boundary re-sort");
 }
 

@@ -4,7 +4,7 @@
  * SPHSolver::insertFluidParticles / neighborhoodSearch, src/SPH2O/SPHSolver/SPHSolver.cpp:170-219).
  *
  * Per step:
- *   1. ns_count        cell key floor(x / h) -> brick-Morton cell index,
+ *   1. ns_count        cell key floor(x / h) -> cell index in brick order,
  *                      per-cell population by atomicAdd (slot = old count)
  *   2. scan_local/add  exclusive scan of the populations -> cellStart[ncells+1]
  *                      (the scan zeroes the populations for the next step)
@@ -140,6 +140,7 @@ __device__ __forceinline__ void build_lists_at(const SimParams& P, const SceneRe
                                                const unsigned* __restrict__ cell_start,
                                                const float4* __restrict__ bpos,
                                                const unsigned* __restrict__ bcell_start,
+                                               const unsigned char* __restrict__ near,
                                                unsigned* __restrict__ nbr_f, unsigned* __restrict__ cnt_f,
                                                unsigned* __restrict__ nbr_b, unsigned* __restrict__ cnt_b,
                                                DevState* st)
@@ -148,24 +149,25 @@ __device__ __forceinline__ void build_lists_at(const SimParams& P, const SceneRe
     /* |r| <= h as the reference rounds it, without the square root */
     const float s2max = P.h2_exact;
     unsigned nF = 0, nB = 0;
-    for_cells27(xi, P.h, grid_for(P, S, (unsigned)i), [&](unsigned c) {
-        const unsigned s = cell_start[c], e = cell_start[c + 1];
-        for (unsigned q = s; q < e; ++q) {
-            if (dist2_exact(xi, pos[q]) <= s2max) {
-                if (nF < P.capF) __stcs(nbr_f + list_index(nF, P.capF, i), q);
-                ++nF;
-            }
-        }
-        if (P.nb > 0) {
-            const unsigned bs = bcell_start[c], be = bcell_start[c + 1];
-            for (unsigned q = bs; q < be; ++q) {
-                if (dist2_exact(xi, bpos[q]) <= s2max) {
-                    if (nB < P.capB) __stcs(nbr_b + list_index(nB, P.capB, i), q);
-                    ++nB;
+    const Grid g = grid_for(P, S, (unsigned)i);
+    const auto list = [&](const unsigned* starts, const float4* xs, unsigned* out, unsigned cap, unsigned& n) {
+        unsigned m = 0; /* accepted candidates of the stretch */
+        for_stretches27(
+            xi, xi, P.h, g, starts, xs,
+            [&](unsigned k, const float (&d)[4], unsigned) {
+                const unsigned t = (d[0] <= s2max ? 1u : 0u) | (d[1] <= s2max ? 2u : 0u) | (d[2] <= s2max ? 4u : 0u) |
+                                   (d[3] <= s2max ? 8u : 0u);
+                m |= t << k;
+            },
+            [&](auto slot) {
+                for (; m; m &= m - 1u) {
+                    if (n < cap) __stcs(out + n * 32u, slot((unsigned)__ffs((int)m) - 1u));
+                    ++n;
                 }
-            }
-        }
-    });
+            });
+    };
+    list(cell_start, pos, nbr_f + list_index(0, P.capF, i), P.capF, nF);
+    if (boundary_near(P, near, xi, g)) list(bcell_start, bpos, nbr_b + list_index(0, P.capB, i), P.capB, nB);
     cnt_f[i] = min(nF, P.capF);
     cnt_b[i] = min(nB, P.capB);
     if (nF > P.capF || nB > P.capB) {
@@ -178,13 +180,14 @@ __global__ void __launch_bounds__(128) k_ns_build_lists(SimParams P, SceneRef S,
                                                         const unsigned* __restrict__ cell_start,
                                                         const float4* __restrict__ bpos,
                                                         const unsigned* __restrict__ bcell_start,
+                                                        const unsigned char* __restrict__ near,
                                                         unsigned* __restrict__ nbr_f, unsigned* __restrict__ cnt_f,
                                                         unsigned* __restrict__ nbr_b, unsigned* __restrict__ cnt_b,
                                                         DevState* st)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= active_n(P, st)) return;
-    build_lists_at(P, S, i, pos, cell_start, bpos, bcell_start, nbr_f, cnt_f, nbr_b, cnt_b, st);
+    build_lists_at(P, S, i, pos, cell_start, bpos, bcell_start, near, nbr_f, cnt_f, nbr_b, cnt_b, st);
 }
 
 /* ---------------------------------------------------------------------- */
@@ -195,11 +198,12 @@ __device__ __noinline__ void build_lists_global(const SimParams& P, int i, const
                                                 const unsigned* __restrict__ cell_start,
                                                 const float4* __restrict__ bpos,
                                                 const unsigned* __restrict__ bcell_start,
+                                                const unsigned char* __restrict__ near,
                                                 unsigned* __restrict__ nbr_f, unsigned* __restrict__ cnt_f,
                                                 unsigned* __restrict__ nbr_b, unsigned* __restrict__ cnt_b,
                                                 DevState* st)
 {
-    build_lists_at(P, SceneRef{}, i, pos, cell_start, bpos, bcell_start, nbr_f, cnt_f, nbr_b, cnt_b, st);
+    build_lists_at(P, SceneRef{}, i, pos, cell_start, bpos, bcell_start, near, nbr_f, cnt_f, nbr_b, cnt_b, st);
 }
 
 /* Fluid particles of one brick's 6 x 6 x 6-cell halo that fit in shared
@@ -217,8 +221,8 @@ constexpr int kStagedBlock = 256;
    ids written, so the lists equal k_ns_build_lists's entry for entry. */
 __global__ void __launch_bounds__(kStagedBlock) k_ns_build_lists_staged(
     SimParams P, const float4* __restrict__ pos, const unsigned* __restrict__ cell_start,
-    const float4* __restrict__ bpos, const unsigned* __restrict__ bcell_start, unsigned* __restrict__ nbr_f,
-    unsigned* __restrict__ cnt_f, unsigned* __restrict__ nbr_b, unsigned* __restrict__ cnt_b, DevState* st)
+    const float4* __restrict__ bpos, const unsigned* __restrict__ bcell_start, const unsigned char* __restrict__ near,
+    unsigned* __restrict__ nbr_f, unsigned* __restrict__ cnt_f, unsigned* __restrict__ nbr_b, unsigned* __restrict__ cnt_b, DevState* st)
 {
     __shared__ float4 s_pos[kHaloCap];
     __shared__ unsigned s_off[217]; /* staged offset of each halo cell; [216] = total */
@@ -236,7 +240,7 @@ __global__ void __launch_bounds__(kStagedBlock) k_ns_build_lists_staged(
         const int cx = 4 * bx - 1 + h % 6, cy = 4 * by - 1 + (h / 6) % 6, cz = 4 * bz - 1 + h / 36;
         unsigned s = 0, e = 0, bs = 0, be = 0;
         if (cx >= 0 && cx < g.dimx && cy >= 0 && cy < g.dimy && cz >= 0 && cz < g.dimz) {
-            const unsigned c = brick_morton(cx, cy, cz, g);
+            const unsigned c = cell_at(cx, cy, cz, g);
             s = cell_start[c];
             e = cell_start[c + 1];
             if (P.nb > 0) {
@@ -291,7 +295,7 @@ __global__ void __launch_bounds__(kStagedBlock) k_ns_build_lists_staged(
         if ((unsigned)lx > 3u || (unsigned)ly > 3u || (unsigned)lz > 3u) {
             /* moved out of its sort cell's brick since the sort: walk the
                cells around its position in global memory */
-            build_lists_global(P, (int)i, pos, cell_start, bpos, bcell_start, nbr_f, cnt_f, nbr_b, cnt_b, st);
+            build_lists_global(P, (int)i, pos, cell_start, bpos, bcell_start, near, nbr_f, cnt_f, nbr_b, cnt_b, st);
             continue;
         }
         unsigned nF = 0, nB = 0;
@@ -330,6 +334,7 @@ __global__ void __launch_bounds__(128) k_ns_build_lists_warp(SimParams P, SceneR
                                                              const unsigned* __restrict__ cell_start,
                                                              const float4* __restrict__ bpos,
                                                              const unsigned* __restrict__ bcell_start,
+                                                             const unsigned char* __restrict__ near,
                                                              unsigned* __restrict__ nbr_f, unsigned* __restrict__ cnt_f,
                                                              unsigned* __restrict__ nbr_b, unsigned* __restrict__ cnt_b,
                                                              DevState* st)
@@ -337,7 +342,7 @@ __global__ void __launch_bounds__(128) k_ns_build_lists_warp(SimParams P, SceneR
     const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     /* the whole warp shares i and leaves together */
     if (i >= active_n(P, st)) return;
-    build_lists_warp_at(P, S, i, pos, cell_start, bpos, bcell_start, nbr_f, cnt_f, nbr_b, cnt_b, st);
+    build_lists_warp_at(P, S, i, pos, cell_start, bpos, bcell_start, near, nbr_f, cnt_f, nbr_b, cnt_b, st);
 }
 
 /* Akinci boundary volume V_b = 1 / sum_b' W(x_b - x_b') over the 27 cells
@@ -351,11 +356,9 @@ __global__ void __launch_bounds__(128) k_boundary_volume(SimParams P, SceneRef S
     if (b >= P.nb) return;
     const float4 xb = bpos[b];
     float delta = 0.0f;
-    for_cells27(xb, P.h, grid_for(P, S, (unsigned)b), [&](unsigned c) {
-        for (unsigned q = bcell_start[c]; q < bcell_start[c + 1]; ++q) {
-            const float s2 = dist2_exact(xb, bpos[q]);
-            if (s2 <= P.h2_guard) delta = __fadd_rn(delta, cs_W_exact(s2, P));
-        }
+    for_candidates27(xb, P.h, grid_for(P, S, (unsigned)b), bcell_start, [&](unsigned q) {
+        const float s2 = dist2_exact(xb, bpos[q]);
+        if (s2 <= P.h2_guard) delta = __fadd_rn(delta, cs_W_exact(s2, P));
     });
     bvol[b] = __fdiv_rn(1.0f, delta);
 }
@@ -433,14 +436,14 @@ void launch_sort(const SimParams& P, const SceneRef& S, int n, const float4* pos
 
 void launch_build_lists(const SimParams& P, const SceneRef& S, const float4* pos, const unsigned* cell_start,
                         const float4* bpos,
-                        const unsigned* bcell_start, unsigned* nbr_f, unsigned* cnt_f, unsigned* nbr_b,
+                        const unsigned* bcell_start, const unsigned char* near, unsigned* nbr_f, unsigned* cnt_f, unsigned* nbr_b,
                         unsigned* cnt_b, DevState* st, cudaStream_t s, bool staged)
 {
     if (P.nf <= 0) return;
     if (staged && !S.scenes && P.cell_order == 0 && P.nf >= (1 << 16)) {
         /* one block per brick; bricks without fluid leave at once */
         const int nbricks = P.nbx * P.nby * (P.dimz / 4);
-        k_ns_build_lists_staged<<<nbricks, kStagedBlock, 0, s>>>(P, pos, cell_start, bpos, bcell_start, nbr_f, cnt_f,
+        k_ns_build_lists_staged<<<nbricks, kStagedBlock, 0, s>>>(P, pos, cell_start, bpos, bcell_start, near, nbr_f, cnt_f,
                                                                   nbr_b, cnt_b, st);
         return;
     }
@@ -450,10 +453,34 @@ void launch_build_lists(const SimParams& P, const SceneRef& S, const float4* pos
        warp's extra instructions cost more (125k: 0.069 vs 0.096 ms). */
     if (P.nf < (1 << 16))
         k_ns_build_lists_warp<<<blocks_for((long long)P.nf * 32, 128), 128, 0, s>>>(
-            P, S, pos, cell_start, bpos, bcell_start, nbr_f, cnt_f, nbr_b, cnt_b, st);
+            P, S, pos, cell_start, bpos, bcell_start, near, nbr_f, cnt_f, nbr_b, cnt_b, st);
     else
-        k_ns_build_lists<<<blocks_for(P.nf, 128), 128, 0, s>>>(P, S, pos, cell_start, bpos, bcell_start, nbr_f,
+        k_ns_build_lists<<<blocks_for(P.nf, 128), 128, 0, s>>>(P, S, pos, cell_start, bpos, bcell_start, near, nbr_f,
                                                                 cnt_f, nbr_b, cnt_b, st);
+}
+
+/* near[c] = 1 for every cell c with a boundary particle in the 27 cells
+   around it (near is zeroed by the caller): fluid particles of the other cells
+   skip the boundary candidates. The boundary does not move, so this is done
+   once per cell order. */
+__global__ void __launch_bounds__(256) k_mark_near(SimParams P, SceneRef S, const float4* __restrict__ bpos,
+                                                   unsigned char* __restrict__ near)
+{
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= P.nb) return;
+    const Grid g = grid_for(P, S, (unsigned)b);
+    const float4 x = bpos[b];
+    const int cx = cell_coord(x.x, P.h, g.cminx, g.dimx);
+    const int cy = cell_coord(x.y, P.h, g.cminy, g.dimy);
+    const int cz = cell_coord(x.z, P.h, g.cminz, g.dimz);
+    for (int xx = max(cx - 1, 0); xx <= min(cx + 1, g.dimx - 1); ++xx)
+        for (int yy = max(cy - 1, 0); yy <= min(cy + 1, g.dimy - 1); ++yy)
+            for (int zz = max(cz - 1, 0); zz <= min(cz + 1, g.dimz - 1); ++zz) near[cell_at(xx, yy, zz, g)] = 1;
+}
+
+void launch_mark_near(const SimParams& P, const SceneRef& S, const float4* bpos, unsigned char* near, cudaStream_t s)
+{
+    if (P.nb > 0) k_mark_near<<<blocks_for(P.nb, 256), 256, 0, s>>>(P, S, bpos, near);
 }
 
 /* bad |= div_h(x) differs from x / h for a mantissa of x (sign and scale of x

@@ -111,6 +111,14 @@ __device__ __forceinline__ void warp_candidates(const float4* __restrict__ xs, u
     }
 }
 
+/* Whether x's cell has boundary particles among its 27 cells (near: see
+   k_mark_near). */
+__device__ __forceinline__ bool boundary_near(const SimParams& P, const unsigned char* __restrict__ near, float4 x,
+                                              const Grid& g)
+{
+    return P.nb > 0 && near[cell_index(x, P.h, g)] != 0;
+}
+
 /* The lists of particle i, built by the whole warp (every lane calls with
    the same i). */
 __device__ __forceinline__ void build_lists_warp_at(const SimParams& P, const SceneRef& S, int i,
@@ -118,6 +126,7 @@ __device__ __forceinline__ void build_lists_warp_at(const SimParams& P, const Sc
                                                     const unsigned* __restrict__ cell_start,
                                                     const float4* __restrict__ bpos,
                                                     const unsigned* __restrict__ bcell_start,
+                                                    const unsigned char* __restrict__ near,
                                                     unsigned* __restrict__ nbr_f, unsigned* __restrict__ cnt_f,
                                                     unsigned* __restrict__ nbr_b, unsigned* __restrict__ cnt_b,
                                                     DevState* st)
@@ -126,15 +135,16 @@ __device__ __forceinline__ void build_lists_warp_at(const SimParams& P, const Sc
     const float4 xi = pos[i];
     const Grid g = grid_for(P, S, (unsigned)i);
     unsigned s = 0, e = 0, bs = 0, be = 0;
+    const bool with_boundary = boundary_near(P, near, xi, g);
     if (lane < 27) {
         const int xx = cell_coord(xi.x, P.h, g.cminx, g.dimx) + (int)lane / 9 - 1;
         const int yy = cell_coord(xi.y, P.h, g.cminy, g.dimy) + ((int)lane / 3) % 3 - 1;
         const int zz = cell_coord(xi.z, P.h, g.cminz, g.dimz) + (int)lane % 3 - 1;
         if (xx >= 0 && xx < g.dimx && yy >= 0 && yy < g.dimy && zz >= 0 && zz < g.dimz) {
-            const unsigned c = brick_morton(xx, yy, zz, g);
+            const unsigned c = cell_at(xx, yy, zz, g);
             s = cell_start[c];
             e = cell_start[c + 1];
-            if (P.nb > 0) {
+            if (with_boundary) {
                 bs = bcell_start[c];
                 be = bcell_start[c + 1];
             }
@@ -142,7 +152,7 @@ __device__ __forceinline__ void build_lists_warp_at(const SimParams& P, const Sc
     }
     unsigned nF = 0, nB = 0;
     warp_candidates(pos, s, e, xi, P.h2_exact, lane, P.capF, nbr_f, i, nF);
-    if (P.nb > 0) warp_candidates(bpos, bs, be, xi, P.h2_exact, lane, P.capB, nbr_b, i, nB);
+    if (with_boundary) warp_candidates(bpos, bs, be, xi, P.h2_exact, lane, P.capB, nbr_b, i, nB);
     if (lane != 0) return;
     cnt_f[i] = min(nF, P.capF);
     cnt_b[i] = min(nB, P.capB);

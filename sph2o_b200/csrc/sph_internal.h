@@ -36,6 +36,7 @@ struct DeviceArrays {
     const unsigned* cell_sorted;   /* cell index of each sorted slot */
     const float4* bpos;
     const unsigned* bcell_start;
+    const unsigned char* near;     /* per cell: boundary particles among its 27 cells */
     const unsigned* nbr_f;
     const unsigned* cnt_f;
     const unsigned* nbr_b;
@@ -78,10 +79,12 @@ void launch_sort(const SimParams& P, const SceneRef& S, int n, const float4* pos
                  const unsigned* orig_in, const GatherSet& g, cudaStream_t s);
 void launch_build_lists(const SimParams& P, const SceneRef& S, const float4* pos, const unsigned* cell_start,
                         const float4* bpos,
-                        const unsigned* bcell_start, unsigned* nbr_f, unsigned* cnt_f, unsigned* nbr_b,
+                        const unsigned* bcell_start, const unsigned char* near, unsigned* nbr_f, unsigned* cnt_f, unsigned* nbr_b,
                         unsigned* cnt_b, DevState* st, cudaStream_t s, bool staged = false);
 void launch_boundary_volume(const SimParams& P, const SceneRef& S, float4* bpos, const unsigned* bcell_start,
                             float* bvol, cudaStream_t s);
+/* cells with boundary particles around them (near: ncells bytes, zeroed by the caller) */
+void launch_mark_near(const SimParams& P, const SceneRef& S, const float4* bpos, unsigned char* near, cudaStream_t s);
 /* *bad (zeroed by the caller) becomes 1 if div_h(x) != x / h for some x */
 void launch_check_div_h(const SimParams& P, unsigned* bad, cudaStream_t s);
 void launch_unsort_v4(int n, const unsigned* orig, const float4* in, float* out3, cudaStream_t s);

@@ -152,19 +152,15 @@ __global__ void __launch_bounds__(128) k_na_density(SimParams P, const float4* _
     const float4 xi = pos[i];
     const Grid g = grid_single(P);
     float rho = 0.0f;
-    for_cells27(xi, P.h, g, [&](unsigned c) {
-        for (unsigned q = cell_start[c]; q < cell_start[c + 1]; ++q) {
-            const float s2 = dist2_exact(xi, pos[q]);
-            if (s2 <= P.h2_guard) rho = __fadd_rn(rho, __fmul_rn(P.mass, cs_W_exact(s2, P)));
-        }
+    for_candidates27(xi, P.h, g, cell_start, [&](unsigned q) {
+        const float s2 = dist2_exact(xi, pos[q]);
+        if (s2 <= P.h2_guard) rho = __fadd_rn(rho, __fmul_rn(P.mass, cs_W_exact(s2, P)));
     });
     if (P.nb > 0)
-        for_cells27(xi, P.h, g, [&](unsigned c) {
-            for (unsigned q = bcell_start[c]; q < bcell_start[c + 1]; ++q) {
-                const float4 xb = bpos[q];
-                const float s2 = dist2_exact(xi, xb);
-                if (s2 <= P.h2_guard) rho = __fadd_rn(rho, __fmul_rn(xb.w, cs_W_exact(s2, P)));
-            }
+        for_candidates27(xi, P.h, g, bcell_start, [&](unsigned q) {
+            const float4 xb = bpos[q];
+            const float s2 = dist2_exact(xi, xb);
+            if (s2 <= P.h2_guard) rho = __fadd_rn(rho, __fmul_rn(xb.w, cs_W_exact(s2, P)));
         });
     rho_out[orig[i]] = rho;
 }
@@ -211,6 +207,7 @@ extern "C" int sph_density_noalloc(float particle_radius, float density0, const 
     P.mass = density0 * (float)std::pow((double)diameter, 3.0);
     const float h3 = P.h * P.h * P.h;
     P.cs_k = 8.0f / ((float)M_PI * h3);
+    P.cs_k2 = 2.0 * (double)P.cs_k;
     P.nf = (int)nf;
     P.nb = (int)nb;
     int cmin[3], dim[3];

@@ -104,21 +104,18 @@ __device__ __forceinline__ void pcib_collide(const SimParams& P, const DeviceArr
     wsum = 0.0f;
     w2sum = 0.0f;
     avg = make_float3(0.0f, 0.0f, 0.0f);
-    for_cells27(x, P.h, grid_single(P), [&](unsigned c) {
-        const unsigned e = A.bcell_start[c + 1];
-        for (unsigned q = A.bcell_start[c]; q < e; ++q) {
-            const float4 xb = A.bpos[q];
-            if (!(glm_length(__fsub_rn(x.x, xb.x), __fsub_rn(x.y, xb.y), __fsub_rn(x.z, xb.z)) < P.rest_r)) continue;
-            const float l = glm_length(__fsub_rn(y.x, xb.x), __fsub_rn(y.y, xb.y), __fsub_rn(y.z, xb.z));
-            const float gap = __fsub_rn(P.rest_r, l);
-            const float w = fmaxf(0.0f, __fdiv_rn(gap, P.rest_r));
-            wsum = __fadd_rn(wsum, w);
-            w2sum = __fadd_rn(w2sum, __fmul_rn(w, gap));
-            const float4 nb = A.bnormal[q];
-            avg.x = __fadd_rn(avg.x, __fmul_rn(w, nb.x));
-            avg.y = __fadd_rn(avg.y, __fmul_rn(w, nb.y));
-            avg.z = __fadd_rn(avg.z, __fmul_rn(w, nb.z));
-        }
+    for_candidates27(x, P.h, grid_single(P), A.bcell_start, [&](unsigned q) {
+        const float4 xb = A.bpos[q];
+        if (!(glm_length(__fsub_rn(x.x, xb.x), __fsub_rn(x.y, xb.y), __fsub_rn(x.z, xb.z)) < P.rest_r)) return;
+        const float l = glm_length(__fsub_rn(y.x, xb.x), __fsub_rn(y.y, xb.y), __fsub_rn(y.z, xb.z));
+        const float gap = __fsub_rn(P.rest_r, l);
+        const float w = fmaxf(0.0f, __fdiv_rn(gap, P.rest_r));
+        wsum = __fadd_rn(wsum, w);
+        w2sum = __fadd_rn(w2sum, __fmul_rn(w, gap));
+        const float4 nb = A.bnormal[q];
+        avg.x = __fadd_rn(avg.x, __fmul_rn(w, nb.x));
+        avg.y = __fadd_rn(avg.y, __fmul_rn(w, nb.y));
+        avg.z = __fadd_rn(avg.z, __fmul_rn(w, nb.z));
     });
 }
 
@@ -161,27 +158,21 @@ __device__ __forceinline__ float boundary_density(const SimParams& P, const Devi
     const float4 xq = A.bpos[q];
     const Grid g = grid_single(P);
     float rho = 0.0f;
-    for_cells27(xq, P.h, g, [&](unsigned c) {
-        const unsigned e = A.cell_start[c + 1];
-        for (unsigned j = A.cell_start[c]; j < e; ++j) {
-            const float4 xj = POLY6 ? A.predr[j] : A.pos[j];
-            const float s2 = dist2_exact(xq, xj);
-            if (!(s2 <= P.h2_guard)) continue;
-            const float w = POLY6 ? poly6_W(__fsub_rn(xq.x, xj.x), __fsub_rn(xq.y, xj.y), __fsub_rn(xq.z, xj.z), P)
-                                  : cs_W_exact(s2, P);
-            rho = __fadd_rn(rho, __fmul_rn(P.mass, w));
-        }
+    for_candidates27(xq, P.h, g, A.cell_start, [&](unsigned j) {
+        const float4 xj = POLY6 ? A.predr[j] : A.pos[j];
+        const float s2 = dist2_exact(xq, xj);
+        if (!(s2 <= P.h2_guard)) return;
+        const float w = POLY6 ? poly6_W(__fsub_rn(xq.x, xj.x), __fsub_rn(xq.y, xj.y), __fsub_rn(xq.z, xj.z), P)
+                              : cs_W_exact(s2, P);
+        rho = __fadd_rn(rho, __fmul_rn(P.mass, w));
     });
-    for_cells27(xq, P.h, g, [&](unsigned c) {
-        const unsigned e = A.bcell_start[c + 1];
-        for (unsigned b = A.bcell_start[c]; b < e; ++b) {
-            const float4 xb = A.bpos[b];
-            const float s2 = dist2_exact(xq, xb);
-            if (!(s2 <= P.h2_guard)) continue;
-            const float w = POLY6 ? poly6_W(__fsub_rn(xq.x, xb.x), __fsub_rn(xq.y, xb.y), __fsub_rn(xq.z, xb.z), P)
-                                  : cs_W_exact(s2, P);
-            rho = __fadd_rn(rho, __fmul_rn(xb.w, w));
-        }
+    for_candidates27(xq, P.h, g, A.bcell_start, [&](unsigned b) {
+        const float4 xb = A.bpos[b];
+        const float s2 = dist2_exact(xq, xb);
+        if (!(s2 <= P.h2_guard)) return;
+        const float w = POLY6 ? poly6_W(__fsub_rn(xq.x, xb.x), __fsub_rn(xq.y, xb.y), __fsub_rn(xq.z, xb.z), P)
+                              : cs_W_exact(s2, P);
+        rho = __fadd_rn(rho, __fmul_rn(xb.w, w));
     });
     return rho;
 }
@@ -1135,8 +1126,11 @@ __device__ __forceinline__ bool pcisph_integrate(const SimParams& P, const Devic
 }
 
 /* Accepted candidates that a thread of k_pcisph_solve collects before it
-   evaluates their kernel terms. */
-constexpr int kPcisphBatch = 32;
+   evaluates their kernel terms: more than the ~33 of a particle inside the
+   fluid, so that all lanes evaluate once, together (32, where most lanes had to
+   evaluate on the way: 1,878 us of solver per 1M step; 40 or 44: 1,084). 44 KB
+   a block, four blocks per SM. */
+constexpr int kPcisphBatch = 44;
 
 /* The loop of PCISPHSolver::step. Neighbours read posd (current position and
    p / rho^2) and predr, never pos, so the pass that ends an iteration also
@@ -1189,30 +1183,37 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
             float rho = 0.0f;
             int n = 0;
             const auto add_fluid = [&]() {
+                /* four independent evaluations at a time; past the end W is 0
+                   and leaves the sum as it is */
 #pragma unroll 1
-                for (int k = 0; k < n; ++k)
-                    rho = __fadd_rn(rho, __fmul_rn(P.mass, cs_W_exact(s_s2[k][threadIdx.x], P)));
+                for (int k = 0; k < n; k += 4) {
+                    float w[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        w[u] = __fmul_rn(P.mass, cs_W_exact(k + u < n ? s_s2[k + u][threadIdx.x] : 4.0f * P.h2, P));
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) rho = __fadd_rn(rho, w[u]);
+                }
                 n = 0;
             };
-            for_cells27(xi, P.h, g, [&](unsigned c) {
-                const unsigned e = A.cell_start[c + 1];
-                for (unsigned q = A.cell_start[c]; q < e; ++q) {
-                    const float s2 = dist2_exact(pi, A.predr[q]);
-                    if (s2 <= P.h2_guard) {
-                        if (n == kPcisphBatch) add_fluid();
-                        s_s2[n++][threadIdx.x] = s2;
+            for_stretches27(
+                xi, pi, P.h, g, A.cell_start, A.predr,
+                [&](unsigned, const float (&d)[4], unsigned) {
+                    if (n > kPcisphBatch - 4) add_fluid();
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        /* a place that is not kept is written over */
+                        s_s2[n][threadIdx.x] = d[u];
+                        n += d[u] <= P.h2_guard ? 1 : 0;
                     }
-                }
-            });
+                },
+                [](auto) {});
             add_fluid();
-            if (P.nb > 0)
-                for_cells27(xi, P.h, g, [&](unsigned c) {
-                    const unsigned e = A.bcell_start[c + 1];
-                    for (unsigned q = A.bcell_start[c]; q < e; ++q) {
-                        const float4 xb = A.bpos[q];
-                        const float s2 = dist2_exact(pi, xb);
-                        if (s2 <= P.h2_guard) rho = __fadd_rn(rho, __fmul_rn(xb.w, cs_W_exact(s2, P)));
-                    }
+            if (boundary_near(P, A.near, xi, g))
+                for_candidates27(xi, P.h, g, A.bcell_start, [&](unsigned q) {
+                    const float4 xb = A.bpos[q];
+                    const float s2 = dist2_exact(pi, xb);
+                    if (s2 <= P.h2_guard) rho = __fadd_rn(rho, __fmul_rn(xb.w, cs_W_exact(s2, P)));
                 });
             A.rho[i] = rho;
             const float err = fmaxf(0.0f, __fsub_rn(rho, P.rho0));
@@ -1246,9 +1247,8 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
             float ax = 0.0f, ay = 0.0f, az = 0.0f;
             const unsigned nF = A.cnt_f[i], nB = A.cnt_b[i];
             if (it == 0) {
-                for (unsigned kk = 0; kk < nF; ++kk) {
-                    const unsigned j = list_at(A.nbr_f, kk, P.capF, i);
-                    const float4 xj = A.posd[j];
+                constexpr int U = 4; /* gathers issued before the first is used */
+                const auto term = [&](unsigned kk, unsigned j, const float4& xj) {
                     float gx, gy, gz;
                     cs_gradW_exact(__fsub_rn(xi.x, xj.x), __fsub_rn(xi.y, xj.y), __fsub_rn(xi.z, xj.z), P, gx, gy, gz);
                     if (more) __stcs(A.pgrad + list_index(kk, P.capF, i), make_float4(__uint_as_float(j), gx, gy, gz));
@@ -1256,6 +1256,21 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
                     ax = __fsub_rn(ax, __fmul_rn(c, gx));
                     ay = __fsub_rn(ay, __fmul_rn(c, gy));
                     az = __fsub_rn(az, __fmul_rn(c, gz));
+                };
+                unsigned kk = 0;
+                for (; kk + U <= nF; kk += U) {
+                    unsigned j[U];
+                    float4 xj[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) j[u] = list_at(A.nbr_f, kk + u, P.capF, i);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) xj[u] = A.posd[j[u]];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) term(kk + u, j[u], xj[u]);
+                }
+                for (; kk < nF; ++kk) {
+                    const unsigned j = list_at(A.nbr_f, kk, P.capF, i);
+                    term(kk, j, A.posd[j]);
                 }
             } else {
                 const float* dp = reinterpret_cast<const float*>(A.posd) + 3;
