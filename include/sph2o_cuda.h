@@ -394,7 +394,7 @@ int sph_debug_barrier_timeout(sph_ctx* ctx);
    takes longer). Work is queued on `stream`
    (a cudaStream_t; NULL = the legacy default stream) and the call returns
    without waiting. Nothing is allocated: the neighbour-search scratch is a
-   fixed file-scope device array of about 9.5 MiB that every GPU loading this
+   fixed file-scope device array of about 6 MiB that every GPU loading this
    library keeps until exit. Sizes above SPH_NOALLOC_MAX_FLUID,
    SPH_NOALLOC_MAX_BOUNDARY or SPH_NOALLOC_MAX_CELLS (cells of edge 4r over
    the domain, padded) return SPH_ERR_CAPACITY with the reason in

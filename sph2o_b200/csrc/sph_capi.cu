@@ -66,7 +66,7 @@ struct sph_ctx {
     float4* pgrad = nullptr; /* PCISPH: gradients of the list entries (DeviceArrays::pgrad) */
     float *rho = nullptr, *alpha = nullptr, *press = nullptr;
     unsigned *cell_of = nullptr, *slot = nullptr, *tmp_key = nullptr, *tmp_src = nullptr, *cell_sorted = nullptr;
-    unsigned *cell_count = nullptr, *cell_start = nullptr, *bcell_start = nullptr, *block_sums = nullptr;
+    unsigned *cell_count = nullptr, *cell_start = nullptr, *bcell_start = nullptr, *chunk_sums = nullptr;
     unsigned char* near = nullptr; /* per cell: boundary particles around it (k_mark_near) */
     float4* bpos = nullptr;
     float* bvol = nullptr;
@@ -467,8 +467,8 @@ int neighbor_search(sph_ctx* c)
         if (c->P.pcib) { g.v4_in[2] = c->normal; g.v4_out[2] = c->normal2; }
     }
     {
-        Phase ph(c, SPH_PROF_SORT, 5);
-        launch_sort(c->P, SceneRef{c->d_scenes, c->d_scene_of}, (int)c->nf, c->pos, c->cell_count, c->cell_start, c->block_sums, c->cell_of, c->slot,
+        Phase ph(c, SPH_PROF_SORT, 4);
+        launch_sort(c->P, SceneRef{c->d_scenes, c->d_scene_of}, (int)c->nf, c->pos, c->cell_count, c->cell_start, c->chunk_sums, c->cell_of, c->slot,
                     c->tmp_key, c->tmp_src, c->orig, g, c->stream);
     }
     std::swap(c->pos, c->pos2);
@@ -1073,7 +1073,7 @@ int sph_init(sph_ctx* c)
     ALLOC(normal, nf); ALLOC(predr, nf); ALLOC(posd, nf);
     ALLOC(cell_of, nmax); ALLOC(slot, nmax); ALLOC(tmp_key, nmax); ALLOC(tmp_src, nmax); ALLOC(cell_sorted, nmax);
     ALLOC(cell_count, (size_t)P.ncells); ALLOC(cell_start, (size_t)P.ncells + 1);
-    ALLOC(bcell_start, (size_t)P.ncells + 1); ALLOC(block_sums, (size_t)P.ncells / 4096 + 1);
+    ALLOC(bcell_start, (size_t)P.ncells + 1); ALLOC(chunk_sums, (size_t)P.ncells / 4096 + 1);
     ALLOC(near, (size_t)P.ncells);
     ALLOC(bpos, nb); ALLOC(bvol, nb); ALLOC(borig, nb);
     ALLOC(cnt_f, nf); ALLOC(cnt_b, nf);
@@ -1139,10 +1139,11 @@ int sph_init(sph_ctx* c)
                 if (c->grid_solve[dv][o][t] <= 0) return fail(c, SPH_ERR_CUDA, "cannot size the persistent solver grid");
             }
 
-    /* the fast division by h, if it is exact for this h (block_sums is free) */
+    /* the fast division by h, if it is exact for this h (chunk_sums is free) */
     unsigned bad_div = 1;
-    launch_check_div_h(P, c->block_sums, c->stream);
-    CUDA_TRY(c, cudaMemcpyAsync(&bad_div, c->block_sums, sizeof bad_div, cudaMemcpyDeviceToHost, c->stream));
+    launch_check_div_h(P, c->chunk_sums, c->stream);
+    CUDA_TRY(c, cudaMemcpyAsync(&bad_div, c->chunk_sums, sizeof bad_div, cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(c, cudaMemsetAsync(c->chunk_sums, 0, sizeof bad_div, c->stream)); /* the sort expects zeros */
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     P.h_div_exact = bad_div ? 0 : 1;
 
@@ -1182,7 +1183,7 @@ int sph_init(sph_ctx* c)
             g.v4_out[1] = c->bnormal;
         }
         const SceneRef bref{c->d_scenes, c->d_bscene_of};
-        launch_sort(P, bref, (int)nb, braw, c->cell_count, c->bcell_start, c->block_sums, c->cell_of, c->slot,
+        launch_sort(P, bref, (int)nb, braw, c->cell_count, c->bcell_start, c->chunk_sums, c->cell_of, c->slot,
                     c->tmp_key, c->tmp_src, bid, g, c->stream);
         if (!P.pcib) launch_boundary_volume(P, bref, c->bpos, c->bcell_start, c->bvol, c->stream);
         launch_mark_near(P, bref, c->bpos, c->near, c->stream);
@@ -1531,7 +1532,7 @@ int resort_boundary(sph_ctx* c)
     g.v4_in[0] = c->braw;
     g.v4_out[0] = c->bpos;
     const SceneRef bref{c->d_scenes, c->d_bscene_of};
-    launch_sort(c->P, bref, (int)c->nb, c->braw, c->cell_count, c->bcell_start, c->block_sums, c->cell_of, c->slot,
+    launch_sort(c->P, bref, (int)c->nb, c->braw, c->cell_count, c->bcell_start, c->chunk_sums, c->cell_of, c->slot,
                 c->tmp_key, c->tmp_src, c->bid, g, c->stream);
     launch_boundary_volume(c->P, bref, c->bpos, c->bcell_start, c->bvol, c->stream);
     CUDA_TRY(c, cudaMemsetAsync(c->near, 0, c->P.ncells, c->stream));

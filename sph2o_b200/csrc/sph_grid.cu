@@ -5,8 +5,9 @@
  *
  * Per step:
  *   1. ns_count        cell key floor(x / h) -> cell index in brick order,
- *                      per-cell population by atomicAdd (slot = old count)
- *   2. scan_local/add  exclusive scan of the populations -> cellStart[ncells+1]
+ *                      per-cell population by atomicAdd (slot = old count),
+ *                      totals of chunks of 4096 cells
+ *   2. scan            exclusive scan of the populations -> cellStart[ncells+1]
  *                      (the scan zeroes the populations for the next step)
  *   3. ns_scatter      (orig id, source index) into its cell segment
  *   4. ns_rank_gather  rank inside the cell by orig id (deterministic, equal
@@ -30,95 +31,36 @@ namespace sph {
 
 __global__ void __launch_bounds__(256) k_ns_count(SimParams P, SceneRef S, int n, const unsigned* n_dev,
                                                   const float4* __restrict__ pos, unsigned* __restrict__ cell_count,
-                                                  unsigned* __restrict__ cell_of, unsigned* __restrict__ slot)
+                                                  unsigned* __restrict__ chunk_sums, unsigned* __restrict__ cell_of,
+                                                  unsigned* __restrict__ slot)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (n_dev ? (int)*n_dev : n)) return;
-    ns_count_at(P, S, i, pos, cell_count, cell_of, slot);
+    const bool on = i < (n_dev ? (int)*n_dev : n);
+    ns_count_at(on, on ? cell_index(pos[i], P.h, grid_for(P, S, (unsigned)i)) : 0u, i, cell_count, chunk_sums, cell_of,
+                slot);
 }
 
-/* Exclusive scan, phase 1: each 256-thread block scans 4096 populations (16
-   per thread, four 16-byte loads in flight), writes block-local exclusive
-   offsets and zeroes the populations. */
-__global__ void __launch_bounds__(256) k_scan_local(unsigned* __restrict__ count, unsigned* __restrict__ start,
-                                                    unsigned* __restrict__ block_sums)
+/* Exclusive scan of the populations in one launch: each 256-thread block scans
+   4096 of them (scan_chunk_at) on top of the totals of the chunks before it,
+   which the count step has summed, and zeroes the populations for the next
+   search. A second launch that added the chunk offsets cost ~3 us per search. */
+__global__ void __launch_bounds__(256) k_scan(unsigned* __restrict__ count, unsigned* __restrict__ start,
+                                              const unsigned* __restrict__ chunk_sums, int nchunks,
+                                              unsigned* __restrict__ total_out)
 {
-    __shared__ unsigned warp_tot[8];
-    const size_t base = (size_t)blockIdx.x * 4096 + (size_t)threadIdx.x * 16;
-    uint4 c[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) c[k] = *reinterpret_cast<const uint4*>(count + base + 4 * k);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(count + base + 4 * k) = make_uint4(0, 0, 0, 0);
-    unsigned t = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) t += (c[k].x + c[k].y) + (c[k].z + c[k].w);
-    unsigned incl = t;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
-    if (lane == 31) warp_tot[wid] = incl;
-    __syncthreads();
-    if (wid == 0) {
-        const unsigned w = lane < 8 ? warp_tot[lane] : 0u;
-        unsigned wi = w;
-        for (int o = 1; o < 8; o <<= 1) {
-            const unsigned v = __shfl_up_sync(0xffffffffu, wi, o);
-            if (lane >= o) wi += v;
-        }
-        if (lane < 8) warp_tot[lane] = wi - w;
-        if (lane == 7) block_sums[blockIdx.x] = wi;
-    }
-    __syncthreads();
-    unsigned run = warp_tot[wid] + incl - t;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        uint4 o;
-        o.x = run; run += c[k].x;
-        o.y = run; run += c[k].y;
-        o.z = run; run += c[k].z;
-        o.w = run; run += c[k].w;
-        *reinterpret_cast<uint4*>(start + base + 4 * k) = o;
-    }
-}
-
-/* Phase 2: each block adds to its chunk the totals of all chunks before it
-   (summed by the block itself, so the chunk totals need no scan of their
-   own), and the last block writes the grand total. */
-__global__ void __launch_bounds__(1024) k_scan_add(unsigned* __restrict__ start,
-                                                   const unsigned* __restrict__ block_sums, int nblocks,
-                                                   unsigned* __restrict__ total_out)
-{
-    __shared__ unsigned warp_tot[32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    unsigned v = 0;
-    for (int k = threadIdx.x; k < (int)blockIdx.x; k += 1024) v += block_sums[k];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) warp_tot[wid] = v;
-    __syncthreads();
-    if (wid == 0) {
-        unsigned w = warp_tot[lane];
-        for (int o = 16; o > 0; o >>= 1) w += __shfl_down_sync(0xffffffffu, w, o);
-        if (lane == 0) warp_tot[0] = w;
-    }
-    __syncthreads();
-    const unsigned off = warp_tot[0];
-    if ((int)blockIdx.x == nblocks - 1 && threadIdx.x == 0) *total_out = off + block_sums[blockIdx.x];
-    const size_t base = (size_t)blockIdx.x * 4096 + (size_t)threadIdx.x * 4;
-    uint4 s = *reinterpret_cast<uint4*>(start + base);
-    s.x += off; s.y += off; s.z += off; s.w += off;
-    *reinterpret_cast<uint4*>(start + base) = s;
+    scan_chunk_at<true>((int)blockIdx.x, count, start, chunk_sums, nchunks, total_out);
 }
 
 __global__ void __launch_bounds__(256) k_ns_scatter(int n, const unsigned* n_dev, const unsigned* __restrict__ cell_of,
                                                     const unsigned* __restrict__ slot,
                                                     const unsigned* __restrict__ cell_start,
                                                     const unsigned* __restrict__ orig,
-                                                    unsigned* __restrict__ tmp_key, unsigned* __restrict__ tmp_src)
+                                                    unsigned* __restrict__ tmp_key, unsigned* __restrict__ tmp_src,
+                                                    unsigned* __restrict__ chunk_sums, int nchunks)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    /* the scan is done with the chunk totals: zero for the next search */
+    for (int k = i; k < nchunks; k += (int)(gridDim.x * blockDim.x)) chunk_sums[k] = 0u;
     if (i >= (n_dev ? (int)*n_dev : n)) return;
     ns_scatter_at(i, cell_of, slot, cell_start, orig, tmp_key, tmp_src);
 }
@@ -418,7 +360,7 @@ static inline int blocks_for(long long n, int bs) { return (int)((n + bs - 1) / 
 
 void launch_sort(const SimParams& P, const SceneRef& S, int n, const float4* pos_for_keys, unsigned* cell_count,
                  unsigned* cell_start,
-                 unsigned* block_sums, unsigned* cell_of, unsigned* slot, unsigned* tmp_key, unsigned* tmp_src,
+                 unsigned* chunk_sums, unsigned* cell_of, unsigned* slot, unsigned* tmp_key, unsigned* tmp_src,
                  const unsigned* orig_in, const GatherSet& g, cudaStream_t s)
 {
     if (n <= 0) {
@@ -426,11 +368,11 @@ void launch_sort(const SimParams& P, const SceneRef& S, int n, const float4* pos
         cudaMemsetAsync(cell_start, 0, ((size_t)P.ncells + 1) * sizeof(unsigned), s);
         return;
     }
-    k_ns_count<<<blocks_for(n, 256), 256, 0, s>>>(P, S, n, g.n_dev, pos_for_keys, cell_count, cell_of, slot);
-    const int nblk = (int)(P.ncells / 4096);
-    k_scan_local<<<nblk, 256, 0, s>>>(cell_count, cell_start, block_sums);
-    k_scan_add<<<nblk, 1024, 0, s>>>(cell_start, block_sums, nblk, cell_start + P.ncells);
-    k_ns_scatter<<<blocks_for(n, 256), 256, 0, s>>>(n, g.n_dev, cell_of, slot, cell_start, orig_in, tmp_key, tmp_src);
+    const int nchunks = (int)(P.ncells / 4096);
+    k_ns_count<<<blocks_for(n, 256), 256, 0, s>>>(P, S, n, g.n_dev, pos_for_keys, cell_count, chunk_sums, cell_of, slot);
+    k_scan<<<nchunks, 256, 0, s>>>(cell_count, cell_start, chunk_sums, nchunks, cell_start + P.ncells);
+    k_ns_scatter<<<blocks_for(n, 256), 256, 0, s>>>(n, g.n_dev, cell_of, slot, cell_start, orig_in, tmp_key, tmp_src,
+                                                    chunk_sums, nchunks);
     k_ns_rank_gather<<<blocks_for(n, 256), 256, 0, s>>>(n, cell_of, cell_start, tmp_key, tmp_src, g);
 }
 

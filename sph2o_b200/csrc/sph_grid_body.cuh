@@ -25,14 +25,74 @@ struct GatherSet {
     float* f_out[2];
 };
 
-/* cell of particle i and its arrival slot in that cell */
-__device__ __forceinline__ void ns_count_at(const SimParams& P, const SceneRef& S, int i, const float4* __restrict__ pos,
-                                            unsigned* __restrict__ cell_count, unsigned* __restrict__ cell_of,
+/* Particle i (where `on`) in cell c: its cell, its arrival slot there, and the
+   population of c's chunk of 4096 cells, added once per warp where its lanes
+   share a chunk (neighbouring particles nearly always do). The whole warp
+   calls. */
+__device__ __forceinline__ void ns_count_at(bool on, unsigned c, int i, unsigned* __restrict__ cell_count,
+                                            unsigned* __restrict__ chunk_sums, unsigned* __restrict__ cell_of,
                                             unsigned* __restrict__ slot)
 {
-    const unsigned c = cell_index(pos[i], P.h, grid_for(P, S, (unsigned)i));
-    cell_of[i] = c;
-    slot[i] = atomicAdd(&cell_count[c], 1u);
+    if (on) {
+        cell_of[i] = c;
+        slot[i] = atomicAdd(&cell_count[c], 1u);
+    }
+    const unsigned active = __ballot_sync(0xffffffffu, on);
+    if (active == 0u) return;
+    const int first = __ffs((int)active) - 1;
+    const unsigned chunk = c >> 12, chunk0 = __shfl_sync(0xffffffffu, chunk, first);
+    const unsigned same = __ballot_sync(0xffffffffu, on && chunk == chunk0);
+    if ((int)(threadIdx.x & 31u) == first) atomicAdd(&chunk_sums[chunk0], (unsigned)__popc(same));
+    else if (on && chunk != chunk0) atomicAdd(&chunk_sums[chunk], 1u);
+}
+
+/* Exclusive scan of chunk b's 4096 populations by 256 threads (16 per thread,
+   four 16-byte loads in flight), offset by the totals of the chunks before it;
+   the last chunk writes the grand total. ZERO: the populations are zeroed
+   (count and start may be one array without it). */
+template <bool ZERO>
+__device__ __forceinline__ void scan_chunk_at(int b, unsigned* count, unsigned* start, const unsigned* chunk_sums,
+                                              int nchunks, unsigned* total_out)
+{
+    __shared__ unsigned warp_tot[8], warp_off[8];
+    const size_t base = (size_t)b * 4096 + (size_t)threadIdx.x * 16;
+    uint4 c[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c[k] = *reinterpret_cast<const uint4*>(count + base + 4 * k);
+    unsigned before = 0;
+    for (int k = (int)threadIdx.x; k < b; k += 256) before += chunk_sums[k];
+    if (ZERO) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(count + base + 4 * k) = make_uint4(0, 0, 0, 0);
+    }
+    unsigned t = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) t += (c[k].x + c[k].y) + (c[k].z + c[k].w);
+    unsigned incl = t;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (lane == 31) {
+        warp_tot[wid] = incl;
+        warp_off[wid] = before;
+    }
+    __syncthreads();
+    unsigned run = incl - t;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) run += warp_off[w] + (w < wid ? warp_tot[w] : 0u);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        uint4 o;
+        o.x = run; run += c[k].x;
+        o.y = run; run += c[k].y;
+        o.z = run; run += c[k].z;
+        o.w = run; run += c[k].w;
+        *reinterpret_cast<uint4*>(start + base + 4 * k) = o;
+    }
+    if (b == nchunks - 1 && threadIdx.x == 255) *total_out = run;
 }
 
 /* (orig id, source index) of particle i into its cell segment */

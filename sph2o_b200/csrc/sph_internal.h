@@ -75,7 +75,7 @@ struct DeviceArrays {
 /* sph_grid.cu */
 void launch_sort(const SimParams& P, const SceneRef& S, int n, const float4* pos_for_keys, unsigned* cell_count,
                  unsigned* cell_start,
-                 unsigned* block_sums, unsigned* cell_of, unsigned* slot, unsigned* tmp_key, unsigned* tmp_src,
+                 unsigned* chunk_sums, unsigned* cell_of, unsigned* slot, unsigned* tmp_key, unsigned* tmp_src,
                  const unsigned* orig_in, const GatherSet& g, cudaStream_t s);
 void launch_build_lists(const SimParams& P, const SceneRef& S, const float4* pos, const unsigned* cell_start,
                         const float4* bpos,

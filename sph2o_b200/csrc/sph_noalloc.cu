@@ -11,7 +11,7 @@
  * How: the neighbour-search scratch (cell table, sort buffers, sorted copies)
  * lives in one file-scope static __device__ array of fixed size, so this path
  * calls no cudaMalloc, cudaFree or allocating library routine. Every GPU that
- * loads the library holds the array (about 9.5 MiB) until the process exits.
+ * loads the library holds the array (about 6 MiB) until the process exits.
  *
  * Rules for callers (also in include/sph2o_cuda.h):
  *   - sizes above SPH_NOALLOC_MAX_FLUID / _BOUNDARY / _CELLS are rejected
@@ -26,7 +26,7 @@
  *     device ordinal and CUDA context id, so after cudaDeviceReset (a new
  *     primary context, the module possibly reloaded elsewhere) the next call
  *     looks it up again -- that call, too, belongs outside a stream capture.
- * The kernels reuse the pipeline's sort (sph_grid.cu) and evaluate each
+ * The kernels reuse the bodies of the pipeline's sort (sph_grid_body.cuh) and evaluate each
  * density over the 27 cells in the same order and with the same exact
  * arithmetic as the context path, so for particles inside domain_min/max the
  * result equals sph_compute_phase(SPH_PHASE_DENSITY) bit for bit. A particle
@@ -50,26 +50,25 @@ namespace {
 constexpr size_t kMaxFluid = SPH_NOALLOC_MAX_FLUID;
 constexpr size_t kMaxBoundary = SPH_NOALLOC_MAX_BOUNDARY;
 constexpr size_t kMaxCells = SPH_NOALLOC_MAX_CELLS;  /* multiple of 4096 */
-constexpr size_t kMaxN = kMaxFluid > kMaxBoundary ? kMaxFluid : kMaxBoundary;
 
 constexpr size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
-/* byte offsets of the regions inside the scratch array */
-constexpr size_t kOffCount = 0;
-constexpr size_t kOffStart = kOffCount + align256(kMaxCells * 4);
-constexpr size_t kOffBStart = kOffStart + align256((kMaxCells + 1) * 4);
-constexpr size_t kOffBlockSums = kOffBStart + align256((kMaxCells + 1) * 4);
-constexpr size_t kOffCellOf = kOffBlockSums + align256((kMaxCells / 4096 + 1) * 4);
-constexpr size_t kOffSlot = kOffCellOf + align256(kMaxN * 4);
-constexpr size_t kOffKey = kOffSlot + align256(kMaxN * 4);
-constexpr size_t kOffSrc = kOffKey + align256(kMaxN * 4);
-constexpr size_t kOffIds = kOffSrc + align256(kMaxN * 4);
-constexpr size_t kOffOrig = kOffIds + align256(kMaxN * 4);
-constexpr size_t kOffBOrig = kOffOrig + align256(kMaxFluid * 4);
-constexpr size_t kOffPosRaw = kOffBOrig + align256(kMaxBoundary * 4);
-constexpr size_t kOffPos = kOffPosRaw + align256(kMaxFluid * 16);
-constexpr size_t kOffBRaw = kOffPos + align256(kMaxFluid * 16);
-constexpr size_t kOffBPos = kOffBRaw + align256(kMaxBoundary * 16);
+/* byte offsets of the regions inside the scratch array: cell tables (counted
+   and scanned in place) with their chunk totals, zeroed together at the start
+   of a call; then the sort buffers and sorted copies */
+constexpr size_t kOffStart = 0;
+constexpr size_t kOffSums = kOffStart + align256((kMaxCells + 1) * 4);
+constexpr size_t kOffBStart = kOffSums + align256(kMaxCells / 4096 * 4);
+constexpr size_t kOffBSums = kOffBStart + align256((kMaxCells + 1) * 4);
+constexpr size_t kOffCellOf = kOffBSums + align256(kMaxCells / 4096 * 4);
+constexpr size_t kOffSlot = kOffCellOf + align256(kMaxFluid * 4);
+constexpr size_t kOffSrc = kOffSlot + align256(kMaxFluid * 4);
+constexpr size_t kOffOrig = kOffSrc + align256(kMaxFluid * 4);
+constexpr size_t kOffBCellOf = kOffOrig + align256(kMaxFluid * 4);
+constexpr size_t kOffBSlot = kOffBCellOf + align256(kMaxBoundary * 4);
+constexpr size_t kOffBSrc = kOffBSlot + align256(kMaxBoundary * 4);
+constexpr size_t kOffPos = kOffBSrc + align256(kMaxBoundary * 4);
+constexpr size_t kOffBPos = kOffPos + align256(kMaxFluid * 16);
 constexpr size_t kScratchBytes = kOffBPos + align256(kMaxBoundary * 16);
 
 } // namespace
@@ -118,44 +117,127 @@ bool current_context_id(unsigned long long* id)
     return get_id(ctx, id) == CUDA_SUCCESS;
 }
 
-__global__ void k_na_pack_fluid(int n, const float* __restrict__ xyz, float4* __restrict__ out,
-                                unsigned* __restrict__ ids)
+/* One particle set (fluid or boundary) on its way through the counting sort.
+   Fluid and boundary go through each step in one launch, the first blocks the
+   fluid's: a call is six launches, where a sort of its own for each set, the
+   packing and a scan in two steps made it fourteen (30,000 + 5,000 particles:
+   123 us per call). */
+struct NaSet {
+    int n, blocks;           /* particles, blocks of 256 */
+    const float* in;         /* the caller's array, `width` floats per particle */
+    int width;
+    unsigned *start, *sums;  /* cell table (populations, then starts) and its chunk totals */
+    unsigned *cell_of, *slot, *src;
+    unsigned* orig;          /* caller index of each sorted slot (fluid only, else NULL) */
+    float4* out;             /* sorted copy */
+};
+
+__device__ __forceinline__ const NaSet& na_pick(const NaSet& f, const NaSet& b, int& i)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    out[i] = make_float4(xyz[3 * (size_t)i], xyz[3 * (size_t)i + 1], xyz[3 * (size_t)i + 2], 0.0f);
-    ids[i] = (unsigned)i;
+    const bool fluid = (int)blockIdx.x < f.blocks;
+    i = (int)((blockIdx.x - (fluid ? 0u : (unsigned)f.blocks)) * blockDim.x + threadIdx.x);
+    return fluid ? f : b;
 }
 
-__global__ void k_na_pack_boundary(int n, const float* __restrict__ xyzw, float4* __restrict__ out,
-                                   unsigned* __restrict__ ids)
+__device__ __forceinline__ float4 na_load(const NaSet& s, int i)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    out[i] = make_float4(xyzw[4 * (size_t)i], xyzw[4 * (size_t)i + 1], xyzw[4 * (size_t)i + 2],
-                         xyzw[4 * (size_t)i + 3]);
-    ids[i] = (unsigned)i;
+    const float* p = s.in + (size_t)i * s.width;
+    return make_float4(p[0], p[1], p[2], s.width == 4 ? p[3] : 0.0f);
+}
+
+__global__ void __launch_bounds__(256) k_na_zero(unsigned* start, unsigned* sums, unsigned* bstart, unsigned* bsums,
+                                                 unsigned ncells)
+{
+    const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < ncells) start[k] = bstart[k] = 0u;
+    if (k < ncells / 4096u) sums[k] = bsums[k] = 0u;
+    if (k == 0u) start[ncells] = bstart[ncells] = 0u; /* an empty set's total */
+}
+
+__global__ void __launch_bounds__(256) k_na_count(SimParams P, NaSet f, NaSet b)
+{
+    int i;
+    const NaSet& s = na_pick(f, b, i);
+    const bool on = i < s.n;
+    ns_count_at(on, on ? cell_index(na_load(s, i), P.h, grid_single(P)) : 0u, i, s.start, s.sums, s.cell_of, s.slot);
+}
+
+__global__ void __launch_bounds__(256) k_na_scan(NaSet f, NaSet b, int nchunks)
+{
+    const bool fluid = (int)blockIdx.x < nchunks;
+    const NaSet& s = fluid ? f : b;
+    scan_chunk_at<false>((int)blockIdx.x - (fluid ? 0 : nchunks), s.start, s.start, s.sums, nchunks,
+                         s.start + (size_t)nchunks * 4096);
+}
+
+__global__ void __launch_bounds__(256) k_na_scatter(NaSet f, NaSet b)
+{
+    int i;
+    const NaSet& s = na_pick(f, b, i);
+    if (i < s.n) s.src[s.start[s.cell_of[i]] + s.slot[i]] = (unsigned)i;
+}
+
+/* Rank inside the cell by caller index, then the sorted copy. */
+__global__ void __launch_bounds__(256) k_na_rank_gather(NaSet f, NaSet b)
+{
+    int p;
+    const NaSet& s = na_pick(f, b, p);
+    if (p >= s.n) return;
+    const unsigned i = s.src[p];
+    const float4 x = na_load(s, (int)i);
+    const unsigned c = s.cell_of[i], first = s.start[c], end = s.start[c + 1];
+    unsigned dst = first;
+    for (unsigned q = first; q < end; ++q) dst += s.src[q] < i ? 1u : 0u;
+    s.out[dst] = x;
+    if (s.orig) s.orig[dst] = i;
 }
 
 /* Density over the 27 cells: every fluid candidate first, then every boundary
    candidate, cells in the reference's offset order, exact W; written to the
-   caller's order. */
-__global__ void __launch_bounds__(128) k_na_density(SimParams P, const float4* __restrict__ pos,
-                                                    const unsigned* __restrict__ cell_start,
-                                                    const unsigned* __restrict__ orig,
-                                                    const float4* __restrict__ bpos,
-                                                    const unsigned* __restrict__ bcell_start,
-                                                    float* __restrict__ rho_out)
+   caller's order. A thread per particle in blocks of 64, so that the blocks of
+   a few thousand particles still reach every SM; accepted candidates are
+   collected and their kernels evaluated four at a time, all lanes together. */
+constexpr int kNaBlock = 64, kNaBatch = 44;
+
+__global__ void __launch_bounds__(kNaBlock) k_na_density(SimParams P, const float4* __restrict__ pos,
+                                                         const unsigned* __restrict__ cell_start,
+                                                         const unsigned* __restrict__ orig,
+                                                         const float4* __restrict__ bpos,
+                                                         const unsigned* __restrict__ bcell_start,
+                                                         float* __restrict__ rho_out)
 {
+    __shared__ float s_s2[kNaBatch][kNaBlock];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.nf) return;
     const float4 xi = pos[i];
     const Grid g = grid_single(P);
     float rho = 0.0f;
-    for_candidates27(xi, P.h, g, cell_start, [&](unsigned q) {
-        const float s2 = dist2_exact(xi, pos[q]);
-        if (s2 <= P.h2_guard) rho = __fadd_rn(rho, __fmul_rn(P.mass, cs_W_exact(s2, P)));
-    });
+    int n = 0;
+    const auto add_fluid = [&]() {
+        /* past the end W is 0 and leaves the sum as it is */
+#pragma unroll 1
+        for (int k = 0; k < n; k += 4) {
+            float w[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                w[u] = __fmul_rn(P.mass, cs_W_exact(k + u < n ? s_s2[k + u][threadIdx.x] : 4.0f * P.h2, P));
+#pragma unroll
+            for (int u = 0; u < 4; ++u) rho = __fadd_rn(rho, w[u]);
+        }
+        n = 0;
+    };
+    for_stretches27(
+        xi, xi, P.h, g, cell_start, pos,
+        [&](unsigned, const float (&d)[4], unsigned) {
+            if (n > kNaBatch - 4) add_fluid();
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                s_s2[n][threadIdx.x] = d[u];
+                n += d[u] <= P.h2_guard ? 1 : 0;
+            }
+        },
+        [](auto) {});
+    add_fluid();
     if (P.nb > 0)
         for_candidates27(xi, P.h, g, bcell_start, [&](unsigned q) {
             const float4 xb = bpos[q];
@@ -260,44 +342,30 @@ extern "C" int sph_density_noalloc(float particle_radius, float density0, const 
     if (nf == 0) return SPH_OK;
 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    unsigned* cell_count = reinterpret_cast<unsigned*>(base + kOffCount);
-    unsigned* cell_start = reinterpret_cast<unsigned*>(base + kOffStart);
-    unsigned* bcell_start = reinterpret_cast<unsigned*>(base + kOffBStart);
-    unsigned* block_sums = reinterpret_cast<unsigned*>(base + kOffBlockSums);
-    unsigned* cell_of = reinterpret_cast<unsigned*>(base + kOffCellOf);
-    unsigned* slot = reinterpret_cast<unsigned*>(base + kOffSlot);
-    unsigned* key = reinterpret_cast<unsigned*>(base + kOffKey);
-    unsigned* src = reinterpret_cast<unsigned*>(base + kOffSrc);
-    unsigned* ids = reinterpret_cast<unsigned*>(base + kOffIds);
-    unsigned* orig = reinterpret_cast<unsigned*>(base + kOffOrig);
-    unsigned* borig = reinterpret_cast<unsigned*>(base + kOffBOrig);
-    float4* pos_raw = reinterpret_cast<float4*>(base + kOffPosRaw);
-    float4* pos = reinterpret_cast<float4*>(base + kOffPos);
-    float4* braw = reinterpret_cast<float4*>(base + kOffBRaw);
-    float4* bpos = reinterpret_cast<float4*>(base + kOffBPos);
-
-    /* the populations must start at zero; the array keeps the last call's contents */
-    e = cudaMemsetAsync(cell_count, 0, (size_t)P.ncells * sizeof(unsigned), s);
-    if (e != cudaSuccess) return na_fail(SPH_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
-
-    if (nb > 0) {
-        k_na_pack_boundary<<<(nb + 255) / 256, 256, 0, s>>>((int)nb, bxyzpsi, braw, ids);
-        GatherSet gb{};
-        gb.orig_out = borig;
-        gb.v4_in[0] = braw;
-        gb.v4_out[0] = bpos;
-        launch_sort(P, SceneRef{}, (int)nb, braw, cell_count, bcell_start, block_sums, cell_of, slot, key, src, ids, gb, s);
-    } else {
-        e = cudaMemsetAsync(bcell_start, 0, ((size_t)P.ncells + 1) * sizeof(unsigned), s);
-        if (e != cudaSuccess) return na_fail(SPH_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
-    }
-    k_na_pack_fluid<<<(nf + 255) / 256, 256, 0, s>>>((int)nf, xyz, pos_raw, ids);
-    GatherSet gf{};
-    gf.orig_out = orig;
-    gf.v4_in[0] = pos_raw;
-    gf.v4_out[0] = pos;
-    launch_sort(P, SceneRef{}, (int)nf, pos_raw, cell_count, cell_start, block_sums, cell_of, slot, key, src, ids, gf, s);
-    k_na_density<<<(nf + 127) / 128, 128, 0, s>>>(P, pos, cell_start, orig, bpos, bcell_start, rho_out);
+    const auto words = [base](size_t off) { return reinterpret_cast<unsigned*>(base + off); };
+    NaSet f{}, b{};
+    f.n = (int)nf;
+    f.in = xyz;
+    f.width = 3;
+    f.start = words(kOffStart); f.sums = words(kOffSums);
+    f.cell_of = words(kOffCellOf); f.slot = words(kOffSlot); f.src = words(kOffSrc);
+    f.orig = words(kOffOrig);
+    f.out = reinterpret_cast<float4*>(base + kOffPos);
+    b.n = (int)nb;
+    b.in = bxyzpsi;
+    b.width = 4;
+    b.start = words(kOffBStart); b.sums = words(kOffBSums);
+    b.cell_of = words(kOffBCellOf); b.slot = words(kOffBSlot); b.src = words(kOffBSrc);
+    b.out = reinterpret_cast<float4*>(base + kOffBPos);
+    f.blocks = (f.n + 255) / 256;
+    b.blocks = (b.n + 255) / 256;
+    const int blocks = f.blocks + b.blocks, nchunks = (int)(P.ncells / 4096);
+    k_na_zero<<<(P.ncells + 255) / 256, 256, 0, s>>>(f.start, f.sums, b.start, b.sums, P.ncells);
+    k_na_count<<<blocks, 256, 0, s>>>(P, f, b);
+    k_na_scan<<<(nb > 0 ? 2 : 1) * nchunks, 256, 0, s>>>(f, b, nchunks);
+    k_na_scatter<<<blocks, 256, 0, s>>>(f, b);
+    k_na_rank_gather<<<blocks, 256, 0, s>>>(f, b);
+    k_na_density<<<(f.n + kNaBlock - 1) / kNaBlock, kNaBlock, 0, s>>>(P, f.out, f.start, f.orig, b.out, b.start, rho_out);
     e = cudaGetLastError();
     if (e != cudaSuccess) return na_fail(SPH_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     return SPH_OK;
