@@ -449,8 +449,9 @@ int alloc_lists(sph_ctx* c)
     return SPH_OK;
 }
 
-/* Sort the fluid into cells and rebuild the neighbour lists. */
-int neighbor_search(sph_ctx* c)
+/* Sort the fluid into cells, rebuild the neighbour lists and compute what
+   `mode` (SearchMode) adds: densities, Tait pressures. */
+int neighbor_search(sph_ctx* c, int mode = SEARCH_LISTS)
 {
     GatherSet g{};
     if (c->P.dynamic) g.n_dev = &c->st->n_active;
@@ -480,10 +481,14 @@ int neighbor_search(sph_ctx* c)
         std::swap(c->kvws, c->kvws2);
         if (c->P.pcib) std::swap(c->normal, c->normal2);
     }
+    bool done = false;
     {
         Phase ph(c, SPH_PROF_LISTS, 1);
-        launch_build_lists(c->P, SceneRef{c->d_scenes, c->d_scene_of}, c->pos, c->cell_start, c->bpos, c->bcell_start, c->near, c->nbr_f, c->cnt_f, c->nbr_b,
-                           c->cnt_b, c->st, c->stream, c->staged_lists);
+        done = launch_search(c->P, SceneRef{c->d_scenes, c->d_scene_of}, arrays(c), mode, c->stream, c->staged_lists);
+    }
+    if (!done && mode != SEARCH_LISTS) {
+        Phase ph(c, SPH_PROF_DENSITY, 1);
+        launch_density(c->P, arrays(c), false, mode == SEARCH_EOS, c->pass_block, c->stream);
     }
     if (c->P.pcib) {
         /* the fluid's cells get candidate lists at this search */
@@ -522,9 +527,8 @@ int zero_accum(sph_ctx* c)
 int step_wcsph(sph_ctx* c)
 {
     int rc;
-    if ((rc = neighbor_search(c)) != SPH_OK) return rc;
+    if ((rc = neighbor_search(c, SEARCH_EOS)) != SPH_OK) return rc;
     DeviceArrays A = arrays(c);
-    { Phase ph(c, SPH_PROF_DENSITY, 1); launch_density(c->P, A, false, true, c->pass_block, c->stream); }
     if (c->P.pcib) { Phase ph(c, SPH_PROF_DENSITY, 1); launch_boundary_density(c->P, A, c->stream); }
     if (c->P.st_on) { Phase ph(c, SPH_PROF_NORMALS, 1); launch_normals(c->P, A, c->pass_block, c->stream); }
     { Phase ph(c, SPH_PROF_FORCES, 1); launch_forces(c->P, A, FORCE_WCSPH, c->pass_block, c->stream); }
@@ -544,9 +548,8 @@ int step_wcsph(sph_ctx* c)
 int step_pcisph(sph_ctx* c)
 {
     int rc;
-    if ((rc = neighbor_search(c)) != SPH_OK) return rc;
+    if ((rc = neighbor_search(c, SEARCH_DENSITY)) != SPH_OK) return rc;
     DeviceArrays A = arrays(c);
-    { Phase ph(c, SPH_PROF_DENSITY, 1); launch_density(c->P, A, false, false, c->pass_block, c->stream); }
     if (c->P.st_on) { Phase ph(c, SPH_PROF_NORMALS, 1); launch_normals(c->P, A, c->pass_block, c->stream); }
     { Phase ph(c, SPH_PROF_FORCES, 1); launch_forces(c->P, A, FORCE_NP, c->pass_block, c->stream); }
     if ((rc = zero_accum(c)) != SPH_OK) return rc;
@@ -617,8 +620,7 @@ int step_dfsph(sph_ctx* c)
            insertion, and evaluate distances at current positions: rebuild
            the lists from the current positions against the same cell table. */
         Phase ph(c, SPH_PROF_LISTS, 2);
-        launch_build_lists(c->P, SceneRef{c->d_scenes, c->d_scene_of}, c->pos, c->cell_start, c->bpos, c->bcell_start, c->near,
-                           c->nbr_f, c->cnt_f, c->nbr_b, c->cnt_b, c->st, c->stream);
+        launch_search(c->P, SceneRef{c->d_scenes, c->d_scene_of}, arrays(c), SEARCH_LISTS, c->stream);
         launch_pair_factors(c->P, arrays(c), c->stream);
     }
     return check_launch(c, "dfsph step");
@@ -1485,10 +1487,11 @@ int sph_compute_phase(sph_ctx* c, int phase, float* out)
     unsigned na = 0;
     int rc = active_count(c, &na);
     if (rc != SPH_OK) return rc;
-    if ((rc = neighbor_search(c)) != SPH_OK) return rc;
-    DeviceArrays A = arrays(c);
     const bool eos = phase == SPH_PHASE_PRESSURE || phase == SPH_PHASE_PRESSURE_ACC;
-    launch_density(c->P, A, phase == SPH_PHASE_ALPHA || c->desc.simulation_method == SPH_DFSPH, eos, c->pass_block, c->stream);
+    const bool alpha = phase == SPH_PHASE_ALPHA || c->desc.simulation_method == SPH_DFSPH;
+    if ((rc = neighbor_search(c, alpha ? SEARCH_LISTS : eos ? SEARCH_EOS : SEARCH_DENSITY)) != SPH_OK) return rc;
+    DeviceArrays A = arrays(c);
+    if (alpha) launch_density(c->P, A, true, eos, c->pass_block, c->stream);
     /* PCISPH boundary method: SPHSolver::computeDensities covers the
        boundary particles too (SPHSolver.cpp:126-137), WCSPH their pressures */
     if (c->P.pcib) launch_boundary_density(c->P, A, c->stream);
@@ -2136,8 +2139,7 @@ int adj_segment_body(sph_ctx* c, int len)
     for (int n = len - 1; n >= 0; --n) {
         if ((rc = copy_state(c, c->pos, c->vel, c->orig, a.sl_pos + n * nf, a.sl_vel + n * nf, a.sl_orig + n * nf)) != SPH_OK)
             return rc;
-        if ((rc = neighbor_search(c)) != SPH_OK) return rc;
-        { Phase ph(c, SPH_PROF_DENSITY, 1); launch_density(c->P, arrays(c), false, true, c->pass_block, c->stream); }
+        if ((rc = neighbor_search(c, SEARCH_EOS)) != SPH_OK) return rc;
         launch_adjoint_step(c->P, adj_arrays(c), c->stream);
         c->launches += 3;
     }

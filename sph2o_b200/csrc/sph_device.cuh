@@ -442,10 +442,11 @@ __device__ __forceinline__ float dist2_exact_packed(float4 a, float4 b)
    (c = 4, or the rest; d is huge past it), then stretch(slot) with slot(k) the
    slot of the stretch's candidate k. Four candidates are loaded before any is
    used, and nothing branches on a candidate: some lane of a warp accepts
-   nearly every one, so a branch would be taken nearly always. */
+   nearly every one, so a branch would be taken nearly always. [row0, row1):
+   the rows to walk, of the 9 in candidate order. */
 template <typename G, typename R>
 __device__ __forceinline__ void for_stretches27(float4 x, float4 y, float h, const Grid& g, const unsigned* cell_start,
-                                                const float4* pos, G&& group, R&& stretch)
+                                                const float4* pos, G&& group, R&& stretch, int row0 = 0, int row1 = 9)
 {
     const int cx = cell_coord(x.x, h, g.cminx, g.dimx);
     const int cy = cell_coord(x.y, h, g.cminy, g.dimy);
@@ -485,27 +486,26 @@ __device__ __forceinline__ void for_stretches27(float4 x, float4 y, float h, con
     };
     const int last = min(z1, z0 | 3);
     const unsigned ra = cell_z(z0, g), rb = cell_z(min(last + 1, g.dimz - 1), g);
-    for (int xx = max(cx - 1, 0); xx <= min(cx + 1, g.dimx - 1); ++xx) {
-        const unsigned bx = g.base + cell_x(xx, g);
-        for (int yy = max(cy - 1, 0); yy <= min(cy + 1, g.dimy - 1); ++yy) {
-            const unsigned* r = cell_start + (bx + cell_y(yy, g));
-            if (g.order == 1) {
-                const unsigned* c0 = r + cell_z(z0, g);
-                const unsigned* c1 = r + cell_z(z0 + 1, g);
-                const unsigned* c2 = r + cell_z(z1, g);
-                /* three cells that are not neighbours in memory: two stretches */
-                row(c0[0], c0[1] - c0[0], c1[0], c0[1] - c0[0] + c1[1] - c1[0]);
-                if (z1 - z0 == 2) row(c2[0], c2[1] - c2[0], c2[1], c2[1] - c2[0]);
-                continue;
-            }
-            const unsigned s1 = r[ra], n1 = r[ra + (unsigned)(last - z0 + 1)] - s1;
-            unsigned s2 = 0, n = n1;
-            if (last < z1) {
-                s2 = r[rb];
-                n += r[rb + (unsigned)(z1 - last)] - s2;
-            }
-            row(s1, n1, s2, n);
+    for (int t = row0; t < row1; ++t) {
+        const int xx = cx - 1 + t / 3, yy = cy - 1 + t % 3;
+        if (xx < 0 || xx >= g.dimx || yy < 0 || yy >= g.dimy) continue;
+        const unsigned* r = cell_start + (g.base + cell_x(xx, g) + cell_y(yy, g));
+        if (g.order == 1) {
+            const unsigned* c0 = r + cell_z(z0, g);
+            const unsigned* c1 = r + cell_z(z0 + 1, g);
+            const unsigned* c2 = r + cell_z(z1, g);
+            /* three cells that are not neighbours in memory: two stretches */
+            row(c0[0], c0[1] - c0[0], c1[0], c0[1] - c0[0] + c1[1] - c1[0]);
+            if (z1 - z0 == 2) row(c2[0], c2[1] - c2[0], c2[1], c2[1] - c2[0]);
+            continue;
         }
+        const unsigned s1 = r[ra], n1 = r[ra + (unsigned)(last - z0 + 1)] - s1;
+        unsigned s2 = 0, n = n1;
+        if (last < z1) {
+            s2 = r[rb];
+            n += r[rb + (unsigned)(z1 - last)] - s2;
+        }
+        row(s1, n1, s2, n);
     }
 }
 

@@ -76,24 +76,75 @@ __global__ void __launch_bounds__(256) k_ns_rank_gather(int n, const unsigned* _
     ns_rank_gather_at(p, cell_of, cell_start, tmp_key, tmp_src, g);
 }
 
-/* Neighbour lists in the reference's candidate order, filtered at |r| <= h. */
-__device__ __forceinline__ void build_lists_at(const SimParams& P, const SceneRef& S, int i,
-                                               const float4* __restrict__ pos,
-                                               const unsigned* __restrict__ cell_start,
-                                               const float4* __restrict__ bpos,
-                                               const unsigned* __restrict__ bcell_start,
-                                               const unsigned char* __restrict__ near,
-                                               unsigned* __restrict__ nbr_f, unsigned* __restrict__ cnt_f,
-                                               unsigned* __restrict__ nbr_b, unsigned* __restrict__ cnt_b,
-                                               DevState* st)
+/* What a search computes beside the lists: nothing, the densities, or the
+   densities and Tait pressures. */
+template <int MODE>
+__device__ __forceinline__ void store_density(const SimParams& P, int i, float rho, float* __restrict__ out_rho,
+                                              float* __restrict__ out_press)
 {
-    const float4 xi = pos[i];
+    if (MODE == SEARCH_LISTS) return;
+    out_rho[i] = rho;
+    if (MODE == SEARCH_EOS) out_press[i] = tait_pressure(rho, P, P.kr_g);
+}
+
+/* The n list entries out[32 k] (one thread wrote them): their density terms
+   added to rho in list order. Four are evaluated at a time, all lanes of the
+   warp together; past the end W is 0 and leaves the sum as it is. */
+template <bool BOUNDARY>
+__device__ __forceinline__ float add_density(const SimParams& P, float4 xi, const float4* __restrict__ xs,
+                                             const unsigned* out, unsigned n, float rho)
+{
+    for (unsigned k = 0; k < n; k += 4) {
+        unsigned q[4];
+        float4 x[4];
+        float w[4];
+#pragma unroll
+        for (unsigned u = 0; u < 4; ++u) q[u] = out[min(k + u, n - 1u) * 32u];
+#pragma unroll
+        for (unsigned u = 0; u < 4; ++u) x[u] = xs[q[u]];
+#pragma unroll
+        for (unsigned u = 0; u < 4; ++u)
+            w[u] = __fmul_rn(BOUNDARY ? x[u].w : P.mass,
+                             cs_W_exact(k + u < n ? dist2_exact(xi, x[u]) : 4.0f * P.h2, P));
+#pragma unroll
+        for (unsigned u = 0; u < 4; ++u) rho = __fadd_rn(rho, w[u]);
+    }
+    return rho;
+}
+
+/* Arrays of a search. */
+struct SearchArrays {
+    const float4* __restrict__ pos;
+    const unsigned* __restrict__ cell_start;
+    const float4* __restrict__ bpos;
+    const unsigned* __restrict__ bcell_start;
+    const unsigned char* __restrict__ near;
+    unsigned *nbr_f, *cnt_f, *nbr_b, *cnt_b;
+    float *rho, *press;
+    DevState* st;
+};
+
+__device__ __forceinline__ void store_counts(const SimParams& P, const SearchArrays& A, int i, unsigned nF, unsigned nB)
+{
+    A.cnt_f[i] = min(nF, P.capF);
+    A.cnt_b[i] = min(nB, P.capB);
+    if (nF > P.capF || nB > P.capB) {
+        atomicAdd(&A.st->overflow, 1u);
+        atomicOr(&A.st->err, ERRBIT_OVERFLOW);
+    }
+}
+
+/* Neighbour lists of particle i in the reference's candidate order, filtered
+   at |r| <= h, and its density (MODE), by one thread. */
+template <int MODE>
+__device__ __forceinline__ void search_at(const SimParams& P, const SceneRef& S, int i, const SearchArrays& A)
+{
+    const float4 xi = A.pos[i];
     /* |r| <= h as the reference rounds it, without the square root */
     const float s2max = P.h2_exact;
-    unsigned nF = 0, nB = 0;
     const Grid g = grid_for(P, S, (unsigned)i);
-    const auto list = [&](const unsigned* starts, const float4* xs, unsigned* out, unsigned cap, unsigned& n) {
-        unsigned m = 0; /* accepted candidates of the stretch */
+    const auto list = [&](const unsigned* starts, const float4* xs, unsigned* out, unsigned cap) {
+        unsigned m = 0, n = 0; /* accepted candidates of the stretch, of all */
         for_stretches27(
             xi, xi, P.h, g, starts, xs,
             [&](unsigned k, const float (&d)[4], unsigned) {
@@ -107,29 +158,211 @@ __device__ __forceinline__ void build_lists_at(const SimParams& P, const SceneRe
                     ++n;
                 }
             });
+        return n;
     };
-    list(cell_start, pos, nbr_f + list_index(0, P.capF, i), P.capF, nF);
-    if (boundary_near(P, near, xi, g)) list(bcell_start, bpos, nbr_b + list_index(0, P.capB, i), P.capB, nB);
-    cnt_f[i] = min(nF, P.capF);
-    cnt_b[i] = min(nB, P.capB);
-    if (nF > P.capF || nB > P.capB) {
-        atomicAdd(&st->overflow, 1u);
-        atomicOr(&st->err, ERRBIT_OVERFLOW);
-    }
+    unsigned* out_f = A.nbr_f + list_index(0, P.capF, i);
+    unsigned* out_b = A.nbr_b + list_index(0, P.capB, i);
+    const unsigned nF = list(A.cell_start, A.pos, out_f, P.capF);
+    const unsigned nB = boundary_near(P, A.near, xi, g) ? list(A.bcell_start, A.bpos, out_b, P.capB) : 0u;
+    store_counts(P, A, i, nF, nB);
+    if (MODE == SEARCH_LISTS) return;
+    float rho = add_density<false>(P, xi, A.pos, out_f, min(nF, P.capF), 0.0f);
+    rho = add_density<true>(P, xi, A.bpos, out_b, min(nB, P.capB), rho);
+    store_density<MODE>(P, i, rho, A.rho, A.press);
 }
 
-__global__ void __launch_bounds__(128) k_ns_build_lists(SimParams P, SceneRef S, const float4* __restrict__ pos,
-                                                        const unsigned* __restrict__ cell_start,
-                                                        const float4* __restrict__ bpos,
-                                                        const unsigned* __restrict__ bcell_start,
-                                                        const unsigned char* __restrict__ near,
-                                                        unsigned* __restrict__ nbr_f, unsigned* __restrict__ cnt_f,
-                                                        unsigned* __restrict__ nbr_b, unsigned* __restrict__ cnt_b,
-                                                        DevState* st)
+template <int MODE>
+__global__ void __launch_bounds__(128) k_search(SimParams P, SceneRef S, SearchArrays A)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= active_n(P, st)) return;
-    build_lists_at(P, S, i, pos, cell_start, bpos, bcell_start, near, nbr_f, cnt_f, nbr_b, cnt_b, st);
+    if (i >= active_n(P, A.st)) return;
+    search_at<MODE>(P, S, i, A);
+}
+
+/* The same search for small scenes, one warp per particle: lane k < 27 loads the
+   range of the particle's k-th cell (the reference's offset order), a warp scan
+   lays the 27 ranges end to end, and the warp then tests the concatenated
+   candidates 32 at a time; a ballot ranks each round's accepted candidates, so
+   entries are written in candidate order. The accepted squared distances (and
+   boundary weights) are collected in shared memory in that order, the kernel
+   terms evaluated by all lanes, and added one after the other. */
+constexpr int kSearchWarps = 4, kWarpBatch = 96;
+
+template <int MODE>
+__global__ void __launch_bounds__(kSearchWarps * 32) k_search_warp(SimParams P, SceneRef S, SearchArrays A)
+{
+    constexpr bool DENSITY = MODE != SEARCH_LISTS;
+    __shared__ float s_w[kSearchWarps][DENSITY ? kWarpBatch : 1], s_psi[kSearchWarps][DENSITY ? kWarpBatch : 1];
+    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    /* the whole warp shares i and leaves together */
+    if (i >= active_n(P, A.st)) return;
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const float4 xi = A.pos[i];
+    const Grid g = grid_for(P, S, (unsigned)i);
+    const bool with_boundary = boundary_near(P, A.near, xi, g);
+    unsigned s = 0, e = 0, bs = 0, be = 0;
+    if (lane < 27) {
+        const int xx = cell_coord(xi.x, P.h, g.cminx, g.dimx) + (int)lane / 9 - 1;
+        const int yy = cell_coord(xi.y, P.h, g.cminy, g.dimy) + ((int)lane / 3) % 3 - 1;
+        const int zz = cell_coord(xi.z, P.h, g.cminz, g.dimz) + (int)lane % 3 - 1;
+        if (xx >= 0 && xx < g.dimx && yy >= 0 && yy < g.dimy && zz >= 0 && zz < g.dimz) {
+            const unsigned c = cell_at(xx, yy, zz, g);
+            s = A.cell_start[c];
+            e = A.cell_start[c + 1];
+            if (with_boundary) {
+                bs = A.bcell_start[c];
+                be = A.bcell_start[c + 1];
+            }
+        }
+    }
+    float rho = 0.0f;
+    unsigned pending = 0; /* collected terms not yet in rho */
+    const auto add_terms = [&](bool boundary) {
+        __syncwarp();
+        for (unsigned k = lane; k < pending; k += 32u)
+            s_w[warp][k] = __fmul_rn(boundary ? s_psi[warp][k] : P.mass, cs_W_exact(s_w[warp][k], P));
+        __syncwarp();
+#pragma unroll 4
+        for (unsigned k = 0; k < pending; ++k) rho = __fadd_rn(rho, s_w[warp][k]);
+        __syncwarp();
+        pending = 0;
+    };
+    const auto walk = [&](const float4* xs, unsigned begin, unsigned end, unsigned* out, unsigned cap, bool boundary) {
+        const unsigned cnt = end - begin;
+        unsigned incl = cnt, n = 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (unsigned)o) incl += v;
+        }
+        const unsigned total = __shfl_sync(0xffffffffu, incl, 31);
+        const unsigned excl = incl - cnt;
+        for (unsigned u0 = 0; u0 < total; u0 += 32) {
+            const unsigned u = min(u0 + lane, total - 1u);
+            /* cell of candidate u: the number of lanes whose ranges end at or before u */
+            unsigned k = 0;
+#pragma unroll
+            for (unsigned step = 16; step >= 1; step >>= 1)
+                if (__shfl_sync(0xffffffffu, incl, k + step - 1) <= u) k += step;
+            const unsigned q = __shfl_sync(0xffffffffu, begin, k) + (u - __shfl_sync(0xffffffffu, excl, k));
+            const float4 x = xs[q];
+            const float d = dist2_exact(xi, x);
+            const bool in = u0 + lane < total && d <= P.h2_exact;
+            const unsigned bits = __ballot_sync(0xffffffffu, in);
+            const unsigned rank = (unsigned)__popc(bits & ((1u << lane) - 1u));
+            if (in && n + rank < cap) {
+                __stcs(out + (n + rank) * 32u, q);
+                if (DENSITY) {
+                    s_w[warp][pending + rank] = d;
+                    if (boundary) s_psi[warp][pending + rank] = x.w;
+                }
+            }
+            const unsigned more = (unsigned)__popc(bits), kept = min(more, cap - min(n, cap));
+            n += more;
+            if (DENSITY) {
+                pending += kept;
+                if (pending > kWarpBatch - 32u) add_terms(boundary);
+            }
+        }
+        if (DENSITY) add_terms(boundary);
+        return n;
+    };
+    const unsigned nF = walk(A.pos, s, e, A.nbr_f + list_index(0, P.capF, (unsigned)i), P.capF, false);
+    const unsigned nB = with_boundary ? walk(A.bpos, bs, be, A.nbr_b + list_index(0, P.capB, (unsigned)i), P.capB, true) : 0u;
+    if (lane != 0) return;
+    store_counts(P, A, i, nF, nB);
+    store_density<MODE>(P, i, rho, A.rho, A.press);
+}
+
+/* The one-thread search, kept out of line: what the lane groups below fall
+   back to. */
+template <int MODE>
+__device__ __noinline__ void search_out_of_line(const SimParams& P, const SceneRef& S, int i, const SearchArrays& A)
+{
+    search_at<MODE>(P, S, i, A);
+}
+
+/* The same search with four lanes per particle: the rows of cells are split
+   3, 2, 2, 2 over the lanes in candidate order, each lane collects its accepted
+   candidates and their squared distances in shared memory, the counts of the
+   lanes before it place its list entries, and the kernel terms, evaluated by
+   all four lanes, are added in list order. A particle with more than kLaneBatch
+   accepted candidates in one lane is left to search_out_of_line. */
+constexpr int kLanes = 4, kLaneBatch = 24, kLaneBlock = 128;
+
+template <int MODE>
+__global__ void __launch_bounds__(kLaneBlock) k_search_lanes(SimParams P, SceneRef S, SearchArrays A)
+{
+    static_assert(MODE != SEARCH_LISTS, "a warp or one lane builds lists alone");
+    __shared__ unsigned s_q[kLaneBatch][kLaneBlock];
+    __shared__ float s_w[kLaneBatch + 1][kLaneBlock]; /* one spare row */
+    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) / kLanes);
+    const unsigned tid = threadIdx.x, lane = tid & 31u, sub = lane % kLanes, first = lane - sub;
+    const bool on = i < active_n(P, A.st);
+    const float4 xi = on ? A.pos[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const Grid g = grid_for(P, S, on ? (unsigned)i : 0u);
+    const float s2max = P.h2_exact;
+    const int row0 = sub == 0 ? 0 : 2 * (int)sub + 1, row1 = 2 * (int)sub + 3;
+    float rho = 0.0f;
+    bool over = false;
+    /* list (and density terms) of one particle set; its length */
+    const auto set = [&](bool walk, const unsigned* starts, const float4* xs, unsigned* out, unsigned cap, bool boundary) {
+        unsigned m = 0, nq = 0, nw = 0;
+        if (walk)
+            for_stretches27(
+                xi, xi, P.h, g, starts, xs,
+                [&](unsigned k, const float (&d)[4], unsigned) {
+                    unsigned bits = 0;
+#pragma unroll
+                    for (unsigned u = 0; u < 4; ++u) {
+                        const bool in = d[u] <= s2max;
+                        bits |= in ? 1u << u : 0u;
+                        s_w[min(nw, (unsigned)kLaneBatch)][tid] = d[u]; /* written over unless kept */
+                        nw += in ? 1u : 0u;
+                    }
+                    m |= bits << k;
+                },
+                [&](auto slot) {
+                    for (; m; m &= m - 1u, ++nq) s_q[min(nq, kLaneBatch - 1u)][tid] = slot((unsigned)__ffs((int)m) - 1u);
+                },
+                row0, row1);
+        over |= ((__ballot_sync(0xffffffffu, nq > kLaneBatch) >> first) & ((1u << kLanes) - 1u)) != 0u;
+        const unsigned own = min(nq, (unsigned)kLaneBatch);
+        unsigned before = 0, total = 0;
+#pragma unroll
+        for (unsigned l = 0; l < kLanes; ++l) {
+            const unsigned c = __shfl_sync(0xffffffffu, nq, first + l);
+            before += l < sub ? c : 0u;
+            total += c;
+        }
+        for (unsigned k = 0; k < own; ++k) {
+            const unsigned q = s_q[k][tid];
+            if (!over && before + k < cap) __stcs(out + (before + k) * 32u, q);
+            s_w[k][tid] = __fmul_rn(boundary ? xs[q].w : P.mass, cs_W_exact(s_w[k][tid], P));
+        }
+        __syncwarp();
+        unsigned left = cap;
+        for (unsigned l = 0; l < kLanes; ++l) {
+            const unsigned c = min(__shfl_sync(0xffffffffu, own, first + l), left);
+            left -= c;
+            for (unsigned k = 0; k < c; ++k) rho = __fadd_rn(rho, s_w[k][tid - sub + l]);
+        }
+        __syncwarp();
+        return total;
+    };
+    const unsigned nF = set(on, A.cell_start, A.pos, A.nbr_f + list_index(0, P.capF, (unsigned)i), P.capF, false);
+    const bool near = on && boundary_near(P, A.near, xi, g);
+    unsigned nB = 0;
+    if (__any_sync(0xffffffffu, near))
+        nB = set(near, A.bcell_start, A.bpos, A.nbr_b + list_index(0, P.capB, (unsigned)i), P.capB, true);
+    __syncwarp(); /* the other lanes' list entries come before the fallback's */
+    if (!on || sub != 0) return;
+    if (over) {
+        search_out_of_line<MODE>(P, S, i, A);
+        return;
+    }
+    store_counts(P, A, i, nF, nB);
+    store_density<MODE>(P, i, rho, A.rho, A.press);
 }
 
 /* ---------------------------------------------------------------------- */
@@ -145,7 +378,8 @@ __device__ __noinline__ void build_lists_global(const SimParams& P, int i, const
                                                 unsigned* __restrict__ nbr_b, unsigned* __restrict__ cnt_b,
                                                 DevState* st)
 {
-    build_lists_at(P, SceneRef{}, i, pos, cell_start, bpos, bcell_start, near, nbr_f, cnt_f, nbr_b, cnt_b, st);
+    search_at<SEARCH_LISTS>(P, SceneRef{}, i, SearchArrays{pos, cell_start, bpos, bcell_start, near, nbr_f, cnt_f, nbr_b,
+                                                           cnt_b, nullptr, nullptr, st});
 }
 
 /* Fluid particles of one brick's 6 x 6 x 6-cell halo that fit in shared
@@ -160,7 +394,7 @@ constexpr int kStagedBlock = 256;
    warp per cell, coalesced), then every thread walks its particles' 27 cells
    in the reference's offset order over the staged copies: the same
    candidates in the same order, the same exact test, the same global slot
-   ids written, so the lists equal k_ns_build_lists's entry for entry. */
+   ids written, so the lists equal k_search's entry for entry. */
 __global__ void __launch_bounds__(kStagedBlock) k_ns_build_lists_staged(
     SimParams P, const float4* __restrict__ pos, const unsigned* __restrict__ cell_start,
     const float4* __restrict__ bpos, const unsigned* __restrict__ bcell_start, const unsigned char* __restrict__ near,
@@ -271,22 +505,6 @@ __global__ void __launch_bounds__(kStagedBlock) k_ns_build_lists_staged(
     }
 }
 
-__global__ void __launch_bounds__(128) k_ns_build_lists_warp(SimParams P, SceneRef S,
-                                                             const float4* __restrict__ pos,
-                                                             const unsigned* __restrict__ cell_start,
-                                                             const float4* __restrict__ bpos,
-                                                             const unsigned* __restrict__ bcell_start,
-                                                             const unsigned char* __restrict__ near,
-                                                             unsigned* __restrict__ nbr_f, unsigned* __restrict__ cnt_f,
-                                                             unsigned* __restrict__ nbr_b, unsigned* __restrict__ cnt_b,
-                                                             DevState* st)
-{
-    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    /* the whole warp shares i and leaves together */
-    if (i >= active_n(P, st)) return;
-    build_lists_warp_at(P, S, i, pos, cell_start, bpos, bcell_start, near, nbr_f, cnt_f, nbr_b, cnt_b, st);
-}
-
 /* Akinci boundary volume V_b = 1 / sum_b' W(x_b - x_b') over the 27 cells
    (AkinciBoundaryObject.cpp:10-34); k_boundary_psi then stores
    psi = rho0 V_b in bpos.w for the fluid kernels. */
@@ -376,29 +594,57 @@ void launch_sort(const SimParams& P, const SceneRef& S, int n, const float4* pos
     k_ns_rank_gather<<<blocks_for(n, 256), 256, 0, s>>>(n, cell_of, cell_start, tmp_key, tmp_src, g);
 }
 
-void launch_build_lists(const SimParams& P, const SceneRef& S, const float4* pos, const unsigned* cell_start,
-                        const float4* bpos,
-                        const unsigned* bcell_start, const unsigned char* near, unsigned* nbr_f, unsigned* cnt_f, unsigned* nbr_b,
-                        unsigned* cnt_b, DevState* st, cudaStream_t s, bool staged)
+/* Which search. A warp per particle in the smallest scenes, where one lane's
+   walk over ~216 candidates is the critical path (1k WCSPH step 34.7 -> 26.8 us
+   with the densities in it, 8k 40.2 -> 36.0); four lanes per particle up to
+   where one lane each fills the GPU (33k WCSPH step 59.1 us, one lane 62.7, a
+   warp 69.4); then one lane, whose instructions are the fewest (64k 80 us, four
+   lanes 96, a warp 118). Lists alone (DFSPH): a warp up to the second line (33k
+   DFSPH step 188 us, one lane 190, four lanes 199). */
+constexpr int kSearchWarpMax = 1 << 14, kSearchLanesMax = 3 << 14;
+/* Densities in the search kernel up to here: with more particles the lists and
+   positions a thread has just walked have left the caches when it comes back
+   for its density terms, and a second kernel is the faster one (125k 58 us
+   against 42 + 27, 216k 86 against 61 + 29; 1M 333 against 209 + 85). */
+constexpr int kSearchDensityMax = 1 << 18;
+
+template <int MODE>
+static void search_mode(const SimParams& P, const SceneRef& S, const SearchArrays& A, cudaStream_t s)
 {
-    if (P.nf <= 0) return;
+    if (P.nf < (MODE == SEARCH_LISTS ? kSearchLanesMax : kSearchWarpMax)) {
+        k_search_warp<MODE><<<blocks_for(P.nf, kSearchWarps), kSearchWarps * 32, 0, s>>>(P, S, A);
+        return;
+    }
+    if constexpr (MODE != SEARCH_LISTS)
+        if (P.nf < kSearchLanesMax) {
+            k_search_lanes<MODE><<<blocks_for((long long)P.nf * kLanes, kLaneBlock), kLaneBlock, 0, s>>>(P, S, A);
+            return;
+        }
+    k_search<MODE><<<blocks_for(P.nf, 128), 128, 0, s>>>(P, S, A);
+}
+
+bool launch_search(const SimParams& P, const SceneRef& S, const DeviceArrays& D, int mode, cudaStream_t s, bool staged)
+{
+    if (P.nf <= 0) return true;
+    const SearchArrays A{D.pos, D.cell_start, D.bpos, D.bcell_start, D.near, D.nbr_f, D.cnt_f, D.nbr_b,
+                         D.cnt_b, D.rho, D.press, D.st};
     if (staged && !S.scenes && P.cell_order == 0 && P.nf >= (1 << 16)) {
         /* one block per brick; bricks without fluid leave at once */
         const int nbricks = P.nbx * P.nby * (P.dimz / 4);
-        k_ns_build_lists_staged<<<nbricks, kStagedBlock, 0, s>>>(P, pos, cell_start, bpos, bcell_start, near, nbr_f, cnt_f,
-                                                                  nbr_b, cnt_b, st);
-        return;
+        k_ns_build_lists_staged<<<nbricks, kStagedBlock, 0, s>>>(P, A.pos, A.cell_start, A.bpos, A.bcell_start, A.near,
+                                                                  A.nbr_f, A.cnt_f, A.nbr_b, A.cnt_b, A.st);
+        return false;
     }
-    /* A warp per particle below 2^16 particles, where one lane's serial walk
-       over ~216 candidates is the critical path (32k: 32 vs 56 us per build);
-       one lane per particle above, where the particles fill the GPU and the
-       warp's extra instructions cost more (125k: 0.069 vs 0.096 ms). */
-    if (P.nf < (1 << 16))
-        k_ns_build_lists_warp<<<blocks_for((long long)P.nf * 32, 128), 128, 0, s>>>(
-            P, S, pos, cell_start, bpos, bcell_start, near, nbr_f, cnt_f, nbr_b, cnt_b, st);
-    else
-        k_ns_build_lists<<<blocks_for(P.nf, 128), 128, 0, s>>>(P, S, pos, cell_start, bpos, bcell_start, near, nbr_f,
-                                                                cnt_f, nbr_b, cnt_b, st);
+    if (P.nf >= kSearchDensityMax) {
+        search_mode<SEARCH_LISTS>(P, S, A, s);
+        return mode == SEARCH_LISTS;
+    }
+    switch (mode) {
+    case SEARCH_DENSITY: search_mode<SEARCH_DENSITY>(P, S, A, s); break;
+    case SEARCH_EOS: search_mode<SEARCH_EOS>(P, S, A, s); break;
+    default: search_mode<SEARCH_LISTS>(P, S, A, s); break;
+    }
+    return true;
 }
 
 /* near[c] = 1 for every cell c with a boundary particle in the 27 cells

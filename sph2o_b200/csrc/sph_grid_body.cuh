@@ -1,7 +1,6 @@
 /*
  * Per-particle bodies of the neighbour search (sph_grid.cu): the counting
- * sort's count, scatter and rank + gather steps and the small-scene list
- * build (a warp per particle), kept apart from their kernels (one thread or
+ * sort's count, scan, scatter and rank + gather steps, kept apart from their kernels (one thread or
  * warp per index) so that other kernels can run the same steps on their own
  * index ranges, and the GatherSet the sort moves state with.
  */
@@ -134,92 +133,12 @@ __device__ __forceinline__ void ns_rank_gather_at(int p, const unsigned* __restr
     if (g.f_in[1]) g.f_out[1][dst] = g.f_in[1][src];
 }
 
-/* The same lists for small scenes, one warp per particle: lane k < 27 loads
-   the range of the particle's k-th cell (the reference's offset order), a
-   warp scan lays the 27 ranges end to end, and the warp then tests the
-   concatenated candidates 32 at a time; a ballot ranks each round's accepted
-   candidates, so entries are written in candidate order. The serial walk of a
-   particle shrinks from ~216 candidates (or 27 cells) to ~7 rounds. */
-__device__ __forceinline__ void warp_candidates(const float4* __restrict__ xs, unsigned s, unsigned e, float4 xi,
-                                                float s2max, unsigned lane, unsigned cap, unsigned* __restrict__ list,
-                                                int i, unsigned& n)
-{
-    const unsigned cnt = e - s;
-    unsigned incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= (unsigned)o) incl += v;
-    }
-    const unsigned total = __shfl_sync(0xffffffffu, incl, 31);
-    const unsigned excl = incl - cnt;
-    for (unsigned u0 = 0; u0 < total; u0 += 32) {
-        const unsigned u = min(u0 + lane, total - 1u);
-        /* cell of candidate u: the number of lanes whose ranges end at or before u */
-        unsigned k = 0;
-#pragma unroll
-        for (unsigned step = 16; step >= 1; step >>= 1)
-            if (__shfl_sync(0xffffffffu, incl, k + step - 1) <= u) k += step;
-        const unsigned q = __shfl_sync(0xffffffffu, s, k) + (u - __shfl_sync(0xffffffffu, excl, k));
-        const bool in = u0 + lane < total && dist2_exact(xi, xs[q]) <= s2max;
-        const unsigned bits = __ballot_sync(0xffffffffu, in);
-        if (in) {
-            const unsigned r = n + __popc(bits & ((1u << lane) - 1u));
-            if (r < cap) __stcs(list + list_index(r, cap, i), q);
-        }
-        n += __popc(bits);
-    }
-}
-
 /* Whether x's cell has boundary particles among its 27 cells (near: see
    k_mark_near). */
 __device__ __forceinline__ bool boundary_near(const SimParams& P, const unsigned char* __restrict__ near, float4 x,
                                               const Grid& g)
 {
     return P.nb > 0 && near[cell_index(x, P.h, g)] != 0;
-}
-
-/* The lists of particle i, built by the whole warp (every lane calls with
-   the same i). */
-__device__ __forceinline__ void build_lists_warp_at(const SimParams& P, const SceneRef& S, int i,
-                                                    const float4* __restrict__ pos,
-                                                    const unsigned* __restrict__ cell_start,
-                                                    const float4* __restrict__ bpos,
-                                                    const unsigned* __restrict__ bcell_start,
-                                                    const unsigned char* __restrict__ near,
-                                                    unsigned* __restrict__ nbr_f, unsigned* __restrict__ cnt_f,
-                                                    unsigned* __restrict__ nbr_b, unsigned* __restrict__ cnt_b,
-                                                    DevState* st)
-{
-    const unsigned lane = threadIdx.x & 31u;
-    const float4 xi = pos[i];
-    const Grid g = grid_for(P, S, (unsigned)i);
-    unsigned s = 0, e = 0, bs = 0, be = 0;
-    const bool with_boundary = boundary_near(P, near, xi, g);
-    if (lane < 27) {
-        const int xx = cell_coord(xi.x, P.h, g.cminx, g.dimx) + (int)lane / 9 - 1;
-        const int yy = cell_coord(xi.y, P.h, g.cminy, g.dimy) + ((int)lane / 3) % 3 - 1;
-        const int zz = cell_coord(xi.z, P.h, g.cminz, g.dimz) + (int)lane % 3 - 1;
-        if (xx >= 0 && xx < g.dimx && yy >= 0 && yy < g.dimy && zz >= 0 && zz < g.dimz) {
-            const unsigned c = cell_at(xx, yy, zz, g);
-            s = cell_start[c];
-            e = cell_start[c + 1];
-            if (with_boundary) {
-                bs = bcell_start[c];
-                be = bcell_start[c + 1];
-            }
-        }
-    }
-    unsigned nF = 0, nB = 0;
-    warp_candidates(pos, s, e, xi, P.h2_exact, lane, P.capF, nbr_f, i, nF);
-    if (with_boundary) warp_candidates(bpos, bs, be, xi, P.h2_exact, lane, P.capB, nbr_b, i, nB);
-    if (lane != 0) return;
-    cnt_f[i] = min(nF, P.capF);
-    cnt_b[i] = min(nB, P.capB);
-    if (nF > P.capF || nB > P.capB) {
-        atomicAdd(&st->overflow, 1u);
-        atomicOr(&st->err, ERRBIT_OVERFLOW);
-    }
 }
 
 } // namespace sph

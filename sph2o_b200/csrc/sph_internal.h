@@ -37,10 +37,10 @@ struct DeviceArrays {
     const float4* bpos;
     const unsigned* bcell_start;
     const unsigned char* near;     /* per cell: boundary particles among its 27 cells */
-    const unsigned* nbr_f;
-    const unsigned* cnt_f;
-    const unsigned* nbr_b;
-    const unsigned* cnt_b;
+    unsigned* nbr_f;
+    unsigned* cnt_f;
+    unsigned* nbr_b;
+    unsigned* cnt_b;
     /* DFSPH: the lists with each entry's kernel factor, (slot, bits of f with
        gradW = f r), in the layout of nbr_f / nbr_b (see k_density) */
     uint2* pair_f;
@@ -77,10 +77,12 @@ void launch_sort(const SimParams& P, const SceneRef& S, int n, const float4* pos
                  unsigned* cell_start,
                  unsigned* chunk_sums, unsigned* cell_of, unsigned* slot, unsigned* tmp_key, unsigned* tmp_src,
                  const unsigned* orig_in, const GatherSet& g, cudaStream_t s);
-void launch_build_lists(const SimParams& P, const SceneRef& S, const float4* pos, const unsigned* cell_start,
-                        const float4* bpos,
-                        const unsigned* bcell_start, const unsigned char* near, unsigned* nbr_f, unsigned* cnt_f, unsigned* nbr_b,
-                        unsigned* cnt_b, DevState* st, cudaStream_t s, bool staged = false);
+/* Neighbour lists at D.pos and, by `mode`, the densities and Tait pressures of
+   the same particles in the same kernel. False when only the lists were built
+   (the staged build) and the densities are left to launch_density. */
+enum SearchMode : int { SEARCH_LISTS = 0, SEARCH_DENSITY = 1, SEARCH_EOS = 2 };
+bool launch_search(const SimParams& P, const SceneRef& S, const DeviceArrays& D, int mode, cudaStream_t s,
+                   bool staged = false);
 void launch_boundary_volume(const SimParams& P, const SceneRef& S, float4* bpos, const unsigned* bcell_start,
                             float* bvol, cudaStream_t s);
 /* cells with boundary particles around them (near: ncells bytes, zeroed by the caller) */

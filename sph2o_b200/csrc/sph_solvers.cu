@@ -257,51 +257,6 @@ __global__ void __launch_bounds__(256) k_pair_factors(SimParams P, DeviceArrays 
     }
 }
 
-/* Density (and the Tait pressure when EOS) of small scenes with TPP lanes per
-   particle: in each round the group's lanes evaluate m W for TPP consecutive
-   list entries, and lane 0 adds the TPP terms in list order (shuffled to
-   it), so the sum is the sequential one bit for bit; the terms of entries
-   past the end are +0, which leaves a non-negative sum unchanged. */
-template <bool EOS, int TPP>
-__device__ __forceinline__ void density_lanes_at(const SimParams& P, const DeviceArrays& A, int t)
-{
-    const int i = t / TPP;
-    /* a group's lanes share i, so a group leaves together */
-    if (i >= active_n(P, A.st)) return;
-    const unsigned lane = threadIdx.x & 31u, sub = lane % TPP, first = lane - sub;
-    const unsigned gmask = ((1u << TPP) - 1u) << first;
-    const float4 xi = A.pos[i];
-    float rho = 0.0f;
-    const unsigned nF = A.cnt_f[i];
-    for (unsigned k0 = 0; k0 < nF; k0 += TPP) {
-        const unsigned kk = k0 + sub;
-        float w = 0.0f;
-        if (kk < nF) w = __fmul_rn(P.mass, cs_W_exact(dist2_exact(xi, A.pos[list_at(A.nbr_f, kk, P.capF, i)]), P));
-#pragma unroll
-        for (int l = 0; l < TPP; ++l) rho = __fadd_rn(rho, __shfl_sync(gmask, w, first + l));
-    }
-    const unsigned nB = A.cnt_b[i];
-    for (unsigned k0 = 0; k0 < nB; k0 += TPP) {
-        const unsigned kk = k0 + sub;
-        float w = 0.0f;
-        if (kk < nB) {
-            const float4 xb = A.bpos[list_at(A.nbr_b, kk, P.capB, i)];
-            w = __fmul_rn(xb.w, cs_W_exact(dist2_exact(xi, xb), P));
-        }
-#pragma unroll
-        for (int l = 0; l < TPP; ++l) rho = __fadd_rn(rho, __shfl_sync(gmask, w, first + l));
-    }
-    if (sub != 0) return;
-    A.rho[i] = rho;
-    if (EOS) A.press[i] = tait_pressure(rho, P, P.kr_g);
-}
-
-template <bool EOS, int TPP>
-__global__ void __launch_bounds__(256) k_density_lanes(SimParams P, DeviceArrays A)
-{
-    density_lanes_at<EOS, TPP>(P, A, blockIdx.x * blockDim.x + threadIdx.x);
-}
-
 __global__ void __launch_bounds__(256, 8) k_normals(SimParams P, DeviceArrays A)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1537,10 +1492,9 @@ int launch_barrier_timeout_probe(DevState* st, cudaStream_t s)
 
 static inline int blocks_for(long long n, int bs) { return (int)((n + bs - 1) / bs); }
 
-/* Lanes per particle for the WCSPH density and force passes: 4 below 2^16
-   particles, where one lane per particle leaves most of the GPU idle and its
-   serial neighbour walk is the critical path (32k particles: forces 42.8 ->
-   18.4 us, density 25 -> 14 us); one lane above. */
+/* Lanes per particle for the WCSPH force pass: 4 below 2^16 particles, where one
+   lane per particle leaves most of the GPU idle and its serial neighbour walk is
+   the critical path (32k particles: 42.8 -> 18.4 us); one lane above. */
 static int small_scene_lanes(int n)
 {
     return n < (1 << 16) ? 4 : 1;
@@ -1553,11 +1507,6 @@ void launch_density(const SimParams& P, const DeviceArrays& A, bool alpha, bool 
     if (alpha && eos) k_density<true, true><<<g, block, 0, s>>>(P, A);
     else if (alpha && A.divres) k_density<true, false, true><<<g, block, 0, s>>>(P, A);
     else if (alpha) k_density<true, false><<<g, block, 0, s>>>(P, A);
-    else if (small_scene_lanes(P.nf) > 1) {
-        const int gl = blocks_for((long long)P.nf * 4, block);
-        if (eos) k_density_lanes<true, 4><<<gl, block, 0, s>>>(P, A);
-        else k_density_lanes<false, 4><<<gl, block, 0, s>>>(P, A);
-    }
     else if (eos) k_density<false, true><<<g, block, 0, s>>>(P, A);
     else k_density<false, false><<<g, block, 0, s>>>(P, A);
 }
