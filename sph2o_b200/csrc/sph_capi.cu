@@ -128,7 +128,7 @@ struct sph_ctx {
     float4 *plo = nullptr, *plo2 = nullptr;
     float4* snap_plo = nullptr;
     float* divres = nullptr;  /* DFSPH: divergence error of the density pass */
-    float4* rec = nullptr;    /* DFSPH: the solvers' working records (DeviceArrays::rec) */
+    float4* rec = nullptr;    /* DeviceArrays::rec */
     /* autotune snapshot */
     float4 *snap_pos = nullptr, *snap_vel = nullptr;
     unsigned* snap_orig = nullptr;
@@ -1092,8 +1092,8 @@ int sph_init(sph_ctx* c)
     if ((rc = alloc_lists(c)) != SPH_OK) return rc;
     if (c->desc.simulation_method == SPH_DFSPH) {
         if ((rc = dalloc(c, &c->divres, nf)) != SPH_OK) return rc;
-        if ((rc = dalloc(c, &c->rec, 2 * nf)) != SPH_OK) return rc;
     }
+    if ((rc = dalloc(c, &c->rec, 2 * nf)) != SPH_OK) return rc;
     if (c->pos_lo) {
         if (c->nscenes) return fail(c, SPH_ERR_ARG, "position residuals apply to single scenes, not to batches");
         if ((rc = dalloc(c, &c->plo, nf)) != SPH_OK) return rc;
@@ -1372,6 +1372,8 @@ int sph_set_state(sph_ctx* c, const float* xyz, const float* v)
         /* DFSPH keeps densities/alpha of the current positions between steps */
         rc = neighbor_search(c);
         if (rc == SPH_OK) launch_density(c->P, arrays(c), true, false, c->pass_block, c->stream);
+    } else if (v && c->desc.simulation_method == SPH_DFSPH) {
+        launch_pair_factors(c->P, arrays(c), c->stream); /* the records carry the velocities */
     }
     /* one wait: the caller's arrays have been read and the search has run */
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));

@@ -553,6 +553,13 @@ __device__ __forceinline__ unsigned list_at(const unsigned* list, unsigned kk, u
     return __ldcs(list + list_index(kk, cap, (unsigned)i));
 }
 
+/* Record i of DeviceArrays::rec: (x, w0), (v, w1). */
+__device__ __forceinline__ void store_rec(float4* rec, int i, float4 x, float w0, float4 v, float w1)
+{
+    rec[2 * (size_t)i] = make_float4(x.x, x.y, x.z, w0);
+    rec[2 * (size_t)i + 1] = make_float4(v.x, v.y, v.z, w1);
+}
+
 /* ---------------------------------------------------------------------- */
 /* Reductions                                                               */
 

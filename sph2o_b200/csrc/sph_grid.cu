@@ -76,17 +76,6 @@ __global__ void __launch_bounds__(256) k_ns_rank_gather(int n, const unsigned* _
     ns_rank_gather_at(p, cell_of, cell_start, tmp_key, tmp_src, g);
 }
 
-/* What a search computes beside the lists: nothing, the densities, or the
-   densities and Tait pressures. */
-template <int MODE>
-__device__ __forceinline__ void store_density(const SimParams& P, int i, float rho, float* __restrict__ out_rho,
-                                              float* __restrict__ out_press)
-{
-    if (MODE == SEARCH_LISTS) return;
-    out_rho[i] = rho;
-    if (MODE == SEARCH_EOS) out_press[i] = tait_pressure(rho, P, P.kr_g);
-}
-
 /* The n list entries out[32 k] (one thread wrote them): their density terms
    added to rho in list order. Four are evaluated at a time, all lanes of the
    warp together; past the end W is 0 and leaves the sum as it is. */
@@ -121,8 +110,26 @@ struct SearchArrays {
     const unsigned char* __restrict__ near;
     unsigned *nbr_f, *cnt_f, *nbr_b, *cnt_b;
     float *rho, *press;
+    const float4* __restrict__ vel;
+    float4* rec;
     DevState* st;
 };
+
+/* What a search computes beside the lists: nothing, or the densities, the Tait
+   pressures (EOS) and the records that the force pass reads. */
+template <int MODE>
+__device__ __forceinline__ void store_density(const SimParams& P, const SearchArrays& A, int i, float4 xi, float rho)
+{
+    if (MODE == SEARCH_LISTS) return;
+    A.rho[i] = rho;
+    float dp = 0.0f;
+    if (MODE == SEARCH_EOS) {
+        const float p = tait_pressure(rho, P, P.kr_g);
+        A.press[i] = p;
+        dp = p / (rho * rho);
+    }
+    store_rec(A.rec, i, xi, rho, A.vel[i], dp);
+}
 
 __device__ __forceinline__ void store_counts(const SimParams& P, const SearchArrays& A, int i, unsigned nF, unsigned nB)
 {
@@ -168,7 +175,7 @@ __device__ __forceinline__ void search_at(const SimParams& P, const SceneRef& S,
     if (MODE == SEARCH_LISTS) return;
     float rho = add_density<false>(P, xi, A.pos, out_f, min(nF, P.capF), 0.0f);
     rho = add_density<true>(P, xi, A.bpos, out_b, min(nB, P.capB), rho);
-    store_density<MODE>(P, i, rho, A.rho, A.press);
+    store_density<MODE>(P, A, i, xi, rho);
 }
 
 template <int MODE>
@@ -271,7 +278,7 @@ __global__ void __launch_bounds__(kSearchWarps * 32) k_search_warp(SimParams P, 
     const unsigned nB = with_boundary ? walk(A.bpos, bs, be, A.nbr_b + list_index(0, P.capB, (unsigned)i), P.capB, true) : 0u;
     if (lane != 0) return;
     store_counts(P, A, i, nF, nB);
-    store_density<MODE>(P, i, rho, A.rho, A.press);
+    store_density<MODE>(P, A, i, xi, rho);
 }
 
 /* The one-thread search, kept out of line: what the lane groups below fall
@@ -362,7 +369,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_search_lanes(SimParams P, SceneR
         return;
     }
     store_counts(P, A, i, nF, nB);
-    store_density<MODE>(P, i, rho, A.rho, A.press);
+    store_density<MODE>(P, A, i, xi, rho);
 }
 
 /* ---------------------------------------------------------------------- */
@@ -379,7 +386,7 @@ __device__ __noinline__ void build_lists_global(const SimParams& P, int i, const
                                                 DevState* st)
 {
     search_at<SEARCH_LISTS>(P, SceneRef{}, i, SearchArrays{pos, cell_start, bpos, bcell_start, near, nbr_f, cnt_f, nbr_b,
-                                                           cnt_b, nullptr, nullptr, st});
+                                                           cnt_b, nullptr, nullptr, nullptr, nullptr, st});
 }
 
 /* Fluid particles of one brick's 6 x 6 x 6-cell halo that fit in shared
@@ -627,7 +634,7 @@ bool launch_search(const SimParams& P, const SceneRef& S, const DeviceArrays& D,
 {
     if (P.nf <= 0) return true;
     const SearchArrays A{D.pos, D.cell_start, D.bpos, D.bcell_start, D.near, D.nbr_f, D.cnt_f, D.nbr_b,
-                         D.cnt_b, D.rho, D.press, D.st};
+                         D.cnt_b, D.rho, D.press, D.vel, D.rec, D.st};
     if (staged && !S.scenes && P.cell_order == 0 && P.nf >= (1 << 16)) {
         /* one block per brick; bricks without fluid leave at once */
         const int nbricks = P.nbx * P.nby * (P.dimz / 4);

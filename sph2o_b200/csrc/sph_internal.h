@@ -45,8 +45,9 @@ struct DeviceArrays {
        gradW = f r), in the layout of nbr_f / nbr_b (see k_density) */
     uint2* pair_f;
     uint2* pair_b;
-    /* DFSPH solvers' working state, two float4 per particle: (x, y, z, k) and
-       (vx, vy, vz, 0), so a neighbour's half or whole record is one load */
+    /* two float4 per particle, so that half or all of a neighbour's record is one
+       load: (x, y, z, rho), (vx, vy, vz, p / rho^2 in WCSPH) for the force and
+       normal passes, with k in the place of rho inside the DFSPH solvers */
     float4* rec;
     unsigned* orig_w;     /* caller-order ids of the sorted slots (emitters write new ones) */
     double* accum;        /* per-iteration residual accumulators, zeroed per solve */
@@ -105,8 +106,8 @@ enum ForceMode : int {
 
 /* block: threads per block of the pass kernels (128 or 256, autotuned) */
 void launch_density(const SimParams& P, const DeviceArrays& A, bool alpha, bool eos, int block, cudaStream_t s);
-/* pair_f / pair_b from the current lists and positions, where a list build is
-   not followed by the density pass that writes them */
+/* DFSPH: pair_f / pair_b and the records from the current lists, positions and
+   velocities, where no density pass follows that writes them */
 void launch_pair_factors(const SimParams& P, const DeviceArrays& A, cudaStream_t s);
 void launch_normals(const SimParams& P, const DeviceArrays& A, int block, cudaStream_t s);
 void launch_forces(const SimParams& P, const DeviceArrays& A, int mode, int block, cudaStream_t s);

@@ -81,6 +81,43 @@ __device__ __forceinline__ void for_fluid_neighbors(const SimParams& P, const De
     }
 }
 
+/* Record j of DeviceArrays::rec, both halves with one 256-bit load. */
+__device__ __forceinline__ void load_rec(const float4* rec, unsigned j, float4& a, float4& b)
+{
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(rec + 2 * (size_t)j)
+                 : "memory");
+}
+
+/* for_fluid_neighbors over the records: f(place, j, (x_j, w), (v_j, w)) with
+   the entry's place: 0 even or 1 odd in an unrolled round, 2 after the rounds. */
+template <int U, int TPP, typename F>
+__device__ __forceinline__ void for_fluid_records(const SimParams& P, const DeviceArrays& A, int i, unsigned n, F&& f,
+                                                  unsigned sub)
+{
+    unsigned kk = sub;
+    for (; kk + (U - 1) * TPP < n; kk += U * TPP) {
+        unsigned jj[U];
+        float4 a[U], b[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) jj[u] = list_at(A.nbr_f, kk + u * TPP, P.capF, i);
+#pragma unroll
+        for (int u = 0; u < U; ++u) load_rec(A.rec, jj[u], a[u], b[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (u % 2 == 0) f(std::integral_constant<int, 0>(), jj[u], a[u], b[u]);
+            else f(std::integral_constant<int, 1>(), jj[u], a[u], b[u]);
+        }
+    }
+    for (; kk < n; kk += TPP) {
+        const unsigned j = list_at(A.nbr_f, kk, P.capF, i);
+        float4 a, b;
+        load_rec(A.rec, j, a, b);
+        f(std::integral_constant<int, 2>(), j, a, b);
+    }
+}
+
 /* Sum over the TPP adjacent lanes of a particle's lane group. */
 template <int TPP>
 __device__ __forceinline__ float group_sum(float v)
@@ -228,18 +265,19 @@ __global__ void __launch_bounds__(256, 8) k_density(SimParams P, DeviceArrays A)
         const float denom = ((sgx * sgx + sgy * sgy) + sgz * sgz) + ssq;
         A.alpha[i] = denom > P.eps ? rho / denom : 0.0f;
     }
-    if (EOS) A.press[i] = tait_pressure(rho, P, P.kr_g);
-    /* fewer than 20 neighbours within h: no correction (DFSPHSolver.cpp:608-611) */
-    if (DIVRES) {
-        A.divres[i] = (nF + nB < 20u) ? 0.0f : fmaxf(div, 0.0f);
-        /* the divergence solver's record */
-        A.rec[2 * (size_t)i] = make_float4(xi.x, xi.y, xi.z, 0.0f);
-        A.rec[2 * (size_t)i + 1] = vi;
+    float dp = 0.0f;
+    if (EOS) {
+        const float p = tait_pressure(rho, P, P.kr_g);
+        A.press[i] = p;
+        dp = p / (rho * rho);
     }
+    store_rec(A.rec, i, xi, rho, DIVRES ? vi : A.vel[i], dp);
+    /* fewer than 20 neighbours within h: no correction (DFSPHSolver.cpp:608-611) */
+    if (DIVRES) A.divres[i] = (nF + nB < 20u) ? 0.0f : fmaxf(div, 0.0f);
 }
 
-/* What the density pass writes into pair_f / pair_b, alone: after a list
-   build that no density pass follows. */
+/* What the density pass writes into pair_f / pair_b and the records, alone:
+   after a list build, or new velocities, that no density pass follows. */
 __global__ void __launch_bounds__(256) k_pair_factors(SimParams P, DeviceArrays A)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -255,26 +293,67 @@ __global__ void __launch_bounds__(256) k_pair_factors(SimParams P, DeviceArrays 
         const Pair p = make_pair(xi, A.bpos[bq]);
         __stcs(A.pair_b + list_index(kk, P.capB, i), make_uint2(bq, __float_as_uint(cs_gradf(p.rl, p.inv_rl, P))));
     }
+    store_rec(A.rec, i, xi, A.rho[i], A.vel[i], 0.0f);
 }
 
-__global__ void __launch_bounds__(256, 8) k_normals(SimParams P, DeviceArrays A)
+/* cs_gradf with every operation written out; FUSED: 1 - q in one operation from
+   |r|. */
+template <bool FUSED>
+__device__ __forceinline__ float cs_gradf_as(float rl, float inv_rl, const SimParams& P)
+{
+    const float q = __fmul_rn(rl, P.inv_h);
+    if (!(rl > 1.0e-9f) || q > 1.0f) return 0.0f;
+    if (q <= 0.5f) return __fmul_rn(P.cs_l_h2, __fmaf_rn(3.0f, q, -2.0f));
+    const float t = FUSED ? __fmaf_rn(-rl, P.inv_h, 1.0f) : __fsub_rn(1.0f, q);
+    return __fmul_rn(__fmul_rn(-P.cs_l_h, __fmul_rn(t, t)), inv_rl);
+}
+
+/* cs_W of |r| with every operation written out. */
+__device__ __forceinline__ float cs_W_fused(float rl, const SimParams& P)
+{
+    const float q = __fmul_rn(rl, P.inv_h);
+    if (q <= 0.5f) {
+        const float q2 = __fmul_rn(q, q);
+        return __fmul_rn(P.cs_k, __fadd_rn(__fmaf_rn(6.0f, __fmul_rn(q2, q), -__fmul_rn(6.0f, q2)), 1.0f));
+    }
+    const float t = fmaxf(__fmaf_rn(-rl, P.inv_h, 1.0f), 0.0f);
+    return __fmul_rn(P.cs_k, __fmul_rn(2.0f, __fmul_rn(__fmul_rn(t, t), t)));
+}
+
+__global__ void __launch_bounds__(256, 4) k_normals(SimParams P, DeviceArrays A)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= active_n(P, A.st)) return;
     const float4 xi = A.pos[i];
     float nx = 0.0f, ny = 0.0f, nz = 0.0f;
     const unsigned nF = A.cnt_f[i];
-    for (unsigned kk = 0; kk < nF; ++kk) {
-        const unsigned j = list_at(A.nbr_f, kk, P.capF, i);
-        const Pair p = make_pair(xi, A.pos[j]);
-        const float f = (P.mass / A.rho[j]) * cs_gradf(p.rl, p.inv_rl, P);
+    const auto term = [&](const float4& xj) {
+        const Pair p = make_pair(xi, xj);
+        const float f = (P.mass / xj.w) * cs_gradf_as<false>(p.rl, p.inv_rl, P);
         nx += f * p.rx; ny += f * p.ry; nz += f * p.rz;
+    };
+    unsigned kk = 0;
+    for (; kk + 4 <= nF; kk += 4) {
+        unsigned jj[4];
+        float4 xj[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) jj[u] = list_at(A.nbr_f, kk + u, P.capF, i);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) xj[u] = A.rec[2 * (size_t)jj[u]];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) term(xj[u]);
     }
+    for (; kk < nF; ++kk) term(A.rec[2 * (size_t)list_at(A.nbr_f, kk, P.capF, i)]);
     A.normal[i] = make_float4(nx * P.h, ny * P.h, nz * P.h, 0.0f);
 }
 
-/* Non-pressure and pressure accelerations (MODE). TPP adjacent lanes share
-   particle i (small scenes), each summing the list entries sub, sub + TPP,
+/* Non-pressure and pressure accelerations (MODE). A neighbour comes as one
+   256-bit record (position and density | velocity and p / rho^2): gathered one
+   by one they are four loads and a division per pair, and the pass is bound by
+   the L1's rate for scattered gathers (69 % of its wavefronts) and their
+   latency. Records, and 64 registers so that nothing is spilled: 306k with
+   standard viscosity, surface tension and adhesion 134 -> 88 us, 64 batched
+   scenes 164 -> 122, 125k DFSPH 48 -> 34. TPP adjacent lanes share particle i (small scenes), each summing the list entries sub, sub + TPP,
    ...; the group's sums are combined by shuffles and lane 0 of the group
    finishes the particle. */
 template <int MODE, int TPP = 1>
@@ -300,35 +379,44 @@ __device__ __forceinline__ void forces_at(const SimParams& P, const DeviceArrays
         const bool np = MODE != FORCE_PRESSURE;
         const int vm = np ? P.visc_method : -1;
         const bool st_on = np && P.st_on;
-        const float dpi = pressure ? A.press[i] / (rho_i * rho_i) : 0.0f;
+        const float dpi = pressure ? A.press[i] / (rho_i * rho_i) : 0.0f; /* as the records hold it */
         const float dpb = pressure ? A.press[i] / (P.rho0 * P.rho0) : 0.0f;
         const float4 ni = st_on ? A.normal[i] : make_float4(0, 0, 0, 0);
         const float eps_h2 = 0.01f * P.h2;
+        /* Which of its two roundings 1 - q takes, by the entry's place: DFSPH and
+           PCISPH amplify a last bit of these accelerations over a few steps (a
+           solver threshold crossed or not), so the roundings are written out and
+           kept as they have been. */
+        constexpr auto fused = [](int place) {
+            return MODE == FORCE_NP ? place == 0 : MODE == FORCE_NP_CFL ? place != 2 : true;
+        };
         float svx = 0.0f, svy = 0.0f, svz = 0.0f; /* standard viscosity sum */
-        for_fluid_neighbors<2, TPP>(P, A, i, nF, [&](unsigned, unsigned j, const float4& xj) {
-            const Pair p = make_pair(xi, xj);
-            const float rho_j = A.rho[j];
-            const float f = cs_gradf(p.rl, p.inv_rl, P);
+        /* one fluid neighbour from its record */
+        const auto term = [&](auto place, unsigned j, const float4& xj, const float4& vj) {
+            Pair p;
+            p.rx = xi.x - xj.x; p.ry = xi.y - xj.y; p.rz = xi.z - xj.z;
+            p.s = __fmaf_rn(p.rz, p.rz, __fmaf_rn(p.rx, p.rx, __fmul_rn(p.ry, p.ry)));
+            len_inv(p.s, p.rl, p.inv_rl);
+            const float rho_j = xj.w;
+            const float f = cs_gradf_as<fused(decltype(place)::value)>(p.rl, p.inv_rl, P);
             if (pressure) {
-                const float pj = A.press[j];
-                const float c = P.mass * (dpi + pj / (rho_j * rho_j)) * f;
+                const float c = P.mass * (dpi + vj.w) * f;
                 ax -= c * p.rx; ay -= c * p.ry; az -= c * p.rz;
             }
             if (vm >= 0) {
-                const float4 vj = A.vel[j];
                 const float dvx = vi.x - vj.x, dvy = vi.y - vj.y, dvz = vi.z - vj.z;
                 if (vm == 1) {
-                    const float dot = (dvx * p.rx + dvy * p.ry) + dvz * p.rz;
+                    const float dot = __fmaf_rn(dvz, p.rz, __fmaf_rn(dvx, p.rx, __fmul_rn(dvy, p.ry)));
                     /* nu (m / rho_j) dot / (|r|^2 + 0.01 h^2) gradW with one fast
                        division (this pass is compared with the reference to a
                        relative tolerance, not bit for bit) */
-                    const float c = visc_c * __fdividef(P.mass * dot, rho_j * (p.s + eps_h2)) * f;
+                    const float c = visc_c * __fdividef(P.mass * dot, rho_j * __fmaf_rn(0.01f, P.h2, p.s)) * f;
                     ax += c * p.rx; ay += c * p.ry; az += c * p.rz;
                 } else if (vm == 0) {
                     const float c = P.mass / rho_j * visco_lapl(p.rl, P);
                     svx -= c * dvx; svy -= c * dvy; svz -= c * dvz;
                 } else {
-                    const float c = visc_c * (P.mass / rho_j) * cs_W(p.rl * P.inv_h, P) / dt;
+                    const float c = visc_c * (P.mass / rho_j) * cs_W_fused(p.rl, P) / dt;
                     ax -= c * dvx; ay -= c * dvy; az -= c * dvz;
                 }
             }
@@ -340,7 +428,8 @@ __device__ __forceinline__ void forces_at(const SimParams& P, const DeviceArrays
                 ay += kij * (-c * p.ry - P.st * (ni.y - nj.y));
                 az += kij * (-c * p.rz - P.st * (ni.z - nj.z));
             }
-        }, sub);
+        };
+        for_fluid_records<2, TPP>(P, A, i, nF, term, sub);
         if (TPP > 1) {
             ax = group_sum<TPP>(ax); ay = group_sum<TPP>(ay); az = group_sum<TPP>(az);
             svx = group_sum<TPP>(svx); svy = group_sum<TPP>(svy); svz = group_sum<TPP>(svz);
@@ -451,7 +540,7 @@ __device__ __forceinline__ void forces_at(const SimParams& P, const DeviceArrays
 }
 
 template <int MODE, int TPP = 1>
-__global__ void __launch_bounds__(256, 6) k_forces(SimParams P, DeviceArrays A)
+__global__ void __launch_bounds__(256, MODE == FORCE_PRESSURE ? 6 : 4) k_forces(SimParams P, DeviceArrays A)
 {
     __shared__ float s_red[32];
     forces_at<MODE, TPP>(P, A, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.x == 0 && threadIdx.x == 0, s_red);
@@ -464,15 +553,6 @@ __global__ void __launch_bounds__(256, 6) k_forces(SimParams P, DeviceArrays A)
 __device__ __forceinline__ uint2 pair_at(const uint2* pairs, unsigned kk, unsigned cap, int i)
 {
     return __ldcs(pairs + list_index(kk, cap, (unsigned)i));
-}
-
-/* Record j of DeviceArrays::rec, both halves with one 256-bit load. */
-__device__ __forceinline__ void load_rec(const float4* rec, unsigned j, float4& a, float4& b)
-{
-    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-                 : "l"(rec + 2 * (size_t)j)
-                 : "memory");
 }
 
 /* One fluid term of the residual: m f (v_i - v_j) . r_ij */
@@ -810,6 +890,7 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
         kws[i] = it == 0 ? 0.0f : kws[i] * scale;
         const float4 v = A.rec[2 * (size_t)i + 1];
         A.vel[i] = v;
+        if (DIV) dfsph_set_k(A, i, A.rho[i]); /* the record as the force pass reads it */
         if (!DIV) {
             float4 x = A.pos[i];
             float4 lo = P.pos_lo ? A.plo[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -991,6 +1072,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams
         kws[i] *= DIV ? dt : dt * dt;
         const float4 v = A.rec[2 * (size_t)i + 1];
         A.vel[i] = v;
+        if (DIV) dfsph_set_k(A, i, A.rho[i]); /* the record as the force pass reads it */
         if (!DIV) {
             float4 x = A.pos[i];
             x.x = __fadd_rn(x.x, __fmul_rn(v.x, dt));
