@@ -24,7 +24,7 @@
  * fixed order: results are bit-reproducible run to run.
  *
  * One backward step, in the cell-sorted order of the recomputed step:
- *   k_adj_load     x~ = xbar', v~ = vbar' + dt xbar', abar = dt v~, A = p / rho^2
+ *   k_adj_load     x~ = xbar', v~ = vbar' + dt xbar', abar = dt v~, records
  *   k_adj_forces   pressure / viscosity adjoint: rhobar, x~ += dF/dx, v~ += dF/dv,
  *                  dL/dk and dL/dnu partial sums
  *   k_adj_density  x~ += sum_j m (rhobar_i + rhobar_j) gradW_ij + boundary,
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(256) k_adj_load(SimParams P, AdjointArrays J)
     J.xacc[i] = make_float4(xb.x, xb.y, xb.z, 0.0f);
     J.vacc[i] = make_float4(vx, vy, vz, 0.0f);
     const float r = J.rho[i];
-    J.Ap[i] = J.press[i] / (r * r);
+    store_rec(J.rec, i, J.pos[i], 1.0f / r, J.vel[i], J.press[i] / (r * r));
 }
 
 /* Adjoint of the pressure and viscosity accelerations (and of the EOS).
@@ -138,28 +138,25 @@ __global__ void __launch_bounds__(256, 4) k_adj_forces(SimParams P, AdjointArray
     float sA = 0.0f, sB = 0.0f, rv = 0.0f, sbv = 0.0f, nup = 0.0f;
     float xrx = 0.0f, xry = 0.0f, xrz = 0.0f, vrx = 0.0f, vry = 0.0f, vrz = 0.0f;
     if (i < P.nf) {
-        const float4 xi = J.pos[i];
-        const float4 vi = J.vel[i];
+        float4 xi, vi;
+        load_rec(J.rec, (unsigned)i, xi, vi);
         const float4 ai = J.abar[i];
-        const float rho_i = J.rho[i], p_i = J.press[i];
-        const float Ai = J.Ap[i];
+        const float p_i = J.press[i];
+        const float Ai = vi.w;
         const float Bi = p_i / (P.rho0 * P.rho0);
         const float m = P.mass;
         const bool visc = P.visc_method == 1;
         const bool bvisc = visc && P.bvisc != 0.0f;
         const float nu = P.visc, nub = P.bvisc;
         const float eps_h2 = 0.01f * P.h2;
-        const float inv_rho_i = 1.0f / rho_i;
+        const float inv_rho_i = xi.w;
         const unsigned nF = J.cnt_f[i];
-        for (unsigned kk = sub; kk < nF; kk += TPP) {
-            const unsigned j = list_at(J.nbr_f, kk, P.capF, i);
-            const float4 xj = J.pos[j];
+        const auto term = [&](const float4& xj, const float4& vj, const float4& aj) {
             float rx, ry, rz, s, rl, inv_rl, f, g;
             pair_of(xi, xj, rx, ry, rz, s, rl, inv_rl);
             cs_grad_fg(rl, inv_rl, P, f, g);
-            if (f == 0.0f && g == 0.0f) continue;
-            const float4 aj = J.abar[j];
-            const float Aj = J.Ap[j];
+            if (f == 0.0f && g == 0.0f) return;
+            const float Aj = vj.w;
             const float dax = ai.x - aj.x, day = ai.y - aj.y, daz = ai.z - aj.z;
             const float rda = (rx * dax + ry * day) + rz * daz;
             sA -= m * f * rda;
@@ -170,14 +167,12 @@ __global__ void __launch_bounds__(256, 4) k_adj_forces(SimParams P, AdjointArray
             xry += c1 * (f * day + gr * ry);
             xrz += c1 * (f * daz + gr * rz);
             if (visc) {
-                const float4 vj = J.vel[j];
-                const float rho_j = J.rho[j];
                 const float vx = vi.x - vj.x, vy = vi.y - vj.y, vz = vi.z - vj.z;
                 const float vr = (vx * rx + vy * ry) + vz * rz;
                 const float invD = 1.0f / (s + eps_h2);
                 const float phi = vr * invD;
                 /* c = nu m (abar_i / rho_j - abar_j / rho_i) */
-                const float inv_rho_j = 1.0f / rho_j;
+                const float inv_rho_j = xj.w;
                 const float cx = nu * m * (ai.x * inv_rho_j - aj.x * inv_rho_i);
                 const float cy = nu * m * (ai.y * inv_rho_j - aj.y * inv_rho_i);
                 const float cz = nu * m * (ai.z * inv_rho_j - aj.z * inv_rho_i);
@@ -192,6 +187,23 @@ __global__ void __launch_bounds__(256, 4) k_adj_forces(SimParams P, AdjointArray
                 rv += phi * f * ((aj.x * rx + aj.y * ry) + aj.z * rz);
                 nup += m * inv_rho_j * phi * f * ((ai.x * rx + ai.y * ry) + ai.z * rz);
             }
+        };
+        /* two neighbours' loads in flight; added in list order */
+        unsigned kk = sub;
+        for (; kk + TPP < nF; kk += 2 * TPP) {
+            const unsigned j0 = list_at(J.nbr_f, kk, P.capF, i), j1 = list_at(J.nbr_f, kk + TPP, P.capF, i);
+            float4 x0, v0, x1, v1;
+            load_rec(J.rec, j0, x0, v0);
+            load_rec(J.rec, j1, x1, v1);
+            const float4 a0 = J.abar[j0], a1 = J.abar[j1];
+            term(x0, v0, a0);
+            term(x1, v1, a1);
+        }
+        if (kk < nF) {
+            const unsigned j = list_at(J.nbr_f, kk, P.capF, i);
+            float4 x, v;
+            load_rec(J.rec, j, x, v);
+            term(x, v, J.abar[j]);
         }
         const unsigned nB = J.cnt_b[i];
         for (unsigned kk = sub; kk < nB; kk += TPP) {
@@ -253,7 +265,8 @@ __global__ void __launch_bounds__(256, 4) k_adj_forces(SimParams P, AdjointArray
         const float rhobar = -2.0f * p_i * sA * inv_rho_i * inv_rho_i * inv_rho_i +
                              nu * m * rv * inv_rho_i * inv_rho_i - nub * sbv * inv_rho_i * inv_rho_i +
                              pbar * dpdrho;
-        J.rhobar[i] = rhobar;
+        const float4 x = J.rec[2 * (size_t)i];
+        J.xrho[i] = make_float4(x.x, x.y, x.z, rhobar);
         float4 xa = J.xacc[i], va = J.vacc[i];
         xa.x += xrx; xa.y += xry; xa.z += xrz;
         va.x += vrx; va.y += vry; va.z += vrz;
@@ -284,26 +297,37 @@ __global__ void __launch_bounds__(256) k_adj_finish(int nblocks, const double* _
 
 /* Adjoint of the density sum; writes the step's input adjoint in caller order. */
 template <int TPP>
-__global__ void __launch_bounds__(256, 6) k_adj_density(SimParams P, AdjointArrays J)
+__global__ void __launch_bounds__(256, 5) k_adj_density(SimParams P, AdjointArrays J)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = t / TPP;
     const unsigned sub = (unsigned)t % TPP;
     /* a group's lanes share i, so a group leaves together */
     if (i >= P.nf) return;
-    const float4 xi = J.pos[i];
-    const float rbi = J.rhobar[i];
+    const float4 xi = J.xrho[i];
+    const float rbi = xi.w;
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
     const unsigned nF = J.cnt_f[i];
-    for (unsigned kk = sub; kk < nF; kk += TPP) {
-        const unsigned j = list_at(J.nbr_f, kk, P.capF, i);
+    const auto term = [&](const float4& xj) {
         float rx, ry, rz, s, rl, inv_rl;
-        pair_of(xi, J.pos[j], rx, ry, rz, s, rl, inv_rl);
+        pair_of(xi, xj, rx, ry, rz, s, rl, inv_rl);
         const float f = cs_gradf(rl, inv_rl, P);
-        if (f == 0.0f) continue;
-        const float c = P.mass * (rbi + J.rhobar[j]) * f;
+        if (f == 0.0f) return;
+        const float c = P.mass * (rbi + xj.w) * f;
         sx += c * rx; sy += c * ry; sz += c * rz;
+    };
+    unsigned kk = sub;
+    for (; kk + 3 * TPP < nF; kk += 4 * TPP) {
+        unsigned j[4];
+        float4 x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) j[u] = list_at(J.nbr_f, kk + u * TPP, P.capF, i);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = J.xrho[j[u]];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) term(x[u]);
     }
+    for (; kk < nF; kk += TPP) term(J.xrho[list_at(J.nbr_f, kk, P.capF, i)]);
     const unsigned nB = J.cnt_b[i];
     for (unsigned kk = sub; kk < nB; kk += TPP) {
         const float4 xb = J.bpos[list_at(J.nbr_b, kk, P.capB, i)];

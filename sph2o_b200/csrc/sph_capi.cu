@@ -168,7 +168,7 @@ struct sph_ctx {
         DevState *st0 = nullptr, *st1 = nullptr;       /* solver state at the start / end of the run */
         float* target = nullptr;
         float4 *xbar = nullptr, *vbar = nullptr, *abar = nullptr, *xacc = nullptr, *vacc = nullptr;
-        float *Ap = nullptr, *rhobar = nullptr;
+        float4* xrho = nullptr;
         double *part = nullptr, *red = nullptr;  /* per-block partial sums, their totals */
         bool ready = false, have_grad = false;
         cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -2022,7 +2022,7 @@ int adj_reserve(sph_ctx* c, int nseg, int every)
         AALLOC(fin_pos, nf); AALLOC(fin_vel, nf); AALLOC(fin_orig, nf);
         AALLOC(st0, 1); AALLOC(st1, 1); AALLOC(target, 3 * nf);
         AALLOC(xbar, nf); AALLOC(vbar, nf); AALLOC(abar, nf); AALLOC(xacc, nf); AALLOC(vacc, nf);
-        AALLOC(Ap, nf); AALLOC(rhobar, nf); AALLOC(red, 4);
+        AALLOC(xrho, nf); AALLOC(red, 4);
         AALLOC(part, 3 * (size_t)adjoint_blocks((int)nf));
         for (auto& e : a.ev) CUDA_TRY(c, cudaEventCreate(&e));
     }
@@ -2086,7 +2086,7 @@ AdjointArrays adj_arrays(sph_ctx* c)
     J.bpos = c->bpos; J.nbr_f = c->nbr_f; J.cnt_f = c->cnt_f; J.nbr_b = c->nbr_b; J.cnt_b = c->cnt_b;
     J.st = c->st;
     J.xbar = a.xbar; J.vbar = a.vbar; J.abar = a.abar; J.xacc = a.xacc; J.vacc = a.vacc;
-    J.Ap = a.Ap; J.rhobar = a.rhobar; J.part = a.part;
+    J.rec = c->rec; J.xrho = a.xrho; J.part = a.part;
     return J;
 }
 

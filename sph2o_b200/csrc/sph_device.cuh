@@ -553,6 +553,15 @@ __device__ __forceinline__ unsigned list_at(const unsigned* list, unsigned kk, u
     return __ldcs(list + list_index(kk, cap, (unsigned)i));
 }
 
+/* Record j of DeviceArrays::rec, both halves with one 256-bit load. */
+__device__ __forceinline__ void load_rec(const float4* rec, unsigned j, float4& a, float4& b)
+{
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(rec + 2 * (size_t)j)
+                 : "memory");
+}
+
 /* Record i of DeviceArrays::rec: (x, w0), (v, w1). */
 __device__ __forceinline__ void store_rec(float4* rec, int i, float4 x, float w0, float4 v, float w1)
 {

@@ -138,7 +138,7 @@ void launch_emit(const SimParams& P, const DeviceArrays& A, EmitterState* E, con
 
 /* sph_adjoint.cu: reverse-mode WCSPH step. Sorted-order arrays of the
    recomputed step (pos .. cnt_b), caller-order adjoint state (xbar, vbar),
-   sorted-order work arrays (abar .. rhobar) and per-block FP64 partial sums
+   sorted-order work arrays (abar .. xrho) and per-block FP64 partial sums
    part[3 b + q] (q = 0: dL/dk, 1: dL/dnu, 2: loss * N), adjoint_blocks(n)
    blocks, which launch_adjoint_finish reduces into red[0..2]. */
 struct AdjointArrays {
@@ -158,8 +158,8 @@ struct AdjointArrays {
     float4* abar;
     float4* xacc;
     float4* vacc;
-    float* Ap;
-    float* rhobar;
+    float4* rec;     /* (x, y, z, 1 / rho), (vx, vy, vz, p / rho^2): a neighbour's state in one load */
+    float4* xrho;    /* (x, y, z, rhobar) */
     double* part;
 };
 int adjoint_blocks(int n);

@@ -81,15 +81,6 @@ __device__ __forceinline__ void for_fluid_neighbors(const SimParams& P, const De
     }
 }
 
-/* Record j of DeviceArrays::rec, both halves with one 256-bit load. */
-__device__ __forceinline__ void load_rec(const float4* rec, unsigned j, float4& a, float4& b)
-{
-    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-                 : "l"(rec + 2 * (size_t)j)
-                 : "memory");
-}
-
 /* for_fluid_neighbors over the records: f(place, j, (x_j, w), (v_j, w)) with
    the entry's place: 0 even or 1 odd in an unrolled round, 2 after the rounds. */
 template <int U, int TPP, typename F>
