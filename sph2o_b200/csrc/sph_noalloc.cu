@@ -156,10 +156,22 @@ __global__ void __launch_bounds__(256) k_na_zero(unsigned* start, unsigned* sums
 
 __global__ void __launch_bounds__(256) k_na_count(SimParams P, NaSet f, NaSet b)
 {
+    /* chunk totals per block first: the caller's order jumps between chunks of
+       cells, and single additions to these few words queue up */
+    __shared__ unsigned s_chunk[kMaxCells / 4096];
+    for (unsigned k = threadIdx.x; k < kMaxCells / 4096; k += blockDim.x) s_chunk[k] = 0u;
+    __syncthreads();
     int i;
     const NaSet& s = na_pick(f, b, i);
-    const bool on = i < s.n;
-    ns_count_at(on, on ? cell_index(na_load(s, i), P.h, grid_single(P)) : 0u, i, s.start, s.sums, s.cell_of, s.slot);
+    if (i < s.n) {
+        const unsigned c = cell_index(na_load(s, i), P.h, grid_single(P));
+        s.cell_of[i] = c;
+        s.slot[i] = atomicAdd(&s.start[c], 1u);
+        atomicAdd(&s_chunk[c >> 12], 1u);
+    }
+    __syncthreads();
+    for (unsigned k = threadIdx.x; k < kMaxCells / 4096; k += blockDim.x)
+        if (s_chunk[k]) atomicAdd(&s.sums[k], s_chunk[k]);
 }
 
 __global__ void __launch_bounds__(256) k_na_scan(NaSet f, NaSet b, int nchunks)
@@ -192,12 +204,34 @@ __global__ void __launch_bounds__(256) k_na_rank_gather(NaSet f, NaSet b)
     if (s.orig) s.orig[dst] = i;
 }
 
-/* Density over the 27 cells: every fluid candidate first, then every boundary
-   candidate, cells in the reference's offset order, exact W; written to the
-   caller's order. A thread per particle in blocks of 64, so that the blocks of
-   a few thousand particles still reach every SM; accepted candidates are
-   collected and their kernels evaluated four at a time, all lanes together. */
-constexpr int kNaBlock = 64, kNaBatch = 44;
+/* Density over the 27 cells by one thread: every fluid candidate first, then
+   every boundary candidate, cells in the reference's offset order, exact W. */
+__device__ __noinline__ float na_density_at(const SimParams& P, float4 xi, const float4* __restrict__ pos,
+                                            const unsigned* __restrict__ cell_start, const float4* __restrict__ bpos,
+                                            const unsigned* __restrict__ bcell_start)
+{
+    const Grid g = grid_single(P);
+    float rho = 0.0f;
+    for_candidates27(xi, P.h, g, cell_start, [&](unsigned q) {
+        const float s2 = dist2_exact(xi, pos[q]);
+        if (s2 <= P.h2_guard) rho = __fadd_rn(rho, __fmul_rn(P.mass, cs_W_exact(s2, P)));
+    });
+    if (P.nb > 0)
+        for_candidates27(xi, P.h, g, bcell_start, [&](unsigned q) {
+            const float4 xb = bpos[q];
+            const float s2 = dist2_exact(xi, xb);
+            if (s2 <= P.h2_guard) rho = __fadd_rn(rho, __fmul_rn(xb.w, cs_W_exact(s2, P)));
+        });
+    return rho;
+}
+
+/* The same sum with four lanes per particle (a call holds at most 65,536
+   particles, too few to fill the GPU with one lane each): the rows of cells are
+   split 3, 2, 2, 2 over the lanes in candidate order, each lane collects its
+   accepted candidates in shared memory, the four evaluate the kernel terms, and
+   the terms are added in candidate order. A particle with more than kNaBatch
+   candidates in one lane is left to na_density_at. Written to the caller's order. */
+constexpr int kNaBlock = 128, kNaLanes = 4, kNaBatch = 24;
 
 __global__ void __launch_bounds__(kNaBlock) k_na_density(SimParams P, const float4* __restrict__ pos,
                                                          const unsigned* __restrict__ cell_start,
@@ -206,44 +240,52 @@ __global__ void __launch_bounds__(kNaBlock) k_na_density(SimParams P, const floa
                                                          const unsigned* __restrict__ bcell_start,
                                                          float* __restrict__ rho_out)
 {
-    __shared__ float s_s2[kNaBatch][kNaBlock];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.nf) return;
-    const float4 xi = pos[i];
+    __shared__ float s_w[kNaBatch + 1][kNaBlock]; /* one spare row */
+    __shared__ unsigned s_q[kNaBatch][kNaBlock];
+    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) / kNaLanes);
+    const unsigned tid = threadIdx.x, lane = tid & 31u, sub = lane % kNaLanes, first = lane - sub;
+    const bool on = i < P.nf;
+    const float4 xi = on ? pos[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const Grid g = grid_single(P);
+    const int row0 = sub == 0 ? 0 : 2 * (int)sub + 1, row1 = 2 * (int)sub + 3;
     float rho = 0.0f;
-    int n = 0;
-    const auto add_fluid = [&]() {
-        /* past the end W is 0 and leaves the sum as it is */
-#pragma unroll 1
-        for (int k = 0; k < n; k += 4) {
-            float w[4];
+    bool over = false;
+    const auto set = [&](const unsigned* starts, const float4* xs, bool boundary) {
+        unsigned m = 0, nq = 0, nw = 0;
+        if (on)
+            for_stretches27(
+                xi, xi, P.h, g, starts, xs,
+                [&](unsigned k, const float (&d)[4], unsigned) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                w[u] = __fmul_rn(P.mass, cs_W_exact(k + u < n ? s_s2[k + u][threadIdx.x] : 4.0f * P.h2, P));
-#pragma unroll
-            for (int u = 0; u < 4; ++u) rho = __fadd_rn(rho, w[u]);
+                    for (unsigned u = 0; u < 4; ++u) {
+                        const bool in = d[u] <= P.h2_guard;
+                        m |= (in ? 1u << u : 0u) << k;
+                        s_w[min(nw, (unsigned)kNaBatch)][tid] = d[u]; /* written over unless kept */
+                        nw += in ? 1u : 0u;
+                    }
+                },
+                [&](auto slot) {
+                    if (boundary)
+                        for (; m; m &= m - 1u, ++nq)
+                            s_q[min(nq, kNaBatch - 1u)][tid] = slot((unsigned)__ffs((int)m) - 1u);
+                    m = 0;
+                },
+                row0, row1);
+        over |= ((__ballot_sync(0xffffffffu, nw > kNaBatch) >> first) & ((1u << kNaLanes) - 1u)) != 0u;
+        const unsigned own = min(nw, (unsigned)kNaBatch);
+        for (unsigned k = 0; k < own; ++k)
+            s_w[k][tid] = __fmul_rn(boundary ? xs[s_q[k][tid]].w : P.mass, cs_W_exact(s_w[k][tid], P));
+        __syncwarp();
+        for (unsigned l = 0; l < kNaLanes; ++l) {
+            const unsigned c = __shfl_sync(0xffffffffu, own, first + l);
+            for (unsigned k = 0; k < c; ++k) rho = __fadd_rn(rho, s_w[k][tid - sub + l]);
         }
-        n = 0;
+        __syncwarp();
     };
-    for_stretches27(
-        xi, xi, P.h, g, cell_start, pos,
-        [&](unsigned, const float (&d)[4], unsigned) {
-            if (n > kNaBatch - 4) add_fluid();
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                s_s2[n][threadIdx.x] = d[u];
-                n += d[u] <= P.h2_guard ? 1 : 0;
-            }
-        },
-        [](auto) {});
-    add_fluid();
-    if (P.nb > 0)
-        for_candidates27(xi, P.h, g, bcell_start, [&](unsigned q) {
-            const float4 xb = bpos[q];
-            const float s2 = dist2_exact(xi, xb);
-            if (s2 <= P.h2_guard) rho = __fadd_rn(rho, __fmul_rn(xb.w, cs_W_exact(s2, P)));
-        });
+    set(cell_start, pos, false);
+    if (P.nb > 0) set(bcell_start, bpos, true);
+    if (!on || sub != 0) return;
+    if (over) rho = na_density_at(P, xi, pos, cell_start, bpos, bcell_start);
     rho_out[orig[i]] = rho;
 }
 
@@ -365,7 +407,8 @@ extern "C" int sph_density_noalloc(float particle_radius, float density0, const 
     k_na_scan<<<(nb > 0 ? 2 : 1) * nchunks, 256, 0, s>>>(f, b, nchunks);
     k_na_scatter<<<blocks, 256, 0, s>>>(f, b);
     k_na_rank_gather<<<blocks, 256, 0, s>>>(f, b);
-    k_na_density<<<(f.n + kNaBlock - 1) / kNaBlock, kNaBlock, 0, s>>>(P, f.out, f.start, f.orig, b.out, b.start, rho_out);
+    k_na_density<<<(f.n * kNaLanes + kNaBlock - 1) / kNaBlock, kNaBlock, 0, s>>>(P, f.out, f.start, f.orig, b.out, b.start,
+                                                                                    rho_out);
     e = cudaGetLastError();
     if (e != cudaSuccess) return na_fail(SPH_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     return SPH_OK;
