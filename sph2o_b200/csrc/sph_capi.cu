@@ -1916,7 +1916,7 @@ int sph_debug_barrier_timeout(sph_ctx* c)
     /* reset the barrier and the flag so the context stays usable */
     DevState fix = s;
     fix.err &= ~ERRBIT_TIMEOUT;
-    fix.bar_count = 0;
+    fix.bar_arrived[0] = fix.bar_arrived[1] = 0;
     CUDA_TRY(c, cudaMemcpyAsync(c->st, &fix, sizeof fix, cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     c->last = fix;

@@ -26,8 +26,8 @@ namespace sph {
 /* error bits in DevState::err */
 enum : int { ERRBIT_NAN = 1, ERRBIT_OVERFLOW = 2, ERRBIT_TIMEOUT = 4 };
 
-/* bounded spin: ~2^22 polls with >= 256 ns sleep each (> 1 s) */
-constexpr unsigned long long kSpinLimit = 1ull << 22;
+/* bounded spin: ~6e6 polls, each a sleep of about 64 ns and a round trip to the L2 (some 4 s) */
+constexpr unsigned kSpinLimit = 3u << 21;
 
 struct SimParams {
     int nf, nb;
@@ -92,10 +92,13 @@ struct DevState {
     unsigned steps;
     int err;
     unsigned overflow;
-    unsigned bar_count, bar_gen;
     float last_vmax;
     unsigned n_active;          /* active fluid particles (emitters append to them) */
     unsigned ns_epoch;          /* neighbour searches so far (PCISPH boundary cell entries) */
+    unsigned bar_sel;           /* which of the two arrival counts the next cooperative kernel uses */
+    unsigned pad_[31];          /* the counts get lines of their own: they are polled */
+    unsigned bar_arrived[2];
+    unsigned pad2_[30];
 };
 
 /* Fluid particles a pass covers: all nf, or with emitters the active prefix
@@ -637,46 +640,66 @@ __device__ __forceinline__ unsigned atom_add_acq_rel_gpu(unsigned* p, unsigned v
     return old;
 }
 
-__device__ __forceinline__ void st_release_gpu(unsigned* p, unsigned v)
-{
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
+/* Grid-wide barrier for cooperative (co-resident) launches, one object per
+   thread of the kernel. Each block's thread 0 arrives with an acquire-release
+   add (releasing its block's writes, ordered by the preceding __syncthreads)
+   and spins on an acquire load of the same count until all blocks of this
+   barrier have arrived: every block sees every other block's writes from
+   before it. The count only grows inside a kernel, because resetting it and
+   publishing a generation were two more round trips to the L2 on the path of
+   every barrier, as was reading the error flag, which only waiters do now. Two
+   counts take turns from kernel to kernel: the constructor zeroes the one that
+   the previous kernel used, leave() hands over. A DFSPH step has 10 to 20
+   barriers: 26k particles 224 -> 207 us per step, 125k 323 -> 312, 1M 1503 ->
+   1485, 24 batched scenes 506 -> 496 (sleeps of 20, 64 and 256 ns within 1 %).
+   The wait is bounded: after kSpinLimit polls the block records ERRBIT_TIMEOUT
+   and sync() returns false, and the caller leaves the kernel; so does every
+   kernel that starts with that bit set, whose counts mean nothing. */
+struct GridBarrier {
+    DevState* st;
+    unsigned* count;
+    unsigned target = 0;
+    bool dead;
 
-/* Grid-wide barrier for cooperative (co-resident) launches. Each block's
-   thread 0 arrives with an acquire-release add (releasing its block's
-   writes, ordered by the preceding __syncthreads), the last arrival resets
-   the count and publishes the next generation with a release store, and the
-   waiters spin on an acquire load of the generation: every block sees every
-   other block's writes from before the barrier. The wait is bounded: after
-   kSpinLimit polls the block records ERRBIT_TIMEOUT and returns false, and
-   the caller leaves the kernel. */
-__device__ __forceinline__ bool grid_barrier(DevState* st)
-{
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned g = ld_acquire_gpu(&st->bar_gen);
-        const unsigned arrived = atom_add_acq_rel_gpu(&st->bar_count, 1u);
-        int ok = 1;
-        if (arrived == gridDim.x - 1) {
-            atomicExch(&st->bar_count, 0u);
-            st_release_gpu(&st->bar_gen, g + 1u);
-        } else {
-            unsigned long long spins = 0;
-            while (ld_acquire_gpu(&st->bar_gen) == g) {
-                __nanosleep(256);
-                if (++spins > kSpinLimit) {
-                    atomicOr(&st->err, ERRBIT_TIMEOUT);
-                    ok = 0;
-                    break;
+    __device__ __forceinline__ explicit GridBarrier(DevState* s) : st(s), dead((s->err & ERRBIT_TIMEOUT) != 0)
+    {
+        const unsigned sel = s->bar_sel & 1u;
+        count = &s->bar_arrived[sel];
+        if (blockIdx.x == 0 && threadIdx.x == 0) s->bar_arrived[sel ^ 1u] = 0u;
+    }
+
+    __device__ __forceinline__ bool sync()
+    {
+        __shared__ int s_ok;
+        target += gridDim.x;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int ok = !dead;
+            if (ok && (int)(atom_add_acq_rel_gpu(count, 1u) + 1u - target) < 0) {
+                unsigned spins = 0;
+                while ((int)(ld_acquire_gpu(count) - target) < 0) {
+                    __nanosleep(64);
+                    ++spins;
+                    /* a block that gave up will not arrive any more */
+                    const bool left = (spins & 1023u) == 0u &&
+                                      (ld_acquire_gpu(reinterpret_cast<const unsigned*>(&st->err)) & ERRBIT_TIMEOUT) != 0u;
+                    if (left || spins > kSpinLimit) {
+                        atomicOr(&st->err, ERRBIT_TIMEOUT);
+                        ok = 0;
+                        break;
+                    }
                 }
             }
+            s_ok = ok;
         }
-        s_ok = ok && ((ld_acquire_gpu(reinterpret_cast<const unsigned*>(&st->err)) & ERRBIT_TIMEOUT) == 0);
+        __syncthreads();
+        return s_ok != 0;
     }
-    __syncthreads();
-    return s_ok != 0;
-}
+
+    /* At the end of a kernel, by one thread of block 0: it has passed every
+       barrier, so every block has read bar_sel (without barriers nobody uses it). */
+    __device__ __forceinline__ void leave() { st->bar_sel ^= 1u; }
+};
 
 /* ---------------------------------------------------------------------- */
 /* PCISPH boundary method helpers, in the reference's float operation order. */

@@ -784,6 +784,7 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
     constexpr int ACC = TPP == 1 ? 2 : 1;
     __shared__ double s_red[32];
     DevState* st = A.st;
+    GridBarrier bar(st);
     const int nfi = active_n(P, st);
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int nthr = gridDim.x * blockDim.x;
@@ -819,7 +820,7 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
             A.rec[2 * (size_t)i] = make_float4(x.x, x.y, x.z, 0.0f);
             A.rec[2 * (size_t)i + 1] = v;
         }
-        if (!grid_barrier(st)) return;
+        if (!bar.sync()) return;
     } else {
         dt = st->dt;
     }
@@ -837,9 +838,9 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
             else dfsph_set_k(A, i, r > P.rho0 ? kws[i] / ts2 : 0.0f);
         }
     });
-    if (!grid_barrier(st)) return;
+    if (!bar.sync()) return;
     for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U>(P, A, i, sub, valid, dt); });
-    if (!grid_barrier(st)) return;
+    if (!bar.sync()) return;
 
     const double limit = DIV ? (double)(P.eta_v / dt) : (double)P.eta;
     const unsigned min_it = DIV ? P.min_it_v : P.min_it;
@@ -866,10 +867,10 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
         });
         const double bs = block_sum(local, s_red);
         if (threadIdx.x == 0) atomicAdd(&A.accum[it], bs);
-        if (!grid_barrier(st)) return;
+        if (!bar.sync()) return;
         avg = *(volatile double*)&A.accum[it] / (double)nfi;
         for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U>(P, A, i, sub, valid, dt); });
-        if (!grid_barrier(st)) return;
+        if (!bar.sync()) return;
         ++it;
     }
 
@@ -895,6 +896,7 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
     }
     if (bad) atomicOr(&st->err, ERRBIT_NAN);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
+        bar.leave();
         if (!DIV) {
             st->dt = dt;
             st->its = it;
@@ -935,6 +937,7 @@ template <bool DIV>
 __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams P, DeviceArrays A)
 {
     DevState* st = A.st;
+    GridBarrier bar(st);
     SceneState* sst = A.sst;
     const SceneInfo* sc = A.sref.scenes;
     const unsigned* so = A.sref.scene_of;
@@ -967,7 +970,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams
         sst[s].dt_next = dt;
         sst[s].active = (min_it > 0u && max_it > 0u) ? 1u : 0u;  /* parity 0: iteration 0 */
     }
-    if (!grid_barrier(st)) return;
+    if (!bar.sync()) return;
     if (!DIV) {
         for (int i = tid; i < nfi; i += nthr) {
             const float dt = sst[so[i]].dt_next;
@@ -980,7 +983,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams
             A.rec[2 * (size_t)i] = make_float4(x.x, x.y, x.z, 0.0f);
             A.rec[2 * (size_t)i + 1] = v;
         }
-        if (!grid_barrier(st)) return;
+        if (!bar.sync()) return;
     }
     float* kws = DIV ? A.kvws : A.kws;
     for (int i = tid; i < nfi; i += nthr) {
@@ -990,12 +993,12 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams
         if (DIV) dfsph_set_k(A, i, r > 0.0f ? kws[i] / dt : 0.0f);
         else dfsph_set_k(A, i, r > P.rho0 ? kws[i] / (dt * dt) : 0.0f);
     }
-    if (!grid_barrier(st)) return;
+    if (!bar.sync()) return;
     for (int i = tid; i < nfi; i += nthr) {
         dfsph_correct(P, A, i, sst[so[i]].dt_next);
         kws[i] = 0.0f;
     }
-    if (!grid_barrier(st)) return;
+    if (!bar.sync()) return;
 
     /* activity for iteration it lives in bit (it & 1) of SceneState::active;
        the convergence test of iteration it keeps that bit (the correction
@@ -1029,7 +1032,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams
             }
             scene_accumulate(A.accum, stride, it, s, on, err);
         }
-        if (!grid_barrier(st)) return;
+        if (!bar.sync()) return;
         /* convergence test per scene for the next iteration */
         const unsigned nbit = 1u << ((it + 1u) & 1u);
         for (int s = tid; s < ns; s += nthr) {
@@ -1052,7 +1055,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams
             const unsigned s = so[i];
             if (sst[s].active & bit) dfsph_correct(P, A, i, sst[s].dt_next);
         }
-        if (!grid_barrier(st)) return;
+        if (!bar.sync()) return;
         any = *(volatile unsigned*)&A.any_active[it + 1u] != 0u;
         ++it;
     }
@@ -1074,6 +1077,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams
         }
     }
     if (bad) atomicOr(&st->err, ERRBIT_NAN);
+    if (tid == 0) bar.leave();
     for (int s = tid; s < ns; s += nthr) {
         if (!DIV) {
             if (min_it == 0u || max_it == 0u) sst[s].its = 0u;
@@ -1168,6 +1172,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
     __shared__ double s_red[32];
     __shared__ float s_s2[kPcisphBatch][kSolverBlock];
     DevState* st = A.st;
+    GridBarrier bar(st);
     const int nfi = active_n(P, st);
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int nthr = gridDim.x * blockDim.x;
@@ -1193,7 +1198,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
     }
     if (P.pcib)
         for (int q = tid; q < P.nb; q += nthr) A.bpress[q] = 0.0f;
-    if (more && !grid_barrier(st)) return;
+    if (more && !bar.sync()) return;
     while (more) {
         /* predictFluidDensities over the start-of-step candidates of the 27
            cells around the particle's current cell, then updatePressure */
@@ -1261,7 +1266,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
             }
         const double bs = block_sum(local, s_red);
         if (threadIdx.x == 0) atomicAdd(&A.accum[it], bs);
-        if (!grid_barrier(st)) return;
+        if (!bar.sync()) return;
         avg = *(volatile double*)&A.accum[it] / (double)nfi;
         more = (avg > (double)P.eta || it + 1u < P.min_it) && it + 1u < P.max_it;
         /* computePressureAcc at the current positions, with the reference's
@@ -1333,10 +1338,11 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
             else bad |= pcisph_integrate(P, A, i, dt, pa);
         }
         ++it;
-        if (more && !grid_barrier(st)) return;
+        if (more && !bar.sync()) return;
     }
     if (bad) atomicOr(&st->err, ERRBIT_NAN);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
+        bar.leave();
         st->its = it;
         st->pcisph_avg = avg;
         st->avg_dens = avg;
@@ -1551,8 +1557,9 @@ void launch_emit(const SimParams& P, const DeviceArrays& A, EmitterState* E, con
 /* Test kernel: block 1 never arrives, so block 0's wait must run out. */
 __global__ void k_barrier_timeout_probe(DevState* st)
 {
+    GridBarrier bar(st);
     if (blockIdx.x == 1) return;
-    grid_barrier(st);
+    bar.sync();
 }
 
 int launch_barrier_timeout_probe(DevState* st, cudaStream_t s)
