@@ -25,7 +25,7 @@ struct DeviceArrays {
     float4* acc;
     float4* normal;
     float4* predr;        /* PCISPH predicted position */
-    float4* posd;         /* PCISPH: (x, y, z, p / rho^2 of the iteration) */
+    float4* posd;         /* PCISPH: (x, y, z, p / rho^2 of the iteration); DFSPH solvers: (x, y, z, k) */
     float4* pgrad;        /* PCISPH: (slot, gradW) of each fluid list entry, in the layout of nbr_f */
     float* rho;
     float* alpha;
@@ -46,8 +46,7 @@ struct DeviceArrays {
     uint2* pair_f;
     uint2* pair_b;
     /* two float4 per particle, so that half or all of a neighbour's record is one
-       load: (x, y, z, rho), (vx, vy, vz, p / rho^2 in WCSPH) for the force and
-       normal passes, with k in the place of rho inside the DFSPH solvers */
+       load: (x, y, z, rho), (vx, vy, vz, p / rho^2 in WCSPH) */
     float4* rec;
     unsigned* orig_w;     /* caller-order ids of the sorted slots (emitters write new ones) */
     double* accum;        /* per-iteration residual accumulators, zeroed per solve */

@@ -624,16 +624,16 @@ __device__ __forceinline__ float dfsph_residual(const SimParams& P, const Device
 
 /* Partial sums over list entries sub, sub + TPP, ... of
    sum_j m (k_i + k_j) gradW  (+ boundary with k_i), the fluid gathers issued
-   U at a time and ACC interleaved sums, as in dfsph_residual_part. k is in
-   the records' w, written inside the same persistent kernel (before a grid
+   U at a time and ACC interleaved sums, as in dfsph_residual_part. Position
+   and k are in posd, written inside the same persistent kernel (before a grid
    barrier): a read-only (non-coherent) load path would be wrong for it. */
 template <int TPP, int ACC, int U>
 __device__ __forceinline__ void dfsph_correct_part(const SimParams& P, const DeviceArrays& A, int i, int sub,
                                                    float& sx, float& sy, float& sz)
 {
     static_assert(U % ACC == 0, "an unrolled round holds whole rounds of partial sums");
-    const float4* rec = A.rec;
-    const float4 xi = rec[2 * (size_t)i];
+    const float4* xk = A.posd;
+    const float4 xi = xk[i];
     const float ki = xi.w;
     float tx[ACC], ty[ACC], tz[ACC];
 #pragma unroll
@@ -646,7 +646,7 @@ __device__ __forceinline__ void dfsph_correct_part(const SimParams& P, const Dev
 #pragma unroll
         for (int u = 0; u < N; ++u) e[u] = pair_at(A.pair_f, kk + u * TPP, P.capF, i);
 #pragma unroll
-        for (int u = 0; u < N; ++u) xj[u] = rec[2 * (size_t)e[u].x];
+        for (int u = 0; u < N; ++u) xj[u] = xk[e[u].x];
 #pragma unroll
         for (int u = 0; u < N; ++u) {
             const float ks = ki + xj[u].w;
@@ -689,10 +689,13 @@ __device__ __forceinline__ void dfsph_apply(const DeviceArrays& A, int i, float 
     A.rec[2 * (size_t)i + 1] = v;
 }
 
-/* k of particle i, where its neighbours' correction reads it */
+/* k of particle i, where its neighbours' correction reads it: with the position
+   in 16 bytes of its own, eight particles to a line, because the correction
+   reads nothing else and the records hold only four to a line */
 __device__ __forceinline__ void dfsph_set_k(const DeviceArrays& A, int i, float k)
 {
-    reinterpret_cast<float*>(A.rec)[8 * (size_t)i + 3] = k;
+    const float4 x = A.rec[2 * (size_t)i];
+    A.posd[i] = make_float4(x.x, x.y, x.z, k);
 }
 
 /* v_i -= dt * sum_j m (k_i + k_j) gradW  (+ boundary with k_i) */
@@ -765,15 +768,17 @@ __device__ __forceinline__ void dfsph_correct_lanes(const SimParams& P, const De
 }
 
 /* What bounds the passes: the L1's rate for scattered gathers. A warp-visit
-   (32 lanes, one list entry each) takes ~28 SM cycles whatever the occupancy
+   (32 lanes, one list entry each) takes ~26 SM cycles whatever the occupancy
    (8, 6, 5, 4 blocks per SM), and halving its instructions by reading the
    kernel factor f from pair_f instead of recomputing it (rsqrt, spline) alone
    left the 1M pass at 107 us. What helped, per pass on the 1M double dam break
-   in motion (5.5 + 1.25 iterations per step), density solver 1,424 -> 1,231 us
-   per step: a neighbour's position, velocity and k in one record, fetched with
-   one 256-bit load (residual) or one 128-bit load (correction) instead of two
-   (109 -> 104 us); lists in contiguous tiles of 32 particles (104 -> 98); one
-   lane per particle with 64 registers and four gathers in flight (98 -> 95).
+   in motion (5.5 + 1.25 iterations per step), density solver 1,424 -> 1,126 us
+   per step: a neighbour's position and velocity in one record, fetched with
+   one 256-bit load (109 -> 104 us); lists in contiguous tiles of 32 particles
+   (104 -> 98); one lane per particle with 64 registers and four gathers in
+   flight (98 -> 95); candidates in z-fastest order and a barrier of fewer round
+   trips (-4 %); position and k of the correction in 16 bytes of their own
+   instead of half of the record (1,187 -> 1,126; 125k 184 -> 171).
    OCC blocks of 256 per SM: 4 (64 registers) by default, 8 (32 registers, two
    gathers) is the autotuner's other candidate. TPP lanes share a particle;
    1 and 2 lanes add the same two interleaved sums, so they agree bit for bit. */
@@ -808,7 +813,6 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
         /* DFSPHSolver::predictVelocities, into the records */
         for (int i = tid; i < nfi; i += nthr) {
             const float4 a = A.acc[i];
-            const float4 x = A.pos[i];
             float4 v = A.vel[i];
             v.x = __fadd_rn(v.x, __fmul_rn(__fadd_rn(a.x, P.gx), dt));
             v.y = __fadd_rn(v.y, __fmul_rn(__fadd_rn(a.y, P.gy), dt));
@@ -817,7 +821,6 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
                with the normals left by the last collision pass (or by the
                surface-tension pass of this step, which shares the array) */
             if (P.pcib) pcib_velocity(P, A.normal[i], v, v);
-            A.rec[2 * (size_t)i] = make_float4(x.x, x.y, x.z, 0.0f);
             A.rec[2 * (size_t)i + 1] = v;
         }
         if (!bar.sync()) return;
@@ -882,7 +885,6 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
         kws[i] = it == 0 ? 0.0f : kws[i] * scale;
         const float4 v = A.rec[2 * (size_t)i + 1];
         A.vel[i] = v;
-        if (DIV) dfsph_set_k(A, i, A.rho[i]); /* the record as the force pass reads it */
         if (!DIV) {
             float4 x = A.pos[i];
             float4 lo = P.pos_lo ? A.plo[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -979,8 +981,6 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams
             v.x = __fadd_rn(v.x, __fmul_rn(__fadd_rn(a.x, P.gx), dt));
             v.y = __fadd_rn(v.y, __fmul_rn(__fadd_rn(a.y, P.gy), dt));
             v.z = __fadd_rn(v.z, __fmul_rn(__fadd_rn(a.z, P.gz), dt));
-            const float4 x = A.pos[i];
-            A.rec[2 * (size_t)i] = make_float4(x.x, x.y, x.z, 0.0f);
             A.rec[2 * (size_t)i + 1] = v;
         }
         if (!bar.sync()) return;
@@ -1066,7 +1066,6 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams
         kws[i] *= DIV ? dt : dt * dt;
         const float4 v = A.rec[2 * (size_t)i + 1];
         A.vel[i] = v;
-        if (DIV) dfsph_set_k(A, i, A.rho[i]); /* the record as the force pass reads it */
         if (!DIV) {
             float4 x = A.pos[i];
             x.x = __fadd_rn(x.x, __fmul_rn(v.x, dt));
