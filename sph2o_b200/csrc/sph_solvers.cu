@@ -546,6 +546,43 @@ __device__ __forceinline__ uint2 pair_at(const uint2* pairs, unsigned kk, unsign
     return __ldcs(pairs + list_index(kk, cap, (unsigned)i));
 }
 
+/* Calls f(kk, N, e, ahead) for rounds of N of the list entries sub, sub + TPP,
+   ... < n of particle i: entry kk + u TPP is e[u], u < N. AHEAD: rounds of U
+   entries, where those at or beyond n are the particle itself and do not count;
+   f calls ahead() once its gathers are issued, which fetches the next round's
+   entries. Without (32 registers are too few): rounds of U, of ACC and of 1. */
+template <int U, int TPP, int ACC, bool AHEAD, typename F>
+__device__ __forceinline__ void pair_rounds(const uint2* pairs, unsigned sub, unsigned n, unsigned cap, int i, F&& f)
+{
+    if (AHEAD) {
+        uint2 e[U];
+        const auto fetch = [&](unsigned kk, uint2(&to)[U]) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                to[u] = kk + u * TPP < n ? pair_at(pairs, kk + u * TPP, cap, i) : make_uint2((unsigned)i, 0u);
+        };
+        fetch(sub, e);
+        for (unsigned kk = sub; kk < n; kk += U * TPP) {
+            uint2 next[U];
+            f(kk, std::integral_constant<int, U>(), e, [&] { fetch(kk + U * TPP, next); });
+#pragma unroll
+            for (int u = 0; u < U; ++u) e[u] = next[u];
+        }
+    } else {
+        unsigned kk = sub;
+        const auto round = [&](auto count) {
+            constexpr int N = decltype(count)::value;
+            uint2 e[N];
+#pragma unroll
+            for (int u = 0; u < N; ++u) e[u] = pair_at(pairs, kk + u * TPP, cap, i);
+            f(kk, count, e, [] {});
+        };
+        for (; kk + (U - 1) * TPP < n; kk += U * TPP) round(std::integral_constant<int, U>());
+        for (; U > ACC && kk + (ACC - 1) * TPP < n; kk += ACC * TPP) round(std::integral_constant<int, ACC>());
+        if (ACC > 1 && kk < n) round(std::integral_constant<int, 1>());
+    }
+}
+
 /* One fluid term of the residual: m f (v_i - v_j) . r_ij */
 __device__ __forceinline__ float dfsph_residual_term(const SimParams& P, float4 xi, float4 vi, float4 xj, float4 vj,
                                                      float f)
@@ -560,7 +597,7 @@ __device__ __forceinline__ float dfsph_residual_term(const SimParams& P, float4 
    using any of them (more loads in flight per lane) and adds the terms in
    list order, so U changes no bit; TPP * ACC = 2 is one order of additions
    whichever way it is split. */
-template <int TPP, int ACC, int U>
+template <int TPP, int ACC, int U, bool AHEAD>
 __device__ __forceinline__ float dfsph_residual_part(const SimParams& P, const DeviceArrays& A, int i, int sub)
 {
     static_assert(U % ACC == 0, "an unrolled round holds whole rounds of partial sums");
@@ -570,21 +607,17 @@ __device__ __forceinline__ float dfsph_residual_part(const SimParams& P, const D
 #pragma unroll
     for (int c = 0; c < ACC; ++c) s[c] = 0.0f;
     const unsigned nF = A.cnt_f[i], nB = A.cnt_b[i];
-    const auto round = [&](unsigned kk, auto count) {
+    pair_rounds<U, TPP, ACC, AHEAD>(A.pair_f, (unsigned)sub, nF, P.capF, i,
+                                    [&](unsigned kk, auto count, const auto& e, auto ahead) {
         constexpr int N = decltype(count)::value;
-        uint2 e[N];
         float4 xj[N], vj[N];
 #pragma unroll
-        for (int u = 0; u < N; ++u) e[u] = pair_at(A.pair_f, kk + u * TPP, P.capF, i);
-#pragma unroll
         for (int u = 0; u < N; ++u) load_rec(A.rec, e[u].x, xj[u], vj[u]);
+        ahead();
 #pragma unroll
-        for (int u = 0; u < N; ++u) s[u % ACC] += dfsph_residual_term(P, xi, vi, xj[u], vj[u], __uint_as_float(e[u].y));
-    };
-    unsigned kk = sub;
-    for (; kk + (U - 1) * TPP < nF; kk += U * TPP) round(kk, std::integral_constant<int, U>());
-    for (; U > ACC && kk + (ACC - 1) * TPP < nF; kk += ACC * TPP) round(kk, std::integral_constant<int, ACC>());
-    if (ACC > 1 && kk < nF) round(kk, std::integral_constant<int, 1>());
+        for (int u = 0; u < N; ++u)
+            if (!AHEAD || kk + u * TPP < nF) s[u % ACC] += dfsph_residual_term(P, xi, vi, xj[u], vj[u], __uint_as_float(e[u].y));
+    });
     for (unsigned kk = sub; kk < nB; kk += TPP * ACC) {
 #pragma unroll
         for (int c = 0; c < ACC; ++c) {
@@ -619,7 +652,7 @@ __device__ __forceinline__ float dfsph_residual_finish(const SimParams& P, const
 template <bool DIV>
 __device__ __forceinline__ float dfsph_residual(const SimParams& P, const DeviceArrays& A, int i, float dt)
 {
-    return dfsph_residual_finish<DIV>(P, A, i, dfsph_residual_part<1, 1, 4>(P, A, i, 0), dt);
+    return dfsph_residual_finish<DIV>(P, A, i, dfsph_residual_part<1, 1, 4, true>(P, A, i, 0), dt);
 }
 
 /* Partial sums over list entries sub, sub + TPP, ... of
@@ -627,7 +660,7 @@ __device__ __forceinline__ float dfsph_residual(const SimParams& P, const Device
    U at a time and ACC interleaved sums, as in dfsph_residual_part. Position
    and k are in posd, written inside the same persistent kernel (before a grid
    barrier): a read-only (non-coherent) load path would be wrong for it. */
-template <int TPP, int ACC, int U>
+template <int TPP, int ACC, int U, bool AHEAD>
 __device__ __forceinline__ void dfsph_correct_part(const SimParams& P, const DeviceArrays& A, int i, int sub,
                                                    float& sx, float& sy, float& sz)
 {
@@ -639,29 +672,24 @@ __device__ __forceinline__ void dfsph_correct_part(const SimParams& P, const Dev
 #pragma unroll
     for (int c = 0; c < ACC; ++c) tx[c] = ty[c] = tz[c] = 0.0f;
     const unsigned nF = A.cnt_f[i];
-    const auto round = [&](unsigned kk, auto count) {
+    pair_rounds<U, TPP, ACC, AHEAD>(A.pair_f, (unsigned)sub, nF, P.capF, i,
+                                    [&](unsigned kk, auto count, const auto& e, auto ahead) {
         constexpr int N = decltype(count)::value;
-        uint2 e[N];
         float4 xj[N];
 #pragma unroll
-        for (int u = 0; u < N; ++u) e[u] = pair_at(A.pair_f, kk + u * TPP, P.capF, i);
-#pragma unroll
         for (int u = 0; u < N; ++u) xj[u] = xk[e[u].x];
+        ahead();
 #pragma unroll
         for (int u = 0; u < N; ++u) {
             const float ks = ki + xj[u].w;
-            if (fabsf(ks) > P.eps) {
+            if ((!AHEAD || kk + u * TPP < nF) && fabsf(ks) > P.eps) {
                 const float c = P.mass * ks * __uint_as_float(e[u].y);
                 tx[u % ACC] += c * (xi.x - xj[u].x);
                 ty[u % ACC] += c * (xi.y - xj[u].y);
                 tz[u % ACC] += c * (xi.z - xj[u].z);
             }
         }
-    };
-    unsigned kk = sub;
-    for (; kk + (U - 1) * TPP < nF; kk += U * TPP) round(kk, std::integral_constant<int, U>());
-    for (; U > ACC && kk + (ACC - 1) * TPP < nF; kk += ACC * TPP) round(kk, std::integral_constant<int, ACC>());
-    if (ACC > 1 && kk < nF) round(kk, std::integral_constant<int, 1>());
+    });
     if (fabsf(ki) > P.eps) {
         const unsigned nB = A.cnt_b[i];
         for (unsigned kk = sub; kk < nB; kk += TPP * ACC) {
@@ -702,7 +730,7 @@ __device__ __forceinline__ void dfsph_set_k(const DeviceArrays& A, int i, float 
 __device__ __forceinline__ void dfsph_correct(const SimParams& P, const DeviceArrays& A, int i, float dt)
 {
     float sx, sy, sz;
-    dfsph_correct_part<1, 1, 4>(P, A, i, 0, sx, sy, sz);
+    dfsph_correct_part<1, 1, 4, true>(P, A, i, 0, sx, sy, sz);
     dfsph_apply(A, i, dt, sx, sy, sz);
 }
 
@@ -743,22 +771,22 @@ __device__ __forceinline__ void for_particles(int n, F&& f)
 }
 
 /* residual of particle i with its list split over TPP lanes (all lanes call) */
-template <bool DIV, int TPP, int ACC, int U>
+template <bool DIV, int TPP, int ACC, int U, bool AHEAD>
 __device__ __forceinline__ float dfsph_residual_lanes(const SimParams& P, const DeviceArrays& A, int i, int sub,
                                                       bool valid, float dt)
 {
-    float part = valid ? dfsph_residual_part<TPP, ACC, U>(P, A, i, sub) : 0.0f;
+    float part = valid ? dfsph_residual_part<TPP, ACC, U, AHEAD>(P, A, i, sub) : 0.0f;
     if (TPP > 1) part = lane_group_sum<TPP>(part);
     return valid ? dfsph_residual_finish<DIV>(P, A, i, part, dt) : 0.0f;
 }
 
 /* velocity correction of particle i with its list split over TPP lanes */
-template <int TPP, int ACC, int U>
+template <int TPP, int ACC, int U, bool AHEAD>
 __device__ __forceinline__ void dfsph_correct_lanes(const SimParams& P, const DeviceArrays& A, int i, int sub,
                                                     bool valid, float dt)
 {
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-    if (valid) dfsph_correct_part<TPP, ACC, U>(P, A, i, sub, sx, sy, sz);
+    if (valid) dfsph_correct_part<TPP, ACC, U, AHEAD>(P, A, i, sub, sx, sy, sz);
     if (TPP > 1) {
         sx = lane_group_sum<TPP>(sx);
         sy = lane_group_sum<TPP>(sy);
@@ -768,17 +796,21 @@ __device__ __forceinline__ void dfsph_correct_lanes(const SimParams& P, const De
 }
 
 /* What bounds the passes: the L1's rate for scattered gathers. A warp-visit
-   (32 lanes, one list entry each) takes ~26 SM cycles whatever the occupancy
+   (32 lanes, one list entry each) touches ~20 lines and takes ~24 SM cycles whatever the occupancy
    (8, 6, 5, 4 blocks per SM), and halving its instructions by reading the
    kernel factor f from pair_f instead of recomputing it (rsqrt, spline) alone
    left the 1M pass at 107 us. What helped, per pass on the 1M double dam break
-   in motion (5.5 + 1.25 iterations per step), density solver 1,424 -> 1,126 us
+   in motion (5.5 + 1.25 iterations per step), density solver 1,424 -> 1,030 us
    per step: a neighbour's position and velocity in one record, fetched with
    one 256-bit load (109 -> 104 us); lists in contiguous tiles of 32 particles
    (104 -> 98); one lane per particle with 64 registers and four gathers in
    flight (98 -> 95); candidates in z-fastest order and a barrier of fewer round
    trips (-4 %); position and k of the correction in 16 bytes of their own
-   instead of half of the record (1,187 -> 1,126; 125k 184 -> 171).
+   instead of half of the record (1,187 -> 1,126; 125k 184 -> 171); the next
+   round's list entries fetched while the gathers of this one are on their way,
+   and one masked round at the end of a list instead of rounds of 2 and 1
+   (1,126 -> 1,030; 125k 171 -> 163; 24 batched scenes 183 -> 158; with 3 blocks
+   and 4, 6, 8 gathers 1,071, 1,210, 1,335; in 32 registers it spills and loses).
    OCC blocks of 256 per SM: 4 (64 registers) by default, 8 (32 registers, two
    gathers) is the autotuner's other candidate. TPP lanes share a particle;
    1 and 2 lanes add the same two interleaved sums, so they agree bit for bit. */
@@ -786,6 +818,7 @@ template <bool DIV, int OCC, int TPP>
 __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, DeviceArrays A)
 {
     constexpr int U = OCC == 4 ? 4 : 2;
+    constexpr bool AHEAD = OCC == 4;
     constexpr int ACC = TPP == 1 ? 2 : 1;
     __shared__ double s_red[32];
     DevState* st = A.st;
@@ -835,14 +868,14 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
        only where the residual is positive */
     for_particles<TPP>(nfi, [&](int i, int sub, bool valid) {
         const float r = DIV ? (valid ? A.divres[i] : 0.0f)
-                            : dfsph_residual_lanes<DIV, TPP, ACC, U>(P, A, i, sub, valid, dt);
+                            : dfsph_residual_lanes<DIV, TPP, ACC, U, AHEAD>(P, A, i, sub, valid, dt);
         if (valid && sub == 0) {
             if (DIV) dfsph_set_k(A, i, r > 0.0f ? kws[i] / dt : 0.0f);
             else dfsph_set_k(A, i, r > P.rho0 ? kws[i] / ts2 : 0.0f);
         }
     });
     if (!bar.sync()) return;
-    for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U>(P, A, i, sub, valid, dt); });
+    for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U, AHEAD>(P, A, i, sub, valid, dt); });
     if (!bar.sync()) return;
 
     const double limit = DIV ? (double)(P.eta_v / dt) : (double)P.eta;
@@ -855,7 +888,7 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
     while ((avg > limit || it < min_it) && it < max_it) {
         double local = 0.0;
         for_particles<TPP>(nfi, [&](int i, int sub, bool valid) {
-            const float r = dfsph_residual_lanes<DIV, TPP, ACC, U>(P, A, i, sub, valid, dt);
+            const float r = dfsph_residual_lanes<DIV, TPP, ACC, U, AHEAD>(P, A, i, sub, valid, dt);
             if (!valid || sub != 0) return;
             float k;
             if (DIV) {
@@ -872,7 +905,7 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
         if (threadIdx.x == 0) atomicAdd(&A.accum[it], bs);
         if (!bar.sync()) return;
         avg = *(volatile double*)&A.accum[it] / (double)nfi;
-        for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U>(P, A, i, sub, valid, dt); });
+        for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U, AHEAD>(P, A, i, sub, valid, dt); });
         if (!bar.sync()) return;
         ++it;
     }
