@@ -55,58 +55,78 @@ __device__ __forceinline__ Pair make_pair(float4 a, float4 b)
     return p;
 }
 
-/* Calls f(kk, j, x_j) for the fluid neighbours (list entry kk) of sorted particle i in list
-   order, issuing the list loads and position gathers of U entries before the
-   first of them is used (more loads in flight per thread; same order, so the
-   sums it feeds are unchanged). With TPP lanes per particle, lane sub visits
-   the entries sub, sub + TPP, ... */
-template <int U, int TPP = 1, typename F>
-__device__ __forceinline__ void for_fluid_neighbors(const SimParams& P, const DeviceArrays& A, int i, unsigned n, F&& f,
-                                                    unsigned sub = 0)
+/* Calls f(kk, j, x_j, v_j) for the fluid list of particle i in list order (v_j 0
+   without VEL). Rounds of U entries whose gathers are issued before the first of
+   them is used, the next round's entries fetched meanwhile: a round that first
+   waits for its entries and then for its gathers has two latencies in a row. The
+   order of the calls does not change, nor do the sums they feed. */
+template <int U, bool VEL = false, typename F>
+__device__ __forceinline__ void for_fluid_neighbors(const SimParams& P, const DeviceArrays& A, int i, unsigned n, F&& f)
 {
-    unsigned kk = sub;
-    for (; kk + (U - 1) * TPP < n; kk += U * TPP) {
-        unsigned jj[U];
-        float4 xj[U];
+    const auto fetch = [&](unsigned kk, unsigned(&to)[U]) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) jj[u] = list_at(A.nbr_f, kk + u * TPP, P.capF, i);
+        for (int u = 0; u < U; ++u) to[u] = kk + u < n ? list_at(A.nbr_f, kk + u, P.capF, i) : (unsigned)i;
+    };
+    const auto velocity = [&](unsigned j) { return VEL ? A.vel[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f); };
+    unsigned jj[U];
+    fetch(0u, jj);
+    unsigned kk = 0;
+    for (; kk + (U - 1) < n; kk += U) {
+        unsigned next[U];
+        float4 xj[U], vj[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) xj[u] = A.pos[jj[u]];
+        if (VEL) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) f(kk + u * TPP, jj[u], xj[u]);
+            for (int u = 0; u < U; ++u) vj[u] = A.vel[jj[u]];
+        }
+        fetch(kk + U, next);
+#pragma unroll
+        for (int u = 0; u < U; ++u) f(kk + u, jj[u], xj[u], vj[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) jj[u] = next[u];
     }
-    for (; kk < n; kk += TPP) {
-        const unsigned j = list_at(A.nbr_f, kk, P.capF, i);
-        f(kk, j, A.pos[j]);
-    }
+#pragma unroll
+    for (int u = 0; u + 1 < U; ++u)
+        if (kk + u < n) f(kk + u, jj[u], A.pos[jj[u]], velocity(jj[u]));
 }
 
 /* for_fluid_neighbors over the records: f(place, j, (x_j, w), (v_j, w)) with
-   the entry's place: 0 even or 1 odd in an unrolled round, 2 after the rounds. */
+   the entry's place: 0 even or 1 odd in an unrolled round, 2 after the rounds.
+   With TPP lanes per particle, lane sub visits the entries sub, sub + TPP, ... */
 template <int U, int TPP, typename F>
 __device__ __forceinline__ void for_fluid_records(const SimParams& P, const DeviceArrays& A, int i, unsigned n, F&& f,
                                                   unsigned sub)
 {
+    const auto fetch = [&](unsigned kk, unsigned(&to)[U]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            to[u] = kk + u * TPP < n ? list_at(A.nbr_f, kk + u * TPP, P.capF, i) : (unsigned)i;
+    };
+    unsigned jj[U];
+    fetch(sub, jj);
     unsigned kk = sub;
     for (; kk + (U - 1) * TPP < n; kk += U * TPP) {
-        unsigned jj[U];
+        unsigned next[U];
         float4 a[U], b[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) jj[u] = list_at(A.nbr_f, kk + u * TPP, P.capF, i);
-#pragma unroll
         for (int u = 0; u < U; ++u) load_rec(A.rec, jj[u], a[u], b[u]);
+        fetch(kk + U * TPP, next);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             if (u % 2 == 0) f(std::integral_constant<int, 0>(), jj[u], a[u], b[u]);
             else f(std::integral_constant<int, 1>(), jj[u], a[u], b[u]);
         }
+#pragma unroll
+        for (int u = 0; u < U; ++u) jj[u] = next[u];
     }
-    for (; kk < n; kk += TPP) {
-        const unsigned j = list_at(A.nbr_f, kk, P.capF, i);
-        float4 a, b;
-        load_rec(A.rec, j, a, b);
-        f(std::integral_constant<int, 2>(), j, a, b);
-    }
+#pragma unroll
+    for (int u = 0; u + 1 < U; ++u)
+        if (kk + u * TPP < n) {
+            float4 a, b;
+            load_rec(A.rec, jj[u], a, b);
+            f(std::integral_constant<int, 2>(), jj[u], a, b);
+        }
 }
 
 /* Sum over the TPP adjacent lanes of a particle's lane group. */
@@ -211,9 +231,13 @@ __device__ __forceinline__ float boundary_density(const SimParams& P, const Devi
    (DFSPHSolver::computeDivergenceError, DFSPHSolver.cpp:538-621), which the
    divergence solver's warm start reads (A.divres) instead of spending a
    neighbour pass on it: the velocities do not change between this pass
-   and that solver. */
+   and that solver. Bound by gathers and their latency,
+   and with alpha by its arithmetic too: with alpha 5 blocks per SM (nothing
+   spilled) and the velocities gathered with the positions, 1M 189 -> 178 us,
+   26k 37 -> 31 (6 blocks 190, 4 181; rounds of 4 190 to 223); densities alone
+   at 8 blocks, 1M 91 -> 84 (6 blocks 97). */
 template <bool ALPHA, bool EOS, bool DIVRES = false>
-__global__ void __launch_bounds__(256, 8) k_density(SimParams P, DeviceArrays A)
+__global__ void __launch_bounds__(256, ALPHA ? 5 : 8) k_density(SimParams P, DeviceArrays A)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= active_n(P, A.st)) return;
@@ -221,7 +245,7 @@ __global__ void __launch_bounds__(256, 8) k_density(SimParams P, DeviceArrays A)
     const float4 vi = DIVRES ? A.vel[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float rho = 0.0f, sgx = 0.0f, sgy = 0.0f, sgz = 0.0f, ssq = 0.0f, div = 0.0f;
     const unsigned nF = A.cnt_f[i];
-    for_fluid_neighbors<2>(P, A, i, nF, [&](unsigned kk, unsigned j, const float4& xj) {
+    for_fluid_neighbors<2, DIVRES>(P, A, i, nF, [&](unsigned kk, unsigned j, const float4& xj, const float4& vj) {
         rho = __fadd_rn(rho, __fmul_rn(P.mass, cs_W_exact(dist2_exact(xi, xj), P)));
         if (ALPHA) {
             const Pair p = make_pair(xi, xj);
@@ -232,7 +256,6 @@ __global__ void __launch_bounds__(256, 8) k_density(SimParams P, DeviceArrays A)
             sgx += gx; sgy += gy; sgz += gz;
             ssq += (gx * gx + gy * gy) + gz * gz;
             if (DIVRES) {
-                const float4 vj = A.vel[j];
                 div += P.mass * (fg * (((vi.x - vj.x) * p.rx + (vi.y - vj.y) * p.ry) + (vi.z - vj.z) * p.rz));
             }
         }
@@ -275,7 +298,7 @@ __global__ void __launch_bounds__(256) k_pair_factors(SimParams P, DeviceArrays 
     if (i >= active_n(P, A.st)) return;
     const float4 xi = A.pos[i];
     const unsigned nF = A.cnt_f[i], nB = A.cnt_b[i];
-    for_fluid_neighbors<2>(P, A, i, nF, [&](unsigned kk, unsigned j, const float4& xj) {
+    for_fluid_neighbors<2>(P, A, i, nF, [&](unsigned kk, unsigned j, const float4& xj, const float4&) {
         const Pair p = make_pair(xi, xj);
         __stcs(A.pair_f + list_index(kk, P.capF, i), make_uint2(j, __float_as_uint(cs_gradf(p.rl, p.inv_rl, P))));
     });
@@ -344,9 +367,11 @@ __global__ void __launch_bounds__(256, 4) k_normals(SimParams P, DeviceArrays A)
    the L1's rate for scattered gathers (69 % of its wavefronts) and their
    latency. Records, and 64 registers so that nothing is spilled: 306k with
    standard viscosity, surface tension and adhesion 134 -> 88 us, 64 batched
-   scenes 164 -> 122, 125k DFSPH 48 -> 34. TPP adjacent lanes share particle i (small scenes), each summing the list entries sub, sub + TPP,
-   ...; the group's sums are combined by shuffles and lane 0 of the group
-   finishes the particle. */
+   scenes 164 -> 122, 125k DFSPH 48 -> 36; the next round's list entries fetched
+   ahead: 88 -> 74, 124 -> 101, 36 -> 33, 1M DFSPH 158 -> 123. TPP adjacent
+   lanes share particle i (small scenes), each summing the list entries sub,
+   sub + TPP, ...; the group's sums are combined by shuffles and lane 0 of the
+   group finishes the particle. */
 template <int MODE, int TPP = 1>
 __device__ __forceinline__ void forces_at(const SimParams& P, const DeviceArrays& A, int t, bool first_thread,
                                           float* s_red)
