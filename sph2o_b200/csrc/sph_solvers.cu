@@ -1337,7 +1337,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
             float ax = 0.0f, ay = 0.0f, az = 0.0f;
             const unsigned nF = A.cnt_f[i], nB = A.cnt_b[i];
             if (it == 0) {
-                constexpr int U = 4; /* gathers issued before the first is used */
+                constexpr int U = 4; /* gathers issued before the first is used, the next entries meanwhile */
                 const auto term = [&](unsigned kk, unsigned j, const float4& xj) {
                     float gx, gy, gz;
                     cs_gradW_exact(__fsub_rn(xi.x, xj.x), __fsub_rn(xi.y, xj.y), __fsub_rn(xi.z, xj.z), P, gx, gy, gz);
@@ -1347,21 +1347,27 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
                     ay = __fsub_rn(ay, __fmul_rn(c, gy));
                     az = __fsub_rn(az, __fmul_rn(c, gz));
                 };
+                unsigned j[U];
+                const auto fetch = [&](unsigned kk, unsigned(&to)[U]) {
+#pragma unroll
+                    for (int u = 0; u < U; ++u) to[u] = kk + u < nF ? list_at(A.nbr_f, kk + u, P.capF, i) : (unsigned)i;
+                };
+                fetch(0u, j);
                 unsigned kk = 0;
-                for (; kk + U <= nF; kk += U) {
-                    unsigned j[U];
+                for (; kk + (U - 1) < nF; kk += U) {
+                    unsigned next[U];
                     float4 xj[U];
 #pragma unroll
-                    for (int u = 0; u < U; ++u) j[u] = list_at(A.nbr_f, kk + u, P.capF, i);
-#pragma unroll
                     for (int u = 0; u < U; ++u) xj[u] = A.posd[j[u]];
+                    fetch(kk + U, next);
 #pragma unroll
                     for (int u = 0; u < U; ++u) term(kk + u, j[u], xj[u]);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) j[u] = next[u];
                 }
-                for (; kk < nF; ++kk) {
-                    const unsigned j = list_at(A.nbr_f, kk, P.capF, i);
-                    term(kk, j, A.posd[j]);
-                }
+#pragma unroll
+                for (int u = 0; u + 1 < U; ++u)
+                    if (kk + u < nF) term(kk + u, j[u], A.posd[j[u]]);
             } else {
                 const float* dp = reinterpret_cast<const float*>(A.posd) + 3;
 #pragma unroll 4
