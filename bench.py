@@ -538,7 +538,7 @@ def neighbor_search_roofline(nf, entries, prof, steps, peak, peak_kind):
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "peak_kind": f"of {peak_kind}", "algorithmic_bytes_per_step": algo, "ms_per_step": ms,
             "list_entries_per_particle": entries / nf,
-            "kernels": "k_ns_count, scan, k_ns_scatter, k_ns_rank_gather (sort); k_ns_build_lists (lists)"}
+            "kernels": "k_ns_count, k_scan, k_ns_scatter, k_ns_rank_gather (sort); k_search (lists)"}
 
 
 def pair_evaluations(entries, its, itsv, prof, steps, window_ms, surface_tension=False):

@@ -1,10 +1,11 @@
 /*
  * Particle-pass kernels of the WCSPH / PCISPH / DFSPH steps (sm_100a).
  *
- * Every pass is one thread per fluid particle walking that particle's
- * neighbour lists (built once per step by sph_grid.cu); positions and
- * velocities of neighbours are gathered as float4 from the cell-sorted
- * arrays, so a warp's gathers fall on a few cache lines of nearby cells.
+ * Every pass walks the neighbour lists of the fluid particles (built once per
+ * step by sph_grid.cu), one lane per particle or, in small scenes, a few;
+ * neighbours come as records of 16 or 32 bytes from the cell-sorted arrays, and
+ * the list entries of the next round are fetched while a round's gathers are on
+ * their way: the L1's rate for scattered gathers and their latency bound them.
  * The DFSPH and PCISPH iteration loops each run as ONE persistent,
  * cooperative kernel: phases are separated by a bounded grid barrier and
  * the convergence residual is reduced in FP64 on the device (warp shuffles,
@@ -36,7 +37,6 @@
 #include "sph_internal.h"
 
 #include <type_traits>
-
 
 namespace sph {
 
