@@ -653,6 +653,20 @@ int status_from_state(sph_ctx* c, const DevState& s)
     return SPH_OK;
 }
 
+/* Fills lists that were allocated anew. WCSPH and PCISPH search at the start
+   of every step; a DFSPH step starts with passes over the lists, densities and
+   alpha of the last search, which are built again here: from the positions and
+   the cell table of that search, without a sort. Where cubes moved particles
+   since, the densities stay those of the search (see step_dfsph). */
+int rebuild_lists(sph_ctx* c)
+{
+    if (c->desc.simulation_method != SPH_DFSPH) return SPH_OK;
+    launch_search(c->P, SceneRef{c->d_scenes, c->d_scene_of}, arrays(c), SEARCH_LISTS, c->stream);
+    if (c->cubes.empty()) launch_density(c->P, arrays(c), true, false, c->pass_block, c->stream);
+    else launch_pair_factors(c->P, arrays(c), c->stream);
+    return check_launch(c, "list rebuild");
+}
+
 /* After an overflow: clear the flag and grow the lists for later steps. */
 int recover_overflow(sph_ctx* c)
 {
@@ -674,7 +688,8 @@ int recover_overflow(sph_ctx* c)
     c->P.capF = c->P.capF + c->P.capF / 2;
     c->P.capB = c->P.capB + c->P.capB / 2;
     c->lists_valid = false;
-    return alloc_lists(c);
+    const int rc = alloc_lists(c);
+    return rc != SPH_OK ? rc : rebuild_lists(c);
 }
 
 int fill_stats(sph_ctx* c, const DevState& before, const DevState& now, sph_step_stats* out)
