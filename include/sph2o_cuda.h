@@ -363,10 +363,16 @@ int sph_debug_neighbors(sph_ctx* ctx, unsigned* f_offsets, unsigned* f_index, si
 
 /* Test hook for the bounded device-side waits (no reference counterpart):
    launches a two-block cooperative kernel in which one block never reaches
-   the grid barrier. The waiting block gives up after its spin limit (about
-   a second), records the timeout and returns; the call then reports
+   the grid barrier. The waiting block gives up after its spin limit (some
+   seconds), records the timeout and returns; the call then reports
    SPH_ERR_TIMEOUT and clears the flag, leaving the context usable. */
 int sph_debug_barrier_timeout(sph_ctx* ctx);
+
+/* Test hook for a full GPU (no reference counterpart): from now on an
+   allocation that would take this context's device memory above `limit` bytes
+   fails as one fails for which the GPU has no room; 0 (default): no limit. The
+   bytes held now are returned in *held (may be NULL). */
+int sph_debug_limit_memory(sph_ctx* ctx, size_t limit, size_t* held);
 
 /* ---- allocation-free density evaluation ------------------------------- */
 

@@ -114,6 +114,7 @@ def lib():
         "sph_debug_neighbors": (I, [P, C.POINTER(U), C.POINTER(U), C.c_size_t, C.POINTER(U), C.POINTER(U),
                                     C.c_size_t, C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]),
         "sph_debug_barrier_timeout": (I, [P]),
+        "sph_debug_limit_memory": (I, [P, C.c_size_t, C.POINTER(C.c_size_t)]),
         "sph_set_option": (I, [P, I, I]),
         "sph_get_option": (I, [P, I, C.POINTER(I)]),
         "sph_autotune": (I, [P, I, C.c_char_p, C.POINTER(I)]),

@@ -56,7 +56,10 @@ struct sph_ctx {
     bool initialized = false;
     unsigned nf = 0, nb = 0;
     std::vector<float> h_fluid, h_vel, h_bound;
-    std::vector<void*> allocations;
+    struct Allocation { void* p; size_t bytes; };
+    std::vector<Allocation> allocations;
+    size_t held = 0;        /* bytes in allocations */
+    size_t held_limit = 0;  /* sph_debug_limit_memory; 0: none */
 
     /* current / spare buffers (swapped by the neighbour-search sort) */
     float4 *pos = nullptr, *vel = nullptr, *pos2 = nullptr, *vel2 = nullptr;
@@ -201,19 +204,38 @@ template <typename T> int dalloc(sph_ctx* c, T** p, size_t count)
 {
     void* v = nullptr;
     const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
-    cudaError_t e = cudaMalloc(&v, bytes);
-    if (e != cudaSuccess) return fail(c, SPH_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    cudaError_t e = c->held_limit && bytes > c->held_limit - std::min(c->held, c->held_limit) ? cudaErrorMemoryAllocation
+                                                                                              : cudaMalloc(&v, bytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError(); /* the caller gets it here: later launch checks should not find it again */
+        return fail(c, SPH_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
+    c->allocations.push_back({v, bytes});
+    c->held += bytes;
     e = cudaMemsetAsync(v, 0, bytes, c->stream);
     if (e != cudaSuccess) return fail(c, SPH_ERR_CUDA, std::string("cudaMemset: ") + cudaGetErrorString(e));
-    c->allocations.push_back(v);
     *p = static_cast<T*>(v);
     return SPH_OK;
 }
 
+/* Frees one allocation of the context and clears the pointer to it. */
+template <typename T> void dfree(sph_ctx* c, T*& p)
+{
+    const auto it = std::find_if(c->allocations.begin(), c->allocations.end(),
+                                 [&](const sph_ctx::Allocation& a) { return a.p == (void*)p; });
+    if (p && it != c->allocations.end()) {
+        cudaFree(p);
+        c->held -= it->bytes;
+        c->allocations.erase(it);
+    }
+    p = nullptr;
+}
+
 void free_all(sph_ctx* c)
 {
-    for (void* p : c->allocations) cudaFree(p);
+    for (const auto& a : c->allocations) cudaFree(a.p);
     c->allocations.clear();
+    c->held = 0;
     if (c->st_host) { cudaFreeHost(c->st_host); c->st_host = nullptr; }
 }
 
@@ -434,19 +456,27 @@ void drain_profile(sph_ctx* c)
     c->pending.clear();
 }
 
+void drop_lists(sph_ctx* c)
+{
+    dfree(c, c->nbr_f); dfree(c, c->nbr_b);
+    dfree(c, c->pair_f); dfree(c, c->pair_b);
+    dfree(c, c->pgrad);
+}
+
+/* The neighbour lists and what is kept beside their entries, for the capacities
+   in c->P: all of them, or none. */
 int alloc_lists(sph_ctx* c)
 {
+    const size_t nf_entries = list_len(c->nf, c->P.capF), nb_entries = list_len(c->nf, c->P.capB);
     int rc;
-    if ((rc = dalloc(c, &c->nbr_f, list_len(c->nf, c->P.capF))) != SPH_OK) return rc;
-    if ((rc = dalloc(c, &c->nbr_b, list_len(c->nf, c->P.capB))) != SPH_OK) return rc;
+    if ((rc = dalloc(c, &c->nbr_f, nf_entries)) == SPH_OK) rc = dalloc(c, &c->nbr_b, nb_entries);
     if (c->desc.simulation_method == SPH_DFSPH) {
-        if ((rc = dalloc(c, &c->pair_f, list_len(c->nf, c->P.capF))) != SPH_OK) return rc;
-        if ((rc = dalloc(c, &c->pair_b, list_len(c->nf, c->P.capB))) != SPH_OK) return rc;
+        if (rc == SPH_OK) rc = dalloc(c, &c->pair_f, nf_entries);
+        if (rc == SPH_OK) rc = dalloc(c, &c->pair_b, nb_entries);
     }
-    if (c->desc.simulation_method == SPH_PCISPH &&
-        (rc = dalloc(c, &c->pgrad, list_len(c->nf, c->P.capF))) != SPH_OK)
-        return rc;
-    return SPH_OK;
+    if (c->desc.simulation_method == SPH_PCISPH && rc == SPH_OK) rc = dalloc(c, &c->pgrad, nf_entries);
+    if (rc != SPH_OK) drop_lists(c);
+    return rc;
 }
 
 /* Sort the fluid into cells, rebuild the neighbour lists and compute what
@@ -667,7 +697,19 @@ int rebuild_lists(sph_ctx* c)
     return check_launch(c, "list rebuild");
 }
 
-/* After an overflow: clear the flag and grow the lists for later steps. */
+/* Before anything that reads or writes the lists: a context whose lists could
+   not be allocated after an overflow holds none, and asks again here. */
+int ensure_lists(sph_ctx* c)
+{
+    if (c->nbr_f) return SPH_OK;
+    const int rc = alloc_lists(c);
+    return rc != SPH_OK ? rc : rebuild_lists(c);
+}
+
+/* After an overflow: clear the flag and grow the lists for later steps. Where
+   the larger lists do not fit, the lists keep their capacity, and where not even
+   these can be had again (another program took the memory) the context has none
+   until they can (ensure_lists). */
 int recover_overflow(sph_ctx* c)
 {
     int zero = 0;
@@ -675,21 +717,19 @@ int recover_overflow(sph_ctx* c)
     CUDA_TRY(c, cudaMemcpyAsync(&c->st->err, &zero, sizeof(int), cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(c, cudaMemcpyAsync(&c->st->overflow, &uzero, sizeof(unsigned), cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-    auto drop = [&](void* p) {
-        auto it = std::find(c->allocations.begin(), c->allocations.end(), p);
-        if (it != c->allocations.end()) { cudaFree(p); c->allocations.erase(it); }
-    };
     drop_graphs(c);
-    drop(c->nbr_f);
-    drop(c->nbr_b);
-    drop(c->pair_f);
-    drop(c->pair_b);
-    drop(c->pgrad);
-    c->P.capF = c->P.capF + c->P.capF / 2;
-    c->P.capB = c->P.capB + c->P.capB / 2;
+    drop_lists(c);
     c->lists_valid = false;
-    const int rc = alloc_lists(c);
-    return rc != SPH_OK ? rc : rebuild_lists(c);
+    const unsigned capF = c->P.capF, capB = c->P.capB;
+    c->P.capF = capF + capF / 2;
+    c->P.capB = capB + capB / 2;
+    int rc = alloc_lists(c);
+    if (rc == SPH_OK) return rebuild_lists(c);
+    const std::string why = "neighbour list capacity exceeded, and there is no room for larger lists: " + c->err;
+    c->P.capF = capF;
+    c->P.capB = capB;
+    if (ensure_lists(c) == SPH_OK) return fail(c, rc, why);
+    return fail(c, rc, why + "; the present ones were given up too, later calls try again");
 }
 
 int fill_stats(sph_ctx* c, const DevState& before, const DevState& now, sph_step_stats* out)
@@ -1254,6 +1294,7 @@ int sph_step_async(sph_ctx* c, int nsteps)
     if (!c) return SPH_ERR_ARG;
     if (!c->initialized) return fail(c, SPH_ERR_STATE, "sph_step before sph_init");
     if (nsteps < 0) return fail(c, SPH_ERR_ARG, "negative step count");
+    if (const int rl = ensure_lists(c); rl != SPH_OK) return rl;
     if (!c->batch_open) {
         CUDA_TRY(c, cudaEventRecord(c->ev_begin, c->stream));
         c->batch_open = true;
@@ -1369,7 +1410,7 @@ int sph_set_state(sph_ctx* c, const float* xyz, const float* v)
     const size_t nf = c->nf;
     unsigned na = 0;
     int rc0 = active_count(c, &na);
-    if (rc0 != SPH_OK) return rc0;
+    if (rc0 != SPH_OK || (rc0 = ensure_lists(c)) != SPH_OK) return rc0;
     float* tmp = c->stage;
     if (xyz) {
         CUDA_TRY(c, cudaMemcpyAsync(tmp, xyz, 3 * nf * sizeof(float), cudaMemcpyHostToDevice, c->stream));
@@ -1503,7 +1544,7 @@ int sph_compute_phase(sph_ctx* c, int phase, float* out)
         return fail(c, SPH_ERR_ARG, "pressure phases exist for WCSPH only");
     unsigned na = 0;
     int rc = active_count(c, &na);
-    if (rc != SPH_OK) return rc;
+    if (rc != SPH_OK || (rc = ensure_lists(c)) != SPH_OK) return rc;
     const bool eos = phase == SPH_PHASE_PRESSURE || phase == SPH_PHASE_PRESSURE_ACC;
     const bool alpha = phase == SPH_PHASE_ALPHA || c->desc.simulation_method == SPH_DFSPH;
     if ((rc = neighbor_search(c, alpha ? SEARCH_LISTS : eos ? SEARCH_EOS : SEARCH_DENSITY)) != SPH_OK) return rc;
@@ -1579,6 +1620,8 @@ int refresh(sph_ctx* c)
 
 int apply_cell_order(sph_ctx* c, int order)
 {
+    int rc = ensure_lists(c);
+    if (rc != SPH_OK) return rc;
     c->P.cell_order = order;
     if (c->nscenes) {
         for (auto& si : c->h_scenes) si.grid.order = order;
@@ -1586,8 +1629,7 @@ int apply_cell_order(sph_ctx* c, int order)
                                     cudaMemcpyHostToDevice, c->stream));
     }
     drop_graphs(c);
-    int rc = resort_boundary(c);
-    if (rc != SPH_OK) return rc;
+    if ((rc = resort_boundary(c)) != SPH_OK) return rc;
     return refresh(c);
 }
 
@@ -1596,14 +1638,19 @@ int snapshot(sph_ctx* c, bool save)
     const size_t nf = c->nf;
     int rc;
     if (!c->snap_pos) {
-        if ((rc = dalloc(c, &c->snap_pos, nf)) != SPH_OK) return rc;
-        if ((rc = dalloc(c, &c->snap_vel, nf)) != SPH_OK) return rc;
-        if ((rc = dalloc(c, &c->snap_orig, nf)) != SPH_OK) return rc;
-        if ((rc = dalloc(c, &c->snap_kws, nf)) != SPH_OK) return rc;
-        if ((rc = dalloc(c, &c->snap_kvws, nf)) != SPH_OK) return rc;
-        if ((rc = dalloc(c, &c->snap_rho, nf)) != SPH_OK) return rc;
-        if ((rc = dalloc(c, &c->snap_st, 1)) != SPH_OK) return rc;
-        if (c->nscenes && (rc = dalloc(c, &c->snap_sst, c->nscenes)) != SPH_OK) return rc;
+        /* the position last: without it a later call allocates all of them again */
+        const auto alloc = [&](auto*& p, size_t n) {
+            dfree(c, p);
+            return dalloc(c, &p, n);
+        };
+        if ((rc = alloc(c->snap_vel, nf)) != SPH_OK) return rc;
+        if ((rc = alloc(c->snap_orig, nf)) != SPH_OK) return rc;
+        if ((rc = alloc(c->snap_kws, nf)) != SPH_OK) return rc;
+        if ((rc = alloc(c->snap_kvws, nf)) != SPH_OK) return rc;
+        if ((rc = alloc(c->snap_rho, nf)) != SPH_OK) return rc;
+        if ((rc = alloc(c->snap_st, 1)) != SPH_OK) return rc;
+        if (c->nscenes && (rc = alloc(c->snap_sst, c->nscenes)) != SPH_OK) return rc;
+        if ((rc = alloc(c->snap_pos, nf)) != SPH_OK) return rc;
     }
     auto cp = [&](void* a, void* b, size_t bytes) -> int {
         CUDA_TRY(c, cudaMemcpyAsync(save ? b : a, save ? a : b, bytes, cudaMemcpyDeviceToDevice, c->stream));
@@ -1778,7 +1825,7 @@ int sph_autotune(sph_ctx* c, int trial_steps, const char* cache_path, int* confi
         if (config) for (int i = 0; i < SPH_TUNE_COUNT; ++i) config[i] = best[i];
         return SPH_OK;
     }
-    if ((rc = snapshot(c, true)) != SPH_OK) return rc;
+    if ((rc = ensure_lists(c)) != SPH_OK || (rc = snapshot(c, true)) != SPH_OK) return rc;
     const DevState last = c->last;
     const std::vector<SceneState> last_sst = c->last_sst;
     const bool graphs = c->use_graphs;
@@ -1939,13 +1986,21 @@ int sph_debug_barrier_timeout(sph_ctx* c)
     return SPH_OK;
 }
 
+int sph_debug_limit_memory(sph_ctx* c, size_t limit, size_t* held)
+{
+    if (!c) return SPH_ERR_ARG;
+    c->held_limit = limit;
+    if (held) *held = c->held;
+    return SPH_OK;
+}
+
 int sph_debug_neighbors(sph_ctx* c, unsigned* f_offsets, unsigned* f_index, size_t f_cap, unsigned* b_offsets,
                         unsigned* b_index, size_t b_cap, size_t* nf_total, size_t* nb_total)
 {
     if (!c) return SPH_ERR_ARG;
     if (!c->initialized) return fail(c, SPH_ERR_STATE, "sph_debug_neighbors before sph_init");
-    int rc = neighbor_search(c);
-    if (rc != SPH_OK) return rc;
+    int rc = ensure_lists(c);
+    if (rc != SPH_OK || (rc = neighbor_search(c)) != SPH_OK) return rc;
     if (c->pair_f) launch_pair_factors(c->P, arrays(c), c->stream); /* the next DFSPH step reads them */
     const size_t nf = c->nf, nb = c->nb;
     std::vector<unsigned> cntf(nf), cntb(nf), orig(nf), borig(nb);
@@ -2002,16 +2057,6 @@ namespace {
 
 constexpr size_t kAdjointListBudget = size_t(8) << 30;
 
-void dfree(sph_ctx* c, void* p)
-{
-    if (!p) return;
-    auto it = std::find(c->allocations.begin(), c->allocations.end(), p);
-    if (it != c->allocations.end()) {
-        cudaFree(p);
-        c->allocations.erase(it);
-    }
-}
-
 int adj_supported(sph_ctx* c)
 {
     if (c->nscenes) return fail(c, SPH_ERR_ARG, "the WCSPH adjoint applies to a single scene, not to a batch");
@@ -2032,18 +2077,25 @@ int adj_reserve(sph_ctx* c, int nseg, int every)
     auto& a = c->adj;
     const size_t nf = c->nf;
     int rc;
-#define AALLOC(ptr, count) if ((rc = dalloc(c, &a.ptr, (count))) != SPH_OK) return rc
-    if (!a.xbar) {
+/* what an earlier call had of it is given back */
+#define AALLOC(ptr, count)                                          \
+    do {                                                            \
+        dfree(c, a.ptr);                                            \
+        if ((rc = dalloc(c, &a.ptr, (count))) != SPH_OK) return rc; \
+    } while (0)
+    if (!a.part) {
         AALLOC(fin_pos, nf); AALLOC(fin_vel, nf); AALLOC(fin_orig, nf);
         AALLOC(st0, 1); AALLOC(st1, 1); AALLOC(target, 3 * nf);
         AALLOC(xbar, nf); AALLOC(vbar, nf); AALLOC(abar, nf); AALLOC(xacc, nf); AALLOC(vacc, nf);
         AALLOC(xrho, nf); AALLOC(red, 4);
+        for (auto& e : a.ev)
+            if (!e) CUDA_TRY(c, cudaEventCreate(&e));
+        /* last: without it a later call allocates all of these again */
         AALLOC(part, 3 * (size_t)adjoint_blocks((int)nf));
-        for (auto& e : a.ev) CUDA_TRY(c, cudaEventCreate(&e));
     }
     if (nseg > a.cap_seg) {
         dfree(c, a.ck_pos); dfree(c, a.ck_vel); dfree(c, a.ck_orig);
-        a.ck_pos = a.ck_vel = nullptr; a.ck_orig = nullptr; a.cap_seg = 0;
+        a.cap_seg = 0;
         AALLOC(ck_pos, (size_t)nseg * nf); AALLOC(ck_vel, (size_t)nseg * nf); AALLOC(ck_orig, (size_t)nseg * nf);
         a.cap_seg = nseg;
     }
@@ -2052,11 +2104,9 @@ int adj_reserve(sph_ctx* c, int nseg, int every)
     if (every > a.cap_every || keep != a.keep_lists ||
         (keep && (a.sl_capF != c->P.capF || a.sl_capB != c->P.capB))) {
         drop_graphs(c);
-        for (void* p : {(void*)a.sl_pos, (void*)a.sl_vel, (void*)a.sl_orig, (void*)a.sl_nbr_f, (void*)a.sl_cnt_f,
-                        (void*)a.sl_nbr_b, (void*)a.sl_cnt_b, (void*)a.sl_rho, (void*)a.sl_press})
-            dfree(c, p);
-        a.sl_pos = a.sl_vel = nullptr; a.sl_orig = a.sl_nbr_f = a.sl_cnt_f = a.sl_nbr_b = a.sl_cnt_b = nullptr;
-        a.sl_rho = a.sl_press = nullptr;
+        dfree(c, a.sl_pos); dfree(c, a.sl_vel); dfree(c, a.sl_orig);
+        dfree(c, a.sl_nbr_f); dfree(c, a.sl_cnt_f); dfree(c, a.sl_nbr_b); dfree(c, a.sl_cnt_b);
+        dfree(c, a.sl_rho); dfree(c, a.sl_press);
         const int cap = std::max(every, a.cap_every);
         a.cap_every = 0;
         AALLOC(sl_pos, (size_t)cap * nf); AALLOC(sl_vel, (size_t)cap * nf); AALLOC(sl_orig, (size_t)cap * nf);
@@ -2225,7 +2275,7 @@ int sph_wcsph_forward(sph_ctx* c, int nsteps, int ckpt_every, const float* targe
     a.have_grad = false;
     const int every = std::min(ckpt_every, nsteps);
     const int nseg = (nsteps + every - 1) / every;
-    if ((rc = adj_reserve(c, nseg, every)) != SPH_OK) return rc;
+    if ((rc = ensure_lists(c)) != SPH_OK || (rc = adj_reserve(c, nseg, every)) != SPH_OK) return rc;
     const size_t nf = c->nf;
     CUDA_TRY(c, cudaMemcpyAsync(a.target, target, 3 * nf * sizeof(float), cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(c, cudaEventRecord(a.ev[0], c->stream));
@@ -2272,7 +2322,7 @@ int sph_wcsph_backward(sph_ctx* c, float* dL_dv0, float* dL_dvisc, float* dL_dk)
     auto& a = c->adj;
     if (!c->initialized || !a.ready) return fail(c, SPH_ERR_STATE, "sph_wcsph_backward before sph_wcsph_forward");
     int rc = adj_supported(c);
-    if (rc != SPH_OK) return rc;
+    if (rc != SPH_OK || (rc = ensure_lists(c)) != SPH_OK) return rc;
     const size_t nf = c->nf;
     CUDA_TRY(c, cudaEventRecord(a.ev[2], c->stream));
     CUDA_TRY(c, cudaMemsetAsync(a.part, 0, 3 * (size_t)adjoint_blocks((int)nf) * sizeof(double), c->stream));

@@ -2,18 +2,23 @@
 it reports the overflow, the capacity grows, and the next step runs on complete
 lists. A context whose lists are built once more from the same positions before
 that step (by a change of the cell order and back) is the reference: the same
-lists in the same order, so the tolerance is zero.
+lists in the same order, so the tolerance is zero. Where there is no room for
+what has to be allocated (a limit on the context's memory stands in for a full
+GPU), the call reports it, the context keeps its state, and once there is room
+it goes on like one that never met the limit.
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 
 from sph2o_b200 import api
 from sph2o_b200 import scenes as S
-from sph2o_b200.api import Scene, Simulation, SphError
+from sph2o_b200.api import Scene, Simulation, SphError, lib
 
 pytestmark = pytest.mark.gpu
 NONE = np.zeros((0, 3), np.float32)
-OVERFLOW = -4
+OVERFLOW, NO_MEMORY = -4, -2
 
 
 def block_of(method, dims=(14, 13, 12), r=0.02):
@@ -24,13 +29,22 @@ def block_of(method, dims=(14, 13, 12), r=0.02):
     return sc.desc(), sc.fluid()[0]
 
 
-def overflowing(desc, x, squeeze):
+def limit_memory(sim, limit):
+    """Sets the limit (0: none); the bytes that the context holds."""
+    held = C.c_size_t()
+    assert lib().sph_debug_limit_memory(sim._h, limit, C.byref(held)) == 0
+    return held.value
+
+
+def overflowing(desc, x, squeeze, limit=None, code=OVERFLOW):
     """A context whose last step met more neighbours (74 at 0.82, 78 at 0.8) than its lists hold (64)."""
     sim = Simulation(desc, x, NONE)
+    if limit is not None:
+        limit_memory(sim, limit_memory(sim, 0) if limit == "held" else limit)
     sim.set_state((np.float32(0.1) + x * np.float32(squeeze)).astype(np.float32), np.zeros_like(x))
     with pytest.raises(SphError) as e:
         sim.step(1)
-    assert e.value.code == OVERFLOW
+    assert e.value.code == code
     return sim
 
 
@@ -49,3 +63,59 @@ def test_step_after_the_capacity_has_grown(method, squeeze):
         sim.close()
     for grown, again in zip(*got):
         assert np.array_equal(grown, again)
+
+
+@pytest.mark.parametrize("method", [S.WCSPH, S.PCISPH, S.DFSPH])
+@pytest.mark.parametrize("limit", ["held", 1])
+def test_no_room_to_grow(method, limit):
+    """With the bytes held as the limit the lists keep their capacity; with one
+    byte not even these can be had again."""
+    desc, x = block_of(method)
+    still = np.zeros_like(x)
+    got = []
+    for full in (False, True):
+        sim = overflowing(desc, x, 0.82, limit if full else None, NO_MEMORY if full else OVERFLOW)
+        before = sim.state()
+        if full and limit == 1:
+            for call in (lambda: sim.step(1), sim.neighbors, lambda: sim.phase(api.PHASE_DENSITY),
+                         lambda: sim.set_state(x, still), lambda: sim.set_option(api.OPT_CELL_ORDER, 1),
+                         lambda: sim.autotune(1)):
+                with pytest.raises(SphError) as e:
+                    call()
+                assert e.value.code == NO_MEMORY
+            for a, b in zip(before, sim.state()):
+                assert np.array_equal(a, b)
+            limit_memory(sim, 0)
+            sim.set_option(api.OPT_CELL_ORDER, 0)
+        sim.set_state(x, still)
+        sim.step(2)
+        got.append(sim.state())
+        sim.close()
+    for roomy, limited in zip(*got):
+        assert np.array_equal(roomy, limited)
+
+
+def test_adjoint_where_each_allocation_fails():
+    desc, x = block_of(S.WCSPH)
+    target = x + np.float32(0.01)
+    got = []
+    for full in (False, True):
+        sim = Simulation(desc, x, NONE)
+        held = limit_memory(sim, 0)
+        failures, limit = 0, held
+        while full:
+            limit_memory(sim, limit)
+            try:
+                sim.wcsph_forward(4, target, ckpt_every=2)
+                break
+            except SphError as e:
+                assert e.code == NO_MEMORY
+                failures += 1
+                limit += 16 * len(x)
+        assert failures > 10 or not full
+        sim.set_state(x, np.zeros_like(x))
+        loss = sim.wcsph_forward(4, target, ckpt_every=2)
+        got.append((loss, *sim.wcsph_backward(want_x0=True).values()))
+        sim.close()
+    for roomy, limited in zip(*got):
+        assert np.array_equal(roomy, limited)
