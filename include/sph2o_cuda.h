@@ -219,12 +219,13 @@ enum sph_option {
     SPH_OPT_CUDA_GRAPHS = 0,      /* 1 (default): steps replay captured CUDA graphs of two steps (one
                                      for an odd remainder), keyed by the buffer assignment */
     SPH_OPT_CELL_ORDER = 1,       /* 0 (default): 4x4x4 cell bricks, z fastest inside; 1: linear, x fastest */
-    SPH_OPT_SOLVER_OCCUPANCY = 2, /* DFSPH persistent solver blocks per SM: 8 or 4; until set it reads 8 and
-                                     the library chooses */
+    SPH_OPT_SOLVER_OCCUPANCY = 2, /* 8 (default) or 4: kept and returned, but the persistent DFSPH solver runs
+                                     with 4 blocks per SM for either; its form with 8 was slower at every
+                                     size and is gone. Results never depended on it. */
     SPH_OPT_PASS_BLOCK = 3,       /* threads per block of the particle-pass kernels: 256 (default) or 128 */
     SPH_OPT_SOLVER_LANES = 4,     /* lanes sharing one particle's neighbour list in the persistent DFSPH
-                                     solver: 1, 2 or 4; 1 and 2 give the same bits; until set it reads 2 and
-                                     the library chooses 1 or 2 by size */
+                                     solver: 1, 2 or 4; 1 and 2 give the same bits. Until set, the library's
+                                     choice: 1 from 2^16 fluid particles on, else 2 */
     SPH_OPT_POSITION_RESIDUAL = 5,/* 1: every position keeps the rounding residual of its integration
                                      (float pair, error-free sums), so long runs of small steps keep about
                                      twice float precision; 0 (default): FP32 positions rounded as the
@@ -240,8 +241,8 @@ enum sph_option {
 int sph_set_option(sph_ctx* ctx, int option, int value);
 int sph_get_option(const sph_ctx* ctx, int option, int* value);
 
-/* Chooses SPH_OPT_CELL_ORDER, SPH_OPT_SOLVER_OCCUPANCY, SPH_OPT_PASS_BLOCK and
-   SPH_OPT_SOLVER_LANES by timing trial_steps steps (CUDA events) of every
+/* Chooses SPH_OPT_CELL_ORDER, SPH_OPT_PASS_BLOCK and SPH_OPT_SOLVER_LANES (and
+   keeps SPH_OPT_SOLVER_OCCUPANCY) by timing trial_steps steps (CUDA events) of every
    combination, each from a snapshot of the current state that is restored
    afterwards: the simulation is left exactly where it was. cache_path (may
    be NULL) names a JSON file keyed by GPU name, method and particle counts;

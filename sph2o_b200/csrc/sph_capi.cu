@@ -81,7 +81,7 @@ struct sph_ctx {
     double* accum = nullptr;
     size_t accum_len = 0;
     int grid_pcisph = 0;
-    int grid_solve[2][2][3] = {};  /* DFSPH solver grid by [divergence][occupancy 8, 4][lanes 1, 2, 4] */
+    int grid_solve[2][3] = {};  /* DFSPH solver grid by [divergence][lanes 1, 2, 4] */
     DevState last{};
     bool lists_valid = false;
     /* timing: batch events + per-phase profiling */
@@ -111,9 +111,9 @@ struct sph_ctx {
     bool use_graphs = true;
     /* tunables (sph_set_option / sph_autotune) */
     int pass_block = 256;
-    int solver_occ = 0;  /* blocks per SM and lanes of the persistent DFSPH solver; 0: not set, by size */
+    int solver_occ = 8;  /* SPH_OPT_SOLVER_OCCUPANCY: kept and returned, no kernel depends on it */
     bool staged_lists = false; /* SPH_OPT_LIST_STAGED */
-    int solver_tpp = 0;
+    int solver_tpp = 0;  /* lanes of the persistent DFSPH solver; 0: not set, by size */
     float* stage = nullptr;      /* 3 max(nf, nb) floats: device side of every host transfer (see sph_get_state) */
     float4* braw = nullptr;      /* boundary in caller order (re-sorted when the cell order changes) */
     unsigned* bid = nullptr;
@@ -592,23 +592,18 @@ int step_pcisph(sph_ctx* c)
     return check_launch(c, "pcisph step");
 }
 
-/* Blocks per SM of the persistent DFSPH solver: 4 (64 registers, four gathers
-   in flight) unless set; 8 (32 registers, two) measured slower at every size
-   (26k 153 against 136 us of density solver per step, 125k 223 against 205,
-   1M 1,282 against 1,231). */
-int solver_occ(const sph_ctx* c) { return c->solver_occ ? c->solver_occ : 4; }
-
 /* Lanes per particle of the persistent DFSPH solver unless set: one from 2^16
-   particles on, where they fill the 148 x 4 x 256 resident threads (125k: 205
-   us of density solver per step against 209 with two lanes; 1M: 1,231 against
-   1,361); two below (26k: 136 against 149). Both give the same bits. */
+   particles on, where they fill the 148 x 4 x 256 resident threads (density and
+   divergence solver per step, 125k: 165 + 62 us against 168 + 64 with two lanes;
+   1M: 1,035 + 296 against 1,144 + 327); two below (26k: 64 + 29 against 71 + 34;
+   at the line, 64k: 100 + 43 against 101 + 47). Both give the same bits. */
 int solver_lanes(const sph_ctx* c) { return c->solver_tpp ? c->solver_tpp : c->nf >= (1u << 16) ? 1 : 2; }
 
 int tpp_index(int tpp) { return tpp == 4 ? 2 : tpp == 2 ? 1 : 0; }
 
 int solve_grid(const sph_ctx* c, bool divergence)
 {
-    return c->grid_solve[divergence ? 1 : 0][solver_occ(c) == 4 ? 1 : 0][tpp_index(solver_lanes(c))];
+    return c->grid_solve[divergence ? 1 : 0][tpp_index(solver_lanes(c))];
 }
 
 int step_dfsph(sph_ctx* c)
@@ -622,7 +617,7 @@ int step_dfsph(sph_ctx* c)
     {
         Phase ph(c, SPH_PROF_DENSITY_SOLVE, 1);
         e = c->nscenes ? launch_dfsph_solve_batch(c->P, A, false, c->grid_batch_density, c->stream)
-                       : launch_dfsph_solve(c->P, A, false, solve_grid(c, false), solver_occ(c), solver_lanes(c), c->stream);
+                       : launch_dfsph_solve(c->P, A, false, solve_grid(c, false), solver_lanes(c), c->stream);
     }
     if (e != 0) return fail(c, SPH_ERR_CUDA, std::string("dfsph density solver launch: ") + cudaGetErrorString((cudaError_t)e));
     if (c->P.pcib) { /* DFSPHSolver.cpp:60-70 */
@@ -638,7 +633,7 @@ int step_dfsph(sph_ctx* c)
     {
         Phase ph(c, SPH_PROF_DIVERGENCE_SOLVE, 1);
         e = c->nscenes ? launch_dfsph_solve_batch(c->P, A, true, c->grid_batch_div, c->stream)
-                       : launch_dfsph_solve(c->P, A, true, solve_grid(c, true), solver_occ(c), solver_lanes(c), c->stream);
+                       : launch_dfsph_solve(c->P, A, true, solve_grid(c, true), solver_lanes(c), c->stream);
     }
     if (e != 0) return fail(c, SPH_ERR_CUDA, std::string("dfsph divergence solver launch: ") + cudaGetErrorString((cudaError_t)e));
     cube_correct(c); /* DFSPHSolver.cpp:94-103 */
@@ -1190,11 +1185,10 @@ int sph_init(sph_ctx* c)
     c->grid_pcisph = persistent_grid(true, false);
     if (c->grid_pcisph <= 0) return fail(c, SPH_ERR_CUDA, "cannot size the persistent solver grid");
     for (int dv = 0; dv < 2; ++dv)
-        for (int o = 0; o < 2; ++o)
-            for (int t = 0; t < 3; ++t) {
-                c->grid_solve[dv][o][t] = persistent_grid(false, dv == 1, false, o ? 4 : 8, 1 << t);
-                if (c->grid_solve[dv][o][t] <= 0) return fail(c, SPH_ERR_CUDA, "cannot size the persistent solver grid");
-            }
+        for (int t = 0; t < 3; ++t) {
+            c->grid_solve[dv][t] = persistent_grid(false, dv == 1, false, 1 << t);
+            if (c->grid_solve[dv][t] <= 0) return fail(c, SPH_ERR_CUDA, "cannot size the persistent solver grid");
+        }
 
     /* the fast division by h, if it is exact for this h (chunk_sums is free) */
     unsigned bad_div = 1;
@@ -1767,7 +1761,6 @@ int sph_set_option(sph_ctx* c, int option, int value)
     case SPH_OPT_SOLVER_OCCUPANCY:
         if (value != 4 && value != 8) return fail(c, SPH_ERR_ARG, "solver occupancy is 4 or 8");
         c->solver_occ = value;
-        drop_graphs(c);
         return SPH_OK;
     case SPH_OPT_PASS_BLOCK:
         if (value != 128 && value != 256) return fail(c, SPH_ERR_ARG, "pass block is 128 or 256");
@@ -1800,9 +1793,9 @@ int sph_get_option(const sph_ctx* c, int option, int* value)
     switch (option) {
     case SPH_OPT_CUDA_GRAPHS: *value = c->use_graphs ? 1 : 0; return SPH_OK;
     case SPH_OPT_CELL_ORDER: *value = c->P.cell_order; return SPH_OK;
-    case SPH_OPT_SOLVER_OCCUPANCY: *value = c->solver_occ ? c->solver_occ : 8; return SPH_OK;
+    case SPH_OPT_SOLVER_OCCUPANCY: *value = c->solver_occ; return SPH_OK;
     case SPH_OPT_PASS_BLOCK: *value = c->pass_block; return SPH_OK;
-    case SPH_OPT_SOLVER_LANES: *value = c->solver_tpp ? c->solver_tpp : 2; return SPH_OK;
+    case SPH_OPT_SOLVER_LANES: *value = solver_lanes(c); return SPH_OK;
     case SPH_OPT_POSITION_RESIDUAL: *value = c->pos_lo; return SPH_OK;
     case SPH_OPT_LIST_STAGED: *value = c->staged_lists ? 1 : 0; return SPH_OK;
     default: return SPH_ERR_ARG;
@@ -1818,7 +1811,7 @@ int sph_autotune(sph_ctx* c, int trial_steps, const char* cache_path, int* confi
         /* trial steps would advance the carried normals and the per-cell search record */
         return fail(c, SPH_ERR_ARG, "sph_autotune is not available with the PCISPH boundary method");
     const std::string key = tune_key(c);
-    int best[SPH_TUNE_COUNT] = {c->P.cell_order, solver_occ(c), c->pass_block, solver_lanes(c)};
+    int best[SPH_TUNE_COUNT] = {c->P.cell_order, c->solver_occ, c->pass_block, solver_lanes(c)};
     int rc;
     if (tune_lookup(cache_path, key, best)) {
         if ((rc = apply_config(c, best)) != SPH_OK) return rc;
@@ -1833,14 +1826,12 @@ int sph_autotune(sph_ctx* c, int trial_steps, const char* cache_path, int* confi
     double best_ms = 1e300;
     const bool dfsph = c->desc.simulation_method == SPH_DFSPH;
     for (int order = 0; order < 2; ++order)
-        for (int occ : {8, 4})
-            for (int tpp : {1, 2, 4}) {
+        for (int tpp : {1, 2, 4}) {
             /* only the single-scene DFSPH solver has these variants */
-            if ((!dfsph || c->nscenes) && (occ == 4 || tpp != 1)) continue;
+            if ((!dfsph || c->nscenes) && tpp != 1) continue;
             for (int blk : {256, 128}) {
-                const int cfg[SPH_TUNE_COUNT] = {order, occ, blk, tpp};
+                const int cfg[SPH_TUNE_COUNT] = {order, c->solver_occ, blk, tpp};
                 if ((rc = snapshot(c, false)) != SPH_OK) return rc;
-                c->solver_occ = occ;
                 c->solver_tpp = tpp;
                 c->pass_block = blk;
                 rc = order != c->P.cell_order ? apply_cell_order(c, order) : refresh(c);
@@ -1860,10 +1851,9 @@ int sph_autotune(sph_ctx* c, int trial_steps, const char* cache_path, int* confi
                     for (int i = 0; i < SPH_TUNE_COUNT; ++i) best[i] = cfg[i];
                 }
             }
-            }
+        }
     /* back to the snapshot with the chosen configuration */
     if ((rc = snapshot(c, false)) != SPH_OK) return rc;
-    c->solver_occ = best[1];
     c->pass_block = best[2];
     c->solver_tpp = best[3];
     rc = best[0] != c->P.cell_order ? apply_cell_order(c, best[0]) : refresh(c);

@@ -571,40 +571,25 @@ __device__ __forceinline__ uint2 pair_at(const uint2* pairs, unsigned kk, unsign
     return __ldcs(pairs + list_index(kk, cap, (unsigned)i));
 }
 
-/* Calls f(kk, N, e, ahead) for rounds of N of the list entries sub, sub + TPP,
-   ... < n of particle i: entry kk + u TPP is e[u], u < N. AHEAD: rounds of U
-   entries, where those at or beyond n are the particle itself and do not count;
-   f calls ahead() once its gathers are issued, which fetches the next round's
-   entries. Without (32 registers are too few): rounds of U, of ACC and of 1. */
-template <int U, int TPP, int ACC, bool AHEAD, typename F>
+/* Calls f(kk, e, ahead) for rounds of U of the list entries sub, sub + TPP, ...
+   < n of particle i: entry kk + u TPP is e[u]; those at or beyond n are the
+   particle itself and do not count. f calls ahead() once its gathers are issued,
+   which fetches the next round's entries. */
+template <int U, int TPP, typename F>
 __device__ __forceinline__ void pair_rounds(const uint2* pairs, unsigned sub, unsigned n, unsigned cap, int i, F&& f)
 {
-    if (AHEAD) {
-        uint2 e[U];
-        const auto fetch = [&](unsigned kk, uint2(&to)[U]) {
+    uint2 e[U];
+    const auto fetch = [&](unsigned kk, uint2(&to)[U]) {
 #pragma unroll
-            for (int u = 0; u < U; ++u)
-                to[u] = kk + u * TPP < n ? pair_at(pairs, kk + u * TPP, cap, i) : make_uint2((unsigned)i, 0u);
-        };
-        fetch(sub, e);
-        for (unsigned kk = sub; kk < n; kk += U * TPP) {
-            uint2 next[U];
-            f(kk, std::integral_constant<int, U>(), e, [&] { fetch(kk + U * TPP, next); });
+        for (int u = 0; u < U; ++u)
+            to[u] = kk + u * TPP < n ? pair_at(pairs, kk + u * TPP, cap, i) : make_uint2((unsigned)i, 0u);
+    };
+    fetch(sub, e);
+    for (unsigned kk = sub; kk < n; kk += U * TPP) {
+        uint2 next[U];
+        f(kk, e, [&] { fetch(kk + U * TPP, next); });
 #pragma unroll
-            for (int u = 0; u < U; ++u) e[u] = next[u];
-        }
-    } else {
-        unsigned kk = sub;
-        const auto round = [&](auto count) {
-            constexpr int N = decltype(count)::value;
-            uint2 e[N];
-#pragma unroll
-            for (int u = 0; u < N; ++u) e[u] = pair_at(pairs, kk + u * TPP, cap, i);
-            f(kk, count, e, [] {});
-        };
-        for (; kk + (U - 1) * TPP < n; kk += U * TPP) round(std::integral_constant<int, U>());
-        for (; U > ACC && kk + (ACC - 1) * TPP < n; kk += ACC * TPP) round(std::integral_constant<int, ACC>());
-        if (ACC > 1 && kk < n) round(std::integral_constant<int, 1>());
+        for (int u = 0; u < U; ++u) e[u] = next[u];
     }
 }
 
@@ -622,7 +607,7 @@ __device__ __forceinline__ float dfsph_residual_term(const SimParams& P, float4 
    using any of them (more loads in flight per lane) and adds the terms in
    list order, so U changes no bit; TPP * ACC = 2 is one order of additions
    whichever way it is split. */
-template <int TPP, int ACC, int U, bool AHEAD>
+template <int TPP, int ACC, int U>
 __device__ __forceinline__ float dfsph_residual_part(const SimParams& P, const DeviceArrays& A, int i, int sub)
 {
     static_assert(U % ACC == 0, "an unrolled round holds whole rounds of partial sums");
@@ -632,16 +617,14 @@ __device__ __forceinline__ float dfsph_residual_part(const SimParams& P, const D
 #pragma unroll
     for (int c = 0; c < ACC; ++c) s[c] = 0.0f;
     const unsigned nF = A.cnt_f[i], nB = A.cnt_b[i];
-    pair_rounds<U, TPP, ACC, AHEAD>(A.pair_f, (unsigned)sub, nF, P.capF, i,
-                                    [&](unsigned kk, auto count, const auto& e, auto ahead) {
-        constexpr int N = decltype(count)::value;
-        float4 xj[N], vj[N];
+    pair_rounds<U, TPP>(A.pair_f, (unsigned)sub, nF, P.capF, i, [&](unsigned kk, const auto& e, auto ahead) {
+        float4 xj[U], vj[U];
 #pragma unroll
-        for (int u = 0; u < N; ++u) load_rec(A.rec, e[u].x, xj[u], vj[u]);
+        for (int u = 0; u < U; ++u) load_rec(A.rec, e[u].x, xj[u], vj[u]);
         ahead();
 #pragma unroll
-        for (int u = 0; u < N; ++u)
-            if (!AHEAD || kk + u * TPP < nF) s[u % ACC] += dfsph_residual_term(P, xi, vi, xj[u], vj[u], __uint_as_float(e[u].y));
+        for (int u = 0; u < U; ++u)
+            if (kk + u * TPP < nF) s[u % ACC] += dfsph_residual_term(P, xi, vi, xj[u], vj[u], __uint_as_float(e[u].y));
     });
     for (unsigned kk = sub; kk < nB; kk += TPP * ACC) {
 #pragma unroll
@@ -677,7 +660,7 @@ __device__ __forceinline__ float dfsph_residual_finish(const SimParams& P, const
 template <bool DIV>
 __device__ __forceinline__ float dfsph_residual(const SimParams& P, const DeviceArrays& A, int i, float dt)
 {
-    return dfsph_residual_finish<DIV>(P, A, i, dfsph_residual_part<1, 1, 4, true>(P, A, i, 0), dt);
+    return dfsph_residual_finish<DIV>(P, A, i, dfsph_residual_part<1, 1, 4>(P, A, i, 0), dt);
 }
 
 /* Partial sums over list entries sub, sub + TPP, ... of
@@ -685,7 +668,7 @@ __device__ __forceinline__ float dfsph_residual(const SimParams& P, const Device
    U at a time and ACC interleaved sums, as in dfsph_residual_part. Position
    and k are in posd, written inside the same persistent kernel (before a grid
    barrier): a read-only (non-coherent) load path would be wrong for it. */
-template <int TPP, int ACC, int U, bool AHEAD>
+template <int TPP, int ACC, int U>
 __device__ __forceinline__ void dfsph_correct_part(const SimParams& P, const DeviceArrays& A, int i, int sub,
                                                    float& sx, float& sy, float& sz)
 {
@@ -697,17 +680,15 @@ __device__ __forceinline__ void dfsph_correct_part(const SimParams& P, const Dev
 #pragma unroll
     for (int c = 0; c < ACC; ++c) tx[c] = ty[c] = tz[c] = 0.0f;
     const unsigned nF = A.cnt_f[i];
-    pair_rounds<U, TPP, ACC, AHEAD>(A.pair_f, (unsigned)sub, nF, P.capF, i,
-                                    [&](unsigned kk, auto count, const auto& e, auto ahead) {
-        constexpr int N = decltype(count)::value;
-        float4 xj[N];
+    pair_rounds<U, TPP>(A.pair_f, (unsigned)sub, nF, P.capF, i, [&](unsigned kk, const auto& e, auto ahead) {
+        float4 xj[U];
 #pragma unroll
-        for (int u = 0; u < N; ++u) xj[u] = xk[e[u].x];
+        for (int u = 0; u < U; ++u) xj[u] = xk[e[u].x];
         ahead();
 #pragma unroll
-        for (int u = 0; u < N; ++u) {
+        for (int u = 0; u < U; ++u) {
             const float ks = ki + xj[u].w;
-            if ((!AHEAD || kk + u * TPP < nF) && fabsf(ks) > P.eps) {
+            if (kk + u * TPP < nF && fabsf(ks) > P.eps) {
                 const float c = P.mass * ks * __uint_as_float(e[u].y);
                 tx[u % ACC] += c * (xi.x - xj[u].x);
                 ty[u % ACC] += c * (xi.y - xj[u].y);
@@ -755,7 +736,7 @@ __device__ __forceinline__ void dfsph_set_k(const DeviceArrays& A, int i, float 
 __device__ __forceinline__ void dfsph_correct(const SimParams& P, const DeviceArrays& A, int i, float dt)
 {
     float sx, sy, sz;
-    dfsph_correct_part<1, 1, 4, true>(P, A, i, 0, sx, sy, sz);
+    dfsph_correct_part<1, 1, 4>(P, A, i, 0, sx, sy, sz);
     dfsph_apply(A, i, dt, sx, sy, sz);
 }
 
@@ -796,22 +777,22 @@ __device__ __forceinline__ void for_particles(int n, F&& f)
 }
 
 /* residual of particle i with its list split over TPP lanes (all lanes call) */
-template <bool DIV, int TPP, int ACC, int U, bool AHEAD>
+template <bool DIV, int TPP, int ACC, int U>
 __device__ __forceinline__ float dfsph_residual_lanes(const SimParams& P, const DeviceArrays& A, int i, int sub,
                                                       bool valid, float dt)
 {
-    float part = valid ? dfsph_residual_part<TPP, ACC, U, AHEAD>(P, A, i, sub) : 0.0f;
+    float part = valid ? dfsph_residual_part<TPP, ACC, U>(P, A, i, sub) : 0.0f;
     if (TPP > 1) part = lane_group_sum<TPP>(part);
     return valid ? dfsph_residual_finish<DIV>(P, A, i, part, dt) : 0.0f;
 }
 
 /* velocity correction of particle i with its list split over TPP lanes */
-template <int TPP, int ACC, int U, bool AHEAD>
+template <int TPP, int ACC, int U>
 __device__ __forceinline__ void dfsph_correct_lanes(const SimParams& P, const DeviceArrays& A, int i, int sub,
                                                     bool valid, float dt)
 {
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-    if (valid) dfsph_correct_part<TPP, ACC, U, AHEAD>(P, A, i, sub, sx, sy, sz);
+    if (valid) dfsph_correct_part<TPP, ACC, U>(P, A, i, sub, sx, sy, sz);
     if (TPP > 1) {
         sx = lane_group_sum<TPP>(sx);
         sy = lane_group_sum<TPP>(sy);
@@ -835,15 +816,16 @@ __device__ __forceinline__ void dfsph_correct_lanes(const SimParams& P, const De
    round's list entries fetched while the gathers of this one are on their way,
    and one masked round at the end of a list instead of rounds of 2 and 1
    (1,126 -> 1,030; 125k 171 -> 163; 24 batched scenes 183 -> 158; with 3 blocks
-   and 4, 6, 8 gathers 1,071, 1,210, 1,335; in 32 registers it spills and loses).
-   OCC blocks of 256 per SM: 4 (64 registers) by default, 8 (32 registers, two
-   gathers) is the autotuner's other candidate. TPP lanes share a particle;
-   1 and 2 lanes add the same two interleaved sums, so they agree bit for bit. */
-template <bool DIV, int OCC, int TPP>
-__global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, DeviceArrays A)
+   and 4, 6, 8 gathers 1,071, 1,210, 1,335). 4 blocks of 256 per SM, 64 registers:
+   8 blocks in 32 registers hold two gathers and no entries ahead, and were slower
+   with the lanes taken at every size (density solver 1k 54 us against 41, 26k 79
+   against 64, 125k 216 against 165, 1M 1,294 against 1,035). TPP lanes share a
+   particle; 1 and 2 lanes add the same two interleaved sums, so they agree bit for
+   bit. */
+template <bool DIV, int TPP>
+__global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve(SimParams P, DeviceArrays A)
 {
-    constexpr int U = OCC == 4 ? 4 : 2;
-    constexpr bool AHEAD = OCC == 4;
+    constexpr int U = 4;
     constexpr int ACC = TPP == 1 ? 2 : 1;
     __shared__ double s_red[32];
     DevState* st = A.st;
@@ -893,14 +875,14 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
        only where the residual is positive */
     for_particles<TPP>(nfi, [&](int i, int sub, bool valid) {
         const float r = DIV ? (valid ? A.divres[i] : 0.0f)
-                            : dfsph_residual_lanes<DIV, TPP, ACC, U, AHEAD>(P, A, i, sub, valid, dt);
+                            : dfsph_residual_lanes<DIV, TPP, ACC, U>(P, A, i, sub, valid, dt);
         if (valid && sub == 0) {
             if (DIV) dfsph_set_k(A, i, r > 0.0f ? kws[i] / dt : 0.0f);
             else dfsph_set_k(A, i, r > P.rho0 ? kws[i] / ts2 : 0.0f);
         }
     });
     if (!bar.sync()) return;
-    for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U, AHEAD>(P, A, i, sub, valid, dt); });
+    for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U>(P, A, i, sub, valid, dt); });
     if (!bar.sync()) return;
 
     const double limit = DIV ? (double)(P.eta_v / dt) : (double)P.eta;
@@ -913,7 +895,7 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
     while ((avg > limit || it < min_it) && it < max_it) {
         double local = 0.0;
         for_particles<TPP>(nfi, [&](int i, int sub, bool valid) {
-            const float r = dfsph_residual_lanes<DIV, TPP, ACC, U, AHEAD>(P, A, i, sub, valid, dt);
+            const float r = dfsph_residual_lanes<DIV, TPP, ACC, U>(P, A, i, sub, valid, dt);
             if (!valid || sub != 0) return;
             float k;
             if (DIV) {
@@ -930,7 +912,7 @@ __global__ void __launch_bounds__(kSolverBlock, OCC) k_dfsph_solve(SimParams P, 
         if (threadIdx.x == 0) atomicAdd(&A.accum[it], bs);
         if (!bar.sync()) return;
         avg = *(volatile double*)&A.accum[it] / (double)nfi;
-        for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U, AHEAD>(P, A, i, sub, valid, dt); });
+        for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U>(P, A, i, sub, valid, dt); });
         if (!bar.sync()) return;
         ++it;
     }
@@ -1682,18 +1664,17 @@ void launch_forces(const SimParams& P, const DeviceArrays& A, int mode, int bloc
     }
 }
 
-/* k_dfsph_solve instance for (divergence, blocks per SM, lanes per particle) */
-static const void* dfsph_solve_fn(bool divergence, int occ, int tpp)
+/* k_dfsph_solve instance for (divergence, lanes per particle) */
+static const void* dfsph_solve_fn(bool divergence, int tpp)
 {
-#define SPH_SOLVE_FN(D, O)                                                                          \
-    (tpp == 4 ? (const void*)k_dfsph_solve<D, O, 4>                                                 \
-              : tpp == 2 ? (const void*)k_dfsph_solve<D, O, 2> : (const void*)k_dfsph_solve<D, O, 1>)
-    if (divergence) return occ == 4 ? SPH_SOLVE_FN(true, 4) : SPH_SOLVE_FN(true, 8);
-    return occ == 4 ? SPH_SOLVE_FN(false, 4) : SPH_SOLVE_FN(false, 8);
+#define SPH_SOLVE_FN(D)                                                                             \
+    (tpp == 4 ? (const void*)k_dfsph_solve<D, 4>                                                    \
+              : tpp == 2 ? (const void*)k_dfsph_solve<D, 2> : (const void*)k_dfsph_solve<D, 1>)
+    return divergence ? SPH_SOLVE_FN(true) : SPH_SOLVE_FN(false);
 #undef SPH_SOLVE_FN
 }
 
-int persistent_grid(bool pcisph, bool divergence, bool batch, int occ, int tpp)
+int persistent_grid(bool pcisph, bool divergence, bool batch, int tpp)
 {
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
@@ -1701,7 +1682,7 @@ int persistent_grid(bool pcisph, bool divergence, bool batch, int occ, int tpp)
     const void* fn = pcisph ? (const void*)k_pcisph_solve
                      : batch ? (divergence ? (const void*)k_dfsph_solve_batch<true>
                                            : (const void*)k_dfsph_solve_batch<false>)
-                             : dfsph_solve_fn(divergence, occ, tpp);
+                             : dfsph_solve_fn(divergence, tpp);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSolverBlock, 0) != cudaSuccess) return 0;
     return per_sm * sms;
 }
@@ -1714,12 +1695,11 @@ static int coop_launch(const void* fn, const SimParams& P, const DeviceArrays& A
     return (int)cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kSolverBlock), args, 0, s);
 }
 
-int launch_dfsph_solve(const SimParams& P, const DeviceArrays& A, bool divergence, int grid, int occ, int tpp,
-                       cudaStream_t s)
+int launch_dfsph_solve(const SimParams& P, const DeviceArrays& A, bool divergence, int grid, int tpp, cudaStream_t s)
 {
     const int need = blocks_for((long long)(P.nf > 0 ? P.nf : 1) * tpp, kSolverBlock);
     const int g = grid < need ? grid : need;
-    return coop_launch(dfsph_solve_fn(divergence, occ, tpp), P, A, g > 0 ? g : 1, s);
+    return coop_launch(dfsph_solve_fn(divergence, tpp), P, A, g > 0 ? g : 1, s);
 }
 
 int launch_dfsph_solve_batch(const SimParams& P, const DeviceArrays& A, bool divergence, int grid, cudaStream_t s)

@@ -79,6 +79,24 @@ def test_options_round_trip_and_reject_bad_values():
     sim.close()
 
 
+# 2^16 fluid particles is where the solver's lanes change by themselves: 65,504; 65,536
+@pytest.mark.parametrize("dims,lanes", [((7, 5, 3), 2), ((89, 46, 16), 2), ((64, 64, 16), 1)])
+def test_options_read_what_runs(dims, lanes):
+    """Options that were never set read what the library has chosen, so writing
+    them back changes nothing."""
+    r = 0.02
+    sim = Simulation.from_scene(Scene.from_dict(S.scene(
+        method=S.DFSPH, radius=r, blocks=[S.block(dims, r, (2 * r,) * 3)],
+        tank=((0, 0, 0), tuple(2 * r * (k + 4) for k in dims)), time_step=5e-4, jitter=0.3, seed=2)))
+    options = [api.OPT_CELL_ORDER, api.OPT_SOLVER_OCCUPANCY, api.OPT_PASS_BLOCK, api.OPT_SOLVER_LANES]
+    read = [sim.get_option(o) for o in options]
+    assert read == [0, 8, 256, lanes]
+    for o, v in zip(options, read):
+        sim.set_option(o, v)
+    assert [sim.get_option(o) for o in options] == read
+    sim.close()
+
+
 @pytest.mark.parametrize("method", METHODS)
 @pytest.mark.parametrize("lanes", [1, 2, 4])
 def test_launch_shape_does_not_change_results(method, lanes):
