@@ -463,20 +463,45 @@ void drop_lists(sph_ctx* c)
     dfree(c, c->pgrad);
 }
 
-/* The neighbour lists and what is kept beside their entries, for the capacities
-   in c->P: all of them, or none. */
+/* Device memory that this context can still take. */
+size_t memory_left(const sph_ctx* c)
+{
+    size_t left = 0, total = 0;
+    if (cudaMemGetInfo(&left, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return c->held_limit ? std::min(left, c->held_limit - std::min(c->held, c->held_limit)) : left;
+}
+
+/* The neighbour lists for the capacities in c->P, both or none, and what the
+   DFSPH and PCISPH solvers keep beside the list entries to save time: kernel
+   factors (8 bytes an entry) or gradients (16), 1,024 bytes per particle beside
+   the 730 of everything else. They are kept only where they take at most half of
+   the memory that is left, so that they refuse no scene that fits without them
+   (110 million DFSPH particles: 80 GB without, out of memory with) and leave room
+   for other programs. A scene that has the GPU to itself keeps them up to about 60
+   million particles; without them the solvers compute the same values again. */
 int alloc_lists(sph_ctx* c)
 {
     const size_t nf_entries = list_len(c->nf, c->P.capF), nb_entries = list_len(c->nf, c->P.capB);
     int rc;
     if ((rc = dalloc(c, &c->nbr_f, nf_entries)) == SPH_OK) rc = dalloc(c, &c->nbr_b, nb_entries);
-    if (c->desc.simulation_method == SPH_DFSPH) {
-        if (rc == SPH_OK) rc = dalloc(c, &c->pair_f, nf_entries);
-        if (rc == SPH_OK) rc = dalloc(c, &c->pair_b, nb_entries);
+    if (rc != SPH_OK) {
+        drop_lists(c);
+        return rc;
     }
-    if (c->desc.simulation_method == SPH_PCISPH && rc == SPH_OK) rc = dalloc(c, &c->pgrad, nf_entries);
-    if (rc != SPH_OK) drop_lists(c);
-    return rc;
+    const bool pairs = c->desc.simulation_method == SPH_DFSPH, gradients = c->desc.simulation_method == SPH_PCISPH;
+    const size_t pair_b_entries = c->nb > 0 ? nb_entries : 1;
+    const size_t bytes = pairs ? (nf_entries + pair_b_entries) * sizeof(uint2) : gradients ? nf_entries * sizeof(float4) : 0;
+    if (bytes == 0 || bytes > memory_left(c) / 2) return SPH_OK;
+    const std::string err = c->err;
+    if (gradients ? dalloc(c, &c->pgrad, nf_entries) != SPH_OK
+                  : dalloc(c, &c->pair_f, nf_entries) != SPH_OK || dalloc(c, &c->pair_b, pair_b_entries) != SPH_OK) {
+        dfree(c, c->pgrad); dfree(c, c->pair_f); dfree(c, c->pair_b);
+        c->err = err;
+    }
+    return SPH_OK;
 }
 
 /* Sort the fluid into cells, rebuild the neighbour lists and compute what
@@ -1122,7 +1147,9 @@ int sph_init(sph_ctx* c)
     ALLOC(orig, nf); ALLOC(orig2, nf);
     ALLOC(kws, nf); ALLOC(kws2, nf); ALLOC(kvws, nf); ALLOC(kvws2, nf);
     ALLOC(acc, nf); ALLOC(rho, nf); ALLOC(alpha, nf); ALLOC(press, nf);
-    ALLOC(normal, nf); ALLOC(predr, nf); ALLOC(posd, nf);
+    if (P.st_on || P.pcib) ALLOC(normal, nf);
+    if (c->desc.simulation_method == SPH_PCISPH) ALLOC(predr, nf);
+    if (c->desc.simulation_method != SPH_WCSPH) ALLOC(posd, nf);
     ALLOC(cell_of, nmax); ALLOC(slot, nmax); ALLOC(tmp_key, nmax); ALLOC(tmp_src, nmax); ALLOC(cell_sorted, nmax);
     ALLOC(cell_count, (size_t)P.ncells); ALLOC(cell_start, (size_t)P.ncells + 1);
     ALLOC(bcell_start, (size_t)P.ncells + 1); ALLOC(chunk_sums, (size_t)P.ncells / 4096 + 1);
@@ -1139,10 +1166,7 @@ int sph_init(sph_ctx* c)
     c->pos_base = c->pos;
     c->orig_base = c->orig;
     c->kws_base = c->kws;
-    if ((rc = alloc_lists(c)) != SPH_OK) return rc;
-    if (c->desc.simulation_method == SPH_DFSPH) {
-        if ((rc = dalloc(c, &c->divres, nf)) != SPH_OK) return rc;
-    }
+    if (c->desc.simulation_method == SPH_DFSPH && (rc = dalloc(c, &c->divres, nf)) != SPH_OK) return rc;
     if ((rc = dalloc(c, &c->rec, 2 * nf)) != SPH_OK) return rc;
     if (c->pos_lo) {
         if (c->nscenes) return fail(c, SPH_ERR_ARG, "position residuals apply to single scenes, not to batches");
@@ -1260,6 +1284,9 @@ int sph_init(sph_ctx* c)
                                         c->stream));
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     }
+
+    /* last of all arrays: what they leave decides what is kept beside the lists */
+    if ((rc = alloc_lists(c)) != SPH_OK) return rc;
 
     /* solver state */
     DevState s0{};
@@ -1991,7 +2018,8 @@ int sph_debug_neighbors(sph_ctx* c, unsigned* f_offsets, unsigned* f_index, size
     if (!c->initialized) return fail(c, SPH_ERR_STATE, "sph_debug_neighbors before sph_init");
     int rc = ensure_lists(c);
     if (rc != SPH_OK || (rc = neighbor_search(c)) != SPH_OK) return rc;
-    if (c->pair_f) launch_pair_factors(c->P, arrays(c), c->stream); /* the next DFSPH step reads them */
+    if (c->desc.simulation_method == SPH_DFSPH)
+        launch_pair_factors(c->P, arrays(c), c->stream); /* the next step reads them */
     const size_t nf = c->nf, nb = c->nb;
     std::vector<unsigned> cntf(nf), cntb(nf), orig(nf), borig(nb);
     std::vector<unsigned> nbrf(list_len(nf, c->P.capF)), nbrb(list_len(nf, c->P.capB));

@@ -26,7 +26,8 @@ struct DeviceArrays {
     float4* normal;
     float4* predr;        /* PCISPH predicted position */
     float4* posd;         /* PCISPH: (x, y, z, p / rho^2 of the iteration); DFSPH solvers: (x, y, z, k) */
-    float4* pgrad;        /* PCISPH: (slot, gradW) of each fluid list entry, in the layout of nbr_f */
+    float4* pgrad;        /* PCISPH: (slot, gradW) of each fluid list entry, in the layout of nbr_f
+                             (NULL: not kept) */
     float* rho;
     float* alpha;
     float* kws;
@@ -42,7 +43,7 @@ struct DeviceArrays {
     unsigned* nbr_b;
     unsigned* cnt_b;
     /* DFSPH: the lists with each entry's kernel factor, (slot, bits of f with
-       gradW = f r), in the layout of nbr_f / nbr_b (see k_density) */
+       gradW = f r), in the layout of nbr_f / nbr_b (see k_density; NULL: not kept) */
     uint2* pair_f;
     uint2* pair_b;
     /* two float4 per particle, so that half or all of a neighbour's record is one
@@ -105,7 +106,7 @@ enum ForceMode : int {
 
 /* block: threads per block of the pass kernels (128 or 256, autotuned) */
 void launch_density(const SimParams& P, const DeviceArrays& A, bool alpha, bool eos, int block, cudaStream_t s);
-/* DFSPH: pair_f / pair_b and the records from the current lists, positions and
+/* DFSPH: pair_f / pair_b (where kept) and the records from the current lists, positions and
    velocities, where no density pass follows that writes them */
 void launch_pair_factors(const SimParams& P, const DeviceArrays& A, cudaStream_t s);
 void launch_normals(const SimParams& P, const DeviceArrays& A, int block, cudaStream_t s);

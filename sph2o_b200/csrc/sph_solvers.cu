@@ -235,8 +235,9 @@ __device__ __forceinline__ float boundary_density(const SimParams& P, const Devi
    and with alpha by its arithmetic too: with alpha 5 blocks per SM (nothing
    spilled) and the velocities gathered with the positions, 1M 189 -> 178 us,
    26k 37 -> 31 (6 blocks 190, 4 181; rounds of 4 190 to 223); densities alone
-   at 8 blocks, 1M 91 -> 84 (6 blocks 97). */
-template <bool ALPHA, bool EOS, bool DIVRES = false>
+   at 8 blocks, 1M 91 -> 84 (6 blocks 97). STORED: the kernel factors are kept
+   beside the list entries for the solvers (pair_f, pair_b). */
+template <bool ALPHA, bool EOS, bool DIVRES = false, bool STORED = DIVRES>
 __global__ void __launch_bounds__(256, ALPHA ? 5 : 8) k_density(SimParams P, DeviceArrays A)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(256, ALPHA ? 5 : 8) k_density(SimParams P, Dev
         if (ALPHA) {
             const Pair p = make_pair(xi, xj);
             const float fg = cs_gradf(p.rl, p.inv_rl, P);
-            if (DIVRES) __stcs(A.pair_f + list_index(kk, P.capF, i), make_uint2(j, __float_as_uint(fg)));
+            if (STORED) __stcs(A.pair_f + list_index(kk, P.capF, i), make_uint2(j, __float_as_uint(fg)));
             const float f = P.mass * fg;
             const float gx = f * p.rx, gy = f * p.ry, gz = f * p.rz;
             sgx += gx; sgy += gy; sgz += gz;
@@ -268,7 +269,7 @@ __global__ void __launch_bounds__(256, ALPHA ? 5 : 8) k_density(SimParams P, Dev
         if (ALPHA) {
             const Pair p = make_pair(xi, xb);
             const float fg = cs_gradf(p.rl, p.inv_rl, P);
-            if (DIVRES) __stcs(A.pair_b + list_index(kk, P.capB, i), make_uint2(bq, __float_as_uint(fg)));
+            if (STORED) __stcs(A.pair_b + list_index(kk, P.capB, i), make_uint2(bq, __float_as_uint(fg)));
             const float f = xb.w * fg;
             sgx += f * p.rx; sgy += f * p.ry; sgz += f * p.rz;
             if (DIVRES) div += xb.w * (fg * ((vi.x * p.rx + vi.y * p.ry) + vi.z * p.rz));
@@ -290,22 +291,25 @@ __global__ void __launch_bounds__(256, ALPHA ? 5 : 8) k_density(SimParams P, Dev
     if (DIVRES) A.divres[i] = (nF + nB < 20u) ? 0.0f : fmaxf(div, 0.0f);
 }
 
-/* What the density pass writes into pair_f / pair_b and the records, alone:
-   after a list build, or new velocities, that no density pass follows. */
+/* What the density pass writes into pair_f / pair_b (STORED) and the records,
+   alone: after a list build, or new velocities, that no density pass follows. */
+template <bool STORED>
 __global__ void __launch_bounds__(256) k_pair_factors(SimParams P, DeviceArrays A)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= active_n(P, A.st)) return;
     const float4 xi = A.pos[i];
-    const unsigned nF = A.cnt_f[i], nB = A.cnt_b[i];
-    for_fluid_neighbors<2>(P, A, i, nF, [&](unsigned kk, unsigned j, const float4& xj, const float4&) {
-        const Pair p = make_pair(xi, xj);
-        __stcs(A.pair_f + list_index(kk, P.capF, i), make_uint2(j, __float_as_uint(cs_gradf(p.rl, p.inv_rl, P))));
-    });
-    for (unsigned kk = 0; kk < nB; ++kk) {
-        const unsigned bq = list_at(A.nbr_b, kk, P.capB, i);
-        const Pair p = make_pair(xi, A.bpos[bq]);
-        __stcs(A.pair_b + list_index(kk, P.capB, i), make_uint2(bq, __float_as_uint(cs_gradf(p.rl, p.inv_rl, P))));
+    if (STORED) {
+        const unsigned nF = A.cnt_f[i], nB = A.cnt_b[i];
+        for_fluid_neighbors<2>(P, A, i, nF, [&](unsigned kk, unsigned j, const float4& xj, const float4&) {
+            const Pair p = make_pair(xi, xj);
+            __stcs(A.pair_f + list_index(kk, P.capF, i), make_uint2(j, __float_as_uint(cs_gradf(p.rl, p.inv_rl, P))));
+        });
+        for (unsigned kk = 0; kk < nB; ++kk) {
+            const unsigned bq = list_at(A.nbr_b, kk, P.capB, i);
+            const Pair p = make_pair(xi, A.bpos[bq]);
+            __stcs(A.pair_b + list_index(kk, P.capB, i), make_uint2(bq, __float_as_uint(cs_gradf(p.rl, p.inv_rl, P))));
+        }
     }
     store_rec(A.rec, i, xi, A.rho[i], A.vel[i], 0.0f);
 }
@@ -565,24 +569,40 @@ __global__ void __launch_bounds__(256, MODE == FORCE_PRESSURE ? 6 : 4) k_forces(
 /* ---------------------------------------------------------------------- */
 /* DFSPH pieces                                                             */
 
-/* Entry kk of particle i in a pair array (evict-first, as list_at). */
-__device__ __forceinline__ uint2 pair_at(const uint2* pairs, unsigned kk, unsigned cap, int i)
+/* Entry kk of particle i in a list of `cap` entries per particle: its slot and,
+   STORED, the bits of its kernel factor (evict-first, as list_at). */
+template <bool STORED>
+__device__ __forceinline__ uint2 pair_at(const uint2* pairs, const unsigned* list, unsigned kk, unsigned cap, int i)
 {
-    return __ldcs(pairs + list_index(kk, cap, (unsigned)i));
+    if (STORED) return __ldcs(pairs + list_index(kk, cap, (unsigned)i));
+    return make_uint2(list_at(list, kk, cap, i), 0u);
+}
+
+/* The kernel factor of an entry: stored, or computed with the roundings of the
+   density pass (k_density), written out so that both give the same bits. */
+template <bool STORED>
+__device__ __forceinline__ float pair_factor(const SimParams& P, uint2 e, float4 xi, float4 xj)
+{
+    if (STORED) return __uint_as_float(e.y);
+    const float rx = __fsub_rn(xi.x, xj.x), ry = __fsub_rn(xi.y, xj.y), rz = __fsub_rn(xi.z, xj.z);
+    float rl, inv_rl;
+    len_inv(__fmaf_rn(rz, rz, __fmaf_rn(rx, rx, __fmul_rn(ry, ry))), rl, inv_rl);
+    return cs_gradf_as<false>(rl, inv_rl, P);
 }
 
 /* Calls f(kk, e, ahead) for rounds of U of the list entries sub, sub + TPP, ...
    < n of particle i: entry kk + u TPP is e[u]; those at or beyond n are the
    particle itself and do not count. f calls ahead() once its gathers are issued,
    which fetches the next round's entries. */
-template <int U, int TPP, typename F>
-__device__ __forceinline__ void pair_rounds(const uint2* pairs, unsigned sub, unsigned n, unsigned cap, int i, F&& f)
+template <int U, int TPP, bool STORED, typename F>
+__device__ __forceinline__ void pair_rounds(const uint2* pairs, const unsigned* list, unsigned sub, unsigned n,
+                                            unsigned cap, int i, F&& f)
 {
     uint2 e[U];
     const auto fetch = [&](unsigned kk, uint2(&to)[U]) {
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            to[u] = kk + u * TPP < n ? pair_at(pairs, kk + u * TPP, cap, i) : make_uint2((unsigned)i, 0u);
+            to[u] = kk + u * TPP < n ? pair_at<STORED>(pairs, list, kk + u * TPP, cap, i) : make_uint2((unsigned)i, 0u);
     };
     fetch(sub, e);
     for (unsigned kk = sub; kk < n; kk += U * TPP) {
@@ -607,7 +627,7 @@ __device__ __forceinline__ float dfsph_residual_term(const SimParams& P, float4 
    using any of them (more loads in flight per lane) and adds the terms in
    list order, so U changes no bit; TPP * ACC = 2 is one order of additions
    whichever way it is split. */
-template <int TPP, int ACC, int U>
+template <int TPP, int ACC, int U, bool STORED>
 __device__ __forceinline__ float dfsph_residual_part(const SimParams& P, const DeviceArrays& A, int i, int sub)
 {
     static_assert(U % ACC == 0, "an unrolled round holds whole rounds of partial sums");
@@ -617,23 +637,25 @@ __device__ __forceinline__ float dfsph_residual_part(const SimParams& P, const D
 #pragma unroll
     for (int c = 0; c < ACC; ++c) s[c] = 0.0f;
     const unsigned nF = A.cnt_f[i], nB = A.cnt_b[i];
-    pair_rounds<U, TPP>(A.pair_f, (unsigned)sub, nF, P.capF, i, [&](unsigned kk, const auto& e, auto ahead) {
+    pair_rounds<U, TPP, STORED>(A.pair_f, A.nbr_f, (unsigned)sub, nF, P.capF, i,
+                                [&](unsigned kk, const auto& e, auto ahead) {
         float4 xj[U], vj[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) load_rec(A.rec, e[u].x, xj[u], vj[u]);
         ahead();
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (kk + u * TPP < nF) s[u % ACC] += dfsph_residual_term(P, xi, vi, xj[u], vj[u], __uint_as_float(e[u].y));
+            if (kk + u * TPP < nF)
+                s[u % ACC] += dfsph_residual_term(P, xi, vi, xj[u], vj[u], pair_factor<STORED>(P, e[u], xi, xj[u]));
     });
     for (unsigned kk = sub; kk < nB; kk += TPP * ACC) {
 #pragma unroll
         for (int c = 0; c < ACC; ++c) {
             if (c > 0 && kk + c * TPP >= nB) break;
-            const uint2 e = pair_at(A.pair_b, kk + c * TPP, P.capB, i);
+            const uint2 e = pair_at<STORED>(A.pair_b, A.nbr_b, kk + c * TPP, P.capB, i);
             const float4 xb = A.bpos[e.x];
             const float rx = xi.x - xb.x, ry = xi.y - xb.y, rz = xi.z - xb.z;
-            s[c] += xb.w * (__uint_as_float(e.y) * ((vi.x * rx + vi.y * ry) + vi.z * rz));
+            s[c] += xb.w * (pair_factor<STORED>(P, e, xi, xb) * ((vi.x * rx + vi.y * ry) + vi.z * rz));
         }
     }
     return ACC == 2 ? s[0] + s[ACC - 1] : s[0];
@@ -657,10 +679,10 @@ __device__ __forceinline__ float dfsph_residual_finish(const SimParams& P, const
 }
 
 /* predicted density (DIV=false) or divergence error (DIV=true) of particle i */
-template <bool DIV>
+template <bool DIV, bool STORED>
 __device__ __forceinline__ float dfsph_residual(const SimParams& P, const DeviceArrays& A, int i, float dt)
 {
-    return dfsph_residual_finish<DIV>(P, A, i, dfsph_residual_part<1, 1, 4>(P, A, i, 0), dt);
+    return dfsph_residual_finish<DIV>(P, A, i, dfsph_residual_part<1, 1, 4, STORED>(P, A, i, 0), dt);
 }
 
 /* Partial sums over list entries sub, sub + TPP, ... of
@@ -668,7 +690,7 @@ __device__ __forceinline__ float dfsph_residual(const SimParams& P, const Device
    U at a time and ACC interleaved sums, as in dfsph_residual_part. Position
    and k are in posd, written inside the same persistent kernel (before a grid
    barrier): a read-only (non-coherent) load path would be wrong for it. */
-template <int TPP, int ACC, int U>
+template <int TPP, int ACC, int U, bool STORED>
 __device__ __forceinline__ void dfsph_correct_part(const SimParams& P, const DeviceArrays& A, int i, int sub,
                                                    float& sx, float& sy, float& sz)
 {
@@ -680,7 +702,8 @@ __device__ __forceinline__ void dfsph_correct_part(const SimParams& P, const Dev
 #pragma unroll
     for (int c = 0; c < ACC; ++c) tx[c] = ty[c] = tz[c] = 0.0f;
     const unsigned nF = A.cnt_f[i];
-    pair_rounds<U, TPP>(A.pair_f, (unsigned)sub, nF, P.capF, i, [&](unsigned kk, const auto& e, auto ahead) {
+    pair_rounds<U, TPP, STORED>(A.pair_f, A.nbr_f, (unsigned)sub, nF, P.capF, i,
+                                [&](unsigned kk, const auto& e, auto ahead) {
         float4 xj[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) xj[u] = xk[e[u].x];
@@ -689,7 +712,7 @@ __device__ __forceinline__ void dfsph_correct_part(const SimParams& P, const Dev
         for (int u = 0; u < U; ++u) {
             const float ks = ki + xj[u].w;
             if (kk + u * TPP < nF && fabsf(ks) > P.eps) {
-                const float c = P.mass * ks * __uint_as_float(e[u].y);
+                const float c = P.mass * ks * pair_factor<STORED>(P, e[u], xi, xj[u]);
                 tx[u % ACC] += c * (xi.x - xj[u].x);
                 ty[u % ACC] += c * (xi.y - xj[u].y);
                 tz[u % ACC] += c * (xi.z - xj[u].z);
@@ -702,9 +725,9 @@ __device__ __forceinline__ void dfsph_correct_part(const SimParams& P, const Dev
 #pragma unroll
             for (int c = 0; c < ACC; ++c) {
                 if (c > 0 && kk + c * TPP >= nB) break;
-                const uint2 e = pair_at(A.pair_b, kk + c * TPP, P.capB, i);
+                const uint2 e = pair_at<STORED>(A.pair_b, A.nbr_b, kk + c * TPP, P.capB, i);
                 const float4 xb = A.bpos[e.x];
-                const float w = xb.w * ki * __uint_as_float(e.y);
+                const float w = xb.w * ki * pair_factor<STORED>(P, e, xi, xb);
                 tx[c] += w * (xi.x - xb.x); ty[c] += w * (xi.y - xb.y); tz[c] += w * (xi.z - xb.z);
             }
         }
@@ -733,10 +756,11 @@ __device__ __forceinline__ void dfsph_set_k(const DeviceArrays& A, int i, float 
 }
 
 /* v_i -= dt * sum_j m (k_i + k_j) gradW  (+ boundary with k_i) */
+template <bool STORED>
 __device__ __forceinline__ void dfsph_correct(const SimParams& P, const DeviceArrays& A, int i, float dt)
 {
     float sx, sy, sz;
-    dfsph_correct_part<1, 1, 4>(P, A, i, 0, sx, sy, sz);
+    dfsph_correct_part<1, 1, 4, STORED>(P, A, i, 0, sx, sy, sz);
     dfsph_apply(A, i, dt, sx, sy, sz);
 }
 
@@ -777,22 +801,22 @@ __device__ __forceinline__ void for_particles(int n, F&& f)
 }
 
 /* residual of particle i with its list split over TPP lanes (all lanes call) */
-template <bool DIV, int TPP, int ACC, int U>
+template <bool DIV, int TPP, int ACC, int U, bool STORED>
 __device__ __forceinline__ float dfsph_residual_lanes(const SimParams& P, const DeviceArrays& A, int i, int sub,
                                                       bool valid, float dt)
 {
-    float part = valid ? dfsph_residual_part<TPP, ACC, U>(P, A, i, sub) : 0.0f;
+    float part = valid ? dfsph_residual_part<TPP, ACC, U, STORED>(P, A, i, sub) : 0.0f;
     if (TPP > 1) part = lane_group_sum<TPP>(part);
     return valid ? dfsph_residual_finish<DIV>(P, A, i, part, dt) : 0.0f;
 }
 
 /* velocity correction of particle i with its list split over TPP lanes */
-template <int TPP, int ACC, int U>
+template <int TPP, int ACC, int U, bool STORED>
 __device__ __forceinline__ void dfsph_correct_lanes(const SimParams& P, const DeviceArrays& A, int i, int sub,
                                                     bool valid, float dt)
 {
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-    if (valid) dfsph_correct_part<TPP, ACC, U>(P, A, i, sub, sx, sy, sz);
+    if (valid) dfsph_correct_part<TPP, ACC, U, STORED>(P, A, i, sub, sx, sy, sz);
     if (TPP > 1) {
         sx = lane_group_sum<TPP>(sx);
         sy = lane_group_sum<TPP>(sy);
@@ -821,8 +845,10 @@ __device__ __forceinline__ void dfsph_correct_lanes(const SimParams& P, const De
    with the lanes taken at every size (density solver 1k 54 us against 41, 26k 79
    against 64, 125k 216 against 165, 1M 1,294 against 1,035). TPP lanes share a
    particle; 1 and 2 lanes add the same two interleaved sums, so they agree bit for
-   bit. */
-template <bool DIV, int TPP>
+   bit. Without STORED the factors are computed again from the slots in the lists,
+   for scenes that leave no room for them: density solver 1M 1,259 us, 125k 201
+   against 165, 26k 122 against 107. */
+template <bool DIV, int TPP, bool STORED>
 __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve(SimParams P, DeviceArrays A)
 {
     constexpr int U = 4;
@@ -875,14 +901,14 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve(SimParams P, De
        only where the residual is positive */
     for_particles<TPP>(nfi, [&](int i, int sub, bool valid) {
         const float r = DIV ? (valid ? A.divres[i] : 0.0f)
-                            : dfsph_residual_lanes<DIV, TPP, ACC, U>(P, A, i, sub, valid, dt);
+                            : dfsph_residual_lanes<DIV, TPP, ACC, U, STORED>(P, A, i, sub, valid, dt);
         if (valid && sub == 0) {
             if (DIV) dfsph_set_k(A, i, r > 0.0f ? kws[i] / dt : 0.0f);
             else dfsph_set_k(A, i, r > P.rho0 ? kws[i] / ts2 : 0.0f);
         }
     });
     if (!bar.sync()) return;
-    for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U>(P, A, i, sub, valid, dt); });
+    for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U, STORED>(P, A, i, sub, valid, dt); });
     if (!bar.sync()) return;
 
     const double limit = DIV ? (double)(P.eta_v / dt) : (double)P.eta;
@@ -895,7 +921,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve(SimParams P, De
     while ((avg > limit || it < min_it) && it < max_it) {
         double local = 0.0;
         for_particles<TPP>(nfi, [&](int i, int sub, bool valid) {
-            const float r = dfsph_residual_lanes<DIV, TPP, ACC, U>(P, A, i, sub, valid, dt);
+            const float r = dfsph_residual_lanes<DIV, TPP, ACC, U, STORED>(P, A, i, sub, valid, dt);
             if (!valid || sub != 0) return;
             float k;
             if (DIV) {
@@ -912,7 +938,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve(SimParams P, De
         if (threadIdx.x == 0) atomicAdd(&A.accum[it], bs);
         if (!bar.sync()) return;
         avg = *(volatile double*)&A.accum[it] / (double)nfi;
-        for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U>(P, A, i, sub, valid, dt); });
+        for_particles<TPP>(nfi, [&](int i, int sub, bool valid) { dfsph_correct_lanes<TPP, ACC, U, STORED>(P, A, i, sub, valid, dt); });
         if (!bar.sync()) return;
         ++it;
     }
@@ -975,7 +1001,7 @@ __device__ __forceinline__ void scene_accumulate(double* accum, unsigned stride,
     }
 }
 
-template <bool DIV>
+template <bool DIV, bool STORED>
 __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams P, DeviceArrays A)
 {
     DevState* st = A.st;
@@ -1029,13 +1055,13 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams
     for (int i = tid; i < nfi; i += nthr) {
         const float dt = sst[so[i]].dt_next;
         /* the divergence error comes from the density pass */
-        const float r = DIV ? A.divres[i] : dfsph_residual<DIV>(P, A, i, dt);
+        const float r = DIV ? A.divres[i] : dfsph_residual<DIV, STORED>(P, A, i, dt);
         if (DIV) dfsph_set_k(A, i, r > 0.0f ? kws[i] / dt : 0.0f);
         else dfsph_set_k(A, i, r > P.rho0 ? kws[i] / (dt * dt) : 0.0f);
     }
     if (!bar.sync()) return;
     for (int i = tid; i < nfi; i += nthr) {
-        dfsph_correct(P, A, i, sst[so[i]].dt_next);
+        dfsph_correct<STORED>(P, A, i, sst[so[i]].dt_next);
         kws[i] = 0.0f;
     }
     if (!bar.sync()) return;
@@ -1056,7 +1082,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams
             double err = 0.0;
             if (on) {
                 const float dt = sst[s].dt_next;
-                const float r = dfsph_residual<DIV>(P, A, i, dt);
+                const float r = dfsph_residual<DIV, STORED>(P, A, i, dt);
                 float k;
                 if (DIV) {
                     k = r * A.alpha[i] / (dt * A.rho[i]);
@@ -1093,7 +1119,7 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_dfsph_solve_batch(SimParams
         }
         for (int i = tid; i < nfi; i += nthr) {
             const unsigned s = so[i];
-            if (sst[s].active & bit) dfsph_correct(P, A, i, sst[s].dt_next);
+            if (sst[s].active & bit) dfsph_correct<STORED>(P, A, i, sst[s].dt_next);
         }
         if (!bar.sync()) return;
         any = *(volatile unsigned*)&A.any_active[it + 1u] != 0u;
@@ -1206,6 +1232,7 @@ constexpr int kPcisphBatch = 44;
 /* The loop of PCISPHSolver::step. Neighbours read posd (current position and
    p / rho^2) and predr, never pos, so the pass that ends an iteration also
    predicts the next one's positions, or integrates when it was the last. */
+template <bool KEEP>
 __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, DeviceArrays A)
 {
     __shared__ double s_red[32];
@@ -1312,18 +1339,20 @@ __global__ void __launch_bounds__(kSolverBlock, 4) k_pcisph_solve(SimParams P, D
            exact gradient arithmetic: the result feeds the next predicted
            positions, whose densities enter the ill-conditioned p update. The
            gradients do not change within a step: the first iteration keeps
-           them beside their list entries for the later ones. */
+           them beside their list entries for the later ones (KEEP; else, where
+           there is no room, each iteration computes them: 1M, two iterations,
+           1,010 us of solver per step against 988). */
         for (int i = tid; i < nfi; i += nthr) {
             const float4 xi = A.posd[i];
             const float dpi = xi.w;
             float ax = 0.0f, ay = 0.0f, az = 0.0f;
             const unsigned nF = A.cnt_f[i], nB = A.cnt_b[i];
-            if (it == 0) {
+            if (!KEEP || it == 0) {
                 constexpr int U = 4; /* gathers issued before the first is used, the next entries meanwhile */
                 const auto term = [&](unsigned kk, unsigned j, const float4& xj) {
                     float gx, gy, gz;
                     cs_gradW_exact(__fsub_rn(xi.x, xj.x), __fsub_rn(xi.y, xj.y), __fsub_rn(xi.z, xj.z), P, gx, gy, gz);
-                    if (more) __stcs(A.pgrad + list_index(kk, P.capF, i), make_float4(__uint_as_float(j), gx, gy, gz));
+                    if (KEEP && more) __stcs(A.pgrad + list_index(kk, P.capF, i), make_float4(__uint_as_float(j), gx, gy, gz));
                     const float c = __fmul_rn(P.mass, __fadd_rn(dpi, xj.w));
                     ax = __fsub_rn(ax, __fmul_rn(c, gx));
                     ay = __fsub_rn(ay, __fmul_rn(c, gy));
@@ -1630,7 +1659,8 @@ void launch_density(const SimParams& P, const DeviceArrays& A, bool alpha, bool 
     if (P.nf <= 0) return;
     const int g = blocks_for(P.nf, block);
     if (alpha && eos) k_density<true, true><<<g, block, 0, s>>>(P, A);
-    else if (alpha && A.divres) k_density<true, false, true><<<g, block, 0, s>>>(P, A);
+    else if (alpha && A.pair_f) k_density<true, false, true><<<g, block, 0, s>>>(P, A);
+    else if (alpha && A.divres) k_density<true, false, true, false><<<g, block, 0, s>>>(P, A);
     else if (alpha) k_density<true, false><<<g, block, 0, s>>>(P, A);
     else if (eos) k_density<false, true><<<g, block, 0, s>>>(P, A);
     else k_density<false, false><<<g, block, 0, s>>>(P, A);
@@ -1638,7 +1668,9 @@ void launch_density(const SimParams& P, const DeviceArrays& A, bool alpha, bool 
 
 void launch_pair_factors(const SimParams& P, const DeviceArrays& A, cudaStream_t s)
 {
-    if (P.nf > 0) k_pair_factors<<<blocks_for(P.nf, 256), 256, 0, s>>>(P, A);
+    if (P.nf <= 0) return;
+    if (A.pair_f) k_pair_factors<true><<<blocks_for(P.nf, 256), 256, 0, s>>>(P, A);
+    else k_pair_factors<false><<<blocks_for(P.nf, 256), 256, 0, s>>>(P, A);
 }
 
 void launch_normals(const SimParams& P, const DeviceArrays& A, int block, cudaStream_t s)
@@ -1664,26 +1696,42 @@ void launch_forces(const SimParams& P, const DeviceArrays& A, int mode, int bloc
     }
 }
 
-/* k_dfsph_solve instance for (divergence, lanes per particle) */
-static const void* dfsph_solve_fn(bool divergence, int tpp)
+/* Solver instances; stored: with what is kept beside the list entries (pair_f /
+   pair_b, pgrad). */
+static const void* dfsph_solve_fn(bool divergence, int tpp, bool stored)
 {
-#define SPH_SOLVE_FN(D)                                                                             \
-    (tpp == 4 ? (const void*)k_dfsph_solve<D, 4>                                                    \
-              : tpp == 2 ? (const void*)k_dfsph_solve<D, 2> : (const void*)k_dfsph_solve<D, 1>)
-    return divergence ? SPH_SOLVE_FN(true) : SPH_SOLVE_FN(false);
+#define SPH_SOLVE_FN(D, S)                                                                          \
+    (tpp == 4 ? (const void*)k_dfsph_solve<D, 4, S>                                                 \
+              : tpp == 2 ? (const void*)k_dfsph_solve<D, 2, S> : (const void*)k_dfsph_solve<D, 1, S>)
+    if (stored) return divergence ? SPH_SOLVE_FN(true, true) : SPH_SOLVE_FN(false, true);
+    return divergence ? SPH_SOLVE_FN(true, false) : SPH_SOLVE_FN(false, false);
 #undef SPH_SOLVE_FN
+}
+
+static const void* dfsph_batch_fn(bool divergence, bool stored)
+{
+    if (stored) return divergence ? (const void*)k_dfsph_solve_batch<true, true> : (const void*)k_dfsph_solve_batch<false, true>;
+    return divergence ? (const void*)k_dfsph_solve_batch<true, false> : (const void*)k_dfsph_solve_batch<false, false>;
+}
+
+static const void* pcisph_fn(bool stored)
+{
+    return stored ? (const void*)k_pcisph_solve<true> : (const void*)k_pcisph_solve<false>;
 }
 
 int persistent_grid(bool pcisph, bool divergence, bool batch, int tpp)
 {
-    int dev = 0, sms = 0, per_sm = 0;
+    int dev = 0, sms = 0, per_sm = 1 << 10;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    const void* fn = pcisph ? (const void*)k_pcisph_solve
-                     : batch ? (divergence ? (const void*)k_dfsph_solve_batch<true>
-                                           : (const void*)k_dfsph_solve_batch<false>)
-                             : dfsph_solve_fn(divergence, tpp);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSolverBlock, 0) != cudaSuccess) return 0;
+    /* a grid that is resident as a whole for either instance */
+    for (bool stored : {false, true}) {
+        int n = 0;
+        const void* fn = pcisph ? pcisph_fn(stored)
+                         : batch ? dfsph_batch_fn(divergence, stored) : dfsph_solve_fn(divergence, tpp, stored);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kSolverBlock, 0) != cudaSuccess) return 0;
+        per_sm = n < per_sm ? n : per_sm;
+    }
     return per_sm * sms;
 }
 
@@ -1699,22 +1747,21 @@ int launch_dfsph_solve(const SimParams& P, const DeviceArrays& A, bool divergenc
 {
     const int need = blocks_for((long long)(P.nf > 0 ? P.nf : 1) * tpp, kSolverBlock);
     const int g = grid < need ? grid : need;
-    return coop_launch(dfsph_solve_fn(divergence, tpp), P, A, g > 0 ? g : 1, s);
+    return coop_launch(dfsph_solve_fn(divergence, tpp, A.pair_f != nullptr), P, A, g > 0 ? g : 1, s);
 }
 
 int launch_dfsph_solve_batch(const SimParams& P, const DeviceArrays& A, bool divergence, int grid, cudaStream_t s)
 {
     const int need = blocks_for(P.nf > 0 ? P.nf : 1, kSolverBlock);
     const int g = grid < need ? grid : need;
-    return coop_launch(divergence ? (const void*)k_dfsph_solve_batch<true> : (const void*)k_dfsph_solve_batch<false>,
-                       P, A, g > 0 ? g : 1, s);
+    return coop_launch(dfsph_batch_fn(divergence, A.pair_f != nullptr), P, A, g > 0 ? g : 1, s);
 }
 
 int launch_pcisph_solve(const SimParams& P, const DeviceArrays& A, int grid, cudaStream_t s)
 {
     const int need = blocks_for(P.nf > 0 ? P.nf : 1, kSolverBlock);
     const int g = grid < need ? grid : need;
-    return coop_launch((const void*)k_pcisph_solve, P, A, g > 0 ? g : 1, s);
+    return coop_launch(pcisph_fn(A.pgrad != nullptr), P, A, g > 0 ? g : 1, s);
 }
 
 } // namespace sph
