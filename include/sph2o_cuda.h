@@ -245,8 +245,8 @@ int sph_get_option(const sph_ctx* ctx, int option, int* value);
    keeps SPH_OPT_SOLVER_OCCUPANCY) by timing trial_steps steps (CUDA events) of every
    combination, each from a snapshot of the current state that is restored
    afterwards: the simulation is left exactly where it was. cache_path (may
-   be NULL) names a JSON file keyed by GPU name, method and particle counts;
-   a hit skips the trials and a miss appends the result. config (may be NULL)
+   be NULL) names a JSON file keyed by GPU name, method, particle counts, force
+   options and the build of the kernels; a hit skips the trials and a miss appends the result. config (may be NULL)
    receives the SPH_TUNE_COUNT chosen values in option order 1..4. */
 int sph_autotune(sph_ctx* ctx, int trial_steps, const char* cache_path, int* config);
 

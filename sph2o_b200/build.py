@@ -11,6 +11,7 @@ nvcc cross-compiles for sm_100a without a GPU. Host code is compiled with
 """
 from __future__ import annotations
 
+import hashlib
 import os
 import shutil
 import subprocess
@@ -50,12 +51,24 @@ def _deps():
     return out
 
 
+def kernel_id():
+    """Identifies the kernel sources: a cached autotuning result holds for the
+    kernels it was measured on."""
+    d = os.path.join(HERE, "csrc")
+    h = hashlib.sha1()
+    for f in sorted(os.listdir(d)):
+        if f.endswith((".cu", ".cuh", ".h")):
+            with open(os.path.join(d, f), "rb") as src:
+                h.update(src.read())
+    return h.hexdigest()[:12]
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     nvcc = nvcc_path()
     deps = _deps()
     if force or _stale(LIB, deps):
         cmd = [nvcc, *ARCH, "-lineinfo", "-O3", "-std=c++17", "-shared", "-Xcompiler", "-fPIC,-ffp-contract=off",
-               "-Xptxas", "-v" if verbose else "-O3", "-o", LIB]
+               f'-DSPH_KERNEL_ID="{kernel_id()}"', "-Xptxas", "-v" if verbose else "-O3", "-o", LIB]
         cmd += [os.path.join(HERE, s) for s in CUDA_SOURCES + HOST_SOURCES]
         subprocess.run(cmd, check=True, cwd=HERE)
     driver_src = os.path.join(HERE, "host", "sph2o_main.cpp")

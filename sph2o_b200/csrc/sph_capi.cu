@@ -1694,12 +1694,21 @@ int snapshot(sph_ctx* c, bool save)
     return SPH_OK;
 }
 
+#ifndef SPH_KERNEL_ID
+#define SPH_KERNEL_ID "unnamed"  /* the build passes a hash of the kernel sources */
+#endif
+
+/* What a tuning result holds for: the GPU, the kernels (an entry of another
+   build would choose among kernels that are no longer the same), the scene's
+   size and the options that change what a step does. */
 std::string tune_key(sph_ctx* c)
 {
     cudaDeviceProp prop{};
     cudaGetDeviceProperties(&prop, c->device);
     std::ostringstream k;
-    k << prop.name << "|m" << c->desc.simulation_method << "|n" << c->nf << "|b" << c->nb << "|s" << c->nscenes;
+    k << prop.name << "|m" << c->desc.simulation_method << "|n" << c->nf << "|b" << c->nb << "|s" << c->nscenes
+      << "|o" << c->P.visc_method << '.' << (c->P.bvisc != 0.0f) << '.' << c->P.st_on << '.' << c->P.adh_on << '.'
+      << c->pos_lo << '.' << c->desc.boundary_method << '.' << c->P.dynamic << "|k" << SPH_KERNEL_ID;
     return k.str();
 }
 

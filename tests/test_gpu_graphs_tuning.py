@@ -178,6 +178,25 @@ def test_autotune_leaves_state_untouched(method, tmp_path):
     sim.close(); ref.close(); other.close()
 
 
+def test_autotune_cache_entries_hold_for_one_build_and_one_scene(tmp_path):
+    """An entry without the build of the kernels (as they once were written), or
+    of a scene with other forces, is not taken and not lost."""
+    import torch
+
+    cache = tmp_path / "tune.json"
+    sim = small_sim(S.WCSPH)
+    old = f"{torch.cuda.get_device_name(0)}|m0|n{sim.nf}|b{sim.nb}|s0"
+    cache.write_text(json.dumps({old: [1, 8, 128, 1]}))
+    sim.autotune(trial_steps=1, cache_path=str(cache))
+    table = json.loads(cache.read_text())
+    assert len(table) == 2 and table[old] == [1, 8, 128, 1]
+    plain = Simulation.from_scene(Scene.from_dict(S.small(method=S.WCSPH)))
+    assert (plain.nf, plain.nb) == (sim.nf, sim.nb)
+    plain.autotune(trial_steps=1, cache_path=str(cache))
+    assert len(json.loads(cache.read_text())) == 3
+    sim.close(); plain.close()
+
+
 def test_autotune_batch_restores_scene_states():
     dims = [(6, 5, 7), (9, 8, 6), (5, 5, 5)]
     b = Batch([Scene.from_dict(S.small(method=S.DFSPH, n=n, radius=0.02, seed=40 + k)) for k, n in enumerate(dims)])
