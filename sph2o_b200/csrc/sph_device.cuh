@@ -21,6 +21,8 @@
 
 #include <cmath>
 
+#include "sph_slots.h"
+
 namespace sph {
 
 /* error bits in DevState::err */
@@ -446,8 +448,9 @@ __device__ __forceinline__ float dist2_exact_packed(float4 a, float4 b)
    slot of the stretch's candidate k. Four candidates are loaded before any is
    used, and nothing branches on a candidate: some lane of a warp accepts
    nearly every one, so a branch would be taken nearly always. [row0, row1):
-   the rows to walk, of the 9 in candidate order. */
-template <typename G, typename R>
+   the rows to walk, of the 9 in candidate order. Off: the type of the byte
+   offsets (sph_slots.h). */
+template <typename Off = unsigned, typename G, typename R>
 __device__ __forceinline__ void for_stretches27(float4 x, float4 y, float h, const Grid& g, const unsigned* cell_start,
                                                 const float4* pos, G&& group, R&& stretch, int row0 = 0, int row1 = 9)
 {
@@ -459,15 +462,8 @@ __device__ __forceinline__ void for_stretches27(float4 x, float4 y, float h, con
     const auto row = [&](unsigned s1, unsigned n1, unsigned s2, unsigned n) {
         for (unsigned k0 = 0; k0 < n; k0 += 32) {
             const unsigned c = min(n - k0, 32u);
-            /* byte offsets: 16 B per slot, below 2^32 for every size that fits the GPU */
-            unsigned o = (k0 < n1 ? s1 + k0 : s2 + (k0 - n1)) * 16u;
-            const unsigned oe = (s1 + n1) * 16u, o2 = s2 * 16u;
-            const auto next = [&]() {
-                const float4 v = *reinterpret_cast<const float4*>(base + o);
-                o += 16u;
-                if (o == oe) o = o2;
-                return v;
-            };
+            SlotWalk<Off> walk(s1, n1, s2, k0);
+            const auto next = [&]() { return *reinterpret_cast<const float4*>(base + walk.next()); };
             unsigned k = 0;
             for (; k + 4 <= c; k += 4) {
                 float4 v[4];

@@ -144,7 +144,7 @@ __device__ __forceinline__ void store_counts(const SimParams& P, const SearchArr
 
 /* Neighbour lists of particle i in the reference's candidate order, filtered
    at |r| <= h, and its density (MODE), by one thread. */
-template <int MODE>
+template <int MODE, typename Off>
 __device__ __forceinline__ void search_at(const SimParams& P, const SceneRef& S, int i, const SearchArrays& A)
 {
     const float4 xi = A.pos[i];
@@ -153,7 +153,7 @@ __device__ __forceinline__ void search_at(const SimParams& P, const SceneRef& S,
     const Grid g = grid_for(P, S, (unsigned)i);
     const auto list = [&](const unsigned* starts, const float4* xs, unsigned* out, unsigned cap) {
         unsigned m = 0, n = 0; /* accepted candidates of the stretch, of all */
-        for_stretches27(
+        for_stretches27<Off>(
             xi, xi, P.h, g, starts, xs,
             [&](unsigned k, const float (&d)[4], unsigned) {
                 const unsigned t = (d[0] <= s2max ? 1u : 0u) | (d[1] <= s2max ? 2u : 0u) | (d[2] <= s2max ? 4u : 0u) |
@@ -179,12 +179,12 @@ __device__ __forceinline__ void search_at(const SimParams& P, const SceneRef& S,
     store_density<MODE>(P, A, i, xi, rho);
 }
 
-template <int MODE>
+template <int MODE, typename Off>
 __global__ void __launch_bounds__(128) k_search(SimParams P, SceneRef S, SearchArrays A)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= active_n(P, A.st)) return;
-    search_at<MODE>(P, S, i, A);
+    search_at<MODE, Off>(P, S, i, A);
 }
 
 /* The same search for small scenes, one warp per particle: lane k < 27 loads the
@@ -284,10 +284,10 @@ __global__ void __launch_bounds__(kSearchWarps * 32) k_search_warp(SimParams P, 
 
 /* The one-thread search, kept out of line: what the lane groups below fall
    back to. */
-template <int MODE>
+template <int MODE, typename Off>
 __device__ __noinline__ void search_out_of_line(const SimParams& P, const SceneRef& S, int i, const SearchArrays& A)
 {
-    search_at<MODE>(P, S, i, A);
+    search_at<MODE, Off>(P, S, i, A);
 }
 
 /* The same search with four lanes per particle: the rows of cells are split
@@ -298,7 +298,7 @@ __device__ __noinline__ void search_out_of_line(const SimParams& P, const SceneR
    accepted candidates in one lane is left to search_out_of_line. */
 constexpr int kLanes = 4, kLaneBatch = 24, kLaneBlock = 128;
 
-template <int MODE>
+template <int MODE, typename Off>
 __global__ void __launch_bounds__(kLaneBlock) k_search_lanes(SimParams P, SceneRef S, SearchArrays A)
 {
     static_assert(MODE != SEARCH_LISTS, "a warp or one lane builds lists alone");
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_search_lanes(SimParams P, SceneR
     const auto set = [&](bool walk, const unsigned* starts, const float4* xs, unsigned* out, unsigned cap, bool boundary) {
         unsigned m = 0, nq = 0, nw = 0;
         if (walk)
-            for_stretches27(
+            for_stretches27<Off>(
                 xi, xi, P.h, g, starts, xs,
                 [&](unsigned k, const float (&d)[4], unsigned) {
                     unsigned bits = 0;
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_search_lanes(SimParams P, SceneR
     __syncwarp(); /* the other lanes' list entries come before the fallback's */
     if (!on || sub != 0) return;
     if (over) {
-        search_out_of_line<MODE>(P, S, i, A);
+        search_out_of_line<MODE, Off>(P, S, i, A);
         return;
     }
     store_counts(P, A, i, nF, nB);
@@ -386,7 +386,7 @@ __device__ __noinline__ void build_lists_global(const SimParams& P, int i, const
                                                 unsigned* __restrict__ nbr_b, unsigned* __restrict__ cnt_b,
                                                 DevState* st)
 {
-    search_at<SEARCH_LISTS>(P, SceneRef{}, i, SearchArrays{pos, cell_start, bpos, bcell_start, near, nbr_f, cnt_f, nbr_b,
+    search_at<SEARCH_LISTS, unsigned long long>(P, SceneRef{}, i, SearchArrays{pos, cell_start, bpos, bcell_start, near, nbr_f, cnt_f, nbr_b,
                                                            cnt_b, nullptr, nullptr, nullptr, nullptr, st});
 }
 
@@ -616,19 +616,24 @@ constexpr int kSearchWarpMax = 1 << 14, kSearchLanesMax = 3 << 14;
    against 42 + 27, 216k 86 against 61 + 29; 1M 333 against 209 + 85). */
 constexpr int kSearchDensityMax = 1 << 18;
 
+template <int MODE, typename Off>
+static void search_by_lanes(const SimParams& P, const SceneRef& S, const SearchArrays& A, cudaStream_t s)
+{
+    if constexpr (MODE != SEARCH_LISTS)
+        if (P.nf < kSearchLanesMax) {
+            k_search_lanes<MODE, Off><<<blocks_for((long long)P.nf * kLanes, kLaneBlock), kLaneBlock, 0, s>>>(P, S, A);
+            return;
+        }
+    k_search<MODE, Off><<<blocks_for(P.nf, 128), 128, 0, s>>>(P, S, A);
+}
+
 template <int MODE>
 static void search_mode(const SimParams& P, const SceneRef& S, const SearchArrays& A, cudaStream_t s)
 {
-    if (P.nf < (MODE == SEARCH_LISTS ? kSearchLanesMax : kSearchWarpMax)) {
+    if (P.nf < (MODE == SEARCH_LISTS ? kSearchLanesMax : kSearchWarpMax))
         k_search_warp<MODE><<<blocks_for(P.nf, kSearchWarps), kSearchWarps * 32, 0, s>>>(P, S, A);
-        return;
-    }
-    if constexpr (MODE != SEARCH_LISTS)
-        if (P.nf < kSearchLanesMax) {
-            k_search_lanes<MODE><<<blocks_for((long long)P.nf * kLanes, kLaneBlock), kLaneBlock, 0, s>>>(P, S, A);
-            return;
-        }
-    k_search<MODE><<<blocks_for(P.nf, 128), 128, 0, s>>>(P, S, A);
+    else if (narrow_slots((unsigned)P.nf, (unsigned)P.nb)) search_by_lanes<MODE, unsigned>(P, S, A, s);
+    else search_by_lanes<MODE, unsigned long long>(P, S, A, s);
 }
 
 bool launch_search(const SimParams& P, const SceneRef& S, const DeviceArrays& D, int mode, cudaStream_t s, bool staged)
