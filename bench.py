@@ -132,7 +132,7 @@ def batched_run(steps, warmup, method=0, count=256, loop_steps=None, indices=Non
     batch = Batch(scs)
     total = batch.nf
     # launch shape and cell order picked by the library's autotuner (trial
-    # steps from a snapshot that is restored), cached per GPU and workload
+    # steps from a snapshot that is restored), cached per GPU, workload and build
     tuned = batch.autotune(trial_steps=3, cache_path=os.path.join(tempfile.gettempdir(), "sph2o_autotune.json"))
     batch.step(warmup)
     torch.cuda.synchronize()
@@ -466,9 +466,8 @@ def config_run(name, steps, warmup, cpu=True, cpu_window=None, tune=True):
     """One named workload on this GPU (device-timed window of `steps` after
     `warmup`) and, when cpu, the reference's OpenMP path on the host cores over
     `cpu_window` = (steps, warmup) (default: the same window). With tune, the
-    library's autotuner picks cell order, solver occupancy, pass block and
-    solver lanes first (trial steps from a restored snapshot, cached per GPU
-    and workload)."""
+    library's autotuner picks cell order, pass block and solver lanes first
+    (trial steps from a restored snapshot, cached per GPU, workload and build)."""
     from sph2o_b200.api import Scene, Simulation
     desc, make = workloads()[name]
     d = make()

@@ -98,8 +98,9 @@ typedef struct sph_step_stats {
    stream). Phases of one step, in launch order: */
 enum sph_profile_phase {
     SPH_PROF_SORT = 0,        /* cell keys, counting sort, reorder        */
-    SPH_PROF_LISTS = 1,       /* neighbour-list build                      */
-    SPH_PROF_DENSITY = 2,     /* density (+alpha, +EOS)                    */
+    SPH_PROF_LISTS = 1,       /* neighbour-list build; in WCSPH and PCISPH scenes below 2^18 fluid
+                                 particles also their densities (+EOS), which the same kernel computes */
+    SPH_PROF_DENSITY = 2,     /* density (+alpha, +EOS) as a pass of its own: 0 in those scenes */
     SPH_PROF_NORMALS = 3,     /* surface-tension normals                   */
     SPH_PROF_FORCES = 4,      /* non-pressure forces (+WCSPH pressure, integrate) */
     SPH_PROF_DENSITY_SOLVE = 5,  /* DFSPH density solver (persistent kernel) */
@@ -193,7 +194,10 @@ int sph_get_num_active(sph_ctx* ctx, unsigned* n);
    masses m = rho0 (2r)^3, boundary volumes (AkinciBoundaryObject::computeVolume,
    AkinciBoundaryObject.cpp:10-34) and the solver's init (DFSPHSolver::init,
    DFSPHSolver.cpp:22-31: neighbour search, densities, alpha;
-   PCISPHSolver::init: scaling factor, PCISPHSolver.cpp:403-436). */
+   PCISPHSolver::init: scaling factor, PCISPHSolver.cpp:403-436). Takes about
+   730 bytes of device memory per fluid particle, and 1,024 more in DFSPH and
+   PCISPH where these are at most half of what is then left (they save time;
+   results do not depend on them). */
 int sph_init(sph_ctx* ctx);
 
 /* Replaces nsteps calls of SPHSolver::step (WCSPHSolver.cpp:14-78,

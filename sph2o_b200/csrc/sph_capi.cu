@@ -1570,7 +1570,7 @@ int sph_compute_phase(sph_ctx* c, int phase, float* out)
     const bool alpha = phase == SPH_PHASE_ALPHA || c->desc.simulation_method == SPH_DFSPH;
     if ((rc = neighbor_search(c, alpha ? SEARCH_LISTS : eos ? SEARCH_EOS : SEARCH_DENSITY)) != SPH_OK) return rc;
     DeviceArrays A = arrays(c);
-    if (alpha) launch_density(c->P, A, true, eos, c->pass_block, c->stream);
+    if (alpha) launch_density(c->P, A, true, false, c->pass_block, c->stream); /* pressures: WCSPH only */
     /* PCISPH boundary method: SPHSolver::computeDensities covers the
        boundary particles too (SPHSolver.cpp:126-137), WCSPH their pressures */
     if (c->P.pcib) launch_boundary_density(c->P, A, c->stream);

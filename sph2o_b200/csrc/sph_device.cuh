@@ -646,8 +646,8 @@ __device__ __forceinline__ unsigned atom_add_acq_rel_gpu(unsigned* p, unsigned v
    every barrier, as was reading the error flag, which only waiters do now. Two
    counts take turns from kernel to kernel: the constructor zeroes the one that
    the previous kernel used, leave() hands over. A DFSPH step has 10 to 20
-   barriers: 26k particles 224 -> 207 us per step, 125k 323 -> 312, 1M 1503 ->
-   1485, 24 batched scenes 506 -> 496 (sleeps of 20, 64 and 256 ns within 1 %).
+   barriers: 26k particles 224 -> 203 us per step, 125k 323 -> 307, 1M 1503 ->
+   1485, 24 batched scenes 506 -> 489 (sleeps of 20, 64 and 256 ns within 1 %).
    The wait is bounded: after kSpinLimit polls the block records ERRBIT_TIMEOUT
    and sync() returns false, and the caller leaves the kernel; so does every
    kernel that starts with that bit set, whose counts mean nothing. */

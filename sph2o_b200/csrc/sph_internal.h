@@ -104,7 +104,8 @@ enum ForceMode : int {
     FORCE_PRESSURE = 3     /* pressure acceleration only -> acc (phase access) */
 };
 
-/* block: threads per block of the pass kernels (128 or 256, autotuned) */
+/* block: threads per block of the pass kernels (128 or 256, autotuned). alpha
+   or eos, not both: a method has the one or the other. */
 void launch_density(const SimParams& P, const DeviceArrays& A, bool alpha, bool eos, int block, cudaStream_t s);
 /* DFSPH: pair_f / pair_b (where kept) and the records from the current lists, positions and
    velocities, where no density pass follows that writes them */

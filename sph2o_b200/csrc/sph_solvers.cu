@@ -1658,8 +1658,7 @@ void launch_density(const SimParams& P, const DeviceArrays& A, bool alpha, bool 
 {
     if (P.nf <= 0) return;
     const int g = blocks_for(P.nf, block);
-    if (alpha && eos) k_density<true, true><<<g, block, 0, s>>>(P, A);
-    else if (alpha && A.pair_f) k_density<true, false, true><<<g, block, 0, s>>>(P, A);
+    if (alpha && A.pair_f) k_density<true, false, true><<<g, block, 0, s>>>(P, A);
     else if (alpha && A.divres) k_density<true, false, true, false><<<g, block, 0, s>>>(P, A);
     else if (alpha) k_density<true, false><<<g, block, 0, s>>>(P, A);
     else if (eos) k_density<false, true><<<g, block, 0, s>>>(P, A);
