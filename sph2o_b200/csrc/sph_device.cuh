@@ -463,7 +463,11 @@ __device__ __forceinline__ void for_stretches27(float4 x, float4 y, float h, con
         for (unsigned k0 = 0; k0 < n; k0 += 32) {
             const unsigned c = min(n - k0, 32u);
             SlotWalk<Off> walk(s1, n1, s2, k0);
-            const auto next = [&]() { return *reinterpret_cast<const float4*>(base + walk.next()); };
+            const auto next = [&]() {
+                const float4 v = *reinterpret_cast<const float4*>(base + walk.at);
+                walk.advance();
+                return v;
+            };
             unsigned k = 0;
             for (; k + 4 <= c; k += 4) {
                 float4 v[4];

@@ -18,9 +18,9 @@ static bool walks(unsigned s1, unsigned n1, unsigned s2, unsigned n2)
 {
     for (unsigned k = 0; k <= n1 + n2; ++k) {
         SlotWalk<Off> w(s1, n1, s2, k);
-        for (unsigned j = k; j < n1 + n2; ++j) {
+        for (unsigned j = k; j < n1 + n2; ++j, w.advance()) {
             const unsigned long long slot = j < n1 ? s1 + j : s2 + (j - n1);
-            if ((unsigned long long)w.next() != 16 * slot) return false;
+            if ((unsigned long long)w.at != 16 * slot) return false;
         }
     }
     return true;
